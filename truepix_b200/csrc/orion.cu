@@ -350,10 +350,26 @@ __device__ __forceinline__ void load_digest(const unsigned char* tree, long long
     w[4] = sha::bswap32(b.x); w[5] = sha::bswap32(b.y); w[6] = sha::bswap32(b.z); w[7] = sha::bswap32(b.w);
 }
 
+// 16 bytes from global to shared memory, asynchronously; zeros when !in
+__device__ __forceinline__ void copy_async16(void* dst, const void* src, bool in)
+{
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    const int n = in ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copy_async_wait()
+{
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
 // Row leaves (linearPC.cpp:61-95,145-168): for row r < cw_len,
 // h <- SHA256(h || rows[r][2j] || rows[r][2j+1]) for j = 0..63 from h = 0.
 // One thread per row; the CTA stages 128 rows x 8 columns (padded to 9, so
-// that 16-byte reads of consecutive rows fall in distinct banks) at a time.
+// that 16-byte reads of consecutive rows fall in distinct banks) at a time, the
+// next 8 columns copied behind the hashes of the present ones (two tiles, 36 KB:
+// six CTAs an SM, what a 1080p commit's 881 CTAs need to run in one wave).
 // A launch covers the column pairs [pair0, pair1) (multiples of kLeafPairs): a
 // chain split over several launches keeps its running state in the row's leaf
 // slot (raw state words) between them, the last launch stores the digest bytes.
@@ -362,29 +378,43 @@ __global__ void __launch_bounds__(kLeafRows) leaf_kernel(const ulonglong2* __res
                                                          unsigned char* __restrict__ tree, long long leaf0,
                                                          uint32_t one, int pair0, int pair1)
 {
-    __shared__ ulonglong2 tile[kLeafRows][2 * kLeafPairs + 1];
+    __shared__ ulonglong2 tile[2][kLeafRows][2 * kLeafPairs + 1];
     const long long r0 = (long long)blockIdx.x * kLeafRows;
     const int tid = threadIdx.x;
     const bool live = r0 + tid < cw_len;
     uint32_t* slot = reinterpret_cast<uint32_t*>(tree + (leaf0 + r0 + tid) * 32);
-    uint32_t st[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) st[i] = (pair0 > 0 && live) ? slot[i] : 0;
-    for (int pair = pair0; pair < pair1; pair += kLeafPairs) {
+    // 16 bytes a thread and step: eight neighbouring threads copy a row's 128 bytes
+    auto fetch = [&](int pair) {
+        ulonglong2(*t)[2 * kLeafPairs + 1] = tile[(pair / kLeafPairs) & 1];
 #pragma unroll
         for (int k = 0; k < 2 * kLeafPairs; ++k) {
             const int i = tid + k * kLeafRows;
             const int rr = i >> 3, cc = i & 7;
-            const long long r = r0 + rr;
-            tile[rr][cc] = r < cw_len ? ldg16(rows + r * kColumns + 2 * pair + cc) : make_ulonglong2(0, 0);
+            const bool in = r0 + rr < cw_len;
+            copy_async16(&t[rr][cc], rows + (in ? r0 + rr : 0) * kColumns + 2 * pair + cc, in);
+        }
+        copy_async_commit();
+    };
+    fetch(pair0);
+    uint32_t st[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) st[i] = (pair0 > 0 && live) ? slot[i] : 0;
+#pragma unroll 1
+    for (int pair = pair0; pair < pair1; pair += kLeafPairs) {
+        if (pair + kLeafPairs < pair1) {
+            fetch(pair + kLeafPairs);
+            copy_async_wait<1>();
+        } else {
+            copy_async_wait<0>();
         }
         __syncthreads();
+        const ulonglong2* mine = tile[(pair / kLeafPairs) & 1][tid];
 #pragma unroll 1
         for (int p = 0; p < kLeafPairs; ++p) {
             uint32_t w[16];
 #pragma unroll
             for (int i = 0; i < 8; ++i) w[i] = st[i];
-            const ulonglong2 x = tile[tid][2 * p], y = tile[tid][2 * p + 1];
+            const ulonglong2 x = mine[2 * p], y = mine[2 * p + 1];
             sha::fe_words(x.x, x.y, w + 8);
             sha::fe_words(y.x, y.y, w + 12);
             sha::hash64(w, st, sha::AddMad{one});
@@ -414,41 +444,40 @@ __global__ void fill_leaves_kernel(unsigned char* __restrict__ tree, long long l
 
 // `levels` tree levels above the n_in nodes at heap positions [n_in, 2 n_in):
 // CTA b reduces the 2^levels nodes from n_in + b * 2^levels to one node
-// (merkle_tree.cpp:64-83: node k = SHA256(node 2k || node 2k + 1)).
+// (merkle_tree.cpp:64-83: node k = SHA256(node 2k || node 2k + 1)). Bound by the
+// latency of one hash after another up the levels.
 __global__ void __launch_bounds__(256) tree_kernel(unsigned char* __restrict__ tree, long long n_in, int levels,
                                                    uint32_t one)
 {
-    __shared__ uint32_t s[256][9];
+    __shared__ uint32_t s[2][256][9];
     const int t = threadIdx.x;
     long long base = n_in + ((long long)blockIdx.x << levels);   // first child of this level
     int cnt = 1 << (levels - 1);                                  // parents at this level
-    uint32_t st[8];
-    if (t < cnt) {
-        uint32_t w[16];
-        load_digest(tree, base + 2 * t, w);
-        load_digest(tree, base + 2 * t + 1, w + 8);
-        sha::hash64(w, st, sha::AddMad{one});
-        store_digest(tree, (base >> 1) + t, st);
-    }
-    for (int lv = 1; lv < levels; ++lv) {
+#pragma unroll 1
+    for (int lv = 0; lv < levels; ++lv) {
         if (t < cnt) {
+            uint32_t w[16], st[8];
+            if (lv == 0) {
+                load_digest(tree, base + 2 * t, w);
+                load_digest(tree, base + 2 * t + 1, w + 8);
+            } else {
+                const uint32_t(*in)[9] = s[lv & 1];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) s[t][i] = st[i];
+                for (int i = 0; i < 8; ++i) {
+                    w[i] = in[2 * t][i];
+                    w[8 + i] = in[2 * t + 1][i];
+                }
+            }
+            // one copy of the rounds for all levels, so that they stay in the
+            // instruction cache (68 us for the 17 levels of a 1080p tree with two)
+            sha::hash64(w, st, sha::AddMad{one});
+#pragma unroll
+            for (int i = 0; i < 8; ++i) s[(lv + 1) & 1][t][i] = st[i];
+            store_digest(tree, (base >> 1) + t, st);
         }
         __syncthreads();
         base >>= 1;
         cnt >>= 1;
-        if (t < cnt) {
-            uint32_t w[16];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                w[i] = s[2 * t][i];
-                w[8 + i] = s[2 * t + 1][i];
-            }
-            sha::hash64(w, st, sha::AddMad{one});
-            store_digest(tree, (base >> 1) + t, st);
-        }
-        __syncthreads();
     }
 }
 

@@ -12,24 +12,38 @@ namespace {
 
 constexpr int kSlices = 64;   // 2^log_slice_number (include/infrastructure/constants.h)
 
-// leaf j: h <- SHA256(x || y || h) over the 64 slices (fri.cpp:96-110: the pair
-// first, the running digest second -- the opposite order of the Orion row leaves)
-__global__ void __launch_bounds__(256) fri_leaf_kernel(const ulonglong2* __restrict__ l_eval, long long slice,
-                                                       unsigned char* __restrict__ tree, uint32_t one)
+constexpr int kLeafThreads = 128;
+
+// The leaf chains of both commit kinds, h <- SHA256(x || y || h) over the 64 slices
+// (fri.cpp:96-110, 396-410: the pair first, the running digest second -- the
+// opposite order of the Orion row leaves): leaf t's x and y of slice i stand at
+// src + t leaf_step + i slice_step and y_off behind it. One thread per leaf; the
+// next pair is loaded behind the hash of the present one. Bound by the chain of
+// 128 compressions while the leaves give a scheduler at most one warp (up to
+// 18,944 of them: CTAs of 128 threads, so that small steps spread over the SMs),
+// by the ALU pipe beyond.
+__global__ void __launch_bounds__(kLeafThreads) pair_leaf_kernel(const ulonglong2* __restrict__ src,
+                                                                 long long n_leaves, long long leaf_step,
+                                                                 long long slice_step, long long y_off,
+                                                                 unsigned char* __restrict__ tree, uint32_t one)
 {
-    const long long half = slice >> 1;
-    const long long j = (long long)blockIdx.x * 256 + threadIdx.x;
-    if (j >= half) return;
+    const long long t = (long long)blockIdx.x * kLeafThreads + threadIdx.x;
+    if (t >= n_leaves) return;
     uint32_t st[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) st[i] = 0;
+    const ulonglong2* p = src + t * leaf_step;
+    ulonglong2 x = __ldg(p), y = __ldg(p + y_off);
 #pragma unroll 1
     for (int i = 0; i < kSlices; ++i) {
-        const ulonglong2 x = __ldg(l_eval + i * slice + j);
-        const ulonglong2 y = __ldg(l_eval + i * slice + j + half);
         uint32_t w[16];
         sha::fe_words(x.x, x.y, w);
         sha::fe_words(y.x, y.y, w + 4);
+        if (i + 1 < kSlices) {
+            p += slice_step;
+            x = __ldg(p);
+            y = __ldg(p + y_off);
+        }
 #pragma unroll
         for (int k = 0; k < 8; ++k) w[8 + k] = st[k];
         sha::hash64(w, st, sha::AddMad{one});
@@ -37,9 +51,17 @@ __global__ void __launch_bounds__(256) fri_leaf_kernel(const ulonglong2* __restr
     uint4 a, b;
     a.x = sha::bswap32(st[0]); a.y = sha::bswap32(st[1]); a.z = sha::bswap32(st[2]); a.w = sha::bswap32(st[3]);
     b.x = sha::bswap32(st[4]); b.y = sha::bswap32(st[5]); b.z = sha::bswap32(st[6]); b.w = sha::bswap32(st[7]);
-    uint4* p = reinterpret_cast<uint4*>(tree + (half + j) * 32);
-    p[0] = a;
-    p[1] = b;
+    uint4* d = reinterpret_cast<uint4*>(tree + (n_leaves + t) * 32);
+    d[0] = a;
+    d[1] = b;
+}
+
+bool launch_pair_leaves(const ulonglong2* src, long long n_leaves, long long leaf_step, long long slice_step,
+                        long long y_off, unsigned char* tree, const char* what, cudaStream_t s)
+{
+    pair_leaf_kernel<<<(unsigned)((n_leaves + kLeafThreads - 1) / kLeafThreads), kLeafThreads, 0, s>>>(
+        src, n_leaves, leaf_step, slice_step, y_off, tree, 1u);
+    return !cuda_failed(cudaGetLastError(), what);
 }
 
 __device__ __forceinline__ fp2 ld_fe(const ulonglong2* p) { const ulonglong2 v = __ldg(p); return mk(v.y, v.x); }
@@ -65,35 +87,6 @@ __global__ void __launch_bounds__(256) fri_fold_kernel(const ulonglong2* __restr
     next[pos] = make_ulonglong2(c.im, c.re);
 }
 
-// leaf i = chain over the 64 pairs of row i of the interleaved witness:
-// h <- SHA256(x || y || h) (fri.cpp:396-410)
-__global__ void __launch_bounds__(256) fri_row_leaf_kernel(const ulonglong2* __restrict__ w, long long n_leaves,
-                                                           unsigned char* __restrict__ tree, uint32_t one)
-{
-    const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
-    if (i >= n_leaves) return;
-    uint32_t st[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) st[k] = 0;
-    const ulonglong2* row = w + (i << 7);
-#pragma unroll 1
-    for (int j = 0; j < kSlices; ++j) {
-        const ulonglong2 x = __ldg(row + 2 * j), y = __ldg(row + 2 * j + 1);
-        uint32_t m[16];
-        sha::fe_words(x.x, x.y, m);
-        sha::fe_words(y.x, y.y, m + 4);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) m[8 + k] = st[k];
-        sha::hash64(m, st, sha::AddMad{one});
-    }
-    uint4 a, b;
-    a.x = sha::bswap32(st[0]); a.y = sha::bswap32(st[1]); a.z = sha::bswap32(st[2]); a.w = sha::bswap32(st[3]);
-    b.x = sha::bswap32(st[4]); b.y = sha::bswap32(st[5]); b.z = sha::bswap32(st[6]); b.w = sha::bswap32(st[7]);
-    uint4* p = reinterpret_cast<uint4*>(tree + (n_leaves + i) * 32);
-    p[0] = a;
-    p[1] = b;
-}
-
 }  // namespace
 
 bool fri_step(const ulonglong2* w, int log_m, fp2 r, ulonglong2* next, unsigned char* tree, cudaStream_t s)
@@ -116,10 +109,10 @@ bool fri_step(const ulonglong2* w, int log_m, fp2 r, ulonglong2* next, unsigned 
     if (cuda_failed(cudaGetLastError(), "fri fold")) return false;
     if (cuda_failed(cudaMemsetAsync(tree, 0, 32, s), "fri tree clear")) return false;
     timer_begin(s, 9211);
-    fri_row_leaf_kernel<<<(unsigned)((n_leaves + 255) / 256), 256, 0, s>>>(next, n_leaves, tree, 1u);
+    // leaf i: the 64 pairs of row i of the interleaved witness
+    const bool leaves = launch_pair_leaves(next, n_leaves, 2 * kSlices, 2, 1, tree, "fri leaves", s);
     timer_end(s);
-    if (cuda_failed(cudaGetLastError(), "fri leaves")) return false;
-    return orion::build_tree(tree, n_leaves, s);
+    return leaves && orion::build_tree(tree, n_leaves, s);
 }
 
 bool commit(const ulonglong2* src, int log_len, ulonglong2* l_eval, unsigned char* tree, cudaStream_t s)
@@ -138,9 +131,7 @@ bool commit(const ulonglong2* src, int log_len, ulonglong2* l_eval, unsigned cha
     if (!ok) return false;
     if (cuda_failed(cudaMemsetAsync(tree, 0, 32, s), "rs tree clear")) return false;
     const long long half = slice >> 1;
-    fri_leaf_kernel<<<(unsigned)((half + 255) / 256), 256, 0, s>>>(l_eval, slice, tree, 1u);
-    if (cuda_failed(cudaGetLastError(), "rs leaves")) return false;
-    return orion::build_tree(tree, half, s);
+    return launch_pair_leaves(l_eval, half, 1, slice, half, tree, "rs leaves", s) && orion::build_tree(tree, half, s);
 }
 
 }  // namespace rs

@@ -150,46 +150,74 @@ __host__ __device__ __forceinline__ void compress_pad64(uint32_t st[8], Add add)
 #ifdef __CUDACC__
 // round constants (and the padding block's k + w) for the device's compact form
 static __constant__ Tables kShaTables = make_tables();
+// AddMad's `one` where no launch hands it in
+static __constant__ uint32_t kShaOne = 1u;
 
-// One compression in compact form: four passes over a 16-round body (the
-// schedule's rolling index and the round variables' rotation repeat every 16
-// rounds, so the body indexes registers statically) with the round constants
-// read from constant memory. A quarter of the fully unrolled code: the leaf and
-// tree kernels, which keep one hash in flight per thread, then run from the
-// instruction cache instead of streaming ~40 KB of straight-line code per hash.
+// One round. The additions are grouped so that behind e only Sigma1 and two of them
+// stand before the next e, and behind a Sigma0 and one before the next a; no group
+// has more than seven. Cycles a round (average over a message and a padding block)
+// at one / two / six warps a scheduler: 38.8 / 67.8 / 194.3; in the order of the
+// standard's text 43.3 / 68.8 / 193.1; that order with eight schedule words made in
+// front of the eight rounds that use them 50.5 / 69.8 / 192.6. The ALU pipe's own
+// bound is 26 a warp (13 instructions a round on 16 lanes).
+template <class Add>
+__device__ __forceinline__ void round_step(uint32_t a, uint32_t b, uint32_t c, uint32_t& d, uint32_t e, uint32_t f,
+                                           uint32_t g, uint32_t& h, uint32_t kw, Add add)
+{
+    const uint32_t s1 = rotr(e, 6) ^ rotr(e, 11) ^ rotr(e, 25);
+    const uint32_t ch = (e & f) ^ (~e & g);
+    const uint32_t s0 = rotr(a, 2) ^ rotr(a, 13) ^ rotr(a, 22);
+    const uint32_t mj = (a & b) ^ (a & c) ^ (b & c);
+    const uint32_t t1 = add(s1, add(ch, add(h, kw)));
+    d = add(d, t1);
+    h = add(s0, add(mj, t1));
+}
+
+// Sixteen rounds from round i0 (a multiple of 16); kUpdate: each schedule word is
+// replaced by the one sixteen rounds on right behind the round that used it, off
+// the chain of the rounds.
+template <bool kSched, bool kUpdate, class Add>
+__device__ __forceinline__ void sixteen_rounds(uint32_t s[8], uint32_t w[16], const uint32_t* K, Add add)
+{
+#pragma unroll
+    for (int t = 0; t < 16; ++t) {
+        const uint32_t kw = kSched ? add(w[t], K[t]) : K[t];
+        round_step(s[(0 - t) & 7], s[(1 - t) & 7], s[(2 - t) & 7], s[(3 - t) & 7], s[(4 - t) & 7], s[(5 - t) & 7],
+                   s[(6 - t) & 7], s[(7 - t) & 7], kw, add);
+        if (kSched && kUpdate) {
+            const uint32_t x = w[(t + 1) & 15], y = w[(t + 14) & 15];
+            w[t] = add(rotr(y, 17) ^ rotr(y, 19) ^ (y >> 10),
+                       add(rotr(x, 7) ^ rotr(x, 18) ^ (x >> 3), add(w[t], w[(t + 9) & 15])));
+        }
+    }
+}
+
+// One compression in compact form: a 16-round body looped (the schedule's rolling
+// index and the round variables' rotation repeat every 16 rounds, so the body
+// indexes registers statically) with the round constants read from constant
+// memory, and for a message block the last 16 rounds, which make no schedule
+// words, behind it. Less than half of the fully unrolled code: the leaf and tree
+// kernels, which keep one hash in flight per thread, run from the instruction
+// cache instead of streaming ~40 KB of straight-line code per hash (65 cycles a
+// round at one warp a scheduler, 254 at six in that form).
 // kSched: message block w (consumed as the rolling schedule); otherwise the
 // constant padding block, K holding its k + w.
 template <bool kSched, class Add>
 __device__ __forceinline__ void compress_compact(uint32_t st[8], uint32_t w[16], const uint32_t* K, Add add)
 {
-    uint32_t a = st[0], b = st[1], c = st[2], d = st[3], e = st[4], f = st[5], g = st[6], h = st[7];
+    uint32_t s[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s[i] = st[i];
+    if (kSched) {
 #pragma unroll 1
-    for (int i = 0; i < 64; i += 16) {
-#pragma unroll
-        for (int j = 0; j < 16; j += 8) {
-            if (kSched && i > 0) {
-#pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    const int t = j + q;    // w[t] holds word i + t - 16 here
-                    const uint32_t x = w[(t + 1) & 15], y = w[(t + 14) & 15];
-                    w[t] = add(add(w[t], rotr(x, 7) ^ rotr(x, 18) ^ (x >> 3)),
-                               add(w[(t + 9) & 15], rotr(y, 17) ^ rotr(y, 19) ^ (y >> 10)));
-                }
-            }
-#define TP_SHA_KW(q) (kSched ? add(w[j + q], K[i + j + q]) : K[i + j + q])
-            TP_SHA_ROUND(a, b, c, d, e, f, g, h, TP_SHA_KW(0));
-            TP_SHA_ROUND(h, a, b, c, d, e, f, g, TP_SHA_KW(1));
-            TP_SHA_ROUND(g, h, a, b, c, d, e, f, TP_SHA_KW(2));
-            TP_SHA_ROUND(f, g, h, a, b, c, d, e, TP_SHA_KW(3));
-            TP_SHA_ROUND(e, f, g, h, a, b, c, d, TP_SHA_KW(4));
-            TP_SHA_ROUND(d, e, f, g, h, a, b, c, TP_SHA_KW(5));
-            TP_SHA_ROUND(c, d, e, f, g, h, a, b, TP_SHA_KW(6));
-            TP_SHA_ROUND(b, c, d, e, f, g, h, a, TP_SHA_KW(7));
-#undef TP_SHA_KW
-        }
+        for (int i = 0; i < 48; i += 16) sixteen_rounds<true, true>(s, w, K + i, add);
+        sixteen_rounds<true, false>(s, w, K + 48, add);
+    } else {
+#pragma unroll 1
+        for (int i = 0; i < 64; i += 16) sixteen_rounds<false, false>(s, w, K + i, add);
     }
-    st[0] = add(st[0], a); st[1] = add(st[1], b); st[2] = add(st[2], c); st[3] = add(st[3], d);
-    st[4] = add(st[4], e); st[5] = add(st[5], f); st[6] = add(st[6], g); st[7] = add(st[7], h);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) st[i] = add(st[i], s[i]);
 }
 #endif
 
