@@ -48,7 +48,7 @@ struct DevPar {
     template <class F>
     __device__ void one(F&& fn) const
     {
-        if (threadIdx.x == 0) fn();
+        if (threadIdx.x < 32) fn();   // the first warp, all lanes (transcript.cuh)
         __syncthreads();
     }
 };

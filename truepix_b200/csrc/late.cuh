@@ -127,7 +127,6 @@ struct Work {
     fp2 A[kMaxGates];
     fp2 red[3][kThreads];
     fp2 w[2 * kMaxInBits];     // the challenges
-    fp2 pt[kMaxInBits];        // a point on the line
     fp2 h[kMaxInBits + 1];     // the line's values
     fp2 hc[kMaxInBits + 1];    // its coefficients
     fp2 vv[kMaxInBits + 1];    // closing: the coefficients' tags
@@ -193,32 +192,55 @@ TP_HD void step_sums(Work& w, const uint32_t* gates, const Shape& sh, int rd, in
     w.red[2][tid] = s2;
 }
 
-// one level of the tree sum: threads below `half` add the slot `half` above
-TP_HD void step_reduce(Work& w, int half, int tid)
+// one level of the sum over the threads' slots: threads below `left` add the three
+// slots left, 2 left and 3 left above theirs (256 slots in four steps)
+TP_HD void step_reduce(Work& w, int left, int tid)
 {
-    if (tid < half)
-        for (int q = 0; q < 3; ++q) w.red[q][tid] = f2add(w.red[q][tid], w.red[q][tid + half]);
+    if (tid < left)
+        for (int q = 0; q < 3; ++q) {
+            fp2* r = w.red[q] + tid;
+            r[0] = f2add(f2add(r[0], r[left]), f2add(r[2 * left], r[3 * left]));
+        }
 }
 
-// thread 0: the round's coefficients and its challenge
+// The steps run by `par.one`: one warp on the device (one call on the host). Its
+// lanes do the same work, each on copies of its own of the transcript and the
+// VOLE state (transcript.cuh), and lane 0 writes. Reads of the workspace that the
+// writes below them would change come before the synchronisation in front of these.
+TP_HD void warp_sync()
+{
+#ifdef __CUDA_ARCH__
+    __syncwarp();
+#endif
+}
+
+// the round's coefficients and its challenge
 TP_HD void step_head(Work& w, const Frame& f, const Shape& sh, int rd)
 {
     fp2 c[3];
     vole::interpolate_quadratic(f2mul(w.red[0][0], w.beta), f2mul(w.red[1][0], w.beta),
                                 f2mul(w.red[2][0], w.beta), c);
-    for (int q = 0; q < 3; ++q) f.coefs[3 * rd + q] = c[q];
     fp2 r;
     if (f.chal) {
         r = f.chal[rd];
     } else {
+        fs::State st = w.st;
+        vole::State vs = w.vs;
         const fs::Label label = vole::sc_label(sh.layer, sh.round0 + rd);
-        if (!vole::round(w.st, w.vs, c, 3, f.u, f.v, sh.count, label, f.proof ? f.proof + 4 * rd : nullptr,
-                         &r))
-            w.bad = 1;
+        const bool ok = vole::round(st, vs, c, 3, f.u, f.v, sh.count, label, f.proof ? f.proof + 4 * rd : nullptr, &r);
+        warp_sync();
+        if (fs::lead()) {
+            w.st = st;
+            w.vs = vs;
+            if (!ok) w.bad = 1;
+        }
     }
-    w.r = r;
-    w.w[rd] = r;
-    f.chal_out[rd] = r;
+    if (fs::lead()) {
+        for (int q = 0; q < 3; ++q) f.coefs[3 * rd + q] = c[q];
+        w.r = r;
+        w.w[rd] = r;
+        f.chal_out[rd] = r;
+    }
 }
 
 // fold T by the challenge into Tn, update the gates' weights
@@ -246,42 +268,134 @@ TP_HD void step_restart(Work& w, const Shape& sh, int tid)
     for (int k = tid; k < (1 << sh.n); k += kThreads) w.T[k] = w.V[k];
 }
 
-// thread 0: the point w1 + t (w2 - w1)
-TP_HD void step_line_point(Work& w, const Shape& sh, int t)
-{
-    for (int j = 0; j < sh.n; ++j) w.pt[j] = f2add(w.w[j], f2scale(f2sub(w.w[sh.n + j], w.w[j]), (u64)t));
-}
+// ---- the line projection: V at the points w1 + t (w2 - w1), t = 2..n, as sums over
+// the wires of eq(point, k) V[k], all points at once (one warp's worth of threads
+// each); eq from two half tables. T and Tn are free by then.
 
-// fold T by coordinate j of the line point into Tn
-TP_HD void step_fold_point(Work& w, const Shape& sh, int j, int tid)
-{
-    const int half = (1 << sh.n) >> (j + 1);
-    const fp2 r = w.pt[j];
-    for (int k = tid; k < half; k += kThreads) w.Tn[k] = f2fold(w.T[2 * k], w.T[2 * k + 1], r);
-}
+TP_HD int line_low_bits(const Shape& sh) { return sh.n >> 1; }
+TP_HD int line_table(const Shape& sh) { return (1 << line_low_bits(sh)) + (1 << (sh.n - line_low_bits(sh))); }
 
-// thread 0: coefficients (constant first) of the polynomial through (t, h[t]),
-// t = 0..n, by Newton's divided differences on the nodes 0..n
-TP_HD void step_interpolate(Work& w, const Frame& f, const Shape& sh)
+// the points' coordinates, Tn[(t - 2) n + j]
+TP_HD void step_line_points(Work& w, const Shape& sh, int tid)
 {
     const int n = sh.n;
-    fp2 d[kMaxInBits + 1], c[kMaxInBits + 1];
-    for (int i = 0; i <= n; ++i) d[i] = w.h[i];
-    for (int lvl = 1; lvl <= n; ++lvl) {
-        const u64 inv = finv((u64)lvl);
-        for (int i = n; i >= lvl; --i) d[i] = f2scale(f2sub(d[i], d[i - 1]), inv);
+    if (tid >= (n - 1) * n) return;
+    const int t = 2 + tid / n, j = tid % n;
+    w.Tn[tid] = f2add(w.w[j], f2scale(f2sub(w.w[n + j], w.w[j]), (u64)t));
+}
+
+// the half tables of eq, T[(t - 2) table + entry]: the low half first
+TP_HD void step_line_eq(Work& w, const Shape& sh, int tid)
+{
+    const int n = sh.n, n1 = line_low_bits(sh), lo = 1 << n1, table = line_table(sh);
+    const fp2 one = mk(1, 0);
+    for (int e = tid; e < (n - 1) * table; e += kThreads) {
+        const int q = e / table, i = e % table;
+        const int first = i < lo ? 0 : n1, last = i < lo ? n1 : n, k = i < lo ? i : i - lo;
+        fp2 v = one;
+        for (int j = first; j < last; ++j) {
+            const fp2 p = w.Tn[q * n + j];
+            v = f2mul(v, ((k >> (j - first)) & 1) ? p : f2sub(one, p));
+        }
+        w.T[e] = v;
     }
-    // c(t) = d[n]; then c(t) <- c(t) (t - i) + d[i] for i = n - 1..0
-    for (int i = 0; i <= n; ++i) c[i] = f2zero();
-    c[0] = d[n];
-    int deg = 0;
-    for (int i = n - 1; i >= 0; --i) {
-        c[deg + 1] = c[deg];
-        for (int k = deg; k >= 1; --k) c[k] = f2sub(c[k - 1], f2scale(c[k], (u64)i));
-        c[0] = f2add(f2sub(f2zero(), f2scale(c[0], (u64)i)), d[i]);
-        ++deg;
+}
+
+// partial sums of point t = 2 + tid / 32
+TP_HD void step_line_sums(Work& w, const Shape& sh, int tid)
+{
+    const int q = tid >> 5, n1 = line_low_bits(sh);
+    fp2 s = f2zero();
+    if (q < sh.n - 1) {
+        const fp2* lo = w.T + q * line_table(sh);
+        const fp2* hi = lo + (1 << n1);
+        for (int k = tid & 31; k < (1 << sh.n); k += 32)
+            s = f2add(s, f2mul(f2mul(lo[k & ((1 << n1) - 1)], hi[k >> n1]), w.V[k]));
     }
-    for (int i = 0; i <= n; ++i) f.h[i] = w.hc[i] = c[i];
+    w.red[0][tid] = s;
+}
+
+// one level of the sums within each 32 slots (32 -> 8 -> 2 -> 1)
+TP_HD void step_line_reduce(Work& w, int left, int tid)
+{
+    if ((tid & 31) >= left) return;
+    fp2* r = w.red[0] + tid;
+    r[0] = left > 1 ? f2add(f2add(r[0], r[left]), f2add(r[2 * left], r[3 * left])) : f2add(r[0], r[1]);
+}
+
+TP_HD void step_line_values(Work& w, const Shape& sh, int tid)
+{
+    if (tid < sh.n - 1) w.h[2 + tid] = w.red[0][32 * tid];
+}
+
+// The coefficients of the polynomial of degree n through (t, h[t]), t = 0..n, are a
+// fixed matrix times the values: row k, column t is the coefficient of x^k in the
+// t-th Lagrange polynomial on the nodes 0..n. The matrices for n <= kMaxInBits are
+// made at compile time.
+constexpr u64 mul_c(u64 a, u64 b)   // canonical a, b -> a b mod p (compile time)
+{
+    const u64 a0 = a & 0xFFFFFFFFull, a1 = a >> 32, b0 = b & 0xFFFFFFFFull, b1 = b >> 32;
+    const u64 lo = a0 * b0, mid = a0 * b1 + a1 * b0, hi = a1 * b1;
+    u64 s = (lo & P61) + (lo >> 61) + (hi << 3) + (mid >> 29) + ((mid & 0x1FFFFFFFull) << 32);
+    s = (s & P61) + (s >> 61);
+    return s >= P61 ? s - P61 : s;
+}
+constexpr u64 neg_c(u64 a) { return a ? P61 - a : 0; }
+// 1 / k mod p for 1 <= k <= 9: (m p + 1) / k for the m that makes it whole
+constexpr u64 inv_c(u64 k)
+{
+    for (u64 m = 0; m < k; ++m)
+        if ((m * P61 + 1) % k == 0) return (m * P61 + 1) / k;
+    return 0;
+}
+struct LineMatrix {
+    u64 m[kMaxInBits + 1][kMaxInBits + 1][kMaxInBits + 1];   // [n][k][t]
+};
+constexpr LineMatrix make_line_matrix()
+{
+    LineMatrix L{};
+    for (int n = 1; n <= kMaxInBits; ++n)
+        for (int t = 0; t <= n; ++t) {
+            u64 c[kMaxInBits + 2] = {1};   // the product of (x - i) / (t - i) over i != t
+            int deg = 0;
+            for (int i = 0; i <= n; ++i) {
+                if (i == t) continue;
+                const u64 inv = t > i ? inv_c((u64)(t - i)) : neg_c(inv_c((u64)(i - t)));
+                for (int k = deg + 1; k >= 0; --k) {
+                    const u64 up = k > 0 ? c[k - 1] : 0, here = k <= deg ? neg_c(mul_c(c[k], (u64)i)) : 0;
+                    const u64 sum = up + here >= P61 ? up + here - P61 : up + here;
+                    c[k] = mul_c(sum, inv);
+                }
+                ++deg;
+            }
+            for (int k = 0; k <= n; ++k) L.m[n][k][t] = c[k];
+        }
+    return L;
+}
+#ifdef __CUDACC__
+static __constant__ LineMatrix kLineMatrixDev = make_line_matrix();
+#endif
+inline u64 line_entry_host(int n, int k, int t)
+{
+    static constexpr LineMatrix L = make_line_matrix();
+    return L.m[n][k][t];
+}
+
+// thread k: coefficient k (constant first) of the polynomial through (t, h[t])
+#pragma nv_exec_check_disable
+TP_HD void step_interpolate(Work& w, const Frame& f, const Shape& sh, int tid)
+{
+    if (tid > sh.n) return;
+    fp2 c = f2zero();
+    for (int t = 0; t <= sh.n; ++t) {
+#ifdef __CUDA_ARCH__
+        const u64 m = kLineMatrixDev.m[sh.n][tid][t];
+#else
+        const u64 m = line_entry_host(sh.n, tid, t);
+#endif
+        c = f2add(c, f2scale(w.h[t], m));
+    }
+    f.h[tid] = w.hc[tid] = c;
 }
 
 // ---- the layer's closing proofs (circuitnizkvec_vole.py:433-500, one layer) ----
@@ -291,65 +405,65 @@ TP_HD void step_interpolate(Work& w, const Frame& f, const Shape& sh)
 // commitments, the product proof's two values and with zk the masks' two)
 TP_HD int close_eq_index(const Shape& sh) { return sh.n + 6 + 5 * (sh.zk != 0); }
 
-// thread 0: create_final_prod_pok (:175-218; the zero-knowledge prover's,
+// create_final_prod_pok (:175-218; the zero-knowledge prover's,
 // circuitnizkvec_vole_ZK.py:188-247, adds three mask commitments of 1 and their
 // product proof) on the line's coefficients
 TP_HD void step_close_commit(Work& w, const Frame& f, const Shape& sh)
 {
     const int n = sh.n;
     const int zk = sh.zk != 0;
-    if (w.vs.bad || w.vs.idx + (unsigned long long)(n + 2 + 3 * zk) > (unsigned long long)sh.count) {
-        w.vs.bad = 1;
-        w.bad = 1;
+    fs::State st = w.st;
+    vole::State vs = w.vs;
+    if (vs.bad || vs.idx + (unsigned long long)(n + 2 + 3 * zk) > (unsigned long long)sh.count) {
+        warp_sync();
+        if (fs::lead()) {
+            w.vs.bad = 1;
+            w.bad = 1;
+        }
         return;
     }
     fp2* out = f.closing;
+    auto put = [&](fp2 v) {   // the next closing value: written out and put
+        fs::put_fp2(st, v.re, v.im);
+        if (fs::lead()) *out = v;
+        ++out;
+    };
     fp2 sval = f2zero();
     for (int k = 0; k <= n; ++k) sval = f2add(sval, w.hc[k]);
     const fp2 prod = f2mul(w.hc[0], sval);
-    fp2 v1, v3;
-    out[0] = vole::commit(w.vs, w.hc[0], f.u, f.v, &v1);
-    out[1] = vole::commit(w.vs, prod, f.u, f.v, &v3);
-    fs::put_fp2(w.st, out[0].re, out[0].im);
-    fs::put_fp2(w.st, out[1].re, out[1].im);
+    fp2 v1, v3, vv[kMaxInBits + 1], mtag[3];
+    const fp2 d0 = vole::commit(vs, w.hc[0], f.u, f.v, &v1);
+    const fp2 d1 = vole::commit(vs, prod, f.u, f.v, &v3);
+    put(d0);
+    put(d1);
     fp2 rest_sum = f2zero(), rest_v = f2zero();
-    w.vv[0] = v1;
+    vv[0] = v1;
     for (int k = 1; k <= n; ++k) {
-        out[1 + k] = vole::commit(w.vs, w.hc[k], f.u, f.v, &w.vv[k]);
-        fs::put_fp2(w.st, out[1 + k].re, out[1 + k].im);
+        put(vole::commit(vs, w.hc[k], f.u, f.v, &vv[k]));
         rest_sum = f2add(rest_sum, w.hc[k]);
-        rest_v = f2add(rest_v, w.vv[k]);
+        rest_v = f2add(rest_v, vv[k]);
     }
-    const fp2 c = fs::rand_fp2(w.st, fs::label_lit("pok-vec"));
-    out[n + 2] = f2mul(rest_sum, c);
-    out[n + 3] = f2mul(rest_v, c);
-    fs::put_fp2(w.st, out[n + 2].re, out[n + 2].im);
-    fs::put_fp2(w.st, out[n + 3].re, out[n + 3].im);
-    int k = n + 4;
-    fp2 mtag[3];
-    if (zk) {
-        for (int q = 0; q < 3; ++q) {
-            out[k] = vole::commit(w.vs, mk(1, 0), f.u, f.v, &mtag[q]);
-            fs::put_fp2(w.st, out[k].re, out[k].im);
-            ++k;
-        }
-    }
-    fp2 vsum = f2zero();
-    for (int q = 0; q <= n; ++q) vsum = f2add(vsum, w.vv[q]);
+    const fp2 c = fs::rand_fp2(st, fs::label_lit("pok-vec"));
+    put(f2mul(rest_sum, c));
+    put(f2mul(rest_v, c));
+    if (zk)
+        for (int q = 0; q < 3; ++q) put(vole::commit(vs, mk(1, 0), f.u, f.v, &mtag[q]));
+    const fp2 vsum = f2add(v1, rest_v);
     // prod_finish on (x, sum, x * sum) with tags (v1, sum of tags, v3)
-    out[k] = f2mul(v1, vsum);
-    out[k + 1] = f2sub(f2add(f2mul(w.hc[0], vsum), f2mul(sval, v1)), v3);
-    fs::put_fp2(w.st, out[k].re, out[k].im);
-    fs::put_fp2(w.st, out[k + 1].re, out[k + 1].im);
+    put(f2mul(v1, vsum));
+    put(f2sub(f2add(f2mul(w.hc[0], vsum), f2mul(sval, v1)), v3));
     if (zk) {   // prod_finish on (1, 1, 1) with the masks' tags
-        out[k + 2] = f2mul(mtag[0], mtag[1]);
-        out[k + 3] = f2sub(f2add(mtag[1], mtag[0]), mtag[2]);
-        fs::put_fp2(w.st, out[k + 2].re, out[k + 2].im);
-        fs::put_fp2(w.st, out[k + 3].re, out[k + 3].im);
+        put(f2mul(mtag[0], mtag[1]));
+        put(f2sub(f2add(mtag[1], mtag[0]), mtag[2]));
     }
+    warp_sync();
+    if (!fs::lead()) return;
+    for (int k = 0; k <= n; ++k) w.vv[k] = vv[k];
     w.pr[0] = v1;
     w.pr[1] = vsum;
     w.pr[2] = v3;
+    w.st = st;
+    w.vs = vs;
 }
 
 // per-thread partial sums of the wiring predicates' multilinear extensions times
@@ -376,12 +490,18 @@ TP_HD void step_close_sums(Work& w, const Frame& f, const uint32_t* gates, const
     w.red[2][tid] = f2zero();
 }
 
-// thread 0: the equality proof against the last round's value, tau, the proof of
-// knowledge of all round coefficients, the input point and its value proof
+// the equality proof against the last round's value, tau, the proof of knowledge
+// of all round coefficients, the input point and its value proof
 TP_HD void step_close_tail(Work& w, const Frame& f, const Shape& sh)
 {
     const int n = sh.n, nb = sh.round0;
-    fp2* out = f.closing + (close_eq_index(sh) - (n + 6));   // out[n + 6]: the equality value
+    fs::State st = w.st;
+    fp2* out = f.closing + close_eq_index(sh);
+    auto put = [&](fp2 v) {
+        fs::put_fp2(st, v.re, v.im);
+        if (fs::lead()) *out = v;
+        ++out;
+    };
     // beta's factor: prod over the early challenges of 2 w z + 1 - (w + z)
     fp2 mz = mk(1, 0);
     for (int k = 0; k < nb; ++k) {
@@ -389,53 +509,51 @@ TP_HD void step_close_tail(Work& w, const Frame& f, const Shape& sh)
         mz = f2mul(mz, f2sub(f2add(f2dbl(f2mul(wk, zk)), mk(1, 0)), f2add(wk, zk)));
     }
     const fp2 tv = f2mul(w.red[0][0], mz);
-    const fp2 e = fs::rand_fp2(w.st, fs::label_lit("eq"));
-    out[n + 6] = f2mul(f2sub(w.vs.prev, tv), e);
-    fs::put_fp2(w.st, out[n + 6].re, out[n + 6].im);
-    const fp2 tau = fs::rand_fp2(w.st, vole::tau_label(sh.layer));
+    const fp2 e = fs::rand_fp2(st, fs::label_lit("eq"));
+    put(f2mul(f2sub(w.vs.prev, tv), e));
+    const fp2 tau = fs::rand_fp2(st, vole::tau_label(sh.layer));
     fp2 tag = w.vv[n];
     for (int k = n - 1; k >= 0; --k) tag = f2add(f2mul(tag, tau), w.vv[k]);
-    for (int j = 0; j < n; ++j) f.point[j] = f2add(w.w[j], f2mul(f2sub(w.w[n + j], w.w[j]), tau));
-    for (int k = 0; k < nb; ++k) f.point[n + k] = f.w3[k * f.w3_stride];
     // create_pok_final
     fp2 osum = f2zero(), vsum = f2zero();
     for (int k = 0; k < 4; ++k) {
         osum = f2add(osum, w.vs.out_elem[k]);
         vsum = f2add(vsum, w.vs.v_elem[k]);
     }
-    const fp2 c = fs::rand_fp2(w.st, fs::label_lit("pok-final"));
-    out[n + 7] = f2mul(osum, c);
-    out[n + 8] = f2mul(vsum, c);
-    fs::put_fp2(w.st, out[n + 7].re, out[n + 7].im);
-    fs::put_fp2(w.st, out[n + 8].re, out[n + 8].im);
+    const fp2 c = fs::rand_fp2(st, fs::label_lit("pok-final"));
+    put(f2mul(osum, c));
+    put(f2mul(vsum, c));
     // put(["gkr_input_point", [[re, im], ...]]): a string, then every coordinate's two ints
-    fs::put_label(w.st, fs::label_lit("gkr_input_point"));
+    fs::put_label(st, fs::label_lit("gkr_input_point"));
     for (int k = 0; k < n + nb; ++k) {
-        fs::absorb_byte(w.st, 0x02);
-        fs::absorb_le(w.st, f.point[k].re, 8);
-        fs::absorb_byte(w.st, 0x02);
-        fs::absorb_le(w.st, f.point[k].im, 8);
+        const fp2 x = k < n ? f2add(w.w[k], f2mul(f2sub(w.w[n + k], w.w[k]), tau)) : f.w3[(k - n) * f.w3_stride];
+        if (fs::lead()) f.point[k] = x;
+        fs::absorb_le(st, 0x02 | (x.re << 8), 8);
+        fs::absorb_le(st, (x.re >> 56) | (0x02 << 8) | (x.im << 16), 8);
+        fs::absorb_le(st, x.im >> 48, 2);
     }
     // create_input_value_proof
-    const fp2 civ = fs::rand_fp2(w.st, fs::label_lit("input-val"));
-    out[n + 9] = f2mul(tag, civ);
-    fs::put_fp2(w.st, out[n + 9].re, out[n + 9].im);
+    const fp2 civ = fs::rand_fp2(st, fs::label_lit("input-val"));
+    put(f2mul(tag, civ));
+    warp_sync();
+    if (!fs::lead()) return;
+    w.st = st;
     w.vs.prev = tag;
     *f.tag = tag;
 }
 
-// thread 0: the VOLE state and transcript back to the frame
+// the VOLE state and transcript back to the frame
 TP_HD void step_store(Work& w, const Frame& f)
 {
-    if (!f.chal) {
+    if (!f.chal && fs::lead()) {
         *f.st = w.st;
         *f.vs = w.vs;
     }
 }
 
 // The whole late phase of one frame. par.all(fn) runs fn(thread index) on every
-// thread of the CTA and then waits at a barrier; par.one(fn) runs fn on thread 0
-// and waits. Every branch below depends only on values all threads read alike
+// thread of the CTA and then waits at a barrier; par.one(fn) runs fn once (on the
+// device: on every lane of the first warp, see above) and waits. Every branch below depends only on values all threads read alike
 // after a barrier.
 #pragma nv_exec_check_disable
 template <class Par>
@@ -445,35 +563,31 @@ TP_HD void run_frame(Work& w, const Frame& f, const Shape& sh, const uint32_t* g
     par.all([&](int tid) { step_load(w, f, sh, tid); });
     for (int rd = 0; rd < 2 * n; ++rd) {
         par.all([&](int tid) { step_sums(w, gates, sh, rd, tid); });
-        for (int half = kThreads / 2; half > 0; half >>= 1) par.all([&](int tid) { step_reduce(w, half, tid); });
+        for (int left = kThreads / 4; left > 0; left >>= 2) par.all([&](int tid) { step_reduce(w, left, tid); });
         par.one([&] { step_head(w, f, sh, rd); });
         if (w.bad) break;
         par.all([&](int tid) { step_fold(w, gates, sh, rd, tid); });
         const int j = rd < n ? rd : rd - n;
         par.all([&](int tid) { step_copy(w, W >> (j + 1), tid); });
         if (rd == n - 1) {
-            par.one([&] { w.v1 = w.h[0] = w.T[0]; });
+            par.all([&](int tid) { if (tid == 0) w.v1 = w.h[0] = w.T[0]; });
             par.all([&](int tid) { step_restart(w, sh, tid); });
         }
-        if (rd == 2 * n - 1) par.one([&] { w.h[1] = w.T[0]; });
+        if (rd == 2 * n - 1) par.all([&](int tid) { if (tid == 0) w.h[1] = w.T[0]; });
     }
     if (!w.bad) {
-        for (int t = 2; t <= n; ++t) {
-            par.one([&] { step_line_point(w, sh, t); });
-            par.all([&](int tid) { step_restart(w, sh, tid); });
-            for (int j = 0; j < n; ++j) {
-                par.all([&](int tid) { step_fold_point(w, sh, j, tid); });
-                par.all([&](int tid) { step_copy(w, W >> (j + 1), tid); });
-            }
-            par.one([&] { w.h[t] = w.T[0]; });
-        }
-        par.one([&] { step_interpolate(w, f, sh); });
+        par.all([&](int tid) { step_line_points(w, sh, tid); });
+        par.all([&](int tid) { step_line_eq(w, sh, tid); });
+        par.all([&](int tid) { step_line_sums(w, sh, tid); });
+        for (int left = 8; left > 0; left = left > 2 ? 2 : left - 1) par.all([&](int tid) { step_line_reduce(w, left, tid); });
+        par.all([&](int tid) { step_line_values(w, sh, tid); });
+        par.all([&](int tid) { step_interpolate(w, f, sh, tid); });
         if (f.closing) {
             par.one([&] { step_close_commit(w, f, sh); });
             if (!w.bad) {
                 par.all([&](int tid) { step_close_sums(w, f, gates, sh, tid); });
-                for (int half = kThreads / 2; half > 0; half >>= 1)
-                    par.all([&](int tid) { step_reduce(w, half, tid); });
+                for (int left = kThreads / 4; left > 0; left >>= 2)
+                    par.all([&](int tid) { step_reduce(w, left, tid); });
                 par.one([&] { step_close_tail(w, f, sh); });
             }
         }

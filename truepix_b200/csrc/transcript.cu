@@ -73,81 +73,95 @@ bool make_device_label(const char* label, tp::fs::Label* L, const char* who)
     return true;
 }
 
-__global__ void put_fp2s_kernel(State* __restrict__ st, int n, const ulonglong2* __restrict__ vals, int k)
+// Device transcripts: one warp (a CTA of 32 threads) per state, see transcript.cuh.
+// The kernels are bound by the latency of the hash's round chain, so a warp of its
+// own costs nothing, transcripts at different offsets do not diverge, and the two
+// digests of a draw are closed side by side.
+constexpr int kFsThreads = 32;
+
+// the warp's state back to memory, once every lane has read it
+__device__ __forceinline__ void store_state(State* st, const State& s)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    __syncwarp();
+    if (tp::fs::lead()) *st = s;
+}
+
+__global__ void __launch_bounds__(kFsThreads) put_fp2s_kernel(State* __restrict__ st,
+                                                              const ulonglong2* __restrict__ vals, int k)
+{
+    const int i = blockIdx.x;
     State s = st[i];
     for (int j = 0; j < k; ++j) {
         const ulonglong2 v = vals[(long long)i * k + j];   // packed {re, im}
         tp::fs::put_fp2(s, v.x, v.y);
     }
-    st[i] = s;
+    store_state(st + i, s);
 }
 
-__global__ void rand_ext_kernel(State* __restrict__ st, int n, tp::fs::Label L, ulonglong2* __restrict__ out)
+__global__ void __launch_bounds__(kFsThreads) rand_ext_kernel(State* __restrict__ st, tp::fs::Label L,
+                                                              ulonglong2* __restrict__ out)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    const int i = blockIdx.x;
     State s = st[i];
     const tp::fp2 r = tp::fs::rand_fp2(s, L);
-    st[i] = s;
-    out[i] = make_ulonglong2(r.re, r.im);
+    store_state(st + i, s);
+    if (tp::fs::lead()) out[i] = make_ulonglong2(r.re, r.im);
 }
 
-// ---- VOLE-committed early round (vole.cuh), one thread per frame ----------------
+// ---- VOLE-committed early round (vole.cuh), one warp per frame ------------------
 using VoleState = tp::vole::State;
 
-// rounds (optional): frame i takes part only while this round k < rounds[i]
-__global__ void vole_round_kernel(State* __restrict__ st, VoleState* __restrict__ vs, int n,
-                                  const tp::fp2* __restrict__ claims, const tp::fp2* __restrict__ u,
-                                  const tp::fp2* __restrict__ v, long long count, tp::fs::Label L,
-                                  tp::fp2* __restrict__ chal, tp::fp2* __restrict__ proof,
-                                  const int* __restrict__ rounds, int k)
+// the round of frame i on its four claims: the states updated in place, the
+// challenge returned (on every lane)
+__device__ __forceinline__ tp::fp2 vole_round_frame(State* st, VoleState* vs, const tp::fp2* claims,
+                                                    const tp::fp2* u, const tp::fp2* v, long long count,
+                                                    const tp::fs::Label& L, tp::fp2* proof)
 {
     using namespace tp;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || (rounds && k >= rounds[i])) return;
-    VoleState w = vs[i];
-    State s = st[i];
-    fp2 coef[4];
-    vole::interpolate_cubic(claims[4 * i], claims[4 * i + 1], claims[4 * i + 2], claims[4 * i + 3], coef);
+    VoleState w = *vs;
+    State s = *st;
+    fp2 coef[4], r;
+    vole::interpolate_cubic(claims[0], claims[1], claims[2], claims[3], coef);
+    vole::round(s, w, coef, 4, u, v, count, L, proof, &r);
+    store_state(st, s);
+    if (fs::lead()) *vs = w;
+    return r;
+}
+
+// rounds (optional): frame i takes part only while this round k < rounds[i]
+__global__ void __launch_bounds__(kFsThreads) vole_round_kernel(
+    State* __restrict__ st, VoleState* __restrict__ vs, const tp::fp2* __restrict__ claims,
+    const tp::fp2* __restrict__ u, const tp::fp2* __restrict__ v, long long count, tp::fs::Label L,
+    tp::fp2* __restrict__ chal, tp::fp2* __restrict__ proof, const int* __restrict__ rounds, int k)
+{
+    const int i = blockIdx.x;
+    if (rounds && k >= rounds[i]) return;
     const long long base = (long long)i * count;
-    fp2 r;
-    vole::round(s, w, coef, 4, u + base, v + base, count, L, proof ? proof + 5 * i : nullptr, &r);
-    st[i] = s;
-    vs[i] = w;
-    chal[i] = r;
+    const tp::fp2 r = vole_round_frame(st + i, vs + i, claims + 4 * i, u + base, v + base, count, L,
+                                       proof ? proof + 5 * i : nullptr);
+    if (tp::fs::lead()) chal[i] = r;
 }
 
 // ---- VOLE-committed rounds of frames each at its own round (the serving loop) ----
 // meta[slot] = {round, rounds}: round < 0 means the slot is idle; after its round
 // the slot moves to round + 1, or to -1 after its last round.
-__global__ void vole_round_slots_kernel(State* __restrict__ st, VoleState* __restrict__ vs, int n,
-                                        int2* __restrict__ meta, const tp::fp2* __restrict__ claims,
-                                        const tp::fp2* __restrict__ u, const tp::fp2* __restrict__ v,
-                                        long long count, int layer, tp::fp2* __restrict__ chal_cur,
-                                        tp::fp2* __restrict__ chal_hist, tp::fp2* __restrict__ proof, int max_rounds)
+__global__ void __launch_bounds__(kFsThreads) vole_round_slots_kernel(
+    State* __restrict__ st, VoleState* __restrict__ vs, int2* __restrict__ meta, const tp::fp2* __restrict__ claims,
+    const tp::fp2* __restrict__ u, const tp::fp2* __restrict__ v, long long count, int layer,
+    tp::fp2* __restrict__ chal_cur, tp::fp2* __restrict__ chal_hist, tp::fp2* __restrict__ proof, int max_rounds)
 {
-    using namespace tp;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    const int i = blockIdx.x;
     const int2 m = meta[i];
     if (m.x < 0 || m.x >= m.y || m.x >= max_rounds) return;
-    VoleState w = vs[i];
-    State s = st[i];
-    fp2 coef[4];
-    vole::interpolate_cubic(claims[4 * i], claims[4 * i + 1], claims[4 * i + 2], claims[4 * i + 3], coef);
     const long long base = (long long)i * count;
-    fp2 r;
     const long long at = (long long)i * max_rounds + m.x;
-    vole::round(s, w, coef, 4, u + base, v + base, count, vole::sc_label(layer, m.x), proof ? proof + 5 * at : nullptr,
-                &r);
-    st[i] = s;
-    vs[i] = w;
-    chal_cur[i] = r;
-    chal_hist[at] = r;
-    meta[i] = make_int2(m.x + 1 < m.y ? m.x + 1 : -1, m.y);
+    const tp::fp2 r = vole_round_frame(st + i, vs + i, claims + 4 * i, u + base, v + base, count,
+                                       tp::vole::sc_label(layer, m.x), proof ? proof + 5 * at : nullptr);
+    if (tp::fs::lead()) {
+        chal_cur[i] = r;
+        chal_hist[at] = r;
+        meta[i] = make_int2(m.x + 1 < m.y ? m.x + 1 : -1, m.y);
+    }
 }
 
 // ---- host absorbs: whole blocks compressed straight from the caller's bytes,
@@ -185,18 +199,21 @@ void host_blocks(uint32_t h[8], const uint8_t* p, size_t nblocks)
     }
 }
 
+// the bytes of the pending partial block
+uint8_t* pending(State& s) { return reinterpret_cast<uint8_t*>(s.unit); }
+
 // the same bytes and state as tp::fs::absorb
 void host_absorb(State& s, const uint8_t* p, uint64_t n)
 {
     s.total += n;
     if (s.nbuf) {
         const uint64_t take = n < 64u - s.nbuf ? n : 64u - s.nbuf;
-        memcpy(s.buf + s.nbuf, p, take);
+        memcpy(pending(s) + s.nbuf, p, take);
         s.nbuf += (uint32_t)take;
         p += take;
         n -= take;
         if (s.nbuf < 64) return;
-        host_blocks(s.h, s.buf, 1);
+        host_blocks(s.h, pending(s), 1);
         s.nbuf = 0;
     }
     const uint64_t nb = n / 64;
@@ -205,7 +222,7 @@ void host_absorb(State& s, const uint8_t* p, uint64_t n)
         p += 64 * nb;
         n -= 64 * nb;
     }
-    memcpy(s.buf, p, n);
+    memcpy(pending(s), p, n);
     s.nbuf = (uint32_t)n;
 }
 
@@ -306,7 +323,7 @@ void put_outputs_group(State* const* st, const uint8_t* const* pix, int k, const
     uint32_t* h[kGroup];
     const uint8_t* p[kGroup];
     size_t fill = st[0]->nbuf;   // equal for every frame of the group
-    for (int c = 0; c < k; ++c) memcpy(&stage[(size_t)c * cap], st[c]->buf, fill);
+    for (int c = 0; c < k; ++c) memcpy(&stage[(size_t)c * cap], pending(*st[c]), fill);
     const uint64_t n_values = (uint64_t)C.n_copies_padded << C.out_bits;
     for (long long c0 = 0; c0 < C.n_copies_padded; c0 += kCopiesPerChunk) {
         const long long nc = C.n_copies_padded - c0 < kCopiesPerChunk ? C.n_copies_padded - c0 : kCopiesPerChunk;
@@ -326,7 +343,7 @@ void put_outputs_group(State* const* st, const uint8_t* const* pix, int k, const
         for (int c = 0; c < k; ++c) memmove(&stage[(size_t)c * cap], &stage[(size_t)c * cap] + 64 * nblk, fill);
     }
     for (int c = 0; c < k; ++c) {
-        memcpy(st[c]->buf, &stage[(size_t)c * cap], fill);
+        memcpy(pending(*st[c]), &stage[(size_t)c * cap], fill);
         st[c]->nbuf = (uint32_t)fill;
         st[c]->total += 8 * n_values;
     }
@@ -382,8 +399,8 @@ bool launch_vole_round_batch(void* d_states, void* d_vole_states, int n, const v
 {
     fs::Label L;
     if (!make_device_label(label, &L, "vole round")) return false;
-    vole_round_kernel<<<(n + 127) / 128, 128, 0, s>>>(
-        static_cast<State*>(d_states), static_cast<VoleState*>(d_vole_states), n, static_cast<const fp2*>(d_claims),
+    vole_round_kernel<<<n, kFsThreads, 0, s>>>(
+        static_cast<State*>(d_states), static_cast<VoleState*>(d_vole_states), static_cast<const fp2*>(d_claims),
         static_cast<const fp2*>(d_u), static_cast<const fp2*>(d_v), count, L, static_cast<fp2*>(d_chal),
         static_cast<fp2*>(d_proof), d_rounds, k);
     return !cuda_failed(cudaGetLastError(), "vole round");
@@ -587,8 +604,8 @@ int tp_fs_put_fp2s_dev(void* d_states, int n, const void* d_vals, int k, void* s
         return -1;
     }
     if (k == 0) return 0;
-    put_fp2s_kernel<<<(n + 127) / 128, 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        static_cast<State*>(d_states), n, static_cast<const ulonglong2*>(d_vals), k);
+    put_fp2s_kernel<<<n, kFsThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+        static_cast<State*>(d_states), static_cast<const ulonglong2*>(d_vals), k);
     return tp::cuda_failed(cudaGetLastError(), "transcript put") ? -1 : 0;
 }
 
@@ -602,8 +619,8 @@ int tp_fs_rand_ext_dev(void* d_states, int n, const char* label, void* d_out, vo
         tp::set_error(tp::TP_ERR_ARG, "tp_fs_rand_ext_dev: bad arguments");
         return -1;
     }
-    rand_ext_kernel<<<(n + 127) / 128, 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        static_cast<State*>(d_states), n, L, static_cast<ulonglong2*>(d_out));
+    rand_ext_kernel<<<n, kFsThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+        static_cast<State*>(d_states), L, static_cast<ulonglong2*>(d_out));
     return tp::cuda_failed(cudaGetLastError(), "transcript rand_ext") ? -1 : 0;
 }
 
@@ -759,8 +776,8 @@ int tp_vole_round_slots_dev(void* d_fs_states, void* d_vole_states, int n_slots,
         tp::set_error(tp::TP_ERR_ARG, "tp_vole_round_slots_dev: bad arguments");
         return -1;
     }
-    vole_round_slots_kernel<<<(n_slots + 127) / 128, 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        static_cast<State*>(d_fs_states), static_cast<VoleState*>(d_vole_states), n_slots, static_cast<int2*>(d_meta),
+    vole_round_slots_kernel<<<n_slots, kFsThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+        static_cast<State*>(d_fs_states), static_cast<VoleState*>(d_vole_states), static_cast<int2*>(d_meta),
         static_cast<const tp::fp2*>(d_claims), static_cast<const tp::fp2*>(d_u), static_cast<const tp::fp2*>(d_v),
         count, layer, static_cast<tp::fp2*>(d_chal_cur), static_cast<tp::fp2*>(d_chal_hist),
         static_cast<tp::fp2*>(d_proof), max_rounds);
@@ -779,8 +796,8 @@ int tp_vole_round_dev(void* d_fs_states, void* d_vole_states, int n, const void*
         tp::set_error(tp::TP_ERR_ARG, "tp_vole_round_dev: bad arguments");
         return -1;
     }
-    vole_round_kernel<<<(n + 127) / 128, 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        static_cast<State*>(d_fs_states), static_cast<VoleState*>(d_vole_states), n,
+    vole_round_kernel<<<n, kFsThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+        static_cast<State*>(d_fs_states), static_cast<VoleState*>(d_vole_states),
         static_cast<const tp::fp2*>(d_claims), static_cast<const tp::fp2*>(d_u), static_cast<const tp::fp2*>(d_v),
         count, L, static_cast<tp::fp2*>(d_chal), static_cast<tp::fp2*>(d_proof), nullptr, 0);
     return tp::cuda_failed(cudaGetLastError(), "vole round") ? -1 : 0;

@@ -96,22 +96,26 @@ TP_HD bool round(fs::State& s, State& w, const fp2* c, int n_coef, const fp2* u,
         *r_out = f2zero();
         return false;
     }
-    fp2 tag[4];
-    for (int k = 0; k < n_coef; ++k) {
-        tag[k] = v[w.idx];
-        const fp2 dm = f2sub(c[k], u[w.idx]);
-        ++w.idx;
-        fs::put_fp2(s, dm.re, dm.im);
-        if (proof) proof[k] = dm;
+    fp2 tag[4], dm[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {     // every load before the first hash
+        if (k >= n_coef) break;
+        tag[k] = v[w.idx + k];
+        dm[k] = f2sub(c[k], u[w.idx + k]);
         w.v_elem[k] = f2add(w.v_elem[k], tag[k]);
         w.out_elem[k] = f2add(w.out_elem[k], c[k]);
+    }
+    w.idx += (unsigned long long)n_coef;
+    for (int k = 0; k < n_coef; ++k) {
+        fs::put_fp2(s, dm[k].re, dm[k].im);
+        if (proof && fs::lead()) proof[k] = dm[k];
     }
     fp2 now = tag[0];
     for (int k = 0; k < n_coef; ++k) now = f2add(now, tag[k]);
     const fp2 e = fs::rand_fp2(s, fs::label_lit("eq"));
     const fp2 vz = w.has_prev ? f2mul(f2sub(w.prev, now), e) : f2mul(now, e);
     fs::put_fp2(s, vz.re, vz.im);
-    if (proof) proof[n_coef] = vz;
+    if (proof && fs::lead()) proof[n_coef] = vz;
     const fp2 r = fs::rand_fp2(s, label);
     fp2 p = tag[n_coef - 1];
     for (int k = n_coef - 2; k >= 0; --k) p = f2add(f2mul(p, r), tag[k]);
