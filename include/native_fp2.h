@@ -216,7 +216,8 @@ int tp_batch_graph_replays(void* batch);
  * (2 to 16 CTAs per SM) and the fastest is kept for this device; launches of a
  * bucket not yet measured use 4 per SM. tp_batch_tune_table lists the measured
  * entries (returns their count), tp_batch_tune_set installs one (e.g. from a
- * saved table). Kinds: 0 table claim, 1 table fold + claim, 2 byte claim, 3 byte
+ * saved table). Kinds: 0 table claim, 1 table fold + claim, 2 byte claim (for layers
+ * of few product groups the launch that sums the bytes per copy), 3 byte
  * fold + claim; bucket = floor(log2 of the launch's pairs x rows). */
 int tp_batch_autotune(int on);
 int tp_batch_tune_table(int* kind, int* bucket, int* ctas_per_sm, int max);

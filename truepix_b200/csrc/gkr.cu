@@ -521,28 +521,45 @@ bool upload_gate_form(const GateForm& g, DevGateForm& d, cudaStream_t s)
     d.K0 = g.K0;
     d.n_wires = (int)g.L.size();
     d.n_terms = (int)g.tc.size();
-    d.L = (fp2*)dev_alloc(sizeof(fp2) * g.L.size(), s);
-    d.ab = (int2*)dev_alloc(sizeof(int2) * std::max<size_t>(1, g.tc.size()), s);
-    d.c = (fp2*)dev_alloc(sizeof(fp2) * std::max<size_t>(1, g.tc.size()), s);
-    if (!d.L || !d.ab || !d.c) return false;
-    if (!upload_async(d.L, g.L.data(), sizeof(fp2) * g.L.size(), s)) return false;
-    if (d.n_terms) {
-        std::vector<int2> ab((size_t)d.n_terms);
-        for (int i = 0; i < d.n_terms; ++i) ab[i] = make_int2(g.ta[i], g.tb[i]);
-        if (!upload_async(d.ab, ab.data(), sizeof(int2) * ab.size(), s)) return false;
-        if (!upload_async(d.c, g.tc.data(), sizeof(fp2) * g.tc.size(), s)) return false;
+    // one upload: L, then the terms' coefficients and wires, then the groups
+    std::vector<int> gptr, gb;
+    for (int i = 0; i < d.n_terms; ++i)
+        if (i == 0 || g.tb[(size_t)i] != g.tb[(size_t)i - 1]) {
+            gptr.push_back(i);
+            gb.push_back(g.tb[(size_t)i]);
+        }
+    d.groups = (int)gb.size();
+    gptr.push_back(d.n_terms);
+    const size_t oL = 0, oc = oL + sizeof(fp2) * g.L.size(), oab = oc + sizeof(fp2) * g.tc.size(),
+                 op = oab + sizeof(int2) * g.tc.size(), ob = op + sizeof(int) * gptr.size(),
+                 bytes = ob + sizeof(int) * gb.size();
+    if (bytes > d.cap) {
+        dev_free(d.mem, s);
+        d.cap = 0;
+        d.mem = dev_alloc(bytes, s);
+        if (!d.mem) return false;
+        d.cap = bytes;
     }
-    return true;
+    unsigned char* m = static_cast<unsigned char*>(d.mem);
+    d.L = reinterpret_cast<fp2*>(m + oL);
+    d.c = reinterpret_cast<fp2*>(m + oc);
+    d.ab = reinterpret_cast<int2*>(m + oab);
+    d.gptr = reinterpret_cast<int*>(m + op);
+    d.gb = reinterpret_cast<int*>(m + ob);
+    std::vector<unsigned char> h(bytes);
+    memcpy(h.data() + oL, g.L.data(), sizeof(fp2) * g.L.size());
+    if (d.n_terms) memcpy(h.data() + oc, g.tc.data(), sizeof(fp2) * g.tc.size());
+    int2* ab = reinterpret_cast<int2*>(h.data() + oab);
+    for (int i = 0; i < d.n_terms; ++i) ab[i] = make_int2(g.ta[(size_t)i], g.tb[(size_t)i]);
+    memcpy(h.data() + op, gptr.data(), sizeof(int) * gptr.size());
+    if (d.groups) memcpy(h.data() + ob, gb.data(), sizeof(int) * gb.size());
+    return upload_async(d.mem, h.data(), bytes, s);
 }
 
 void free_gate_form(DevGateForm& d, cudaStream_t s)
 {
-    dev_free(d.L, s);
-    dev_free(d.ab, s);
-    dev_free(d.c, s);
-    d.L = nullptr;
-    d.ab = nullptr;
-    d.c = nullptr;
+    dev_free(d.mem, s);
+    d = DevGateForm();
 }
 
 bool workspace_init(ClaimWorkspace& w, size_t blocks, cudaStream_t s)

@@ -25,14 +25,19 @@ struct GateForm {
 bool build_gate_form(int n_gates, const int* type, const int* in0, const int* in1,
                      const u64* z_re, const u64* z_im, int n_wires, GateForm& out);
 
-// Device copy of a GateForm.
+// Device copy of a GateForm, one block of memory kept for the next form.
 struct DevGateForm {
     fp2 K0;
     fp2* L = nullptr;
     int2* ab = nullptr;
     fp2* c = nullptr;
+    int* gptr = nullptr;   // [groups + 1] terms that share their wire b
+    int* gb = nullptr;     // [groups] that wire
     int n_terms = 0;
     int n_wires = 0;
+    int groups = 0;
+    void* mem = nullptr;
+    size_t cap = 0;
 };
 bool upload_gate_form(const GateForm& g, DevGateForm& d, cudaStream_t s);
 void free_gate_form(DevGateForm& d, cudaStream_t s);
@@ -69,7 +74,17 @@ struct Frame {
     fp2* fin = nullptr;    // [n_wires + 1]: wires, then beta
     u64* out8 = nullptr;   // default claim slot
     bool configured = false;
+    bool loaded = false;   // its table, bytes or vectors are in place
     size_t cap0 = 0, cap1 = 0, capb = 0, capfin = 0;  // element capacities kept across resets
+    // rounds on vectors (gkr_linear.cu): the source stays as it is (bytes copied
+    // aside by the forms launch, or the table in buf[0]) until the finish
+    bool linear = false, forms_done = false;
+    int folds = 0;                            // folds applied to the vectors, recorded in rs
+    fp2* vec[2] = {nullptr, nullptr};         // 1 + 2 groups vectors of n / n/2 copies
+    unsigned char* bytes = nullptr;
+    fp2* rs = nullptr;                        // [64] challenges applied, [64] given ones
+    fp2* fpart = nullptr;
+    size_t capv = 0, cap_bytes = 0, cap_part = 0;
 };
 
 // A batch of frames advanced together: one launch per round for all frames
@@ -112,6 +127,9 @@ bool batch_load_pixels(Batch* B, int i, const PixSrc& px, const fp2* d_beta);
 // claims of all unfinished frames; d_claims[i] (8 u64, device) or the frame's slot
 bool batch_claim(Batch* B, u64* const* d_claims);
 bool batch_fold(Batch* B, int i, fp2 r);
+// a one-frame batch: n_rounds claims (d_claims + 8 k u64, or null: the frame's slot),
+// each followed by the fold by challenges[2 k], [2 k + 1]
+bool batch_given_rounds(Batch* B, int n_rounds, const u64* challenges, u64* d_claims);
 // the same with the challenge in device memory (read in stream order when the
 // next claim or finish is queued); needs a claim or finish before the next fold
 bool batch_fold_dev(Batch* B, int i, const fp2* d_r);
@@ -121,8 +139,8 @@ bool batch_finish(Batch* B, fp2* const* d_wires, fp2* const* d_beta);
 // Every early round of a batch on device transcripts, as one CUDA graph: per
 // round the claims (d_claims + 8 B k u64), the VOLE-committed round
 // (tp_vole_round_dev: challenge d_chal + B k, proof d_proof + 5 B k, labels
-// "sc-<layer>-<k>"), the fold by the drawn challenge; then the finish. All
-// frames must have the same number of rounds. The jobs of all rounds are planned
+// "sc-<layer>-<k>"), the fold by the drawn challenge; then the finish. Frames of
+// different sizes leave after their own last round. The jobs of all rounds are planned
 // on the host and uploaded in one copy; the graph is captured on the first call
 // of a shape and replayed while the shape and the buffers stay the same.
 bool batch_vole_rounds_graph(Batch* B, u64* d_claims, void* d_states, void* d_vole_states, const fp2* d_u,

@@ -1,0 +1,781 @@
+// Early rounds whose per-copy sums stay in vectors.
+//
+// A round's claim at copy c needs, besides beta, only
+//   s(c) = sum_w L[w] V[w][c]                     (the layer's linear part)
+//   M_g(c) = sum_{terms of group g} coef V[a][c]  and  V[b_g][c]
+// per group g of product terms that share their wire b. Folding the copies by a
+// challenge is linear, so these 1 + 2 G vectors fold by themselves, and the table
+// of all wires is not needed until the end, where the wire values are sums over
+// the copies weighted with eq(challenges, c). For the layers of TruePix's circuits
+// (G = 0, or 1 to 3 for mask and crop) a round then moves 32 B per copy and vector
+// instead of 32 B per copy and wire: over 64 1080p frames the rounds after the
+// first took 2.95 ms (12.9 GB of folded tables written and read) and now 0.1 ms.
+// The sums are exact field sums, so every value is the same.
+//
+//   forms     the vectors from the source. From bytes: an integer matrix product
+//             (copies x wires bytes) x (wires x 16 byte-planes of a form's
+//             coefficients, eight for each limb) on the tensor cores, u8 x u8
+//             accumulated in 32 bits (512 * 255 * 255 < 2^31), recombined mod p;
+//             bound by reading the bytes. The bytes are also copied aside (rows of
+//             a multiple of 32 bytes), so that the caller's buffer is free after
+//             the first claim or fold as before. From a table: one warp a slice of
+//             rows, 32 copies wide; bound by reading the table.
+//   rounds    one thread a pair of copies, one launch a round (vec_round_kernel), or
+//             all rounds of a frame in one CTA once few pairs are left
+//             (vec_rounds_kernel), with the challenges given or drawn by the
+//             VOLE-committed round on the frame's transcript.
+//   finish    wires from bytes: (16 byte-planes of eq) x (copies x wires) the same
+//             way; from a table: a warp per wire.
+#include "gkr.h"
+#include "gkr_internal.cuh"
+#include "runtime.h"
+#include "vole.cuh"
+
+#include <algorithm>
+
+namespace tp {
+
+namespace {
+
+constexpr int kTileRows = 64;        // copies staged at a time by the byte forms
+constexpr int kFormThreads = 128;    // a warp per 16 of them
+constexpr int kVecThreads = 256;
+constexpr int kRoundsThreads = 512;
+constexpr int kFinCopies = 512;      // copies per CTA of the finish from bytes
+
+__device__ __forceinline__ void read_job(const Job* jobs, Job& sj)
+{
+    const int* src = reinterpret_cast<const int*>(jobs + blockIdx.y);
+    int* dst = reinterpret_cast<int*>(&sj);
+    for (int i = threadIdx.x; i < (int)(sizeof(Job) / 4); i += blockDim.x) dst[i] = __ldg(src + i);
+    __syncthreads();
+}
+
+// D += A B for a 16 x 32 tile of A and a 32 x 8 tile of B, bytes: lane (g = lane / 4,
+// j = lane % 4) holds A[g][4j..], A[g + 8][4j..], A[g][16 + 4j..], A[g + 8][16 + 4j..],
+// B[4j..][g], B[16 + 4j..][g] and D[g][2j], D[g][2j + 1], D[g + 8][2j], D[g + 8][2j + 1]
+__device__ __forceinline__ void mma_u8(int (&d)[4], u32 a0, u32 a1, u32 a2, u32 a3, u32 b0, u32 b1)
+{
+    asm volatile(
+        "mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+        "{%0, %1, %2, %3};"
+        : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// 4 x 4 bytes transposed: byte i of out[m] = byte m of in[i]
+__device__ __forceinline__ void transpose4(const u32 (&in)[4], u32 (&out)[4])
+{
+    const u32 a = __byte_perm(in[0], in[1], 0x5140), b = __byte_perm(in[2], in[3], 0x5140);   // bytes 0, 1
+    const u32 c = __byte_perm(in[0], in[1], 0x7362), d = __byte_perm(in[2], in[3], 0x7362);   // bytes 2, 3
+    out[0] = __byte_perm(a, b, 0x5410);
+    out[1] = __byte_perm(a, b, 0x7632);
+    out[2] = __byte_perm(c, d, 0x5410);
+    out[3] = __byte_perm(c, d, 0x7632);
+}
+
+// v 2^sh mod p (nearly) for 0 <= v < 2^36, 0 <= sh < 61
+__device__ __forceinline__ u64 shift_mod(u64 v, int sh)
+{
+    return ((v << sh) & P61) + (sh ? v >> (61 - sh) : 0);
+}
+
+__device__ __forceinline__ void async16(void* dst, const void* src, bool in)
+{
+    const u32 d = (u32)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+
+// ---- forms from bytes ---------------------------------------------------------
+// Dynamic shared memory: two tiles of 64 rows, then the 16 planes of one form, all
+// with rows of kp + 16 bytes (kp = J.stride, the copy size rounded up to 32), so that
+// the fragments' words of eight rows fall in distinct banks.
+
+// tile t's rows into buf (asynchronously where whole 16-byte vectors can be read)
+__device__ void stage_tile(const Job& J, int t, unsigned char* buf, int pitch)
+{
+    const int c0 = t * kTileRows;
+    if (J.vec) {
+        const int per = J.cs >> 4;
+        for (int i = threadIdx.x; i < kTileRows * per; i += kFormThreads) {
+            const int r = i / per, q = i - r * per;
+            const bool in = c0 + r < J.n_real;
+            async16(buf + r * pitch + 16 * q, J.pix + (size_t)(in ? c0 + r : 0) * J.cs + 16 * q, in);
+        }
+    } else {
+        const int words = J.stride >> 2;
+        for (int i = threadIdx.x; i < kTileRows * words; i += kFormThreads) {
+            const int r = i / words, q = 4 * (i - r * words);
+            u32 v = 0;
+            if (c0 + r < J.n_real) {
+                const unsigned char* p = J.pix + (size_t)(c0 + r) * J.cs;
+#pragma unroll
+                for (int b = 0; b < 4; ++b)
+                    if (q + b < J.cs) v |= (u32)__ldg(p + q + b) << (8 * b);
+            }
+            *reinterpret_cast<u32*>(buf + r * pitch + q) = v;
+        }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+__global__ void __launch_bounds__(kFormThreads) forms_bytes_kernel(const Job* __restrict__ jobs)
+{
+    __shared__ __align__(16) Job J;
+    __shared__ fp2 s_const;    // the form's term of the constant wire
+    extern __shared__ __align__(16) unsigned char dsm[];
+    read_job(jobs, J);
+    const int tiles = (J.n_in + kTileRows - 1) / kTileRows;
+    const int t0 = blockIdx.x * J.wpg, t1 = min(tiles, t0 + J.wpg);
+    if (t0 >= t1) return;
+    const int kp = J.stride, pitch = kp + 16, cs = J.cs;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, j = lane & 3;
+    unsigned char* tile[2] = {dsm, dsm + kTileRows * pitch};
+    unsigned char* planes = dsm + 2 * kTileRows * pitch;
+    if (J.vec) {   // the columns behind the copied vectors stay zero
+        const int pad = (kp - cs) >> 2;
+        for (int i = tid; i < 2 * kTileRows * pad; i += kFormThreads)
+            *reinterpret_cast<u32*>(dsm + (i / pad) * pitch + cs + 4 * (i % pad)) = 0u;
+    }
+    for (int form = 0; form <= J.G; ++form) {
+        stage_tile(J, t0, tile[0], pitch);
+        // the form's planes: byte l of a coefficient's limbs in plane l (re), 8 + l (im)
+        if (tid == 0) s_const = form == 0 && J.const_idx >= 0 ? J.Lc : f2zero();
+        if (form == 0) {
+            for (int q = tid; 4 * q < kp; q += kFormThreads) {
+                u32 re[2][4], im[2][4], o[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const fp2 l = 4 * q + k < cs ? ld2(J.L + 4 * q + k) : f2zero();
+                    re[0][k] = (u32)l.re;
+                    re[1][k] = (u32)(l.re >> 32);
+                    im[0][k] = (u32)l.im;
+                    im[1][k] = (u32)(l.im >> 32);
+                }
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    transpose4(re[h], o);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) *reinterpret_cast<u32*>(planes + (4 * h + k) * pitch + 4 * q) = o[k];
+                    transpose4(im[h], o);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        *reinterpret_cast<u32*>(planes + (8 + 4 * h + k) * pitch + 4 * q) = o[k];
+                }
+            }
+        } else {
+            for (int i = tid; i < 16 * (kp >> 2); i += kFormThreads)
+                *reinterpret_cast<u32*>(planes + (i / (kp >> 2)) * pitch + 4 * (i % (kp >> 2))) = 0u;
+            __syncthreads();
+            // the group's terms: one per wire a
+            for (int e = J.gptr[form - 1] + tid; e < J.gptr[form]; e += kFormThreads) {
+                const int a = J.ab[e].x;
+                const fp2 c = ld2(J.cf + e);
+                if (a < cs) {
+#pragma unroll
+                    for (int l = 0; l < 8; ++l) {
+                        planes[l * pitch + a] = (unsigned char)(c.re >> (8 * l));
+                        planes[(8 + l) * pitch + a] = (unsigned char)(c.im >> (8 * l));
+                    }
+                } else if (a == J.const_idx) {
+                    s_const = l2canon(mk(lmul(c.re, J.const_val), lmul(c.im, J.const_val)));
+                }
+            }
+        }
+        fp2* out = const_cast<fp2*>(J.A) + (size_t)(form == 0 ? 0 : 2 * form - 1) * J.n_in;
+        for (int t = t0; t < t1; ++t) {
+            const unsigned char* buf = tile[(t - t0) & 1];
+            if (t + 1 < t1) {
+                stage_tile(J, t + 1, tile[(t + 1 - t0) & 1], pitch);
+                asm volatile("cp.async.wait_group 1;" ::: "memory");
+            } else {
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
+            }
+            __syncthreads();
+            if (form == 0) {   // the copy of the bytes that the finish reads
+                for (int i = tid; i < kTileRows * (kp >> 4); i += kFormThreads) {
+                    const int r = i / (kp >> 4), q = i - r * (kp >> 4);
+                    if (t * kTileRows + r < J.n_real)
+                        *reinterpret_cast<uint4*>(J.bytes + (size_t)(t * kTileRows + r) * kp + 16 * q) =
+                            *reinterpret_cast<const uint4*>(buf + r * pitch + 16 * q);
+                }
+            } else if (tid < kTileRows) {   // the group's wire b
+                const int c = t * kTileRows + tid, b = J.gb[form - 1];
+                if (c < J.n_in) {
+                    const u64 v = c >= J.n_real ? 0 : b < cs ? buf[tid * pitch + b] : b == J.const_idx ? J.const_val : 0;
+                    st2(out + J.n_in + c, mk(v, 0));
+                }
+            }
+            int d[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};   // limbs of re, of im
+            const unsigned char* ar = buf + (16 * warp + g) * pitch + 4 * j;
+            const unsigned char* br = planes + g * pitch + 4 * j;
+            auto word = [](const unsigned char* p) { return *reinterpret_cast<const u32*>(p); };
+            for (int k = 0; k < kp; k += 32) {
+                const u32 a0 = word(ar + k), a1 = word(ar + 8 * pitch + k), a2 = word(ar + k + 16),
+                          a3 = word(ar + 8 * pitch + k + 16);
+                mma_u8(d[0], a0, a1, a2, a3, word(br + k), word(br + k + 16));
+                mma_u8(d[1], a0, a1, a2, a3, word(br + 8 * pitch + k), word(br + 8 * pitch + k + 16));
+            }
+            // limbs 2j, 2j + 1 of rows g (d[.][0, 1]) and g + 8 (d[.][2, 3])
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                u64 re = shift_mod((u64)(u32)d[0][2 * h] + ((u64)(u32)d[0][2 * h + 1] << 8), 16 * j);
+                u64 im = shift_mod((u64)(u32)d[1][2 * h] + ((u64)(u32)d[1][2 * h + 1] << 8), 16 * j);
+#pragma unroll
+                for (int o = 1; o < 4; o <<= 1) {
+                    re += __shfl_xor_sync(0xffffffffu, re, o);
+                    im += __shfl_xor_sync(0xffffffffu, im, o);
+                }
+                const int c = t * kTileRows + 16 * warp + g + 8 * h;
+                if (j == h && c < J.n_in) {
+                    fp2 v = mk(fold61(re), fold61(im));
+                    if (c < J.n_real) v = l2add(v, s_const);
+                    st2(out + c, v);
+                }
+            }
+            __syncthreads();
+        }
+    }
+}
+
+// ---- forms from a table ---------------------------------------------------------
+// CTA = 32 copies; its warps take slices of the rows and of each group's terms
+__global__ void __launch_bounds__(kVecThreads) forms_table_kernel(const Job* __restrict__ jobs)
+{
+    __shared__ __align__(16) Job J;
+    __shared__ fp2 red[kVecThreads / 32][32];
+    read_job(jobs, J);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int kW = kVecThreads / 32;
+    if ((int)blockIdx.x * 32 >= J.n_in) return;
+    const int c = blockIdx.x * 32 + lane;
+    const bool live = c < J.n_in;
+    const fp2* src = J.src + (live ? c : 0);
+    fp2* out = const_cast<fp2*>(J.A);
+    auto at = [&](int w) {
+        const fp2 v = w < J.W_rows ? ld2(src + (size_t)w * J.n_in) : f2zero();
+        return mk(fold61(v.re), fold61(v.im));
+    };
+    for (int form = 0; form <= J.G; ++form) {
+        const int n = form == 0 ? J.W_rows : J.gptr[form] - J.gptr[form - 1];
+        const int base = form == 0 ? 0 : J.gptr[form - 1];
+        const int per = (n + kW - 1) / kW;
+        const int e0 = min(n, warp * per), e1 = min(n, e0 + per);
+        u64 re = 0, im = 0;
+        int e = e0;
+        for (; e + 4 <= e1; e += 4) {   // four rows' loads before their products
+            fp2 x[4], l[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                x[k] = at(form == 0 ? e + k : J.ab[base + e + k].x);
+                l[k] = ld2((form == 0 ? J.L : J.cf + base) + e + k);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const fp2 v = l2mul(l[k], x[k]);
+                re = fold61(re + v.re);
+                im = fold61(im + v.im);
+            }
+        }
+        for (; e < e1; ++e) {
+            const fp2 v = l2mul(ld2((form == 0 ? J.L : J.cf + base) + e), at(form == 0 ? e : J.ab[base + e].x));
+            re = fold61(re + v.re);
+            im = fold61(im + v.im);
+        }
+        red[warp][lane] = mk(re, im);
+        __syncthreads();
+        fp2* o = out + (size_t)(form == 0 ? 0 : 2 * form - 1) * J.n_in;
+        if (warp == 0 && live) {
+            fp2 s = red[0][lane];
+            for (int k = 1; k < kW; ++k) s = l2add(s, red[k][lane]);
+            st2(o + c, s);
+        }
+        if (form > 0 && warp == 1 && live) st2(o + J.n_in + c, at(J.gb[form - 1]));
+        __syncthreads();
+    }
+}
+
+// ---- rounds ---------------------------------------------------------------------
+
+// loads of vectors: read-only in a launch of one round, written by the same CTA
+// between its rounds in the launch of all
+template <bool kSame>
+__device__ __forceinline__ fp2 ldv(const fp2* p)
+{
+    if (!kSame) return ld2(p);
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
+    return mk(v.x, v.y);
+}
+
+__device__ __forceinline__ void four_points(fp2 v0, fp2 v1, fp2 (&o)[4])
+{
+    o[0] = v0;
+    o[1] = v1;
+    o[2] = l2at_m1(v0, v1);
+    o[3] = l2at_2(v0, v1);
+}
+
+// entries 2p, 2p + 1 of a vector of n_in entries (fold: of its fold by r, stored)
+template <bool kSame>
+__device__ __forceinline__ void pair_of(const fp2* in, fp2* out, int p, bool fold, fp2 r, fp2& x0, fp2& x1)
+{
+    if (!fold) {
+        x0 = ldv<kSame>(in + 2 * (size_t)p);
+        x1 = ldv<kSame>(in + 2 * (size_t)p + 1);
+        return;
+    }
+    const fp2* q = in + 4 * (size_t)p;
+    const fp2 a0 = ldv<kSame>(q), a1 = ldv<kSame>(q + 1), a2 = ldv<kSame>(q + 2), a3 = ldv<kSame>(q + 3);
+    x0 = l2fold(a0, a1, r);
+    x1 = l2fold(a2, a3, r);
+    st2(out + 2 * (size_t)p, x0);
+    st2(out + 2 * (size_t)p + 1, x1);
+}
+
+// the claim's four points at pair p of the (folded) vectors, nearly canonical
+template <bool kSame>
+__device__ __forceinline__ void pair_claim(const Job& J, const fp2* in, fp2* out, const fp2* beta, fp2* beta_out,
+                                           int n_in, int p, bool fold, fp2 r, fp2 (&acc)[4])
+{
+    const size_t n = (size_t)n_in, no = n >> 1;
+    fp2 x0, x1, V[4], b4[4];
+    pair_of<kSame>(in, out, p, fold, r, x0, x1);
+    four_points(x0, x1, V);
+#pragma unroll
+    for (int t = 0; t < 4; ++t) V[t] = l2add(V[t], J.K0);
+    for (int g = 0; g < J.G; ++g) {
+        fp2 m[4], y[4];
+        pair_of<kSame>(in + (2 * g + 1) * n, out + (2 * g + 1) * no, p, fold, r, x0, x1);
+        four_points(x0, x1, m);
+        pair_of<kSame>(in + (2 * g + 2) * n, out + (2 * g + 2) * no, p, fold, r, x0, x1);
+        four_points(x0, x1, y);
+#pragma unroll
+        for (int t = 0; t < 4; ++t) V[t] = l2add(V[t], l2mul(m[t], y[t]));
+    }
+    pair_of<kSame>(beta, beta_out, p, fold, r, x0, x1);
+    four_points(x0, x1, b4);
+#pragma unroll
+    for (int t = 0; t < 4; ++t) acc[t] = l2add(acc[t], l2mul(b4[t], V[t]));
+}
+
+// the CTA's sum of acc (canonical), valid on the threads of warp 0
+template <int kWarps>
+__device__ __forceinline__ void cta_sum(fp2 (&acc)[4], fp2 (*ws)[4])
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+    for (int t = 0; t < 4; ++t) acc[t] = warp_sum(l2canon(acc[t]));
+    if (lane == 0)
+#pragma unroll
+        for (int t = 0; t < 4; ++t) ws[warp][t] = acc[t];
+    __syncthreads();
+    if (warp == 0)
+#pragma unroll
+        for (int t = 0; t < 4; ++t) acc[t] = warp_sum(lane < kWarps ? ws[lane][t] : f2zero());
+}
+
+// one round of every job: a thread per pair; the job's last CTA (ticket) adds the
+// CTAs' sums. A fold's challenge is recorded for the finish.
+template <bool kFold>
+__global__ void __launch_bounds__(kVecThreads) vec_round_kernel(const Job* __restrict__ jobs)
+{
+    __shared__ __align__(16) Job J;
+    __shared__ fp2 ws[kVecThreads / 32][4];
+    __shared__ bool s_last;
+    read_job(jobs, J);
+    if ((int)blockIdx.x >= J.tiles) return;
+    const int p = blockIdx.x * kVecThreads + threadIdx.x;
+    fp2 acc[4] = {f2zero(), f2zero(), f2zero(), f2zero()};
+    if (p < J.n_pairs) pair_claim<false>(J, J.A, J.Aout, J.beta, J.beta_out, J.n_in, p, kFold, J.r, acc);
+    cta_sum<kVecThreads / 32>(acc, ws);
+    const int tid = threadIdx.x;
+    if (kFold && blockIdx.x == 0 && tid == 0) st2(J.rs + J.nf, J.r);
+    if (J.tiles > 1) {
+        if (tid == 0) {
+#pragma unroll
+            for (int t = 0; t < 4; ++t) stcg2(J.partials + (size_t)blockIdx.x * 4 + t, acc[t]);
+            __threadfence();
+            s_last = atomicAdd(J.ticket, 1u) == (unsigned)(J.tiles - 1);
+        }
+        __syncthreads();
+        if (!s_last) return;
+        __threadfence();
+#pragma unroll
+        for (int t = 0; t < 4; ++t) acc[t] = f2zero();
+        for (int i = tid; i < J.tiles; i += kVecThreads)
+#pragma unroll
+            for (int t = 0; t < 4; ++t) acc[t] = f2add(acc[t], ldcg2(J.partials + (size_t)i * 4 + t));
+        cta_sum<kVecThreads / 32>(acc, ws);
+        if (tid == 0) *J.ticket = 0u;
+    }
+    if (tid == 0)
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            J.out8[2 * t] = acc[t].re;
+            J.out8[2 * t + 1] = acc[t].im;
+        }
+}
+
+// All rounds of a frame that are left, one CTA per frame: job J with n_in copies
+// (pending fold by J.r when J.has_r), J.n_rounds claims from round k0 on. The last
+// challenge's fold is left to the finish. The challenges: J.given[q], or drawn by
+// the VOLE-committed round (a.st set). Claims at J.out8 + q a.claim_stride.
+struct RoundsArgs {
+    fs::State* st;
+    vole::State* vs;
+    const fp2* u;
+    const fp2* v;
+    fp2* chal;       // [round][frame]
+    fp2* proof;      // [round][frame][5], optional
+    long long count;
+    long long claim_stride;   // u64s between a frame's claims of successive rounds
+    int n_frames, layer, k0;
+};
+
+template <bool kVole>
+__global__ void __launch_bounds__(kRoundsThreads, 1) vec_rounds_kernel(const Job* __restrict__ jobs, const RoundsArgs a)
+{
+    __shared__ __align__(16) Job J;
+    __shared__ fp2 ws[kRoundsThreads / 32][4];
+    __shared__ fp2 s_r;
+    read_job(jobs, J);
+    const int tid = threadIdx.x;
+    const fp2* in = J.A;
+    const fp2* beta = J.beta;
+    fp2 *out = J.Aout, *beta_out = J.beta_out;
+    int n = J.n_in, nf = J.nf;
+    bool fold = J.has_r != 0;
+    fp2 r = J.r;
+    for (int q = 0; q < J.n_rounds; ++q) {
+        fp2 acc[4] = {f2zero(), f2zero(), f2zero(), f2zero()};
+        const int pairs = fold ? n >> 2 : n >> 1;
+        for (int p = tid; p < pairs; p += kRoundsThreads)
+            pair_claim<true>(J, in, out, beta, beta_out, n, p, fold, r, acc);
+        if (fold) {
+            if (tid == 0) st2(J.rs + nf, r);
+            ++nf;
+            n >>= 1;
+            const fp2 *ti = in, *tb = beta;
+            in = out;
+            beta = beta_out;
+            out = const_cast<fp2*>(ti);
+            beta_out = const_cast<fp2*>(tb);
+        }
+        cta_sum<kRoundsThreads / 32>(acc, ws);
+        if (tid < 32) {
+            u64* o = J.out8 + q * a.claim_stride;
+            if (tid == 0)
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    o[2 * t] = acc[t].re;
+                    o[2 * t + 1] = acc[t].im;
+                }
+            fp2 c;
+            if (kVole) {
+                const int i = J.frame, k = a.k0 + q;
+                const size_t at = (size_t)a.n_frames * k + i;
+                fp2 coef[4];
+                fs::State s = a.st[i];
+                vole::State w = a.vs[i];
+                vole::interpolate_cubic(acc[0], acc[1], acc[2], acc[3], coef);
+                vole::round(s, w, coef, 4, a.u + i * a.count, a.v + i * a.count, a.count, vole::sc_label(a.layer, k),
+                            a.proof ? a.proof + 5 * at : nullptr, &c);
+                __syncwarp();
+                if (tid == 0) {
+                    a.st[i] = s;
+                    a.vs[i] = w;
+                    a.chal[at] = c;
+                }
+                __syncwarp();
+            } else {
+                c = ld2(J.given + q);
+            }
+            if (tid == 0) s_r = c;
+        }
+        __syncthreads();
+        r = s_r;
+        fold = true;
+    }
+}
+
+// ---- finish ---------------------------------------------------------------------
+
+// eq(challenges, c) for the copies c of a chunk: the products over bits 0..3 and 4..8
+// of c and over the chunk's higher bits, in shared memory (49 threads or more)
+struct EqParts {
+    fp2 r[64];
+    fp2 lo[16], mid[32], hi;
+};
+__device__ void eq_parts(const Job& J, int chunk, EqParts& e)
+{
+    const int tid = threadIdx.x, kf = J.nf + (J.has_r != 0);
+    for (int k = tid; k < kf; k += blockDim.x) e.r[k] = k < J.nf ? ldcg2(J.rs + k) : J.r;
+    __syncthreads();
+    const fp2 one = mk(1, 0);
+    auto prod = [&](int idx, int first, int last) {
+        fp2 v = one;
+        for (int b = first; b < last && b < kf; ++b)
+            v = l2mul(v, ((idx >> (b - first)) & 1) ? e.r[b] : l2sub(one, e.r[b]));
+        return v;
+    };
+    if (tid < 16) e.lo[tid] = prod(tid, 0, 4);
+    else if (tid < 48) e.mid[tid - 16] = prod(tid - 16, 4, 9);
+    else if (tid == 48) e.hi = prod(chunk, 9, kf);
+    __syncthreads();
+}
+__device__ __forceinline__ fp2 eq_of(const EqParts& e, int c) { return l2mul(l2mul(e.lo[c & 15], e.mid[c >> 4]), e.hi); }
+
+// beta's value: entry 0 after the pending fold
+__device__ __forceinline__ void finish_beta(const Job& J)
+{
+    const fp2 b = J.has_r ? l2fold(ld2(J.beta), ld2(J.beta + 1), J.r) : ld2(J.beta);
+    st2(J.fin_beta, l2canon(b));
+}
+
+// wires from the copied bytes. CTA = 512 copies, a warp per 32 wires: the planes of
+// eq are the mma's rows, the wires its columns (word loads of four copies' four
+// wires, transposed in registers); partial sums per chunk, the job's last CTA adds
+// them up.
+__global__ void __launch_bounds__(512) finish_bytes_kernel(const Job* __restrict__ jobs)
+{
+    constexpr int kPitch = kFinCopies + 16;
+    __shared__ __align__(16) Job J;
+    __shared__ EqParts e;
+    __shared__ __align__(16) unsigned char E[16 * kPitch];
+    __shared__ fp2 ws[16];
+    __shared__ bool s_last;
+    read_job(jobs, J);
+    const int chunk = blockIdx.x;
+    if (chunk >= J.chunks) return;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, j = lane & 3;
+    const int kf = J.nf + (J.has_r != 0);
+    const int c0 = chunk * kFinCopies;
+    const int lim = min(J.n_real, 1 << kf) - c0;   // copies of this chunk that count
+    eq_parts(J, chunk, e);
+    fp2 sum = f2zero();
+    for (int c = tid; c < kFinCopies; c += blockDim.x) {
+        fp2 v = f2zero();
+        if (c < lim) {
+            v = l2canon(eq_of(e, c));
+            sum = l2add(sum, v);
+        }
+#pragma unroll
+        for (int l = 0; l < 8; ++l) {
+            E[l * kPitch + c] = (unsigned char)(v.re >> (8 * l));
+            E[(8 + l) * kPitch + c] = (unsigned char)(v.im >> (8 * l));
+        }
+    }
+    sum = warp_sum(l2canon(sum));
+    if (lane == 0) ws[warp] = sum;
+    __syncthreads();
+    const int Wp = J.W_rows;
+    fp2* part = J.fpart + (size_t)chunk * Wp;
+    const int kp = J.stride, warps = blockDim.x >> 5;
+    const int steps = min(kFinCopies, (lim + 31) & ~31);
+    for (int wb = warp; 32 * wb < kp; wb += warps) {
+        const unsigned char* src = J.bytes + (size_t)(c0 + 4 * j) * kp + 32 * wb + 4 * g;
+        int d[4][4] = {};
+        for (int k = 0; k < steps; k += 32) {
+            u32 x[4], y[4], b0[4], b1[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                x[i] = *reinterpret_cast<const u32*>(src + (size_t)(k + i) * kp);
+                y[i] = *reinterpret_cast<const u32*>(src + (size_t)(k + 16 + i) * kp);
+            }
+            const unsigned char* er = E + g * kPitch + k + 4 * j;
+            auto word = [](const unsigned char* p) { return *reinterpret_cast<const u32*>(p); };
+            const u32 a0 = word(er), a1 = word(er + 8 * kPitch), a2 = word(er + 16), a3 = word(er + 8 * kPitch + 16);
+            transpose4(x, b0);
+            transpose4(y, b1);
+#pragma unroll
+            for (int m = 0; m < 4; ++m) mma_u8(d[m], a0, a1, a2, a3, b0[m], b1[m]);
+        }
+        // lane (g, j): limb g of re (d[m][0, 1]) and im (d[m][2, 3]) of the wires
+        // 32 wb + 4 (2j) + m and 32 wb + 4 (2j + 1) + m
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                u64 re = shift_mod((u64)(u32)d[m][h], 8 * g), im = shift_mod((u64)(u32)d[m][2 + h], 8 * g);
+#pragma unroll
+                for (int o = 4; o < 32; o <<= 1) {
+                    re = fold61(re + __shfl_xor_sync(0xffffffffu, re, o));
+                    im = fold61(im + __shfl_xor_sync(0xffffffffu, im, o));
+                }
+                const int w = 32 * wb + 4 * (2 * j + h) + m;
+                if (g == 2 * (m & 1) + h && w < J.cs) stcg2(part + w, l2canon(mk(re, im)));
+            }
+    }
+    if (tid == 0) {
+        fp2 s = f2zero();
+        for (int k = 0; k < warps; ++k) s = f2add(s, ws[k]);
+        if (J.const_idx >= J.cs) stcg2(part + J.const_idx, f2scale(s, J.const_val));
+    }
+    __syncthreads();
+    if (tid == 0) {
+        __threadfence();
+        s_last = atomicAdd(J.ticket, 1u) == (unsigned)(J.chunks - 1);
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    for (int w = tid; w < J.W; w += blockDim.x) {
+        fp2 v = f2zero();
+        if (w < J.cs || (w == J.const_idx && w < Wp))
+            for (int k = 0; k < J.chunks; ++k) v = f2add(v, ldcg2(J.fpart + (size_t)k * Wp + w));
+        st2(J.fin + w, v);
+    }
+    if (tid == 0) {
+        finish_beta(J);
+        *J.ticket = 0u;
+    }
+}
+
+// eq(challenges, c) of all copies of a table's frame
+__global__ void __launch_bounds__(kFinCopies) finish_eq_kernel(const Job* __restrict__ jobs)
+{
+    __shared__ __align__(16) Job J;
+    __shared__ EqParts e;
+    read_job(jobs, J);
+    const int kf = J.nf + (J.has_r != 0);
+    const int c = blockIdx.x * kFinCopies + threadIdx.x;
+    if ((long long)blockIdx.x * kFinCopies >= (1LL << kf)) return;
+    eq_parts(J, blockIdx.x, e);
+    if (c < (1 << kf)) st2(J.fpart + c, eq_of(e, threadIdx.x));
+    if (c == 0) finish_beta(J);
+}
+
+// wires from a table: a warp per wire
+__global__ void __launch_bounds__(kVecThreads) finish_table_kernel(const Job* __restrict__ jobs)
+{
+    __shared__ __align__(16) Job J;
+    read_job(jobs, J);
+    const int w = blockIdx.x * (kVecThreads / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (w >= J.W) return;
+    const int n = 1 << (J.nf + (J.has_r != 0));
+    fp2 s = f2zero();
+    if (w < J.W_rows) {
+        const fp2* row = J.src + (size_t)w * J.n_table;
+        for (int c = lane; c < n; c += 32) {
+            const fp2 v = ld2(row + c);
+            s = l2add(s, l2mul(ld2(J.fpart + c), mk(fold61(v.re), fold61(v.im))));
+        }
+    }
+    s = warp_sum(l2canon(s));
+    if (lane == 0) st2(J.fin + w, s);
+}
+
+size_t form_smem(int kp) { return (size_t)(2 * kTileRows + 16) * (kp + 16); }
+
+}  // namespace
+
+int lin_stride(int cs) { return (cs + 31) & ~31; }
+size_t lin_bytes(int cs, int n_real)
+{
+    const size_t rows = ((size_t)std::max(1, n_real) + kFinCopies - 1) / kFinCopies * kFinCopies;
+    return rows * lin_stride(cs);
+}
+int lin_chunks(int n_real, int folds)
+{
+    const long long lim = std::min<long long>(n_real, 1LL << folds);
+    return (int)std::max<long long>(1, (lim + kFinCopies - 1) / kFinCopies);
+}
+
+bool prepare_linear_kernels()
+{
+    static bool done = false;
+    if (done) return true;
+    TP_CUDA_OK(cudaFuncSetAttribute(forms_bytes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)form_smem(512)),
+               "forms smem attr");
+    done = true;
+    return true;
+}
+
+// target: CTAs for the byte forms, which take up to 16 tiles each
+void plan_linear_job(Job& j, int kind, int target)
+{
+    if (kind == kFormsBytes) {
+        const int tiles = (j.n_in + kTileRows - 1) / kTileRows;
+        j.wpg = std::max(1, std::min(16, tiles / target));
+        j.tiles = (tiles + j.wpg - 1) / j.wpg;
+    } else if (kind == kFormsTable) {
+        j.tiles = (j.n_in + 31) / 32;
+    } else {
+        j.tiles = std::max(1, (j.n_pairs + kVecThreads - 1) / kVecThreads);
+    }
+    j.groups = 1;
+}
+
+bool launch_linear(const Job* d_jobs, const std::vector<Job>& jobs, int kind, cudaStream_t s, int* launches)
+{
+    if (jobs.empty()) return true;
+    if (!prepare_linear_kernels()) return false;
+    unsigned ctas = 1;
+    int kp = 0;
+    for (const Job& j : jobs) {
+        ctas = std::max(ctas, (unsigned)j.tiles);
+        kp = std::max(kp, j.stride);
+    }
+    const dim3 grid(ctas, (unsigned)jobs.size());
+    if (kind == kFormsBytes) forms_bytes_kernel<<<grid, kFormThreads, form_smem(kp), s>>>(d_jobs);
+    else if (kind == kFormsTable) forms_table_kernel<<<grid, kVecThreads, 0, s>>>(d_jobs);
+    else if (kind == kVecClaim) vec_round_kernel<false><<<grid, kVecThreads, 0, s>>>(d_jobs);
+    else vec_round_kernel<true><<<grid, kVecThreads, 0, s>>>(d_jobs);
+    ++*launches;
+    return !cuda_failed(cudaGetLastError(), "linear round launch");
+}
+
+bool launch_linear_rounds(const Job* d_jobs, int n_jobs, const VoleRounds* v, int k0, long long claim_stride,
+                          cudaStream_t s, int* launches)
+{
+    RoundsArgs a = {};
+    a.k0 = k0;
+    a.claim_stride = claim_stride;
+    const dim3 grid(1, (unsigned)n_jobs);
+    if (v) {
+        a.st = static_cast<fs::State*>(v->states);
+        a.vs = static_cast<vole::State*>(v->vole_states);
+        a.u = v->u;
+        a.v = v->v;
+        a.chal = v->chal;
+        a.proof = v->proof;
+        a.count = v->count;
+        a.n_frames = v->n_frames;
+        a.layer = v->layer;
+        vec_rounds_kernel<true><<<grid, kRoundsThreads, 0, s>>>(d_jobs, a);
+    } else {
+        vec_rounds_kernel<false><<<grid, kRoundsThreads, 0, s>>>(d_jobs, a);
+    }
+    ++*launches;
+    return !cuda_failed(cudaGetLastError(), "linear rounds launch");
+}
+
+bool launch_linear_finish(const Job* d_jobs, const std::vector<Job>& jobs, bool bytes, cudaStream_t s, int* launches)
+{
+    if (jobs.empty()) return true;
+    if (bytes) {
+        int chunks = 1, kp = 32;
+        for (const Job& j : jobs) {
+            chunks = std::max(chunks, j.chunks);
+            kp = std::max(kp, j.stride);
+        }
+        const unsigned threads = (unsigned)std::max(64, std::min(512, kp));   // a warp per 32 wires
+        finish_bytes_kernel<<<dim3((unsigned)chunks, (unsigned)jobs.size()), threads, 0, s>>>(d_jobs);
+        ++*launches;
+    } else {
+        int kf = 0, w = 1;
+        for (const Job& j : jobs) {
+            kf = std::max(kf, j.nf + (j.has_r != 0));
+            w = std::max(w, j.W);
+        }
+        const unsigned eq = (unsigned)(((1LL << kf) + kFinCopies - 1) / kFinCopies);
+        finish_eq_kernel<<<dim3(eq, (unsigned)jobs.size()), kFinCopies, 0, s>>>(d_jobs);
+        finish_table_kernel<<<dim3(blocks_for((size_t)w, kVecThreads / 32), (unsigned)jobs.size()), kVecThreads, 0, s>>>(
+            d_jobs);
+        *launches += 2;
+    }
+    return !cuda_failed(cudaGetLastError(), "linear finish launch");
+}
+
+}  // namespace tp

@@ -51,7 +51,57 @@ bool frame_alloc(Frame* f, size_t rows0, size_t rows1, cudaStream_t s)
     f->pending = false;
     f->r_dev = nullptr;
     f->pix_cur = false;
-    return (!rows0 || f->buf[0]) && f->buf[1] && f->beta[0] && f->beta[1];
+    f->linear = false;
+    f->loaded = (!rows0 || f->buf[0]) && (!rows1 || f->buf[1]) && f->beta[0] && f->beta[1];
+    return f->loaded;
+}
+
+template <class T>
+bool grow(T*& p, size_t& cap, size_t n, cudaStream_t s)
+{
+    if (n <= cap) return true;
+    dev_free(p, s);
+    p = static_cast<T*>(dev_alloc(sizeof(T) * n, s));
+    cap = p ? n : 0;
+    return p != nullptr;
+}
+
+// Whether the frame's rounds run on vectors (gkr_linear.cu): 1 + 2 groups vectors
+// in place of W_rows rows. A round moves so many times less, against one more pass
+// over the source at the end; below a quarter of the rows that always pays (gray
+// and crop: 1 and 3 against 385 and 386).
+bool wants_linear(const Frame* f)
+{
+    return f->form.groups <= kMaxLinGroups && 4 * (1 + 2 * f->form.groups) <= f->W_rows;
+}
+
+// the vectors' buffers of a frame; `part`: elements of the finish's scratch
+bool linear_alloc(Frame* f, size_t part, cudaStream_t s)
+{
+    const size_t C = (size_t)f->n_copies0, nv = 1 + 2 * (size_t)f->form.groups;
+    // one block: vectors of C copies, then of C / 2
+    fp2* base = f->vec[0];
+    if (!grow(base, f->capv, nv * C + nv * std::max<size_t>(1, C / 2), s)) {
+        f->vec[0] = nullptr;
+        return false;
+    }
+    f->vec[0] = base;
+    f->vec[1] = base + nv * C;
+    if (!f->rs) f->rs = static_cast<fp2*>(dev_alloc(sizeof(fp2) * 128, s));
+    f->linear = true;
+    f->forms_done = false;
+    f->folds = 0;
+    return f->rs && grow(f->fpart, f->cap_part, part, s);
+}
+
+void linear_free(Frame* f, cudaStream_t s)
+{
+    dev_free(f->vec[0], s);
+    dev_free(f->bytes, s);
+    dev_free(f->fpart, s);
+    f->vec[0] = f->vec[1] = f->fpart = nullptr;
+    f->bytes = nullptr;
+    f->capv = f->cap_bytes = f->cap_part = 0;
 }
 
 // apply a recorded fold without a claim
@@ -161,7 +211,34 @@ Job base_job(const Frame* f)
     j.W_rows = f->W_rows;
     j.n_in = f->n_phys;
     j.beta = f->beta[f->cur];
-    if (f->pix_cur) {
+    if (f->linear) {
+        j.A = f->vec[f->cur];
+        j.Aout = f->vec[f->cur ^ 1];
+        j.beta_out = f->beta[f->cur ^ 1];
+        j.G = f->form.groups;
+        j.gptr = f->form.gptr;
+        j.gb = f->form.gb;
+        j.rs = f->rs;
+        j.given = f->rs + 64;
+        j.nf = f->folds;
+        j.has_r = f->pending ? 1 : 0;
+        j.fpart = f->fpart;
+        j.n_table = f->n_copies0;
+        j.const_idx = -1;
+        if (f->px.pix) {
+            j.pix = f->px.pix;
+            j.n_real = f->px.n_real;
+            j.cs = f->px.cs;
+            j.const_idx = f->px.const_idx;
+            j.const_val = f->px.const_val;
+            j.bytes = f->bytes;
+            j.stride = lin_stride(f->px.cs);
+            j.chunks = lin_chunks(f->px.n_real, f->folds + j.has_r);
+            j.vec = ((j.cs & 15) == 0 && (reinterpret_cast<size_t>(j.pix) & 15) == 0) ? 1 : 0;
+        } else {
+            j.src = f->buf[0];
+        }
+    } else if (f->pix_cur) {
         j.pix = f->px.pix;
         j.n_real = f->px.n_real;
         j.cs = f->px.cs;
@@ -171,6 +248,17 @@ Job base_job(const Frame* f)
         j.A = f->buf[f->cur];
     }
     return j;
+}
+
+// the fold that a claim launch applies has been planned into it
+void advance_fold(Frame* f)
+{
+    f->cur = f->pix_cur ? 1 : (f->cur ^ 1);
+    f->pix_cur = false;
+    f->n_phys >>= 1;
+    f->pending = false;
+    f->r_dev = nullptr;
+    if (f->linear) ++f->folds;
 }
 
 }  // namespace
@@ -207,7 +295,7 @@ bool batch_set_gates(Batch* B, int i, int n_gates, const int* type, const int* i
     }
     GateForm g;
     if (!build_gate_form(n_gates, type, in0, in1, z_re, z_im, n_wires, g)) return false;
-    free_gate_form(f->form, B->stream);
+    f->loaded = false;
     f->n_wires = f->W_rows = n_wires;
     f->n_copies0 = f->n_copies = f->n_phys = n_copies;
     f->L_host = g.L;
@@ -230,6 +318,8 @@ bool batch_load_host(Batch* B, int i, const u64* v_re, const u64* v_im, const u6
     cudaStream_t s = B->stream;
     const size_t vn = (size_t)f->n_wires * (size_t)f->n_copies0;
     if (!frame_alloc(f, vn, vn / 2, s)) return false;
+    f->px = PixSrc{};
+    if (wants_linear(f) && !linear_alloc(f, (size_t)f->n_copies0, s)) return false;
     // stage the real limbs in the half-size buffer (exactly vn u64), the
     // imaginary limbs in a temporary, then pack
     u64* stage_re = reinterpret_cast<u64*>(f->buf[1]);
@@ -254,7 +344,10 @@ bool batch_load_device(Batch* B, int i, const fp2* d_values, const fp2* d_beta, 
     Frame* f = B->frames[(size_t)i];
     cudaStream_t s = B->stream;
     const size_t vn = (size_t)f->n_wires * (size_t)f->n_copies0;
-    if (!frame_alloc(f, borrow ? 0 : vn, vn / 2, s)) return false;
+    f->px = PixSrc{};
+    const bool linear = wants_linear(f);
+    if (!frame_alloc(f, borrow ? 0 : vn, linear ? 0 : vn / 2, s)) return false;
+    if (linear && !linear_alloc(f, (size_t)f->n_copies0, s)) return false;
     if (borrow) {
         f->buf[0] = const_cast<fp2*>(d_values);
         f->borrowed0 = true;
@@ -275,9 +368,17 @@ bool batch_load_pixels(Batch* B, int i, const PixSrc& px, const fp2* d_beta)
     f->px = px;
     f->W_rows = pixsrc_rows(px);
     const size_t C = (size_t)f->n_copies0, R = (size_t)f->W_rows;
-    // first fold writes R x C/2 into buf[1]; later folds alternate with buf[0]
-    if (!frame_alloc(f, R * std::max<size_t>(1, C / 4), R * (C / 2), s)) return false;
-    f->pix_cur = true;
+    if (wants_linear(f)) {
+        if (!frame_alloc(f, 0, 0, s) || !linear_alloc(f, (size_t)lin_chunks(px.n_real, 30) * R, s) ||
+            !grow(f->bytes, f->cap_bytes, lin_bytes(px.cs, px.n_real), s)) {
+            f->loaded = false;
+            return false;
+        }
+    } else {
+        // first fold writes R x C/2 into buf[1]; later folds alternate with buf[0]
+        if (!frame_alloc(f, R * std::max<size_t>(1, C / 4), R * (C / 2), s)) return false;
+        f->pix_cur = true;
+    }
     if (px.const_idx >= 0) f->Lc = f2scale(f->L_host[(size_t)px.const_idx], px.const_val);
     TP_CUDA_OK(cudaMemcpyAsync(f->beta[0], d_beta, sizeof(fp2) * C, cudaMemcpyDeviceToDevice, s),
                "copy beta");
@@ -296,7 +397,8 @@ namespace {
 int work_bucket(const std::vector<Job>& jobs, int kind)
 {
     double total = 0;
-    for (const Job& j : jobs) total += (double)j.n_pairs * (kind < 2 ? j.W_rows : j.cs);
+    for (const Job& j : jobs)
+        total += kind == kFormsBytes ? 0.5 * j.n_in * j.cs : (double)j.n_pairs * (kind < 2 ? j.W_rows : j.cs);
     int b = 0;
     while (b < 62 && (double)(1ull << (b + 1)) <= total) ++b;
     return b;
@@ -365,6 +467,30 @@ void plan_jobs(std::vector<Job>& jobs, int kind, int target)
     }
 }
 
+// the same for the launches of frames on vectors: only the forms from bytes have a
+// split (copies per CTA) to choose
+void plan_linear_jobs(std::vector<Job>& jobs, int kind, int target)
+{
+    double total = 0;
+    for (const Job& j : jobs) total += j.n_in;
+    int cta = 0;
+    for (Job& j : jobs) {
+        plan_linear_job(j, kind, std::max(1, (int)(target * (double)j.n_in / total + 0.5)));
+        j.cta0 = cta;
+        cta += j.tiles;
+    }
+}
+
+void plan_launch(std::vector<Job>& jobs, int kind, int target)
+{
+    if (kind < 4) plan_jobs(jobs, kind, target);
+    else plan_linear_jobs(jobs, kind, target);
+}
+
+// the tuner's kind of a launch (the forms from bytes stand for the byte claim they
+// replace), or -1 for one without a split
+int tune_kind(int kind) { return kind < 4 ? kind : kind == kFormsBytes ? 2 : -1; }
+
 size_t launch_ctas(const std::vector<Job>& jobs)
 {
     size_t n = 0;
@@ -380,26 +506,56 @@ void set_workspace_ptrs(Batch* B, std::vector<Job>& jobs)
     }
 }
 
+// the launch that makes the vectors of frames which have none yet; appended to out
+void plan_forms(const std::vector<Frame*>& frames, std::vector<RoundLaunch>& out, int n_sm)
+{
+    for (int kind : {(int)kFormsBytes, (int)kFormsTable}) {
+        RoundLaunch L;
+        L.kind = kind;
+        int lg = 0;
+        for (Frame* f : frames) {
+            if (!f->linear || f->forms_done || (f->px.pix != nullptr) != (kind == kFormsBytes)) continue;
+            Job j = base_job(f);
+            j.kind = kind;
+            L.jobs.push_back(j);
+            L.rdev.push_back(nullptr);
+            f->forms_done = true;
+            lg = 0;
+            while ((1 << lg) < f->n_copies0) ++lg;
+        }
+        if (L.jobs.empty()) continue;
+        if (kind == kFormsBytes) L.bucket = work_bucket(L.jobs, kind);
+        plan_linear_jobs(L.jobs, kind, (kind == kFormsBytes ? tuned_mult(2, L.bucket) : 4) * n_sm);
+        L.timer_tag = (kind == kFormsBytes ? 1000 : 0) + lg;
+        out.push_back(std::move(L));
+    }
+}
+
+constexpr int kKinds = 6;   // 0..3 on tables and bytes, kVecClaim, kVecFold
+
 // the claim launches of one round: per kind, its jobs and the device challenges
 // of their pending folds; advances the frames past the round's folds
 bool plan_claims(Batch* B, u64* const* d_claims, std::vector<RoundLaunch>& out)
 {
     Ctx* c = ctx();
     if (!c) return false;
-    RoundLaunch by_kind[4];
-    std::vector<Frame*> fr[4];
-    for (int k = 0; k < 4; ++k) by_kind[k].kind = k;
+    RoundLaunch by_kind[kKinds];
+    std::vector<Frame*> fr[kKinds], fresh;
+    for (int k = 0; k < kKinds; ++k) by_kind[k].kind = k;
+    bool any = false;
     for (size_t i = 0; i < B->frames.size(); ++i) {
         Frame* f = B->frames[i];
         if (!f->configured) continue;
-        if (!f->buf[1]) {
+        if (!f->loaded) {
             set_error(TP_ERR_ARG, "frame %zu has no table", i);
             return false;
         }
         if (f->n_copies < 2) continue;
+        any = true;
+        if (f->linear && !f->forms_done) fresh.push_back(f);
         Job j = base_job(f);
-        j.kind = (f->pix_cur ? 2 : 0) + (f->pending ? 1 : 0);
-        if (f->pending) {
+        j.kind = f->linear ? (f->pending ? kVecFold : kVecClaim) : (f->pix_cur ? 2 : 0) + (f->pending ? 1 : 0);
+        if (f->pending && !f->linear) {
             const int nxt = f->pix_cur ? 1 : (f->cur ^ 1);
             j.Aout = f->buf[nxt];
             j.beta_out = f->beta[nxt];
@@ -410,31 +566,30 @@ bool plan_claims(Batch* B, u64* const* d_claims, std::vector<RoundLaunch>& out)
         by_kind[j.kind].rdev.push_back(f->pending ? f->r_dev : nullptr);
         fr[j.kind].push_back(f);
     }
-    if (B->frames.size() == 1 && by_kind[0].jobs.empty() && by_kind[1].jobs.empty() && by_kind[2].jobs.empty() &&
-        by_kind[3].jobs.empty()) {
+    if (B->frames.size() == 1 && !any) {
         set_error(TP_ERR_ARG, "claim needs at least 2 copies (have %d)", B->frames[0]->n_copies);
         return false;
     }
-    for (int k = 0; k < 4; ++k) {
+    plan_forms(fresh, out, c->n_sm);
+    for (int k = 0; k < kKinds; ++k) {
         RoundLaunch& L = by_kind[k];
         if (L.jobs.empty()) continue;
-        L.bucket = work_bucket(L.jobs, k);
-        plan_jobs(L.jobs, k, tuned_mult(k, L.bucket) * c->n_sm);
+        if (k < 4) L.bucket = work_bucket(L.jobs, k);
+        plan_launch(L.jobs, k, (k < 4 ? tuned_mult(k, L.bucket) : 4) * c->n_sm);
         int lg = 0;
         while ((1 << lg) < 2 * L.jobs[0].n_pairs) ++lg;
-        L.timer_tag = 1000 * (k >> 1) + 100 * (k & 1) + lg;
-        for (Frame* f : fr[k]) {
-            if (f->pending) {
-                f->cur = f->pix_cur ? 1 : (f->cur ^ 1);
-                f->pix_cur = false;
-                f->n_phys >>= 1;
-                f->pending = false;
-                f->r_dev = nullptr;
-            }
-        }
+        L.timer_tag = (k < 4 ? 1000 * (k >> 1) : 0) + 100 * (k & 1) + lg;
+        for (Frame* f : fr[k])
+            if (f->pending) advance_fold(f);
         out.push_back(std::move(L));
     }
     return true;
+}
+
+bool launch_any(const Job* d_jobs, const RoundLaunch& L, cudaStream_t s, int* launches)
+{
+    return L.kind < 4 ? launch_round(d_jobs, L.jobs, L.kind, s, launches)
+                      : launch_linear(d_jobs, L.jobs, L.kind, s, launches);
 }
 
 // time one round launch under each candidate split, keep the fastest for its
@@ -452,7 +607,7 @@ bool tune_launch(Batch* B, RoundLaunch& L)
     bool ok = true;
     for (int mult : kTuneMults) {
         std::vector<Job> jobs = L.jobs;
-        plan_jobs(jobs, L.kind, mult * c->n_sm);
+        plan_launch(jobs, L.kind, mult * c->n_sm);
         if (!ensure_workspace(B, jobs.size(), launch_ctas(jobs))) {
             ok = false;
             break;
@@ -463,9 +618,12 @@ bool tune_launch(Batch* B, RoundLaunch& L)
             break;
         }
         int dummy = 0;
-        ok = launch_round(B->d_jobs, jobs, L.kind, s, &dummy);   // warm
+        RoundLaunch tried;
+        tried.kind = L.kind;
+        tried.jobs = std::move(jobs);
+        ok = launch_any(B->d_jobs, tried, s, &dummy);   // warm
         ok = ok && !cuda_failed(cudaEventRecord(e0, s), "tune event");
-        for (int rep = 0; ok && rep < 3; ++rep) ok = launch_round(B->d_jobs, jobs, L.kind, s, &dummy);
+        for (int rep = 0; ok && rep < 3; ++rep) ok = launch_any(B->d_jobs, tried, s, &dummy);
         ok = ok && !cuda_failed(cudaEventRecord(e1, s), "tune event") &&
              !cuda_failed(cudaEventSynchronize(e1), "tune sync");
         if (!ok) break;
@@ -481,25 +639,108 @@ bool tune_launch(Batch* B, RoundLaunch& L)
     if (!ok) return false;
     {
         std::lock_guard<std::mutex> lk(tune_mutex());
-        tune_table()[TuneKey{c->device, L.kind, L.bucket}] = best;
+        tune_table()[TuneKey{c->device, tune_kind(L.kind), L.bucket}] = best;
     }
-    plan_jobs(L.jobs, L.kind, best * c->n_sm);
+    plan_launch(L.jobs, L.kind, best * c->n_sm);
     return true;
 }
 
 bool launch_planned(Batch* B, RoundLaunch& L)
 {
-    if (g_tune_on && !tune_known(L.kind, L.bucket) && !tune_launch(B, L)) return false;
+    const int tk = tune_kind(L.kind);
+    if (g_tune_on && tk >= 0 && !tune_known(tk, L.bucket) && !tune_launch(B, L)) return false;
     if (!ensure_workspace(B, L.jobs.size(), launch_ctas(L.jobs))) return false;
     set_workspace_ptrs(B, L.jobs);
     if (!upload_jobs(B, L.jobs.data(), L.jobs.size(), L.rdev)) return false;
     timer_begin(B->stream, L.timer_tag);
-    const bool ok = launch_round(B->d_jobs, L.jobs, L.kind, B->stream, &B->launches);
+    const bool ok = launch_any(B->d_jobs, L, B->stream, &B->launches);
     timer_end(B->stream);
     return ok;
 }
 
+// a linear frame's recorded fold without a claim of the caller's: the claim launch
+// that applies it, its claim left in the frame's own slot
+bool apply_fold_linear(Batch* B, Frame* f)
+{
+    Ctx* c = ctx();
+    if (!c) return false;
+    std::vector<RoundLaunch> plan;
+    plan_forms({f}, plan, c->n_sm);
+    RoundLaunch L;
+    L.kind = kVecFold;
+    Job j = base_job(f);
+    j.kind = kVecFold;
+    j.n_pairs = f->n_phys / 4;
+    j.out8 = f->out8;
+    plan_linear_job(j, kVecFold, 1);
+    L.jobs.push_back(j);
+    L.rdev.push_back(f->r_dev);
+    advance_fold(f);
+    plan.push_back(std::move(L));
+    for (RoundLaunch& q : plan)
+        if (!launch_planned(B, q)) return false;
+    return true;
+}
+
+// Rounds of a linear frame whose challenges (device memory at its given[]) are all
+// known: n_rounds claims, each followed by its fold, in one launch; the last fold
+// stays recorded (host challenge `last`). Planned into L.
+void plan_given(Frame* f, int n_rounds, u64* out8, fp2 last, RoundLaunch& L)
+{
+    Job j = base_job(f);
+    j.kind = kVecFold;
+    j.n_rounds = n_rounds;
+    j.out8 = out8;
+    j.tiles = j.groups = 1;
+    L.kind = kVecFold;
+    L.jobs.push_back(j);
+    L.rdev.push_back(f->pending ? f->r_dev : nullptr);
+    if (f->pending) advance_fold(f);
+    for (int q = 0; q < n_rounds; ++q) {
+        f->n_copies >>= 1;
+        if (q + 1 < n_rounds) advance_fold(f);
+    }
+    f->pending = true;
+    f->r = last;
+    f->r_dev = nullptr;
+}
+
 }  // namespace
+
+bool batch_given_rounds(Batch* B, int n_rounds, const u64* challenges, u64* d_claims)
+{
+    Frame* f = B->frames[0];
+    for (int k = 0; k < n_rounds; ++k) {
+        // from here on in one launch: few pairs left, two rounds or more to go
+        const int left = n_rounds - k;
+        if (f->configured && f->loaded && f->linear && d_claims && left > 1 && left <= 63 &&
+            f->n_copies / 2 <= kFusePairs && (f->n_copies >> left) >= 1) {
+            std::vector<fp2> r;
+            for (int q = k; q < n_rounds; ++q) {
+                r.push_back(mk(challenges[2 * q], challenges[2 * q + 1]));
+                if (r.back().re >= P61 || r.back().im >= P61) {
+                    set_error(TP_ERR_ARG, "fold challenge is not a canonical field element");
+                    return false;
+                }
+            }
+            Ctx* c = ctx();
+            if (!c) return false;
+            std::vector<RoundLaunch> plan;
+            plan_forms({f}, plan, c->n_sm);
+            for (RoundLaunch& L : plan)
+                if (!launch_planned(B, L)) return false;
+            RoundLaunch L;
+            if (!upload_async(f->rs + 64, r.data(), sizeof(fp2) * r.size(), B->stream)) return false;
+            plan_given(f, left, d_claims + 8 * (size_t)k, r.back(), L);
+            return ensure_workspace(B, 1, 1) && upload_jobs(B, L.jobs.data(), 1, L.rdev) &&
+                   launch_linear_rounds(B->d_jobs, 1, nullptr, 0, 8, B->stream, &B->launches);
+        }
+        u64* p = d_claims ? d_claims + 8 * (size_t)k : nullptr;
+        if (!batch_claim(B, &p)) return false;
+        if (!batch_fold(B, 0, mk(challenges[2 * k], challenges[2 * k + 1]))) return false;
+    }
+    return true;
+}
 
 bool batch_claim(Batch* B, u64* const* d_claims)
 {
@@ -526,7 +767,7 @@ bool batch_fold(Batch* B, int i, fp2 r)
         return false;
     }
     if (device_fold_blocked(f)) return false;
-    if (f->pending && !apply_fold(f, B->stream, &B->launches)) return false;
+    if (f->pending && !(f->linear ? apply_fold_linear(B, f) : apply_fold(f, B->stream, &B->launches))) return false;
     f->pending = true;
     f->r = r;
     f->r_dev = nullptr;
@@ -562,29 +803,68 @@ bool batch_fold_dev(Batch* B, int i, const fp2* d_r)
 
 namespace {
 
-// the finish launch: wires and beta of every configured frame (a pending fold of
-// the last two copies applied by it); a pending fold of more copies is applied
-// first (host challenges only)
-bool plan_finish(Batch* B, fp2* const* d_wires, fp2* const* d_beta, RoundLaunch& L)
+// The finish launches: wires and beta of every configured frame (a pending fold of
+// the last two copies applied by it). A pending fold of more copies is applied
+// first (host challenges only) on a table of all wires; linear frames take copy 0
+// after the pending fold from the source at once. out: [0] frames on tables, [1]
+// linear ones from bytes, [2] from a table; `forms` (if any) come before them.
+constexpr int kFinishKinds = 3;
+
+bool plan_finish_frame(Batch* B, Frame* f, fp2* d_wires, fp2* d_beta, RoundLaunch (&out)[kFinishKinds])
 {
-    L.kind = 4;
-    L.max_w = 0;
+    if (f->pending && !f->linear && f->n_phys > 2 &&
+        (device_fold_blocked(f) || !apply_fold(f, B->stream, &B->launches)))
+        return false;
+    Job j = base_job(f);
+    j.kind = f->pending ? 1 : 0;  // a pending fold of the last two copies
+    j.fin = d_wires ? d_wires : f->fin;
+    j.fin_beta = d_beta ? d_beta : f->fin + f->n_wires;
+    RoundLaunch& L = out[!f->linear ? 0 : f->px.pix ? 1 : 2];
+    L.kind = 8;
+    j.tiles = j.groups = 1;
+    L.max_w = std::max(L.max_w, f->n_wires);
+    L.jobs.push_back(j);
+    L.rdev.push_back(f->pending ? f->r_dev : nullptr);
+    return true;
+}
+
+bool plan_finish(Batch* B, fp2* const* d_wires, fp2* const* d_beta, std::vector<RoundLaunch>& forms,
+                 RoundLaunch (&out)[kFinishKinds])
+{
+    Ctx* c = ctx();
+    if (!c) return false;
+    std::vector<Frame*> fresh;
     for (size_t i = 0; i < B->frames.size(); ++i) {
         Frame* f = B->frames[i];
         if (!f->configured) continue;
-        if (!f->buf[1]) {
+        if (!f->loaded) {
             set_error(TP_ERR_ARG, "frame %zu has no table", i);
             return false;
         }
-        if (f->pending && f->n_phys > 2 && (device_fold_blocked(f) || !apply_fold(f, B->stream, &B->launches)))
-            return false;
-        Job j = base_job(f);
-        j.kind = f->pending ? 1 : 0;  // a pending fold of the last two copies
-        j.fin = (d_wires && d_wires[i]) ? d_wires[i] : f->fin;
-        j.fin_beta = (d_beta && d_beta[i]) ? d_beta[i] : f->fin + f->n_wires;
-        L.max_w = std::max(L.max_w, f->n_wires);
-        L.jobs.push_back(j);
-        L.rdev.push_back(f->pending ? f->r_dev : nullptr);
+        if (f->linear && !f->forms_done && f->px.pix) fresh.push_back(f);   // their bytes are copied by the forms
+        if (!plan_finish_frame(B, f, d_wires ? d_wires[i] : nullptr, d_beta ? d_beta[i] : nullptr, out)) return false;
+    }
+    plan_forms(fresh, forms, c->n_sm);
+    return true;
+}
+
+bool launch_finish_kind(const Job* d_jobs, const RoundLaunch& L, int which, cudaStream_t s, int* launches)
+{
+    return which == 0 ? launch_finish(d_jobs, (int)L.jobs.size(), L.max_w, s, launches)
+                      : launch_linear_finish(d_jobs, L.jobs, which == 1, s, launches);
+}
+
+bool launch_finishes(Batch* B, std::vector<RoundLaunch>& forms, RoundLaunch (&fin)[kFinishKinds])
+{
+    for (RoundLaunch& L : forms)
+        if (!launch_planned(B, L)) return false;
+    for (int q = 0; q < kFinishKinds; ++q) {
+        RoundLaunch& L = fin[q];
+        if (L.jobs.empty()) continue;
+        if (!ensure_workspace(B, L.jobs.size(), 1)) return false;
+        set_workspace_ptrs(B, L.jobs);
+        if (!upload_jobs(B, L.jobs.data(), L.jobs.size(), L.rdev)) return false;
+        if (!launch_finish_kind(B->d_jobs, L, q, B->stream, &B->launches)) return false;
     }
     return true;
 }
@@ -593,17 +873,16 @@ bool plan_finish(Batch* B, fp2* const* d_wires, fp2* const* d_beta, RoundLaunch&
 
 bool batch_finish(Batch* B, fp2* const* d_wires, fp2* const* d_beta)
 {
-    RoundLaunch L;
-    if (!plan_finish(B, d_wires, d_beta, L)) return false;
-    if (!ensure_workspace(B, L.jobs.size(), 1)) return false;
-    if (!upload_jobs(B, L.jobs.data(), L.jobs.size(), L.rdev)) return false;
-    return launch_finish(B->d_jobs, (int)L.jobs.size(), L.max_w, B->stream, &B->launches);
+    std::vector<RoundLaunch> forms;
+    RoundLaunch fin[kFinishKinds];
+    return plan_finish(B, d_wires, d_beta, forms, fin) && launch_finishes(B, forms, fin);
 }
 
 namespace {
 
 struct GraphOp {
-    int type = 0;          // 0 round launch, 1 VOLE round, 2 finish
+    int type = 0;          // 0 round launch, 1 VOLE round, 2 finish, 3 all rounds left in one launch
+    int fin = 0;           // 2: which of the finish kinds
     RoundLaunch L;
     size_t job_off = 0, patch_off = 0, n_patch = 0;
     int round = 0;
@@ -655,16 +934,25 @@ bool batch_vole_rounds_graph(Batch* B, u64* d_claims, void* d_states, void* d_vo
     // ---- plan every launch (advances the frames as the launches will)
     std::vector<GraphOp> ops;
     std::vector<u64*> claim_ptrs((size_t)nB);
-    for (int k = 0; k < rounds; ++k) {
+    bool all_linear = true;
+    for (const Frame* f : B->frames) all_linear = all_linear && f->loaded && f->linear;
+    auto push = [&](RoundLaunch& L, int type) {
+        GraphOp op;
+        op.type = type;
+        op.L = std::move(L);
+        ops.push_back(std::move(op));
+    };
+    int k = 0;
+    for (; k < rounds; ++k) {
+        // frames on vectors: once no frame has many pairs left, each runs the rest of
+        // its rounds, transcript included, in one CTA
+        int most = 0;
+        for (const Frame* f : B->frames) most = std::max(most, f->n_copies / 2);
+        if (all_linear && most <= kFusePairs) break;
         for (int i = 0; i < nB; ++i) claim_ptrs[(size_t)i] = d_claims + 8 * ((size_t)nB * k + i);
         std::vector<RoundLaunch> plan;
         if (!plan_claims(B, claim_ptrs.data(), plan)) return false;
-        for (RoundLaunch& L : plan) {
-            GraphOp op;
-            op.type = 0;
-            op.L = std::move(L);
-            ops.push_back(std::move(op));
-        }
+        for (RoundLaunch& L : plan) push(L, 0);
         GraphOp v;
         v.type = 1;
         v.round = k;
@@ -672,11 +960,36 @@ bool batch_vole_rounds_graph(Batch* B, u64* d_claims, void* d_states, void* d_vo
         for (int i = 0; i < nB; ++i)
             if (k < fr_rounds[(size_t)i] && !batch_fold_dev(B, i, d_chal + (size_t)nB * k + i)) return false;
     }
+    if (k < rounds) {
+        std::vector<RoundLaunch> plan;
+        plan_forms(B->frames, plan, c->n_sm);
+        for (RoundLaunch& L : plan) push(L, 0);
+        RoundLaunch L;
+        for (int i = 0; i < nB; ++i) {
+            Frame* f = B->frames[(size_t)i];
+            const int left = fr_rounds[(size_t)i] - k;
+            if (left <= 0) continue;
+            RoundLaunch one;
+            plan_given(f, left, d_claims + 8 * ((size_t)nB * k + i), f2zero(), one);
+            one.jobs[0].frame = i;
+            f->r_dev = d_chal + (size_t)nB * (fr_rounds[(size_t)i] - 1) + i;   // the last fold's challenge
+            L.kind = one.kind;
+            L.jobs.push_back(one.jobs[0]);
+            L.rdev.push_back(one.rdev[0]);
+        }
+        push(L, 3);
+        ops.back().round = k;
+    }
     {
-        GraphOp fin;
-        fin.type = 2;
-        if (!plan_finish(B, d_wires, d_beta, fin.L)) return false;
-        ops.push_back(std::move(fin));
+        std::vector<RoundLaunch> forms;
+        RoundLaunch fin[kFinishKinds];
+        if (!plan_finish(B, d_wires, d_beta, forms, fin)) return false;
+        for (RoundLaunch& L : forms) push(L, 0);
+        for (int q = 0; q < kFinishKinds; ++q)
+            if (!fin[q].jobs.empty()) {
+                push(fin[q], 2);
+                ops.back().fin = q;
+            }
     }
     // ---- workspace, one job table and one patch table
     size_t max_jobs = 1, max_ctas = 1, n_jobs = 0, n_patch = 0;
@@ -688,7 +1001,7 @@ bool batch_vole_rounds_graph(Batch* B, u64* d_claims, void* d_states, void* d_vo
     if (!ensure_workspace(B, max_jobs, max_ctas)) return false;
     for (GraphOp& op : ops) {
         if (op.type == 1) continue;
-        if (op.type == 0) set_workspace_ptrs(B, op.L.jobs);
+        if (op.type != 3) set_workspace_ptrs(B, op.L.jobs);
         op.job_off = n_jobs;
         op.patch_off = n_patch;
         for (const fp2* r : op.L.rdev) op.n_patch += r ? 1 : 0;
@@ -745,7 +1058,7 @@ bool batch_vole_rounds_graph(Batch* B, u64* d_claims, void* d_states, void* d_vo
                                   (long long)(size_t)d_states, (long long)(size_t)d_vole_states,
                                   (long long)(size_t)d_u, (long long)(size_t)d_v, count, layer,
                                   (long long)(size_t)d_chal, (long long)(size_t)d_proof, (long long)nB,
-                                  (long long)uneven};
+                                  (long long)uneven, (long long)(size_t)d_claims};
     int kernels = 0;
     for (const GraphOp& op : ops) {
         key.push_back(op.type);
@@ -755,20 +1068,26 @@ bool batch_vole_rounds_graph(Batch* B, u64* d_claims, void* d_states, void* d_vo
         key.push_back((long long)op.patch_off);
         key.push_back((long long)op.n_patch);
         key.push_back(op.L.max_w);
+        key.push_back(op.fin);
+        key.push_back(op.round);
         for (const Job& j : op.L.jobs) {
             key.push_back(j.tiles);
             key.push_back(j.groups);
             key.push_back(j.wpg);
             key.push_back(j.pw);
+            key.push_back(j.stride);
+            key.push_back(j.chunks);
+            key.push_back(j.W);
+            key.push_back(j.nf + j.has_r);
         }
-        kernels += (op.type == 1) ? 1 : 1 + (op.n_patch ? 1 : 0);
+        kernels += (op.type == 1) ? 1 : 1 + (op.n_patch ? 1 : 0) + (op.type == 2 && op.fin == 2 ? 1 : 0);
     }
     if (!B->graph || key != B->graph_key) {
         if (B->graph) {
             cudaGraphExecDestroy(B->graph);
             B->graph = nullptr;
         }
-        if (!prepare_round_kernels()) return false;
+        if (!prepare_round_kernels() || !prepare_linear_kernels()) return false;
         TP_CUDA_OK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "begin capture");
         bool ok = true;
         int dummy = 0;
@@ -789,10 +1108,15 @@ bool batch_vole_rounds_graph(Batch* B, u64* d_claims, void* d_states, void* d_vo
                 ok = !cuda_failed(cudaGetLastError(), "challenge patch");
             }
             if (!ok) break;
-            if (op.type == 0)
-                ok = launch_round(B->d_table + op.job_off, op.L.jobs, op.L.kind, s, &dummy);
-            else
-                ok = launch_finish(B->d_table + op.job_off, (int)op.L.jobs.size(), op.L.max_w, s, &dummy);
+            if (op.type == 0) {
+                ok = launch_any(B->d_table + op.job_off, op.L, s, &dummy);
+            } else if (op.type == 3) {
+                const VoleRounds v = {d_states, d_vole_states, d_u, d_v, d_chal, d_proof, count, nB, layer};
+                ok = launch_linear_rounds(B->d_table + op.job_off, (int)op.L.jobs.size(), &v, op.round,
+                                          8 * (long long)nB, s, &dummy);
+            } else {
+                ok = launch_finish_kind(B->d_table + op.job_off, op.L, op.fin, s, &dummy);
+            }
         }
         cudaGraph_t g = nullptr;
         const cudaError_t e = cudaStreamEndCapture(s, &g);
@@ -854,19 +1178,18 @@ bool batch_finish_frame(Batch* B, int i, fp2* d_wires, fp2* d_beta)
         return false;
     }
     Frame* f = B->frames[(size_t)i];
-    if (!f->configured || !f->buf[1]) {
+    if (!f->configured || !f->loaded) {
         set_error(TP_ERR_ARG, "frame %d is not configured", i);
         return false;
     }
-    if (f->pending && f->n_phys > 2 && (device_fold_blocked(f) || !apply_fold(f, B->stream, &B->launches)))
-        return false;
-    Job j = base_job(f);
-    j.kind = f->pending ? 1 : 0;
-    j.fin = d_wires ? d_wires : f->fin;
-    j.fin_beta = d_beta ? d_beta : f->fin + f->n_wires;
-    if (!ensure_workspace(B, 1, 1)) return false;
-    if (!upload_jobs(B, &j, 1, std::vector<const fp2*>{f->pending ? f->r_dev : nullptr})) return false;
-    if (!launch_finish(B->d_jobs, 1, f->n_wires, B->stream, &B->launches)) return false;
+    Ctx* c = ctx();
+    if (!c) return false;
+    std::vector<RoundLaunch> forms;
+    RoundLaunch fin[kFinishKinds];
+    const bool fresh = f->linear && !f->forms_done && f->px.pix;
+    if (!plan_finish_frame(B, f, d_wires, d_beta, fin)) return false;
+    if (fresh) plan_forms({f}, forms, c->n_sm);
+    if (!launch_finishes(B, forms, fin)) return false;
     batch_release(B, i, false);
     return true;
 }
@@ -875,7 +1198,7 @@ void batch_release(Batch* B, int i, bool free_buffers)
 {
     if (i < 0 || i >= (int)B->frames.size()) return;
     Frame* f = B->frames[(size_t)i];
-    f->configured = false;
+    f->configured = f->loaded = false;
     f->n_copies = 0;
     f->pending = false;
     f->r_dev = nullptr;
@@ -888,13 +1211,14 @@ void batch_release(Batch* B, int i, bool free_buffers)
         f->buf[0] = f->buf[1] = f->beta[0] = f->beta[1] = nullptr;
         f->cap0 = f->cap1 = f->capb = 0;
         f->borrowed0 = false;
+        linear_free(f, s);
     }
 }
 
 void batch_reset(Batch* B)
 {
     for (Frame* f : B->frames) {
-        f->configured = false;
+        f->configured = f->loaded = false;
         f->n_copies = 0;
     }
 }
@@ -910,6 +1234,8 @@ void batch_destroy(Batch* B)
         dev_free(f->beta[1], s);
         dev_free(f->fin, s);
         dev_free(f->out8, s);
+        linear_free(f, s);
+        dev_free(f->rs, s);
         free_gate_form(f->form, s);
         delete f;
     }

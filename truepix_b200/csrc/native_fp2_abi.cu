@@ -456,13 +456,9 @@ int tp_early_rounds_dev(void* handle, int n_rounds, const uint64_t* challenges, 
     tp::clear_error();
     if (!handle || n_rounds < 0) return -1;
     tp::Batch* S = static_cast<tp::Batch*>(handle);
-    u64* out = static_cast<u64*>(d_claims);
-    for (int k = 0; k < n_rounds; ++k) {
-        u64* p = out ? out + 8 * (size_t)k : nullptr;
-        if (!tp::batch_claim(S, &p)) return -1;
-        if (!tp::batch_fold(S, 0, mk(challenges[2 * k], challenges[2 * k + 1]))) return -1;
-    }
-    return 0;
+    return tp::batch_given_rounds(S, n_rounds, reinterpret_cast<const u64*>(challenges), static_cast<u64*>(d_claims))
+               ? 0
+               : -1;
 }
 
 // ---- batches of frames -------------------------------------------------------

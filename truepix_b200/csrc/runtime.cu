@@ -120,7 +120,7 @@ struct Ring {
     std::vector<bool> used;
     int next = 0;
 };
-Ring g_small{1024, 16 * 1024};
+Ring g_small{1024, 20 * 1024};   // a 512-wire layer's linear form with 384 product terms is 17 KB
 Ring g_large{64, 256 * 1024};
 std::mutex g_ring_mu;
 
