@@ -438,8 +438,15 @@ __global__ void __launch_bounds__(kRoundsThreads, 1) vec_rounds_kernel(const Job
     __shared__ __align__(16) Job J;
     __shared__ fp2 ws[kRoundsThreads / 32][4];
     __shared__ fp2 s_r;
+    __shared__ fs::TxMem tx;
+    __shared__ fs::State s_st;      // the transcript between the rounds
+    __shared__ vole::State s_vs;
     read_job(jobs, J);
     const int tid = threadIdx.x;
+    if (kVole && tid == 0) {
+        s_st = a.st[J.frame];
+        s_vs = a.vs[J.frame];
+    }
     const fp2* in = J.A;
     const fp2* beta = J.beta;
     fp2 *out = J.Aout, *beta_out = J.beta_out;
@@ -475,18 +482,16 @@ __global__ void __launch_bounds__(kRoundsThreads, 1) vec_rounds_kernel(const Job
                 const int i = J.frame, k = a.k0 + q;
                 const size_t at = (size_t)a.n_frames * k + i;
                 fp2 coef[4];
-                fs::State s = a.st[i];
-                vole::State w = a.vs[i];
+                vole::State w = s_vs;
+                fs::Writer s(s_st, &tx);
                 vole::interpolate_cubic(acc[0], acc[1], acc[2], acc[3], coef);
                 vole::round(s, w, coef, 4, a.u + i * a.count, a.v + i * a.count, a.count, vole::sc_label(a.layer, k),
                             a.proof ? a.proof + 5 * at : nullptr, &c);
-                __syncwarp();
+                s.store(s_st);
                 if (tid == 0) {
-                    a.st[i] = s;
-                    a.vs[i] = w;
+                    s_vs = w;
                     a.chal[at] = c;
                 }
-                __syncwarp();
             } else {
                 c = ld2(J.given + q);
             }
@@ -495,6 +500,10 @@ __global__ void __launch_bounds__(kRoundsThreads, 1) vec_rounds_kernel(const Job
         __syncthreads();
         r = s_r;
         fold = true;
+    }
+    if (kVole && tid == 0) {
+        a.st[J.frame] = s_st;
+        a.vs[J.frame] = s_vs;
     }
 }
 

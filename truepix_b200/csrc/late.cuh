@@ -125,7 +125,10 @@ struct Work {
     fp2 T[kMaxWires];
     fp2 Tn[kMaxWires / 2];
     fp2 A[kMaxGates];
-    fp2 red[3][kThreads];
+    union {                    // the sums' slots; a step that hashes has read them before
+        fp2 red[3][kThreads];
+        fs::TxMem tx;
+    };
     fp2 w[2 * kMaxInBits];     // the challenges
     fp2 h[kMaxInBits + 1];     // the line's values
     fp2 hc[kMaxInBits + 1];    // its coefficients
@@ -204,9 +207,10 @@ TP_HD void step_reduce(Work& w, int left, int tid)
 }
 
 // The steps run by `par.one`: one warp on the device (one call on the host). Its
-// lanes do the same work, each on copies of its own of the transcript and the
-// VOLE state (transcript.cuh), and lane 0 writes. Reads of the workspace that the
-// writes below them would change come before the synchronisation in front of these.
+// lanes do the same work, with the transcript in a Writer (transcript.cuh) and each
+// on a copy of its own of the VOLE state, and lane 0 writes. Reads of the workspace
+// that the writes below them would change come before the synchronisation in front
+// of these.
 TP_HD void warp_sync()
 {
 #ifdef __CUDA_ARCH__
@@ -215,6 +219,7 @@ TP_HD void warp_sync()
 }
 
 // the round's coefficients and its challenge
+#pragma nv_exec_check_disable
 TP_HD void step_head(Work& w, const Frame& f, const Shape& sh, int rd)
 {
     fp2 c[3];
@@ -224,13 +229,13 @@ TP_HD void step_head(Work& w, const Frame& f, const Shape& sh, int rd)
     if (f.chal) {
         r = f.chal[rd];
     } else {
-        fs::State st = w.st;
         vole::State vs = w.vs;
+        fs::Writer st(w.st, &w.tx);
         const fs::Label label = vole::sc_label(sh.layer, sh.round0 + rd);
         const bool ok = vole::round(st, vs, c, 3, f.u, f.v, sh.count, label, f.proof ? f.proof + 4 * rd : nullptr, &r);
         warp_sync();
+        st.store(w.st);
         if (fs::lead()) {
-            w.st = st;
             w.vs = vs;
             if (!ok) w.bad = 1;
         }
@@ -408,11 +413,11 @@ TP_HD int close_eq_index(const Shape& sh) { return sh.n + 6 + 5 * (sh.zk != 0); 
 // create_final_prod_pok (:175-218; the zero-knowledge prover's,
 // circuitnizkvec_vole_ZK.py:188-247, adds three mask commitments of 1 and their
 // product proof) on the line's coefficients
+#pragma nv_exec_check_disable
 TP_HD void step_close_commit(Work& w, const Frame& f, const Shape& sh)
 {
     const int n = sh.n;
     const int zk = sh.zk != 0;
-    fs::State st = w.st;
     vole::State vs = w.vs;
     if (vs.bad || vs.idx + (unsigned long long)(n + 2 + 3 * zk) > (unsigned long long)sh.count) {
         warp_sync();
@@ -422,9 +427,10 @@ TP_HD void step_close_commit(Work& w, const Frame& f, const Shape& sh)
         }
         return;
     }
+    fs::Writer st(w.st, &w.tx);
     fp2* out = f.closing;
     auto put = [&](fp2 v) {   // the next closing value: written out and put
-        fs::put_fp2(st, v.re, v.im);
+        st.put_fp2(v.re, v.im);
         if (fs::lead()) *out = v;
         ++out;
     };
@@ -443,7 +449,7 @@ TP_HD void step_close_commit(Work& w, const Frame& f, const Shape& sh)
         rest_sum = f2add(rest_sum, w.hc[k]);
         rest_v = f2add(rest_v, vv[k]);
     }
-    const fp2 c = fs::rand_fp2(st, fs::label_lit("pok-vec"));
+    const fp2 c = st.rand_fp2(fs::label_lit("pok-vec"));
     put(f2mul(rest_sum, c));
     put(f2mul(rest_v, c));
     if (zk)
@@ -457,12 +463,12 @@ TP_HD void step_close_commit(Work& w, const Frame& f, const Shape& sh)
         put(f2sub(f2add(mtag[1], mtag[0]), mtag[2]));
     }
     warp_sync();
+    st.store(w.st);
     if (!fs::lead()) return;
     for (int k = 0; k <= n; ++k) w.vv[k] = vv[k];
     w.pr[0] = v1;
     w.pr[1] = vsum;
     w.pr[2] = v3;
-    w.st = st;
     w.vs = vs;
 }
 
@@ -492,16 +498,10 @@ TP_HD void step_close_sums(Work& w, const Frame& f, const uint32_t* gates, const
 
 // the equality proof against the last round's value, tau, the proof of knowledge
 // of all round coefficients, the input point and its value proof
+#pragma nv_exec_check_disable
 TP_HD void step_close_tail(Work& w, const Frame& f, const Shape& sh)
 {
     const int n = sh.n, nb = sh.round0;
-    fs::State st = w.st;
-    fp2* out = f.closing + close_eq_index(sh);
-    auto put = [&](fp2 v) {
-        fs::put_fp2(st, v.re, v.im);
-        if (fs::lead()) *out = v;
-        ++out;
-    };
     // beta's factor: prod over the early challenges of 2 w z + 1 - (w + z)
     fp2 mz = mk(1, 0);
     for (int k = 0; k < nb; ++k) {
@@ -509,9 +509,17 @@ TP_HD void step_close_tail(Work& w, const Frame& f, const Shape& sh)
         mz = f2mul(mz, f2sub(f2add(f2dbl(f2mul(wk, zk)), mk(1, 0)), f2add(wk, zk)));
     }
     const fp2 tv = f2mul(w.red[0][0], mz);
-    const fp2 e = fs::rand_fp2(st, fs::label_lit("eq"));
+    warp_sync();
+    fs::Writer st(w.st, &w.tx);
+    fp2* out = f.closing + close_eq_index(sh);
+    auto put = [&](fp2 v) {
+        st.put_fp2(v.re, v.im);
+        if (fs::lead()) *out = v;
+        ++out;
+    };
+    const fp2 e = st.rand_fp2(fs::label_lit("eq"));
     put(f2mul(f2sub(w.vs.prev, tv), e));
-    const fp2 tau = fs::rand_fp2(st, vole::tau_label(sh.layer));
+    const fp2 tau = st.rand_fp2(vole::tau_label(sh.layer));
     fp2 tag = w.vv[n];
     for (int k = n - 1; k >= 0; --k) tag = f2add(f2mul(tag, tau), w.vv[k]);
     // create_pok_final
@@ -520,24 +528,24 @@ TP_HD void step_close_tail(Work& w, const Frame& f, const Shape& sh)
         osum = f2add(osum, w.vs.out_elem[k]);
         vsum = f2add(vsum, w.vs.v_elem[k]);
     }
-    const fp2 c = fs::rand_fp2(st, fs::label_lit("pok-final"));
+    const fp2 c = st.rand_fp2(fs::label_lit("pok-final"));
     put(f2mul(osum, c));
     put(f2mul(vsum, c));
     // put(["gkr_input_point", [[re, im], ...]]): a string, then every coordinate's two ints
-    fs::put_label(st, fs::label_lit("gkr_input_point"));
+    st.put_label(fs::label_lit("gkr_input_point"));
     for (int k = 0; k < n + nb; ++k) {
         const fp2 x = k < n ? f2add(w.w[k], f2mul(f2sub(w.w[n + k], w.w[k]), tau)) : f.w3[(k - n) * f.w3_stride];
         if (fs::lead()) f.point[k] = x;
-        fs::absorb_le(st, 0x02 | (x.re << 8), 8);
-        fs::absorb_le(st, (x.re >> 56) | (0x02 << 8) | (x.im << 16), 8);
-        fs::absorb_le(st, x.im >> 48, 2);
+        st.absorb_le(0x02 | (x.re << 8), 8);
+        st.absorb_le((x.re >> 56) | (0x02 << 8) | (x.im << 16), 8);
+        st.absorb_le(x.im >> 48, 2);
     }
     // create_input_value_proof
-    const fp2 civ = fs::rand_fp2(st, fs::label_lit("input-val"));
+    const fp2 civ = st.rand_fp2(fs::label_lit("input-val"));
     put(f2mul(tag, civ));
     warp_sync();
+    st.store(w.st);
     if (!fs::lead()) return;
-    w.st = st;
     w.vs.prev = tag;
     *f.tag = tag;
 }

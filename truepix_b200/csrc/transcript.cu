@@ -73,38 +73,32 @@ bool make_device_label(const char* label, tp::fs::Label* L, const char* who)
     return true;
 }
 
-// Device transcripts: one warp (a CTA of 32 threads) per state, see transcript.cuh.
-// The kernels are bound by the latency of the hash's round chain, so a warp of its
-// own costs nothing, transcripts at different offsets do not diverge, and the two
-// digests of a draw are closed side by side.
+// Device transcripts: one warp (a CTA of 32 threads) per state, see Writer in
+// transcript.cuh. The kernels are bound by the latency of the hash's round chain, so
+// a warp of its own costs nothing and transcripts at different offsets do not diverge.
 constexpr int kFsThreads = 32;
-
-// the warp's state back to memory, once every lane has read it
-__device__ __forceinline__ void store_state(State* st, const State& s)
-{
-    __syncwarp();
-    if (tp::fs::lead()) *st = s;
-}
 
 __global__ void __launch_bounds__(kFsThreads) put_fp2s_kernel(State* __restrict__ st,
                                                               const ulonglong2* __restrict__ vals, int k)
 {
+    __shared__ tp::fs::TxMem mem;
     const int i = blockIdx.x;
-    State s = st[i];
+    tp::fs::Writer s(st[i], &mem);
     for (int j = 0; j < k; ++j) {
         const ulonglong2 v = vals[(long long)i * k + j];   // packed {re, im}
-        tp::fs::put_fp2(s, v.x, v.y);
+        s.put_fp2(v.x, v.y);
     }
-    store_state(st + i, s);
+    s.store(st[i]);
 }
 
 __global__ void __launch_bounds__(kFsThreads) rand_ext_kernel(State* __restrict__ st, tp::fs::Label L,
                                                               ulonglong2* __restrict__ out)
 {
+    __shared__ tp::fs::TxMem mem;
     const int i = blockIdx.x;
-    State s = st[i];
-    const tp::fp2 r = tp::fs::rand_fp2(s, L);
-    store_state(st + i, s);
+    tp::fs::Writer s(st[i], &mem);
+    const tp::fp2 r = s.rand_fp2(L);
+    s.store(st[i]);
     if (tp::fs::lead()) out[i] = make_ulonglong2(r.re, r.im);
 }
 
@@ -118,12 +112,13 @@ __device__ __forceinline__ tp::fp2 vole_round_frame(State* st, VoleState* vs, co
                                                     const tp::fs::Label& L, tp::fp2* proof)
 {
     using namespace tp;
+    __shared__ fs::TxMem mem;
     VoleState w = *vs;
-    State s = *st;
+    fs::Writer s(*st, &mem);
     fp2 coef[4], r;
     vole::interpolate_cubic(claims[0], claims[1], claims[2], claims[3], coef);
     vole::round(s, w, coef, 4, u, v, count, L, proof, &r);
-    store_state(st, s);
+    s.store(*st);
     if (fs::lead()) *vs = w;
     return r;
 }

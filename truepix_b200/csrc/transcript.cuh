@@ -38,9 +38,7 @@ static_assert(sizeof(State) == 120, "transcript state layout");
 // the low k bytes of a unit
 TP_HD uint64_t low_bytes(int k) { return ((uint64_t)1 << (8 * k)) - 1; }   // 0 <= k < 8
 
-// Device code runs a transcript on a whole warp: every lane holds the same state
-// and does the same work on it, except where a draw lets two lanes close two
-// digests side by side (rand_fp2). Lane 0 writes what leaves the warp.
+// Lane 0 writes what leaves a warp that runs a transcript (Writer below).
 TP_HD bool lead()
 {
 #ifdef __CUDA_ARCH__
@@ -50,24 +48,8 @@ TP_HD bool lead()
 #endif
 }
 
-#ifdef __CUDA_ARCH__
-// One compression of the 64 bytes in `unit`. Not inlined: a proof's closing steps
-// hash in dozens of places, and one copy of the rounds stays in the instruction
-// cache.
-static __device__ __noinline__ void compress_units(uint32_t* h, const uint64_t* unit)
-{
-    uint32_t st[8], w[16];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        st[i] = h[i];
-        w[2 * i] = sha::bswap32((uint32_t)unit[i]);
-        w[2 * i + 1] = sha::bswap32((uint32_t)(unit[i] >> 32));
-    }
-    sha::compress_compact<true>(st, w, sha::kShaTables.k, sha::AddMad{sha::kShaOne});
-#pragma unroll
-    for (int i = 0; i < 8; ++i) h[i] = st[i];
-}
-#else
+// ---- the state's operations (host) ----------------------------------------------
+
 inline void compress_units(uint32_t* h, const uint64_t* unit)
 {
     uint32_t w[16];
@@ -77,14 +59,10 @@ inline void compress_units(uint32_t* h, const uint64_t* unit)
     }
     sha::compress(h, w, sha::AddAlu{});
 }
-#endif
 
-// The low `bytes` bytes of v (1 <= bytes <= 8), least significant first: one or
-// two 8-byte units are updated, not byte by byte (the byte-wise form, its buffer
-// indexed dynamically, took ten times as long as the compressions: a committed
-// round of a batch 146 us against 13 us here). Bytes behind the pending ones keep
-// what they held.
-TP_HD void absorb_le(State& s, uint64_t v, int bytes)
+// The low `bytes` bytes of v (1 <= bytes <= 8), least significant first. Bytes
+// behind the pending ones keep what they held.
+inline void absorb_le(State& s, uint64_t v, int bytes)
 {
     const uint64_t all = bytes < 8 ? low_bytes(bytes) : ~(uint64_t)0;
     const int q = (int)(s.nbuf >> 3), r = (int)(s.nbuf & 7);
@@ -104,19 +82,17 @@ TP_HD void absorb_le(State& s, uint64_t v, int bytes)
 }
 
 // one byte into the running hash
-TP_HD void absorb_byte(State& s, uint8_t b) { absorb_le(s, b, 1); }
+inline void absorb_byte(State& s, uint8_t b) { absorb_le(s, b, 1); }
 
 // bytes from memory (the host entry points' caller-owned data)
-TP_HD void absorb(State& s, const uint8_t* p, uint64_t n)
+inline void absorb(State& s, const uint8_t* p, uint64_t n)
 {
     for (uint64_t i = 0; i < n; ++i) absorb_byte(s, p[i]);
 }
 
 // A label of at most 32 bytes held by value in four 64-bit words (byte i in
-// bits 8 (i mod 8) of word i / 8). Device code builds, passes and absorbs labels
-// only in this form: no pointer to a local byte array is handed to the inlined
-// hash code (on sm_100a such a pointer, passed down through the fully inlined
-// draw, was observed to read the wrong bytes).
+// bits 8 (i mod 8) of word i / 8): device code builds, passes and absorbs labels
+// only in this form.
 struct Label {
     uint64_t w0, w1, w2, w3;
     uint32_t len;
@@ -167,7 +143,7 @@ TP_HD void label_decimal(Label& L, long long v)
     }
 }
 
-TP_HD void init(State& s)
+inline void init(State& s)
 {
     sha::init(s.h);
     s.nbuf = 0;
@@ -177,21 +153,21 @@ TP_HD void init(State& s)
 }
 
 // put(list of ints), every value below 2^64 (the reference's array('Q') path)
-TP_HD void put_u64s(State& s, const uint64_t* v, uint64_t n)
+inline void put_u64s(State& s, const uint64_t* v, uint64_t n)
 {
     absorb_byte(s, 0x01);
     absorb_le(s, n, 4);
     for (uint64_t i = 0; i < n; ++i) absorb_le(s, v[i], 8);
 }
 
-TP_HD void put_fp2(State& s, uint64_t re, uint64_t im)
+inline void put_fp2(State& s, uint64_t re, uint64_t im)
 {
     absorb_le(s, 0x03 | (re << 8), 8);
     absorb_le(s, (re >> 56) | (im << 8), 8);
     absorb_le(s, im >> 56, 1);
 }
 
-TP_HD void put_str(State& s, const uint8_t* p, uint32_t len)
+inline void put_str(State& s, const uint8_t* p, uint32_t len)
 {
     absorb_byte(s, 0x04);
     absorb_le(s, len, 4);
@@ -199,11 +175,10 @@ TP_HD void put_str(State& s, const uint8_t* p, uint32_t len)
 }
 
 // put(str) of a label held by value
-TP_HD void put_label(State& s, const Label& L)
+inline void put_label(State& s, const Label& L)
 {
     absorb_le(s, 0x04 | ((uint64_t)L.len << 8), 5);
     const uint64_t w[4] = {L.w0, L.w1, L.w2, L.w3};
-#pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int left = (int)L.len - 8 * i;
         if (left > 0) absorb_le(s, w[i], left < 8 ? left : 8);
@@ -212,10 +187,9 @@ TP_HD void put_label(State& s, const Label& L)
 
 // The chaining words after the SHA-256 padding: the digest of everything
 // absorbed so far. The running state is unchanged.
-TP_HD void digest_words(const State& s, uint32_t h[8])
+inline void digest_words(const State& s, uint32_t h[8])
 {
     uint64_t u[8];
-#pragma unroll
     for (int i = 0; i < 8; ++i) {
         h[i] = s.h[i];
         const int k = (int)s.nbuf - 8 * i;   // pending bytes in this unit and behind it
@@ -223,7 +197,6 @@ TP_HD void digest_words(const State& s, uint32_t h[8])
     }
     if (s.nbuf >= 56) {   // no room for the length
         compress_units(h, u);
-#pragma unroll
         for (int i = 0; i < 8; ++i) u[i] = 0;
     }
     const uint64_t bits = s.total * 8;   // big-endian in the last eight bytes
@@ -232,7 +205,7 @@ TP_HD void digest_words(const State& s, uint32_t h[8])
 }
 
 // the digest bytes (big-endian words)
-TP_HD void digest(const State& s, uint8_t out[32])
+inline void digest(const State& s, uint8_t out[32])
 {
     uint32_t h[8];
     digest_words(s, h);
@@ -245,7 +218,7 @@ TP_HD void digest(const State& s, uint8_t out[32])
 }
 
 // put([rnum]): a one-int list of the counter, which then moves on
-TP_HD void put_counter(State& s)
+inline void put_counter(State& s)
 {
     absorb_le(s, 0x01 | (1ull << 8) | (s.rnum << 40), 8);
     absorb_le(s, s.rnum >> 24, 5);
@@ -253,7 +226,7 @@ TP_HD void put_counter(State& s)
 }
 
 // the low 61 bits of the big-endian digest (its last two words)
-TP_HD uint64_t draw_bits(const State& s)
+inline uint64_t draw_bits(const State& s)
 {
     uint32_t h[8];
     digest_words(s, h);
@@ -262,7 +235,7 @@ TP_HD uint64_t draw_bits(const State& s)
 
 // A draw is redrawn only when its 61 bits are all ones (probability 2^-61); the
 // loop is bounded all the same, and past the bound returns the value reduced.
-TP_HD uint64_t rand_scalar(State& s)
+inline uint64_t rand_scalar(State& s)
 {
     uint64_t v = 0;
     for (int it = 0; it < 1000; ++it) {
@@ -275,7 +248,7 @@ TP_HD uint64_t rand_scalar(State& s)
 
 // rand_ext(label) as an Fp2: "ext", label, "real" -> the real limb; "ext",
 // label, "imag" -> the imaginary limb
-TP_HD fp2 rand_fp2_serial(State& s, const Label& L)
+inline fp2 rand_fp2(State& s, const Label& L)
 {
     const Label ext = label_lit("ext"), real = label_lit("real"), imag = label_lit("imag");
     put_label(s, ext);
@@ -289,35 +262,8 @@ TP_HD fp2 rand_fp2_serial(State& s, const Label& L)
     return mk(re, im);
 }
 
-#ifdef __CUDA_ARCH__
-// The same draw on a warp whose lanes hold the same state. The real limb's value
-// does not enter the transcript, so the state runs on to the imaginary limb's
-// draw at once and the two digests are closed by an even and an odd lane in the
-// same instructions. All-ones values (probability 2^-60) redraw one after the other.
-static __device__ __noinline__ fp2 rand_fp2(State& s, const Label& L)
-{
-    State both[2];   // at the real limb's draw, at the imaginary limb's
-    const State s0 = s;
-    const Label ext = label_lit("ext");
-    for (int q = 0; q < 2; ++q) {
-        put_label(s, ext);
-        put_label(s, L);
-        put_label(s, q ? label_lit("imag") : label_lit("real"));
-        put_counter(s);
-        both[q] = s;
-    }
-    const uint64_t v = draw_bits(both[threadIdx.x & 1]);
-    const uint64_t re = __shfl_sync(0xffffffffu, v, 0), im = __shfl_sync(0xffffffffu, v, 1);
-    if (re < P61 && im < P61) return mk(re, im);
-    s = s0;
-    return rand_fp2_serial(s, L);
-}
-#else
-inline fp2 rand_fp2(State& s, const Label& L) { return rand_fp2_serial(s, L); }
-#endif
-
 // the same draw with a label in memory (host entry points: labels of any length)
-TP_HD void rand_ext(State& s, const uint8_t* label, uint32_t len, uint64_t* re, uint64_t* im)
+inline void rand_ext(State& s, const uint8_t* label, uint32_t len, uint64_t* re, uint64_t* im)
 {
     const Label ext = label_lit("ext"), real = label_lit("real"), imag = label_lit("imag");
     put_label(s, ext);
@@ -329,6 +275,279 @@ TP_HD void rand_ext(State& s, const uint8_t* label, uint32_t len, uint64_t* re, 
     put_label(s, imag);
     *im = rand_scalar(s);
 }
+
+// ---- a transcript at work ---------------------------------------------------------
+// Writer runs a state: opened from it, put to and drawn from, stored back to it. The
+// host form is the state itself.
+//
+// On the device a warp runs it: every lane makes the same calls. What is put gathers
+// in shared memory (TxMem) without being hashed; a draw hashes the whole stretch at
+// once. The message words of all its blocks are known by then, so their schedules
+// are made side by side, one lane per block, and the rounds run on k + w from shared
+// memory: 31 cycles a round against 49 with the schedule in line. The real limb of a
+// draw does not enter the transcript, so the stretch runs on to the imaginary limb's
+// draw and an even and an odd lane close the two digests in the same instructions,
+// each with its own padding. Per committed round (243 bytes, two draws): ~5.6
+// compressions' rounds one after the other and two schedules, 11 us; a thread that
+// appended byte by byte and hashed block by block took 146 us.
+
+constexpr int kTxUnits = 72;     // 8-byte units a stretch may hold (9 blocks)
+constexpr int kTxBlocks = 8;     // blocks hashed at once, padding included
+
+struct TxMem {
+    uint64_t buf[kTxUnits];      // the stretch, from the pending block's first byte
+    uint64_t prev[8];            // the block before it (what a state holds behind its pending bytes)
+    uint32_t h[8], h_next[8];    // chaining words in front of the stretch; behind its last whole block
+    uint64_t out[2];             // the two digests' low 61 bits
+    __align__(16) uint32_t kw[2 * kTxBlocks][68];   // k + w of block b as digest v closes it: row 2 b + v
+};
+
+#ifdef __CUDACC__
+#ifdef __CUDA_ARCH__
+// Hash the stretch's bytes: digest v (the lanes of parity v) closes after its first
+// n_v bytes, total_v bytes into the transcript; with close unset only its whole
+// blocks are taken. m->h_next: the chaining words behind the whole blocks of n_1.
+static __device__ __noinline__ void tx_hash(TxMem* m, uint32_t n0, uint32_t n1, uint64_t total1, bool close)
+{
+    const uint32_t lane = threadIdx.x & 31, v = lane & 1;
+    const int n = (int)(v ? n1 : n0), whole = n >> 6;
+    const int blocks = close ? whole + ((n & 63) >= 56 ? 2 : 1) : whole;
+    const sha::AddMad add{sha::kShaOne};
+    __syncwarp();
+    {
+        const int b = (int)(lane >> 1);
+        if (b < blocks) {
+            uint32_t w[16];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int k = n - 64 * b - 8 * i;   // bytes of this unit and behind it
+                uint64_t u = m->buf[8 * min(b, kTxUnits / 8 - 1) + i];
+                if (k < 8) u = k > 0 ? (u & low_bytes(k)) | ((uint64_t)0x80 << (8 * k)) : k == 0 ? 0x80 : 0;
+                w[2 * i] = sha::bswap32((uint32_t)u);
+                w[2 * i + 1] = sha::bswap32((uint32_t)(u >> 32));
+            }
+            if (close && b == blocks - 1) {
+                const uint64_t bits = 8 * (total1 - (n1 - (uint32_t)n));
+                w[14] = (uint32_t)(bits >> 32);
+                w[15] = (uint32_t)bits;
+            }
+            uint32_t* kw = m->kw[lane];
+#pragma unroll 1
+            for (int i = 0; i < 48; i += 16)
+#pragma unroll
+                for (int t = 0; t < 16; ++t) {
+                    kw[i + t] = add(w[t], sha::kShaTables.k[i + t]);
+                    const uint32_t x = w[(t + 1) & 15], y = w[(t + 14) & 15];
+                    w[t] = add(sha::rotr(y, 17) ^ sha::rotr(y, 19) ^ (y >> 10),
+                               add(sha::rotr(x, 7) ^ sha::rotr(x, 18) ^ (x >> 3), add(w[t], w[(t + 9) & 15])));
+                }
+#pragma unroll
+            for (int t = 0; t < 16; ++t) kw[48 + t] = add(w[t], sha::kShaTables.k[48 + t]);
+        }
+    }
+    __syncwarp();
+    uint32_t st[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) st[i] = m->h[i];
+#pragma unroll 1
+    for (int b = 0; b < blocks; ++b) {
+        if (b == whole && lane == 1)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) m->h_next[i] = st[i];
+        const uint4* kw = reinterpret_cast<const uint4*>(m->kw[2 * b + v]);
+        uint32_t s[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) s[i] = st[i];
+#pragma unroll 1
+        for (int i = 0; i < 16; i += 4) {
+            uint32_t k[16];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint4 x = kw[i + q];
+                k[4 * q] = x.x;
+                k[4 * q + 1] = x.y;
+                k[4 * q + 2] = x.z;
+                k[4 * q + 3] = x.w;
+            }
+#pragma unroll
+            for (int t = 0; t < 16; ++t)
+                sha::round_step(s[(0 - t) & 7], s[(1 - t) & 7], s[(2 - t) & 7], s[(3 - t) & 7], s[(4 - t) & 7],
+                                s[(5 - t) & 7], s[(6 - t) & 7], s[(7 - t) & 7], k[t], add);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) st[i] = add(st[i], s[i]);
+    }
+    if (!close && lane == 1)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) m->h_next[i] = st[i];
+    if (lane < 2) m->out[lane] = (((uint64_t)st[6] << 32) | st[7]) & P61;
+    __syncwarp();
+}
+
+// the whole blocks of the stretch's n bytes are hashed (m->h_next): the rest to its front
+static __device__ __noinline__ void tx_advance(TxMem* m, uint32_t n)
+{
+    const uint32_t lane = threadIdx.x & 31, whole = n >> 6;
+    uint64_t p = 0, u = 0;
+    if (whole && lane < 8) {
+        p = m->buf[8 * (whole - 1) + lane];
+        u = m->buf[8 * whole + lane];
+    }
+    const uint32_t h = m->h_next[lane & 7];
+    __syncwarp();
+    if (whole && lane < 8) {
+        m->prev[lane] = p;
+        m->buf[lane] = u;
+        m->h[lane] = h;
+    }
+    __syncwarp();
+}
+
+class Writer {
+public:
+    __device__ Writer(const State& s, TxMem* mem) : m(mem), total(s.total), rnum(s.rnum), n(s.nbuf)
+    {
+        const uint32_t lane = threadIdx.x & 31;
+        cur = n & 7 ? s.unit[n >> 3] & low_bytes(n & 7) : 0;
+        __syncwarp();
+        if (lane < 8) {
+            m->buf[lane] = m->prev[lane] = s.unit[lane];
+            m->h[lane] = s.h[lane];
+        }
+        __syncwarp();
+    }
+    __device__ void absorb_le(uint64_t v, int bytes)
+    {
+        if (bytes < 8) v &= low_bytes(bytes);
+        const int r = (int)(n & 7);
+        cur |= v << (8 * r);
+        total += (uint64_t)bytes;
+        n += (uint32_t)bytes;
+        if (r + bytes >= 8) {
+            if (lead()) m->buf[(n >> 3) - 1] = cur;
+            cur = r ? v >> (8 * (8 - r)) : 0;
+            if (n >= 64 * (kTxBlocks - 1)) take_whole();
+        }
+    }
+    __device__ void put_fp2(uint64_t re, uint64_t im)
+    {
+        absorb_le(0x03 | (re << 8), 8);
+        absorb_le((re >> 56) | (im << 8), 8);
+        absorb_le(im >> 56, 1);
+    }
+    __device__ void put_label(const Label& L)
+    {
+        absorb_le(0x04 | ((uint64_t)L.len << 8), 5);
+        const uint64_t w[4] = {L.w0, L.w1, L.w2, L.w3};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int left = (int)L.len - 8 * i;
+            if (left > 0) absorb_le(w[i], left < 8 ? left : 8);
+        }
+    }
+    // rand_ext(label)
+    __device__ fp2 rand_fp2(const Label& L)
+    {
+        if (n > 256) take_whole();   // a draw puts at most 134 bytes, its padding at most 72
+        const uint32_t n_start = n;
+        const uint64_t total_start = total, rnum_start = rnum;
+        part(L, label_lit("real"));
+        put_counter();
+        const uint32_t n_real = n;
+        part(L, label_lit("imag"));
+        put_counter();
+        if (lead()) m->buf[n >> 3] = cur;
+        tx_hash(m, n_real, n, total, true);
+        uint64_t re = m->out[0], im = m->out[1];
+        if (re < P61 && im < P61) {
+            tx_advance(m, n);
+            n &= 63;
+            return mk(re, im);
+        }
+        // a limb of all ones is drawn again (probability 2^-60): one after the other
+        n = n_start;
+        total = total_start;
+        rnum = rnum_start;
+        cur = n & 7 ? m->buf[n >> 3] & low_bytes(n & 7) : 0;
+        part(L, label_lit("real"));
+        re = scalar();
+        part(L, label_lit("imag"));
+        im = scalar();
+        return mk(re, im);
+    }
+    // the state at this point back to s (lanes 0..7 write)
+    __device__ void store(State& s)
+    {
+        if (n >= 64) take_whole();
+        const uint32_t lane = threadIdx.x & 31;
+        if (lead()) m->buf[n >> 3] = cur;
+        __syncwarp();
+        if (lane < 8) {
+            const int k = (int)n - 8 * (int)lane;
+            const uint64_t mask = k >= 8 ? ~(uint64_t)0 : k > 0 ? low_bytes(k) : 0;
+            s.unit[lane] = (m->buf[lane] & mask) | (m->prev[lane] & ~mask);
+            s.h[lane] = m->h[lane];
+        }
+        if (lead()) {
+            s.total = total;
+            s.rnum = rnum;
+            s.nbuf = n;
+        }
+        __syncwarp();
+    }
+
+private:
+    __device__ void part(const Label& L, const Label& limb)
+    {
+        put_label(label_lit("ext"));
+        put_label(L);
+        put_label(limb);
+    }
+    __device__ void put_counter()
+    {
+        absorb_le(0x01 | (1ull << 8) | (rnum << 40), 8);
+        absorb_le(rnum >> 24, 5);
+        rnum += 1;
+    }
+    __device__ void take_whole()
+    {
+        tx_hash(m, n, n, total, false);
+        tx_advance(m, n);
+        n &= 63;
+    }
+    __device__ uint64_t scalar()
+    {
+        uint64_t v = 0;
+        for (int it = 0; it < 1000; ++it) {
+            put_counter();
+            if (lead()) m->buf[n >> 3] = cur;
+            tx_hash(m, n, n, total, true);
+            v = m->out[1];
+            tx_advance(m, n);
+            n &= 63;
+            if (v < P61) return v;
+        }
+        return v % P61;
+    }
+    TxMem* m;
+    uint64_t total, rnum, cur;   // cur: the unit that is not full yet
+    uint32_t n;                  // bytes of the stretch
+};
+#else
+class Writer {
+public:
+    Writer(const State& state, TxMem*) : s(state) {}
+    void absorb_le(uint64_t v, int bytes) { fs::absorb_le(s, v, bytes); }
+    void put_fp2(uint64_t re, uint64_t im) { fs::put_fp2(s, re, im); }
+    void put_label(const Label& L) { fs::put_label(s, L); }
+    fp2 rand_fp2(const Label& L) { return fs::rand_fp2(s, L); }
+    void store(State& out) { out = s; }
+
+private:
+    State s;
+};
+#endif
+#endif
 
 }  // namespace fs
 }  // namespace tp

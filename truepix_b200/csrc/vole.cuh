@@ -88,7 +88,9 @@ TP_HD fp2 commit(State& w, fp2 m, const fp2* u, const fp2* v, fp2* tag)
 // frame's correlations u, v (count entries). Returns false, sets w.bad and
 // leaves the transcript untouched when fewer than n_coef correlations remain.
 // proof (optional): the n_coef values d, then the equality value.
-TP_HD bool round(fs::State& s, State& w, const fp2* c, int n_coef, const fp2* u, const fp2* v, long long count,
+#pragma nv_exec_check_disable
+template <class Tx>
+TP_HD bool round(Tx& s, State& w, const fp2* c, int n_coef, const fp2* u, const fp2* v, long long count,
                  const fs::Label& label, fp2* proof, fp2* r_out)
 {
     if (w.bad || w.idx + (unsigned long long)n_coef > (unsigned long long)count) {
@@ -107,16 +109,16 @@ TP_HD bool round(fs::State& s, State& w, const fp2* c, int n_coef, const fp2* u,
     }
     w.idx += (unsigned long long)n_coef;
     for (int k = 0; k < n_coef; ++k) {
-        fs::put_fp2(s, dm[k].re, dm[k].im);
+        s.put_fp2(dm[k].re, dm[k].im);
         if (proof && fs::lead()) proof[k] = dm[k];
     }
     fp2 now = tag[0];
     for (int k = 0; k < n_coef; ++k) now = f2add(now, tag[k]);
-    const fp2 e = fs::rand_fp2(s, fs::label_lit("eq"));
+    const fp2 e = s.rand_fp2(fs::label_lit("eq"));
     const fp2 vz = w.has_prev ? f2mul(f2sub(w.prev, now), e) : f2mul(now, e);
-    fs::put_fp2(s, vz.re, vz.im);
+    s.put_fp2(vz.re, vz.im);
     if (proof && fs::lead()) proof[n_coef] = vz;
-    const fp2 r = fs::rand_fp2(s, label);
+    const fp2 r = s.rand_fp2(label);
     fp2 p = tag[n_coef - 1];
     for (int k = n_coef - 2; k >= 0; --k) p = f2add(f2mul(p, r), tag[k]);
     w.prev = p;
