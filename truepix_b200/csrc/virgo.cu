@@ -16,6 +16,8 @@
 #include <type_traits>
 #include <vector>
 
+#include <cooperative_groups.h>
+
 #include "fp2.cuh"
 #include "runtime.h"
 #include "virgo.h"
@@ -62,6 +64,117 @@ __device__ __forceinline__ fp2 shfl_down2(fp2 v, int o)
     return w;
 }
 
+// The CTA's sum of (qa, qb, qc), valid on thread 0 (canonical on return there). The
+// nine 64-bit adds and shuffles of a butterfly over six limbs a step stay small
+// beside the entry's nine multiplications.
+__device__ __forceinline__ void cta_sum3(fp2& qa, fp2& qb, fp2& qc, fp2 (*red)[3])
+{
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        qa = l2add(qa, shfl_down2(qa, o));
+        qb = l2add(qb, shfl_down2(qb, o));
+        qc = l2add(qc, shfl_down2(qc, o));
+    }
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (lane == 0) {
+        red[w][0] = qa;
+        red[w][1] = qb;
+        red[w][2] = qc;
+    }
+    __syncthreads();
+    if (w == 0) {
+        const bool in = lane < (int)(blockDim.x >> 5);
+        qa = in ? red[lane][0] : f2zero();
+        qb = in ? red[lane][1] : f2zero();
+        qc = in ? red[lane][2] : f2zero();
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            qa = l2add(qa, shfl_down2(qa, o));
+            qb = l2add(qb, shfl_down2(qb, o));
+            qc = l2add(qc, shfl_down2(qc, o));
+        }
+    }
+}
+
+__device__ __forceinline__ void update_entry(const ulonglong2* __restrict__ vma, const ulonglong2* __restrict__ addv,
+                                             const ulonglong2* __restrict__ ams, long long i, fp2 r, bool bit,
+                                             ulonglong2* __restrict__ vma_out, ulonglong2* __restrict__ addv_out,
+                                             ulonglong2* __restrict__ ams_out, fp2& qa, fp2& qb, fp2& qc)
+{
+    const LP v = fold(vma, i, r, bit), a = fold(addv, i, r, bit), m = fold(ams, i, r, bit);
+    st_lp(vma_out, i, v);
+    st_lp(addv_out, i, a);
+    st_lp(ams_out, i, m);
+    qa = l2add(qa, l2mul(m.a, v.a));
+    qb = l2add(qb, l2add(l2add(l2mul(m.a, v.b), l2mul(m.b, v.a)), a.a));
+    qc = l2add(qc, l2add(l2mul(m.b, v.b), a.b));
+}
+
+__device__ __forceinline__ void store_poly(ulonglong2* ret, fp2 qa, fp2 qb, fp2 qc)
+{
+    const fp2 a = l2canon(qa), b = l2canon(qb), c = l2canon(qc);
+    ret[0] = make_ulonglong2(a.im, a.re);
+    ret[1] = make_ulonglong2(b.im, b.re);
+    ret[2] = make_ulonglong2(c.im, c.re);
+}
+
+// Tables of up to 2,048 folded entries: one cluster of up to eight CTAs, a thread an
+// entry, the CTAs' sums added in the first one's shared memory: no partial sums in
+// memory, no ticket to clear. A round of so few entries is launch latency: 10.6 us
+// with the cleared ticket and the grid's sum added up by three threads, 6.5 us so.
+constexpr int kClusterMax = 8, kSmall = kClusterMax * kThreads;
+
+__global__ void __launch_bounds__(kThreads) update_small_kernel(const ulonglong2* __restrict__ vma,
+                                                                const ulonglong2* __restrict__ addv,
+                                                                const ulonglong2* __restrict__ ams, int half, fp2 r,
+                                                                int bit, ulonglong2* __restrict__ vma_out,
+                                                                ulonglong2* __restrict__ addv_out,
+                                                                ulonglong2* __restrict__ ams_out,
+                                                                ulonglong2* __restrict__ ret)
+{
+    namespace cg = cooperative_groups;
+    __shared__ fp2 red[kThreads / 32][3];
+    __shared__ fp2 sums[kClusterMax][3];
+    const cg::cluster_group cluster = cg::this_cluster();
+    fp2 qa = f2zero(), qb = f2zero(), qc = f2zero();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < half) update_entry(vma, addv, ams, i, r, bit, vma_out, addv_out, ams_out, qa, qb, qc);
+    cta_sum3(qa, qb, qc, red);
+    if (threadIdx.x == 0) {
+        fp2* to = cluster.map_shared_rank(&sums[blockIdx.x][0], 0);
+        to[0] = qa;
+        to[1] = qb;
+        to[2] = qc;
+    }
+    cluster.sync();
+    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+    for (unsigned k = 1; k < gridDim.x; ++k) {
+        qa = l2add(qa, sums[k][0]);
+        qb = l2add(qb, sums[k][1]);
+        qc = l2add(qc, sums[k][2]);
+    }
+    store_poly(ret, qa, qb, qc);
+}
+
+bool launch_small(const ulonglong2* vma, const ulonglong2* addv, const ulonglong2* ams, int half, fp2 r, int bit,
+                  ulonglong2* vma_out, ulonglong2* addv_out, ulonglong2* ams_out, ulonglong2* ret, cudaStream_t s)
+{
+    cudaLaunchConfig_t cfg = {};
+    const unsigned blocks = (unsigned)((half + kThreads - 1) / kThreads);
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(blocks > 1 ? kThreads : (unsigned)((half + 31) / 32 * 32));
+    cfg.stream = s;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = blocks;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return !cuda_failed(cudaLaunchKernelEx(&cfg, update_small_kernel, vma, addv, ams, half, r, bit, vma_out, addv_out,
+                                           ams_out, ret),
+                        "virgo update");
+}
+
 __global__ void __launch_bounds__(kThreads) update_kernel(const ulonglong2* __restrict__ vma,
                                                           const ulonglong2* __restrict__ addv,
                                                           const ulonglong2* __restrict__ ams, long long half,
@@ -71,53 +184,35 @@ __global__ void __launch_bounds__(kThreads) update_kernel(const ulonglong2* __re
                                                           unsigned* __restrict__ ticket,
                                                           ulonglong2* __restrict__ ret)
 {
-    __shared__ fp2 red[3][kThreads / 32];
+    __shared__ fp2 red[kThreads / 32][3];
     __shared__ bool last;
     fp2 qa = f2zero(), qb = f2zero(), qc = f2zero();
     const long long stride = (long long)gridDim.x * kThreads;
-    for (long long i = (long long)blockIdx.x * kThreads + threadIdx.x; i < half; i += stride) {
-        const LP v = fold(vma, i, r, bit), a = fold(addv, i, r, bit), m = fold(ams, i, r, bit);
-        st_lp(vma_out, i, v);
-        st_lp(addv_out, i, a);
-        st_lp(ams_out, i, m);
-        qa = l2add(qa, l2mul(m.a, v.a));
-        qb = l2add(qb, l2add(l2add(l2mul(m.a, v.b), l2mul(m.b, v.a)), a.a));
-        qc = l2add(qc, l2add(l2mul(m.b, v.b), a.b));
-    }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-        qa = l2add(qa, shfl_down2(qa, o));
-        qb = l2add(qb, shfl_down2(qb, o));
-        qc = l2add(qc, shfl_down2(qc, o));
-    }
-    const int w = threadIdx.x >> 5;
-    if ((threadIdx.x & 31) == 0) {
-        red[0][w] = qa;
-        red[1][w] = qb;
-        red[2][w] = qc;
-    }
-    __syncthreads();
-    if (threadIdx.x < 3) {
-        fp2 s = f2zero();
-        for (int k = 0; k < kThreads / 32; ++k) s = l2add(s, red[threadIdx.x][k]);
-        part[3 * blockIdx.x + threadIdx.x] = s;
-    }
-    __syncthreads();
+    for (long long i = (long long)blockIdx.x * kThreads + threadIdx.x; i < half; i += stride)
+        update_entry(vma, addv, ams, i, r, bit, vma_out, addv_out, ams_out, qa, qb, qc);
+    cta_sum3(qa, qb, qc, red);
     if (threadIdx.x == 0) {
+        fp2* p = part + 3 * blockIdx.x;
+        p[0] = qa;
+        p[1] = qb;
+        p[2] = qc;
         __threadfence();
         last = atomicAdd(ticket, 1u) == gridDim.x - 1;
     }
     __syncthreads();
-    if (last && threadIdx.x < 3) {
-        __threadfence();
-        const volatile u64* pv = reinterpret_cast<const volatile u64*>(part);
-        fp2 s = f2zero();
-        for (unsigned b = 0; b < gridDim.x; ++b)
-            s = l2add(s, mk(pv[2 * (3 * b + threadIdx.x)], pv[2 * (3 * b + threadIdx.x) + 1]));
-        s = l2canon(s);
-        ret[threadIdx.x] = make_ulonglong2(s.im, s.re);
-        if (threadIdx.x == 0) *ticket = 0;
+    if (!last) return;
+    // the last CTA adds the CTAs' sums, all threads taking part
+    __threadfence();
+    qa = qb = qc = f2zero();
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += kThreads) {
+        const ulonglong2* p = reinterpret_cast<const ulonglong2*>(part + 3 * b);
+        const ulonglong2 x = __ldcg(p), y = __ldcg(p + 1), z = __ldcg(p + 2);
+        qa = l2add(qa, mk(x.x, x.y));
+        qb = l2add(qb, mk(y.x, y.y));
+        qc = l2add(qc, mk(z.x, z.y));
     }
+    cta_sum3(qa, qb, qc, red);
+    if (threadIdx.x == 0) store_poly(ret, qa, qb, qc);
 }
 
 }  // namespace
@@ -136,6 +231,12 @@ bool update(const ulonglong2* vma, const ulonglong2* addv, const ulonglong2* ams
         return false;
     }
     const long long half = n / 2;
+    if (half <= kSmall) {
+        timer_begin(s, 9300);
+        const bool done = launch_small(vma, addv, ams, (int)half, r, bit ? 1 : 0, vma_out, addv_out, ams_out, ret, s);
+        timer_end(s);
+        return done;
+    }
     const long long want = (half + kThreads - 1) / kThreads;
     const unsigned blocks = (unsigned)std::min<long long>(want, (long long)c->n_sm * 8);
     fp2* part = static_cast<fp2*>(dev_alloc(sizeof(fp2) * 3 * blocks + 256, s));
@@ -304,11 +405,20 @@ __global__ void __launch_bounds__(kThreads) phase2_sum_kernel(Layer L, HalfEq g0
         last = atomicAdd(ticket, 1u) == gridDim.x - 1;
     }
     __syncthreads();
-    if (last && threadIdx.x == 0) {
-        __threadfence();
-        const volatile u64* pv = reinterpret_cast<const volatile u64*>(part);
+    if (!last) return;
+    __threadfence();
+    acc = f2zero();
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += kThreads) {
+        const ulonglong2 x = __ldcg(reinterpret_cast<const ulonglong2*>(part + b));
+        acc = l2add(acc, mk(x.x, x.y));
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) acc = l2add(acc, shfl_down2(acc, o));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
         fp2 sum = ld_fe(addv + 1);
-        for (unsigned b = 0; b < gridDim.x; ++b) sum = l2add(sum, mk(pv[2 * b], pv[2 * b + 1]));
+        for (int k = 0; k < kThreads / 32; ++k) sum = l2add(sum, red[k]);
         sum = l2canon(sum);
         addv[1] = make_ulonglong2(sum.im, sum.re);
         *ticket = 0;
