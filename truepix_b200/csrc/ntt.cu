@@ -23,7 +23,6 @@ struct Tables {
     fp2* lo = nullptr;
     fp2* hi = nullptr;
     int h = 0;
-    int quarter = 0;   // w^(n/4) = +i (1) or -i (-1); 0 for n < 4
 };
 
 std::mutex g_mu;
@@ -39,7 +38,6 @@ struct Pass {
     int n_dig;                        // last pass: the earlier digits
     int dig_bits[3];
     int dig_shift[3];
-    int quarter;                      // w_R^(R/4) = +i (1) or -i (-1)
 };
 
 __device__ __forceinline__ fp2 ld_fe(const ulonglong2* p) { const ulonglong2 v = *p; return mk(v.y, v.x); }
@@ -60,22 +58,93 @@ __device__ __forceinline__ int bitrev(int j, int bits) { return bits ? (int)(__b
 // distinct banks.
 __device__ __forceinline__ int at(int r, int c, int log_g) { return (r << log_g) + c + (r >> 3); }
 
-// y * (+i) or y * (-i): the 4th root of unity of the pass, by a swap and a negation
-__device__ __forceinline__ fp2 times_quarter(fp2 y, int quarter)
+// ---- a stage group in registers ---------------------------------------------------
+// K consecutive radix-2 stages lh0 .. lh0 + K - 1: a work item is one column and the
+// 2^K rows base + m 2^lh0 (m < 2^K) that these stages combine. Their twiddles are
+// w_(2^(lh0+j+1))^lo for the stage times a power of the 2^(j+1)-th root; the first
+// factor is taken out of the butterflies: row m is multiplied by T^rev(m), T =
+// w_(2^(lh0+K))^lo, up front (7 multiplications for 8 rows, none in the first group,
+// where lo = 0), and what is left is a plain 2^K-point DFT. Up to 8 points that needs
+// no multiplication in this field: the 4th root is -i (forward; +i inverse) and the
+// 8th 2^30 (1 -+ i), since 2^61 = 1 makes 2^30 = 2^(-31) a square root of 1/2, so
+// they are swaps, negations and rotations by 30 bits. (12 multiplications per 8 rows
+// and group before, two in the first: 2^20 points 47.4 -> see ntt.h.)
+//
+// Bounds: rows come in below 2^61 + 8. The first two levels are left unreduced
+// (differences add 2p, then 4p, and stay below 2^64), folded, and the third level's
+// sums folded again.
+
+// a + w b and a - w b, w = the 4th root; b below 4 p
+template <bool INV>
+__device__ __forceinline__ void quarter_pair(fp2 a, fp2 b, fp2& sum, fp2& diff)
 {
-    return quarter > 0 ? mk(lsub(0, y.im), y.re) : mk(y.im, lsub(0, y.re));
+    const fp2 u = mk(a.re + b.im, a.im + (4 * P61 - b.re));   // a - i b
+    const fp2 v = mk(a.re + (4 * P61 - b.im), a.im + b.re);   // a + i b
+    sum = INV ? v : u;
+    diff = INV ? u : v;
+}
+__device__ __forceinline__ fp2 fold2(fp2 a) { return mk(fold61(a.re), fold61(a.im)); }
+__device__ __forceinline__ u64 rot30(u64 x) { return ((x << 30) & P61) + (x >> 31); }   // x < 2^63 -> < 2^61 + 2^32
+// y w8 and y w8^3 for y below 2^61 + 8
+template <bool INV>
+__device__ __forceinline__ fp2 times_w8(fp2 y)
+{
+    const u64 s = y.re + y.im, d = y.re + (2 * P61 - y.im), e = y.im + (2 * P61 - y.re);
+    return INV ? mk(rot30(d), rot30(s)) : mk(rot30(s), rot30(e));
+}
+template <bool INV>
+__device__ __forceinline__ fp2 times_w8_3(fp2 y)
+{
+    const u64 s = y.re + y.im, n = 4 * P61 - s, d = y.re + (2 * P61 - y.im), e = y.im + (2 * P61 - y.re);
+    return INV ? mk(rot30(n), rot30(d)) : mk(rot30(e), rot30(n));
 }
 
-// K consecutive radix-2 stages lh0 .. lh0 + K - 1 in registers: a work item is one
-// column and the 2^K rows base + m 2^lh0 (m < 2^K) that these stages combine.
-// The butterfly of stage lh on rows (u, u + 2^lh) uses w_R^(pin R / 2^(lh+1)),
-// pin = u mod 2^lh; FIRST (lh0 = 0) makes every pin a compile-time constant, so
-// the multiplications by w^0 = 1 vanish and those by w_R^(R/4) = +-i become a
-// swap and a negation.
-template <int K, bool FIRST>
-__device__ __forceinline__ void stage_group(fp2* sm, const fp2* tws, int log_r, int log_g, int lh0, int quarter)
+// the 2^K-point DFT of x (rows in bit-reversed order, results in natural order);
+// rows below 2^61 + 8 in and out
+template <int K, bool INV>
+__device__ __forceinline__ void dft_rows(fp2 (&x)[1 << K])
 {
-    const int G = 1 << log_g;
+    constexpr int N = 1 << K;
+#pragma unroll
+    for (int m = 0; m < N; m += 2) {
+        const fp2 a = x[m], b = x[m + 1];
+        x[m] = mk(a.re + b.re, a.im + b.im);                                   // < 2^62 + 16
+        x[m + 1] = mk(a.re + (2 * P61 - b.re), a.im + (2 * P61 - b.im));       // < 3 2^61 + 8
+    }
+    if (K >= 2) {
+#pragma unroll
+        for (int m = 0; m < N; m += 4) {
+            const fp2 a = x[m], b = x[m + 2], c = x[m + 1], d = x[m + 3];
+            x[m] = mk(a.re + b.re, a.im + b.im);
+            x[m + 2] = mk(a.re + (4 * P61 - b.re), a.im + (4 * P61 - b.im));   // < 2^64
+            quarter_pair<INV>(c, d, x[m + 1], x[m + 3]);
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < N; ++m) x[m] = fold2(x[m]);
+    if (K >= 3) {
+        const fp2 y1 = times_w8<INV>(x[(5) & (N - 1)]), y3 = times_w8_3<INV>(x[(7) & (N - 1)]);
+        const fp2 y0 = x[4 & (N - 1)], y2 = x[6 & (N - 1)], a0 = x[0], a1 = x[1], a2 = x[2 & (N - 1)],
+                  a3 = x[3 & (N - 1)];
+        auto sum = [](fp2 a, fp2 b) { return fold2(mk(a.re + b.re, a.im + b.im)); };
+        auto dif = [](fp2 a, fp2 b) { return fold2(mk(a.re + (4 * P61 - b.re), a.im + (4 * P61 - b.im))); };
+        x[0] = sum(a0, y0);
+        x[4 & (N - 1)] = dif(a0, y0);
+        x[1] = sum(a1, y1);
+        x[5 & (N - 1)] = dif(a1, y1);
+        fp2 s, d;
+        quarter_pair<INV>(a2, y2, s, d);
+        x[2 & (N - 1)] = fold2(s);
+        x[6 & (N - 1)] = fold2(d);
+        x[3 & (N - 1)] = sum(a3, y3);
+        x[7 & (N - 1)] = dif(a3, y3);
+    }
+}
+
+template <int K, bool FIRST, bool INV>
+__device__ __forceinline__ void stage_group(fp2* sm, const fp2* tws, int log_r, int log_g, int lh0)
+{
+    const int G = 1 << log_g, half = 1 << (log_r - 1);
     const int items = ((1 << log_r) >> K) << log_g;
     for (int it = threadIdx.x; it < items; it += kThreads) {
         const int c = it & (G - 1);
@@ -85,22 +154,17 @@ __device__ __forceinline__ void stage_group(fp2* sm, const fp2* tws, int log_r, 
         const int base = ((q >> sh) << (sh + K)) + lo;
         fp2 x[1 << K];
 #pragma unroll
-        for (int m = 0; m < (1 << K); ++m) x[m] = sm[at(base + (m << sh), c, log_g)];
-#pragma unroll
-        for (int j = 0; j < K; ++j) {
-            const int lh = sh + j;
-#pragma unroll
-            for (int m = 0; m < (1 << K); ++m) {
-                if (m & (1 << j)) continue;
-                const int pin = ((m & ((1 << j) - 1)) << sh) + lo;
-                fp2 y = x[m + (1 << j)];
-                if (FIRST && lh >= 1 && pin == (1 << (lh - 1)) && quarter) y = times_quarter(y, quarter);
-                else if (pin) y = l2mul(tws[pin << (log_r - 1 - lh)], y);
-                const fp2 a = x[m];
-                x[m] = l2add(a, y);
-                x[m + (1 << j)] = l2sub(a, y);
+        for (int m = 0; m < (1 << K); ++m) {
+            x[m] = sm[at(base + (m << sh), c, log_g)];
+            if (!FIRST && m) {
+                const int e = K == 1 ? 1 : K == 2 ? ((m & 1) << 1) | (m >> 1) : ((m & 1) << 2) | (m & 2) | (m >> 2);
+                const int idx = (lo * e) << (log_r - lh0 - K);
+                fp2 w = tws[idx & (half - 1)];
+                if (e > (1 << K) / 2 && idx >= half) w = mk(P61 - w.re, P61 - w.im);   // w^(R/2) = -1
+                x[m] = l2mul(w, x[m]);
             }
         }
+        dft_rows<K, INV>(x);
 #pragma unroll
         for (int m = 0; m < (1 << K); ++m) sm[at(base + (m << sh), c, log_g)] = x[m];
     }
@@ -109,6 +173,7 @@ __device__ __forceinline__ void stage_group(fp2* sm, const fp2* tws, int log_r, 
 // One pass: a CTA transforms G = 2^log_g columns of R = 2^log_r elements.
 // src and dst may be the same buffer (in-place middle pass): every CTA reads its
 // own columns completely before it writes them, and no other CTA touches them.
+template <bool INV>
 __global__ void __launch_bounds__(kThreads, 3) pass_kernel(const ulonglong2* src, ulonglong2* dst, Pass p,
                                                         const fp2* __restrict__ lo,
                                                         const fp2* __restrict__ hi, int h)
@@ -176,13 +241,13 @@ __global__ void __launch_bounds__(kThreads, 3) pass_kernel(const ulonglong2* src
     for (int lh0 = 0; lh0 < p.log_r; lh0 += 3) {
         const int k = min(3, p.log_r - lh0);
         if (lh0 == 0) {
-            if (k == 3) stage_group<3, true>(sm, tws, p.log_r, p.log_g, 0, p.quarter);
-            else if (k == 2) stage_group<2, true>(sm, tws, p.log_r, p.log_g, 0, p.quarter);
-            else stage_group<1, true>(sm, tws, p.log_r, p.log_g, 0, p.quarter);
+            if (k == 3) stage_group<3, true, INV>(sm, tws, p.log_r, p.log_g, 0);
+            else if (k == 2) stage_group<2, true, INV>(sm, tws, p.log_r, p.log_g, 0);
+            else stage_group<1, true, INV>(sm, tws, p.log_r, p.log_g, 0);
         } else {
-            if (k == 3) stage_group<3, false>(sm, tws, p.log_r, p.log_g, lh0, p.quarter);
-            else if (k == 2) stage_group<2, false>(sm, tws, p.log_r, p.log_g, lh0, p.quarter);
-            else stage_group<1, false>(sm, tws, p.log_r, p.log_g, lh0, p.quarter);
+            if (k == 3) stage_group<3, false, INV>(sm, tws, p.log_r, p.log_g, lh0);
+            else if (k == 2) stage_group<2, false, INV>(sm, tws, p.log_r, p.log_g, lh0);
+            else stage_group<1, false, INV>(sm, tws, p.log_r, p.log_g, lh0);
         }
         __syncthreads();
     }
@@ -245,10 +310,6 @@ const Tables* tables(int logn, bool inv)
     const fp2 step = nlo < ((size_t)1 << logn) ? f2mul(lo[nlo - 1], w) : mk(1, 0);   // w^(2^h)
     hi[0] = mk(1, 0);
     for (size_t i = 1; i < nhi; ++i) hi[i] = f2mul(hi[i - 1], step);
-    if (logn >= 2) {
-        const fp2 q = f2pow(w, 1ull << (logn - 2));
-        t.quarter = (q.re == 0 && q.im == 1) ? 1 : (q.re == 0 && q.im == P61 - 1) ? -1 : 0;
-    }
     if (cuda_failed(cudaMalloc(&t.lo, sizeof(fp2) * nlo), "ntt twiddle alloc") ||
         cuda_failed(cudaMalloc(&t.hi, sizeof(fp2) * nhi), "ntt twiddle alloc") ||
         cuda_failed(cudaMemcpy(t.lo, lo.data(), sizeof(fp2) * nlo, cudaMemcpyHostToDevice), "ntt twiddle upload") ||
@@ -306,11 +367,11 @@ bool run(const ulonglong2* in, long long in_len, long long in_step, int logn, bo
     if (!tb) return false;
     Ctx* c = ctx();
     if (c->device >= 0 && c->device < 64 && !g_attr_set[c->device]) {
-        if (cuda_failed(cudaFuncSetAttribute(pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (kTileElems + kTileElems / 8 + 1 + (1 << kMaxLogR) / 2) *
-                                                 (int)sizeof(fp2)),
-                        "ntt smem attribute"))
-            return false;
+        const int most = (kTileElems + kTileElems / 8 + 1 + (1 << kMaxLogR) / 2) * (int)sizeof(fp2);
+        for (auto k : {pass_kernel<false>, pass_kernel<true>})
+            if (cuda_failed(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most),
+                            "ntt smem attribute"))
+                return false;
         g_attr_set[c->device] = true;
     }
     const std::vector<int> d = split(logn);
@@ -336,7 +397,6 @@ bool run(const ulonglong2* in, long long in_len, long long in_step, int logn, bo
         p.in_len = in_len;
         p.in_step = in_step;
         p.scale = p.last ? scale : 0;
-        p.quarter = tb->quarter;
         const ulonglong2* src = t == 0 ? in : tmp;
         ulonglong2* dst = p.last ? out : tmp;
         p.src_batch = t == 0 ? in_batch : n;
@@ -358,7 +418,8 @@ bool run(const ulonglong2* in, long long in_len, long long in_step, int logn, bo
         const long long ctas = n >> (p.log_r + p.log_g);
         const size_t smem = sizeof(fp2) * (((size_t)1 << (p.log_r + p.log_g)) + ((size_t)1 << p.log_r) / 8 + 1 +
                                            ((size_t)1 << p.log_r) / 2);
-        pass_kernel<<<dim3((unsigned)ctas, (unsigned)batch), kThreads, smem, s>>>(src, dst, p, tb->lo, tb->hi, tb->h);
+        auto kernel = inv ? pass_kernel<true> : pass_kernel<false>;
+        kernel<<<dim3((unsigned)ctas, (unsigned)batch), kThreads, smem, s>>>(src, dst, p, tb->lo, tb->hi, tb->h);
         ++g_launches;
         ok = !cuda_failed(cudaGetLastError(), "ntt pass");
     }
