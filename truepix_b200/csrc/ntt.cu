@@ -43,12 +43,11 @@ struct Pass {
 __device__ __forceinline__ fp2 ld_fe(const ulonglong2* p) { const ulonglong2 v = *p; return mk(v.y, v.x); }
 __device__ __forceinline__ void st_fe(ulonglong2* p, fp2 a) { *p = make_ulonglong2(a.im, a.re); }
 
-__device__ __forceinline__ fp2 tw_pow(const fp2* __restrict__ lo, const fp2* __restrict__ hi, int h,
-                                      unsigned long long e)
+__device__ __forceinline__ fp2 tw_pow(const fp2* __restrict__ lo, const fp2* __restrict__ hi, int h, u32 e)
 {
-    const fp2 a = lo[e & ((1ull << h) - 1)];
-    const unsigned long long q = e >> h;
-    return q ? l2mul(a, hi[q]) : a;
+    const u32 l = e & ((1u << h) - 1), q = e >> h;
+    if (l == 0) return hi[q];
+    return q ? l2mul(lo[l], hi[q]) : lo[l];
 }
 
 __device__ __forceinline__ int bitrev(int j, int bits) { return bits ? (int)(__brev((unsigned)j) >> (32 - bits)) : 0; }
@@ -174,7 +173,7 @@ __device__ __forceinline__ void stage_group(fp2* sm, const fp2* tws, int log_r, 
 // src and dst may be the same buffer (in-place middle pass): every CTA reads its
 // own columns completely before it writes them, and no other CTA touches them.
 template <bool INV>
-__global__ void __launch_bounds__(kThreads, 3) pass_kernel(const ulonglong2* src, ulonglong2* dst, Pass p,
+__global__ void __launch_bounds__(kThreads, 4) pass_kernel(const ulonglong2* src, ulonglong2* dst, Pass p,
                                                         const fp2* __restrict__ lo,
                                                         const fp2* __restrict__ hi, int h)
 {
@@ -184,56 +183,79 @@ __global__ void __launch_bounds__(kThreads, 3) pass_kernel(const ulonglong2* src
     const int tid = threadIdx.x;
     src += (long long)blockIdx.y * p.src_batch;
     dst += (long long)blockIdx.y * p.dst_batch;
-    const long long S = 1LL << p.log_s;
+    // every element index of a transform (2^28 points at most) fits 32 bits
+    __shared__ u32 s_base[16];
 
     // twiddles of the R-point DFT: w_R^t = w_n^(t n / R), t < R / 2
-    for (int t = tid; t < R / 2; t += kThreads) tws[t] = tw_pow(lo, hi, h, (unsigned long long)t << (p.logn - p.log_r));
+    for (int t = tid; t < R / 2; t += kThreads) tws[t] = tw_pow(lo, hi, h, (u32)t << (p.logn - p.log_r));
 
     // columns of this CTA
-    long long col_base = 0, s0 = 0, c0 = 0;
+    u32 col_base = 0, s0 = 0;
+    const u32 c0 = blockIdx.x << p.log_g;
     if (!p.last) {
-        const long long groups = S >> p.log_g;   // column groups per outer index
-        const long long a = blockIdx.x / groups;
-        s0 = (blockIdx.x % groups) << p.log_g;
-        col_base = a * ((long long)R << p.log_s) + s0;
+        const int lg = p.log_s - p.log_g;   // column groups per outer index
+        s0 = (blockIdx.x & ((1u << lg) - 1)) << p.log_g;
+        col_base = ((blockIdx.x >> lg) << (p.log_r + p.log_s)) + s0;
     } else {
-        c0 = (long long)blockIdx.x << p.log_g;
-    }
-
-    // load (bit-reversed into shared memory)
-    for (int idx = tid; idx < (R << p.log_g); idx += kThreads) {
-        int c, j;
-        long long pos;
-        if (!p.last) {
-            c = idx & (G - 1);
-            j = idx >> p.log_g;
-            pos = col_base + c + (long long)j * S;
-        } else {
-            // the element of the column: for R >= 2^6, the three lowest lane bits
-            // become bits log_r - 6 .. log_r - 4 of j, so that the eight threads of
-            // a quarter warp write rows bitrev(j) whose bits 3..5 differ (eight
-            // distinct bank groups of the padded tile) while every 64 bytes of
-            // the row are still read by four neighbouring lanes
-            const int u = idx & (R - 1);
-            const int at_bit = p.log_r - 6;
-            const int hi = u >> 3;
-            j = at_bit < 0 ? u : (hi & ((1 << at_bit) - 1)) | ((u & 7) << at_bit) | ((hi >> at_bit) << (at_bit + 3));
-            c = idx >> p.log_r;
-            const long long cc = c0 + c;
-            long long base = 0;
+        if (tid < G) {   // where the column's row starts: its index, digits reversed
+            const u32 cc = c0 + tid;
+            u32 base = 0;
             int sh = 0;
             for (int t = 0; t < p.n_dig; ++t) {
-                base += ((cc >> sh) & ((1LL << p.dig_bits[t]) - 1)) << p.dig_shift[t];
+                base += ((cc >> sh) & ((1u << p.dig_bits[t]) - 1)) << p.dig_shift[t];
                 sh += p.dig_bits[t];
             }
-            pos = base + j;
+            s_base[tid] = base;
         }
-        fp2 v;
-        if (p.first)
-            v = pos < p.in_len ? ld_fe(src + pos * p.in_step) : f2zero();
-        else
-            v = ld_fe(src + pos);
-        sm[at(bitrev(j, p.log_r), c, p.log_g)] = v;
+        __syncthreads();
+    }
+
+    // load (bit-reversed into shared memory), four elements' loads before their stores
+    const int tile = R << p.log_g;
+    const u32 in_len = (u32)p.in_len, in_step = (u32)p.in_step;
+    for (int i0 = tid; i0 < tile; i0 += 4 * kThreads) {
+        fp2 v[4];
+        int slot[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int idx = i0 + q * kThreads;
+            slot[q] = -1;
+            if (idx >= tile) continue;
+            int c, j;
+            u32 pos;
+            if (!p.last) {
+                // fewer than eight columns: the lanes of a quarter warp that share a column
+                // take elements whose bit-reversed rows are neighbours, not R / 2 apart
+                c = idx & (G - 1);
+                j = idx >> p.log_g;
+                if (p.log_g < 3 && p.log_r >= 3) {
+                    const int b = 3 - p.log_g;
+                    j = ((j & ((1 << b) - 1)) << (p.log_r - b)) | (j >> b);
+                }
+                pos = col_base + c + ((u32)j << p.log_s);
+            } else {
+                // the element of the column: for R >= 2^6, the three lowest lane bits
+                // become bits log_r - 6 .. log_r - 4 of j, so that the eight threads of
+                // a quarter warp write rows bitrev(j) whose bits 3..5 differ (eight
+                // distinct bank groups of the padded tile) while every 64 bytes of
+                // the row are still read by four neighbouring lanes
+                const int u = idx & (R - 1);
+                const int at_bit = p.log_r - 6;
+                const int hi = u >> 3;
+                j = at_bit < 0 ? u
+                               : (hi & ((1 << at_bit) - 1)) | ((u & 7) << at_bit) | ((hi >> at_bit) << (at_bit + 3));
+                c = idx >> p.log_r;
+                pos = s_base[c] + j;
+            }
+            if (p.first)
+                v[q] = pos < in_len ? ld_fe(src + pos * in_step) : f2zero();
+            else
+                v[q] = ld_fe(src + pos);
+            slot[q] = at(bitrev(j, p.log_r), c, p.log_g);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (slot[q] >= 0) sm[slot[q]] = v[q];
     }
     __syncthreads();
 
@@ -253,20 +275,18 @@ __global__ void __launch_bounds__(kThreads, 3) pass_kernel(const ulonglong2* src
     }
 
     // store
-    for (int idx = tid; idx < (R << p.log_g); idx += kThreads) {
+    for (int idx = tid; idx < tile; idx += kThreads) {
         const int c = idx & (G - 1);
         const int k = idx >> p.log_g;
         fp2 val = sm[at(k, c, p.log_g)];
         if (!p.last) {
             // w_{R S}^(k s) = w_n^((k s mod R S) n / (R S))
-            const unsigned long long e =
-                (((unsigned long long)k * (unsigned long long)(s0 + c)) & ((1ull << (p.log_r + p.log_s)) - 1))
-                << (p.logn - p.log_r - p.log_s);
+            const u32 e = (((u32)k * (s0 + c)) & ((1u << (p.log_r + p.log_s)) - 1)) << (p.logn - p.log_r - p.log_s);
             if (e) val = l2mul(val, tw_pow(lo, hi, h, e));
-            st_fe(dst + col_base + c + (long long)k * S, val);
+            st_fe(dst + (col_base + c + ((u32)k << p.log_s)), val);
         } else {
             if (p.scale) val = mk(lmul(val.re, p.scale), lmul(val.im, p.scale));
-            st_fe(dst + (c0 + c) + ((long long)k << (p.logn - p.log_r)), l2canon(val));
+            st_fe(dst + (c0 + c + ((u32)k << (p.logn - p.log_r))), l2canon(val));
         }
     }
 }
@@ -405,6 +425,16 @@ bool run(const ulonglong2* in, long long in_len, long long in_step, int logn, bo
         if (log_g > 4) log_g = 4;
         if (!p.last && log_g > p.log_s) log_g = p.log_s;
         if (p.last && log_g > logn - p.log_r) log_g = logn - p.log_r;
+        // Columns per CTA: sixteen (a tile of 4,096 elements at most), halved down to two
+        // (32-byte runs in memory) while there are fewer CTAs than SMs, or fewer than
+        // four an SM and the tile stays at 2,048 elements (a row group per thread).
+        // 2^16 points 53 -> 18 us (16 -> 128 CTAs a pass), 2^18 59 -> 27, 2^20 85 -> 77;
+        // 64 transforms of 2^12 points, 256 CTAs of 1,024 elements, stay (24.7 us
+        // against 30.9 with four columns).
+        auto ctas_of = [&](int g) { return (n >> (p.log_r + g)) * batch; };
+        while (log_g > 1 && (ctas_of(log_g) < c->n_sm ||
+                             (ctas_of(log_g) < 4LL * c->n_sm && p.log_r + log_g - 1 >= 11)))
+            --log_g;
         p.log_g = log_g;
         if (p.last) {
             p.n_dig = P - 1;
