@@ -430,6 +430,26 @@ __global__ void __launch_bounds__(kLeafRows) leaf_kernel(const ulonglong2* __res
     }
 }
 
+// The whole chains of few rows with a warp for the rounds and a warp for the schedule
+// of 32 (sha256.cuh, ChainMem). A row's 32 bytes per hash are loaded by its lane, one
+// hash ahead; every sector is read once.
+__global__ void __launch_bounds__(sha::kFewThreads) leaf_few_kernel(const ulonglong2* __restrict__ rows,
+                                                                    long long cw_len,
+                                                                    unsigned char* __restrict__ tree,
+                                                                    long long leaf0, uint32_t one)
+{
+    __shared__ sha::ChainMem mem;
+    const long long r = (long long)blockIdx.x * sha::kFewRows + (threadIdx.x & 31);
+    const ulonglong2* p = rows + (r < cw_len ? r : cw_len - 1) * kColumns;
+    uint32_t st[8];
+    const bool mine = sha::chain_pair<false>(mem, kColumns / 2, st, sha::AddMad{one}, [&](int n, uint32_t w[8]) {
+        const ulonglong2 x = ldg16(p + 2 * n), y = ldg16(p + 2 * n + 1);
+        sha::fe_words(x.x, x.y, w);
+        sha::fe_words(y.x, y.y, w + 4);
+    });
+    if (mine && r < cw_len) store_digest(tree, leaf0 + r, st);
+}
+
 // tree[leaf0 + i] for i in [from, to): `a` below `split`, `b` from there on
 __global__ void fill_leaves_kernel(unsigned char* __restrict__ tree, long long leaf0, long long from,
                                    long long split, long long to, ulonglong2 a0, ulonglong2 a1,
@@ -649,6 +669,19 @@ bool launch_ok(const char* what)
 {
     ++g_launches;
     return !cuda_failed(cudaGetLastError(), what);
+}
+
+// the leaf chains of `count` rows, column pairs [pair0, pair1)
+void launch_leaves(const ulonglong2* rows, long long count, unsigned char* digests, long long leaf0, int pair0,
+                   int pair1, cudaStream_t s)
+{
+    const long long few = (count + sha::kFewRows - 1) / sha::kFewRows;
+    Ctx* c = ctx();
+    if (c && few <= (long long)sha::kFewPerSm * c->n_sm && pair0 == 0 && pair1 == kColumns / 2)
+        leaf_few_kernel<<<(unsigned)few, sha::kFewThreads, 0, s>>>(rows, count, digests, leaf0, 1u);
+    else
+        leaf_kernel<<<(unsigned)((count + kLeafRows - 1) / kLeafRows), kLeafRows, 0, s>>>(rows, count, digests, leaf0,
+                                                                                         1u, pair0, pair1);
 }
 
 }  // namespace
@@ -880,8 +913,7 @@ bool commit(const Encoder& enc, const ulonglong2* src, const PixelInput* px, ulo
     const int chunks = g_leaf_chunks.load();
     for (int k = 0; k < chunks; ++k) {
         timer_begin(s, kTagLeaf);
-        leaf_kernel<<<(unsigned)((cw_len + kLeafRows - 1) / kLeafRows), kLeafRows, 0, s>>>(
-            rows, cw_len, tree, size, 1u, k * (kColumns / 2) / chunks, (k + 1) * (kColumns / 2) / chunks);
+        launch_leaves(rows, cw_len, tree, size, k * (kColumns / 2) / chunks, (k + 1) * (kColumns / 2) / chunks, s);
         timer_end(s);
         if (!launch_ok("orion leaves")) return false;
     }
@@ -904,8 +936,7 @@ bool commit(const Encoder& enc, const ulonglong2* src, const PixelInput* px, ulo
 bool leaf_digests(const ulonglong2* rows, long long count, unsigned char* digests, cudaStream_t s)
 {
     if (count <= 0) return true;
-    leaf_kernel<<<(unsigned)((count + kLeafRows - 1) / kLeafRows), kLeafRows, 0, s>>>(rows, count, digests, 0, 1u, 0,
-                                                                                       kColumns / 2);
+    launch_leaves(rows, count, digests, 0, 0, kColumns / 2, s);
     return launch_ok("orion column leaves");
 }
 

@@ -14,6 +14,16 @@ constexpr int kSlices = 64;   // 2^log_slice_number (include/infrastructure/cons
 
 constexpr int kLeafThreads = 128;
 
+__device__ __forceinline__ void store_leaf(unsigned char* tree, long long node, const uint32_t st[8])
+{
+    uint4 a, b;
+    a.x = sha::bswap32(st[0]); a.y = sha::bswap32(st[1]); a.z = sha::bswap32(st[2]); a.w = sha::bswap32(st[3]);
+    b.x = sha::bswap32(st[4]); b.y = sha::bswap32(st[5]); b.z = sha::bswap32(st[6]); b.w = sha::bswap32(st[7]);
+    uint4* d = reinterpret_cast<uint4*>(tree + node * 32);
+    d[0] = a;
+    d[1] = b;
+}
+
 // The leaf chains of both commit kinds, h <- SHA256(x || y || h) over the 64 slices
 // (fri.cpp:96-110, 396-410: the pair first, the running digest second -- the
 // opposite order of the Orion row leaves): leaf t's x and y of slice i stand at
@@ -48,19 +58,41 @@ __global__ void __launch_bounds__(kLeafThreads) pair_leaf_kernel(const ulonglong
         for (int k = 0; k < 8; ++k) w[8 + k] = st[k];
         sha::hash64(w, st, sha::AddMad{one});
     }
-    uint4 a, b;
-    a.x = sha::bswap32(st[0]); a.y = sha::bswap32(st[1]); a.z = sha::bswap32(st[2]); a.w = sha::bswap32(st[3]);
-    b.x = sha::bswap32(st[4]); b.y = sha::bswap32(st[5]); b.z = sha::bswap32(st[6]); b.w = sha::bswap32(st[7]);
-    uint4* d = reinterpret_cast<uint4*>(tree + (n_leaves + t) * 32);
-    d[0] = a;
-    d[1] = b;
+    store_leaf(tree, n_leaves + t, st);
+}
+
+// The same chains with a warp for the rounds and a warp for the schedule of 32
+// (sha256.cuh, ChainMem).
+__global__ void __launch_bounds__(sha::kFewThreads) pair_leaf_few_kernel(const ulonglong2* __restrict__ src,
+                                                                         long long n_leaves, long long leaf_step,
+                                                                         long long slice_step, long long y_off,
+                                                                         unsigned char* __restrict__ tree,
+                                                                         uint32_t one)
+{
+    __shared__ sha::ChainMem mem;
+    const long long t = (long long)blockIdx.x * sha::kFewRows + (threadIdx.x & 31);
+    const ulonglong2* p = src + (t < n_leaves ? t : n_leaves - 1) * leaf_step;
+    uint32_t st[8];
+    const bool mine = sha::chain_pair<true>(mem, kSlices, st, sha::AddMad{one}, [&](int n, uint32_t w[8]) {
+        const ulonglong2 x = __ldg(p + n * slice_step), y = __ldg(p + n * slice_step + y_off);
+        sha::fe_words(x.x, x.y, w);
+        sha::fe_words(y.x, y.y, w + 4);
+    });
+    if (mine && t < n_leaves) store_leaf(tree, n_leaves + t, st);
 }
 
 bool launch_pair_leaves(const ulonglong2* src, long long n_leaves, long long leaf_step, long long slice_step,
                         long long y_off, unsigned char* tree, const char* what, cudaStream_t s)
 {
-    pair_leaf_kernel<<<(unsigned)((n_leaves + kLeafThreads - 1) / kLeafThreads), kLeafThreads, 0, s>>>(
-        src, n_leaves, leaf_step, slice_step, y_off, tree, 1u);
+    Ctx* c = ctx();
+    if (!c) return false;
+    const long long few = (n_leaves + sha::kFewRows - 1) / sha::kFewRows;
+    if (few <= (long long)sha::kFewPerSm * c->n_sm)
+        pair_leaf_few_kernel<<<(unsigned)few, sha::kFewThreads, 0, s>>>(src, n_leaves, leaf_step, slice_step, y_off,
+                                                                        tree, 1u);
+    else
+        pair_leaf_kernel<<<(unsigned)((n_leaves + kLeafThreads - 1) / kLeafThreads), kLeafThreads, 0, s>>>(
+            src, n_leaves, leaf_step, slice_step, y_off, tree, 1u);
     return !cuda_failed(cudaGetLastError(), what);
 }
 
