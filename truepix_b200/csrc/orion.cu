@@ -567,7 +567,8 @@ __device__ __forceinline__ void edge31(Acc3& A, Acc3& Bd, Acc3& S, ulonglong2 v,
     mac32(S, sum, w);
 }
 
-template <int CPL>
+// kDepth edges' rows are loaded before their products.
+template <int CPL, int kDepth>
 __global__ void __launch_bounds__(256) gather31_kernel(ulonglong2* __restrict__ rows, long long src_row,
                                                        long long dst_row, long long n_targets,
                                                        const unsigned* __restrict__ ptr,
@@ -596,30 +597,39 @@ __global__ void __launch_bounds__(256) gather31_kernel(ulonglong2* __restrict__ 
         for (int h = 0; h < cnt; h += 8) {
             const int end = min(cnt, h + 8);
             int j = h;
-            for (; j + 2 <= end; j += 2) {
-                const unsigned s0 = __shfl_sync(0xffffffffu, my_s, j), s1 = __shfl_sync(0xffffffffu, my_s, j + 1);
-                const u32 c0 = __shfl_sync(0xffffffffu, my_w.x, j), d0 = __shfl_sync(0xffffffffu, my_w.y, j);
-                const u32 c1 = __shfl_sync(0xffffffffu, my_w.x, j + 1), d1 = __shfl_sync(0xffffffffu, my_w.y, j + 1);
-                const ulonglong2* p0 = src + (long long)s0 * kColumns;
-                const ulonglong2* p1 = src + (long long)s1 * kColumns;
-                ulonglong2 v0[CPL], v1[CPL];
+            for (; j + kDepth <= end; j += kDepth) {
+                u32 c[kDepth], d[kDepth];
+                ulonglong2 v[kDepth][CPL];
 #pragma unroll
-                for (int k = 0; k < CPL; ++k) {
-                    v0[k] = ldg16(p0 + 32 * k);
-                    v1[k] = ldg16(p1 + 32 * k);
+                for (int q = 0; q < kDepth; ++q) {
+                    const ulonglong2* p = src + (long long)__shfl_sync(0xffffffffu, my_s, j + q) * kColumns;
+                    c[q] = __shfl_sync(0xffffffffu, my_w.x, j + q);
+                    d[q] = __shfl_sync(0xffffffffu, my_w.y, j + q);
+#pragma unroll
+                    for (int k = 0; k < CPL; ++k) v[q][k] = ldg16(p + 32 * k);
                 }
 #pragma unroll
-                for (int k = 0; k < CPL; ++k) {
-                    edge31(A[k], Bd[k], S[k], v0[k], c0, d0, c0 + d0);
-                    edge31(A[k], Bd[k], S[k], v1[k], c1, d1, c1 + d1);
-                }
+                for (int q = 0; q < kDepth; ++q)
+#pragma unroll
+                    for (int k = 0; k < CPL; ++k) edge31(A[k], Bd[k], S[k], v[q][k], c[q], d[q], c[q] + d[q]);
             }
-            if (j < end) {
-                const unsigned s0 = __shfl_sync(0xffffffffu, my_s, j);
-                const u32 c0 = __shfl_sync(0xffffffffu, my_w.x, j), d0 = __shfl_sync(0xffffffffu, my_w.y, j);
-                const ulonglong2* p0 = src + (long long)s0 * kColumns;
+            if (j < end) {   // the last few: loads predicated, weights zero past the end
+                u32 c[kDepth], d[kDepth];
+                ulonglong2 v[kDepth][CPL];
 #pragma unroll
-                for (int k = 0; k < CPL; ++k) edge31(A[k], Bd[k], S[k], ldg16(p0 + 32 * k), c0, d0, c0 + d0);
+                for (int q = 0; q < kDepth; ++q) {
+                    const bool in = j + q < end;
+                    const int at = in ? j + q : j;
+                    const ulonglong2* p = src + (long long)__shfl_sync(0xffffffffu, my_s, at) * kColumns;
+                    c[q] = in ? __shfl_sync(0xffffffffu, my_w.x, at) : 0u;
+                    d[q] = in ? __shfl_sync(0xffffffffu, my_w.y, at) : 0u;
+#pragma unroll
+                    for (int k = 0; k < CPL; ++k) v[q][k] = in ? ldg16(p + 32 * k) : make_ulonglong2(0, 0);
+                }
+#pragma unroll
+                for (int q = 0; q < kDepth; ++q)
+#pragma unroll
+                    for (int k = 0; k < CPL; ++k) edge31(A[k], Bd[k], S[k], v[q][k], c[q], d[q], c[q] + d[q]);
             }
 #pragma unroll
             for (int k = 0; k < CPL; ++k) {
@@ -637,6 +647,93 @@ __global__ void __launch_bounds__(256) gather31_kernel(ulonglong2* __restrict__ 
     }
 }
 
+// ---- the inner levels in shared memory ----------------------------------------------
+// The encoder works on every column alone, and from a message of a few thousand rows
+// on a column's whole remaining codeword fits in shared memory: one CTA takes one
+// column through all levels from there inwards and back, instead of two launches a
+// level whose few targets leave the chip idle (4 to 9 launches of 5 to 18 us each).
+// A lane sums one target; the edges of 32 targets (sorted by in-degree, so that a
+// warp's targets are nearly equally long) are stored step by step, so that the lanes
+// read them side by side. Bound by the edges' instructions.
+constexpr int kInnerThreads = 512;
+
+struct InnerLevels {
+    int count;
+    long long row0;                   // first row of the outermost level's message
+    int n0;                           // the message's length
+    struct {
+        int at, n, L;                 // at: the message's first row, from row0
+        InnerGraph c, d;
+    } lv[kMaxInner];
+};
+
+__device__ void inner_gather(ulonglong2* sm, ulonglong2* __restrict__ rows, int src0, int dst0, const InnerGraph& g)
+{
+    const int lane = threadIdx.x & 31;
+    const ulonglong2* in = sm + src0;
+    for (int sl = threadIdx.x >> 5; sl < g.slices; sl += kInnerThreads / 32) {
+        const int t = g.target[32 * sl + lane];
+        const int e0 = g.step[sl], e1 = g.step[sl + 1];
+        Acc3 A = {0, 0, 0}, Bd = {0, 0, 0}, S = {0, 0, 0};
+        const unsigned* es = g.src + 32 * e0 + lane;
+        const uint2* ew = g.w + 32 * e0 + lane;
+        const int steps = e1 - e0;
+        // eight steps' edges are read while the eight before them are summed
+        unsigned s[2][8];
+        uint2 w[2][8];
+        auto fetch = [&](int e, unsigned (&fs)[8], uint2 (&fw)[8]) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {   // past the slice's end: weight zero
+                const bool more = e + q < steps;
+                fs[q] = more ? __ldg(es + 32 * (e + q)) : 0;
+                fw[q] = more ? __ldg(ew + 32 * (e + q)) : make_uint2(0, 0);
+            }
+        };
+        auto sum = [&](const unsigned (&fs)[8], const uint2 (&fw)[8]) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) edge31(A, Bd, S, in[fs[q]], fw[q].x, fw[q].y, fw[q].x + fw[q].y);
+            settle(A);
+            settle(Bd);
+            settle(S);
+        };
+        fetch(0, s[0], w[0]);
+        for (int e = 0; e < steps; e += 16) {
+            fetch(e + 8, s[1], w[1]);
+            sum(s[0], w[0]);
+            if (e + 8 >= steps) break;
+            fetch(e + 16, s[0], w[0]);
+            sum(s[1], w[1]);
+        }
+        if (t >= 0) {
+            const u64 ac = settle(A), bd = settle(Bd), sw = settle(S);
+            const ulonglong2 v =
+                make_ulonglong2(canon61(fold61(sw + (4 * P61 - ac - bd))), canon61(fold61(ac + (2 * P61 - bd))));
+            sm[dst0 + t] = v;
+            rows[(long long)(dst0 + t) * kColumns] = v;
+        }
+    }
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(kInnerThreads, 1) inner_kernel(ulonglong2* __restrict__ all_rows,
+                                                                 const __grid_constant__ InnerLevels P)
+{
+    extern __shared__ ulonglong2 inner_sm[];
+    ulonglong2* sm = inner_sm;
+    ulonglong2* rows = all_rows + P.row0 * kColumns + blockIdx.x;
+    for (int i = threadIdx.x; i < P.n0; i += kInnerThreads) sm[i] = rows[(long long)i * kColumns];
+    __syncthreads();
+    for (int k = 0; k < P.count; ++k) inner_gather(sm, rows, P.lv[k].at, P.lv[k].at + P.lv[k].n, P.lv[k].c);
+    for (int k = P.count - 1; k >= 0; --k) {
+        const int next = P.lv[k].at + P.lv[k].n;
+        inner_gather(sm, rows, next, next + P.lv[k].L, P.lv[k].d);
+    }
+}
+
+// Edges in flight per warp: with two, the 42 edges of an inner graph's target were 21
+// waits for L2 one after the other (a 360p frame's gathers 140 -> 124 us, 1080p 384 ->
+// 355; eight for two columns a lane takes too many registers, 375).
+constexpr int kD1 = 8, kD2 = 4;
 // graphs with fewer targets than this get four warps per target
 constexpr long long kSmallGraph = 8192;
 
@@ -647,13 +744,13 @@ void launch_gather(ulonglong2* rows, long long src_row, long long dst_row, long 
     if (ew32) {
         const int cpl = n_targets < kSmallGraph ? 1 : g_gather_cpl.load();
         if (cpl == 1)
-            gather31_kernel<1><<<(unsigned)((4 * n_targets + 7) / 8), 256, 0, s>>>(rows, src_row, dst_row,
+            gather31_kernel<1, kD1><<<(unsigned)((4 * n_targets + 7) / 8), 256, 0, s>>>(rows, src_row, dst_row,
                                                                                    n_targets, ptr, esrc, ew32);
         else if (cpl == 2)
-            gather31_kernel<2><<<(unsigned)((2 * n_targets + 7) / 8), 256, 0, s>>>(rows, src_row, dst_row,
+            gather31_kernel<2, kD2><<<(unsigned)((2 * n_targets + 7) / 8), 256, 0, s>>>(rows, src_row, dst_row,
                                                                                    n_targets, ptr, esrc, ew32);
         else
-            gather31_kernel<4><<<(unsigned)((n_targets + 7) / 8), 256, 0, s>>>(rows, src_row, dst_row, n_targets,
+            gather31_kernel<4, 2><<<(unsigned)((n_targets + 7) / 8), 256, 0, s>>>(rows, src_row, dst_row, n_targets,
                                                                                ptr, esrc, ew32);
         return;
     }
@@ -669,6 +766,38 @@ bool launch_ok(const char* what)
 {
     ++g_launches;
     return !cuda_failed(cudaGetLastError(), what);
+}
+
+bool launch_inner(const Encoder& enc, ulonglong2* rows, cudaStream_t s)
+{
+    InnerLevels P = {};
+    const size_t from = enc.inner_from;
+    const Level& top = enc.levels[from];
+    P.row0 = top.off;
+    P.n0 = (int)top.n;
+    for (size_t k = from; k < enc.levels.size(); ++k) {
+        const Level& lv = enc.levels[k];
+        auto& v = P.lv[P.count++];
+        v.at = (int)(lv.off - top.off);
+        v.n = (int)lv.n;
+        v.L = (int)lv.L;
+        v.c = enc.inner[2 * (k - from)];
+        v.d = enc.inner[2 * (k - from) + 1];
+    }
+    static std::atomic<bool> attr[64];
+    Ctx* c = ctx();
+    if (!c) return false;
+    const bool known = c->device >= 0 && c->device < 64;
+    if (!known || !attr[c->device].load()) {
+        TP_CUDA_OK(cudaFuncSetAttribute(inner_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        kInnerRows * (int)sizeof(ulonglong2)),
+                   "inner smem");
+        if (known) attr[c->device].store(true);
+    }
+    timer_begin(s, kTagGather);
+    inner_kernel<<<kColumns, kInnerThreads, (size_t)(top.n + top.L + top.RD) * sizeof(ulonglong2), s>>>(rows, P);
+    timer_end(s);
+    return launch_ok("orion inner levels");
 }
 
 // the leaf chains of `count` rows, column pairs [pair0, pair1)
@@ -712,6 +841,72 @@ void zero_block_hash(unsigned char out[32])
     uint32_t w[16] = {0}, st[8];
     sha::hash64(w, st);
     state_to_bytes(st, out);
+}
+
+// The graphs of the levels that run in shared memory, step by step for 32 targets at
+// a time (sorted by in-degree), in one block of device memory.
+static bool inner_graphs(Encoder* e, const std::vector<HostGraph>& C, const std::vector<HostGraph>& D)
+{
+    size_t from = 0;
+    const size_t n_levels = e->levels.size();
+    auto fits = [&](const Level& lv) { return lv.n + lv.L + lv.RD <= kInnerRows; };
+    while (from < n_levels && (!fits(e->levels[from]) || n_levels - from > (size_t)kMaxInner)) ++from;
+    if (from == n_levels) return true;
+    struct Host {
+        std::vector<int> target, step;
+        std::vector<unsigned> src;
+        std::vector<uint2> w;
+    };
+    std::vector<Host> hosts;
+    size_t bytes = 0;
+    auto round16 = [](size_t n) { return (n + 15) / 16 * 16; };
+    for (size_t k = from; k < n_levels; ++k)
+        for (const HostGraph* g : {&C[k], &D[k]}) {
+            Host h;
+            const int R = (int)g->R;
+            auto deg = [&](int t) { return g->ptr[(size_t)t + 1] - g->ptr[(size_t)t]; };
+            for (int t = 0; t < R; ++t) h.target.push_back(t);
+            std::stable_sort(h.target.begin(), h.target.end(), [&](int a, int b) { return deg(a) > deg(b); });
+            h.target.resize((size_t)(R + 31) / 32 * 32, -1);
+            h.step.push_back(0);
+            for (size_t sl = 0; sl < h.target.size(); sl += 32) {
+                const int steps = (int)deg(h.target[sl]);   // the slice's longest
+                for (int q = 0; q < steps; ++q)
+                    for (size_t l = 0; l < 32; ++l) {
+                        const int t = h.target[sl + l];
+                        const bool in = t >= 0 && (unsigned)q < deg(t);
+                        const size_t at = in ? g->ptr[(size_t)t] + (size_t)q : 0;
+                        h.src.push_back(in ? g->src[at] : 0u);
+                        h.w.push_back(in ? make_uint2((unsigned)g->w[at].y, (unsigned)g->w[at].x) : make_uint2(0, 0));
+                    }
+                h.step.push_back(h.step.back() + steps);
+            }
+            bytes += round16(4 * h.target.size()) + round16(4 * h.step.size()) + round16(4 * h.src.size()) +
+                     round16(8 * h.w.size());
+            hosts.push_back(std::move(h));
+        }
+    std::vector<unsigned char> blob(bytes);
+    if (cuda_failed(cudaMalloc(&e->d_inner, std::max<size_t>(16, bytes)), "orion inner graphs")) return false;
+    size_t at = 0;
+    auto put = [&](const void* p, size_t n) {
+        const size_t o = at;
+        if (n) memcpy(blob.data() + o, p, n);
+        at += round16(n);
+        return e->d_inner + o;
+    };
+    for (const Host& h : hosts) {
+        InnerGraph g;
+        g.slices = (int)h.step.size() - 1;
+        g.target = reinterpret_cast<const int*>(put(h.target.data(), 4 * h.target.size()));
+        g.step = reinterpret_cast<const int*>(put(h.step.data(), 4 * h.step.size()));
+        g.src = reinterpret_cast<const unsigned*>(put(h.src.data(), 4 * h.src.size()));
+        g.w = reinterpret_cast<const uint2*>(put(h.w.data(), 8 * h.w.size()));
+        e->inner.push_back(g);
+    }
+    if (cuda_failed(cudaMemcpy(e->d_inner, blob.data(), bytes, cudaMemcpyHostToDevice), "orion inner upload"))
+        return false;
+    e->inner_from = from;
+    return true;
 }
 
 const Encoder* encoder(long long col_len)
@@ -779,6 +974,7 @@ const Encoder* encoder(long long col_len)
                           "orion graph upload") &&
              !cuda_failed(cudaMemcpy(e->d_w, w.data(), sizeof(ulonglong2) * w.size(), cudaMemcpyHostToDevice),
                           "orion graph upload");
+    e->inner_from = e->levels.size();
     bool small = ok && e->n_edges > 0;
     for (size_t i = 0; small && i < w.size(); ++i) small = w[i].x < (1ull << 31) && w[i].y < (1ull << 31);
     if (small) {
@@ -788,11 +984,13 @@ const Encoder* encoder(long long col_len)
              !cuda_failed(cudaMemcpy(e->d_w32, w32.data(), sizeof(uint2) * w32.size(), cudaMemcpyHostToDevice),
                           "orion graph upload");
     }
+    if (small) ok = ok && inner_graphs(e, C, D);
     if (!ok) {
         cudaFree(e->d_ptr);
         cudaFree(e->d_src);
         cudaFree(e->d_w);
         cudaFree(e->d_w32);
+        cudaFree(e->d_inner);
         delete e;
         return nullptr;
     }
@@ -855,6 +1053,7 @@ bool commit(const Encoder& enc, const ulonglong2* src, const PixelInput* px, ulo
     if (cuda_failed(cudaMemsetAsync(tree, 0, 32, s), "orion tree clear")) return false;
     // 1. the message: column-major input -> rows [0, col_len)
     unsigned char* bytes = nullptr;
+    const size_t inner = enc.inner_from;
     if (src) {
         timer_begin(s, kTagLoad);
         transpose_kernel<<<transpose_grid(kColumns, col_len), 256, 0, s>>>(src, rows, kColumns, col_len);
@@ -865,7 +1064,7 @@ bool commit(const Encoder& enc, const ulonglong2* src, const PixelInput* px, ulo
         while ((1 << w_shift) < px->W) ++w_shift;
         const long long n = col_len * kColumns;
         // byte path of the depth-0 C multiplication: values < 2^8, in-degree < 2^16
-        if (px->mask_mode == kMaskNone && px->const_val < 256 && !enc.levels.empty() &&
+        if (inner > 0 && px->mask_mode == kMaskNone && px->const_val < 256 && !enc.levels.empty() &&
             enc.max_c0_in_degree < (1u << 16)) {
             bytes = static_cast<unsigned char*>(dev_alloc((size_t)n, s));
             if (!bytes) return false;
@@ -879,7 +1078,8 @@ bool commit(const Encoder& enc, const ulonglong2* src, const PixelInput* px, ulo
         }
     }
     // 2. C multiplications, outermost depth first
-    for (const Level& lv : enc.levels) {
+    for (size_t k = 0; k < inner; ++k) {
+        const Level& lv = enc.levels[k];
         if (lv.R == 0) continue;
         if (bytes && lv.off == 0) {
             timer_begin(s, kTagGatherBytes);
@@ -898,9 +1098,10 @@ bool commit(const Encoder& enc, const ulonglong2* src, const PixelInput* px, ulo
         if (!launch_ok("orion C gather")) return false;
     }
     if (bytes) dev_free(bytes, s);
+    if (inner < enc.levels.size() && !launch_inner(enc, rows, s)) return false;
     // 3. D multiplications, innermost depth first
-    for (auto it = enc.levels.rbegin(); it != enc.levels.rend(); ++it) {
-        const Level& lv = *it;
+    for (size_t k = inner; k-- > 0;) {
+        const Level& lv = enc.levels[k];
         if (lv.RD == 0) continue;
         const long long next = lv.off + lv.n;
         timer_begin(s, kTagGather);

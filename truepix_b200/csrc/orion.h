@@ -36,6 +36,21 @@ struct Level {
     long long d_ptr, d_edge;   // same for the D graph
 };
 
+constexpr int kInnerRows = 7000;   // codeword rows (112 KB of shared memory)
+constexpr int kMaxInner = 8;       // levels
+
+// A graph's edges, 32 targets (a slice) at a time and step by step: lane l of slice s
+// sums target[32 s + l] (-1: none) over the steps [step[s], step[s + 1]) of src / w
+// (32 entries a step; weight zero past a target's last edge).
+struct InnerGraph {
+    const int* target = nullptr;
+    const int* step = nullptr;
+    const unsigned* src = nullptr;
+    const uint2* w = nullptr;
+    int slices = 0;
+};
+
+
 // Graphs of one column length, transposed to CSR by target on the host and kept
 // on the device (the reference draws them from glibc rand() in its default seed
 // state; the same draws are replayed here).
@@ -54,6 +69,12 @@ struct Encoder {
     // every weight is, they are also kept as {real, img} 32-bit pairs and the
     // gathers multiply 61 x 31 bits (d_w32 non-null).
     uint2* d_w32 = nullptr;            // [n_edges]
+    // Levels inner_from and inwards (codewords of kInnerRows rows at most) run in
+    // shared memory; their graphs, C then D of each level, laid out for it in one block
+    // of device memory. inner_from = levels.size(): none.
+    size_t inner_from = 0;
+    std::vector<InnerGraph> inner;
+    unsigned char* d_inner = nullptr;
 };
 
 // cached per (device, col_len); nullptr and the error set on failure
