@@ -661,7 +661,9 @@ __global__ void __launch_bounds__(256) gather31_kernel(ulonglong2* __restrict__ 
 // level whose few targets leave the chip idle (4 to 9 launches of 5 to 18 us each).
 // A lane sums one target; the edges of 32 targets (sorted by in-degree, so that a
 // warp's targets are nearly equally long) are stored step by step, so that the lanes
-// read them side by side. Bound by the edges' instructions.
+// read them side by side. Bound by the edges' instructions and, inside, by the levels'
+// latency. A 360p commit's levels took 118 us as launches of their own, 46 here; a
+// 1080p commit's 100 us, now 58.
 constexpr int kInnerThreads = 512;
 
 struct InnerLevels {
