@@ -159,7 +159,8 @@ constexpr int kMaxLinGroups = 16;   // more product groups keep the table of all
 constexpr int kFusePairs = 4096;    // from this many pairs on a frame's rounds run in one CTA
 int lin_stride(int cs);
 size_t lin_bytes(int cs, int n_real);        // bytes of a frame's copied rows
-int lin_chunks(int n_real, int folds);       // CTAs of the finish from bytes
+int lin_chunks(int n_real, int folds);       // pieces of 512 copies of the finish from bytes
+void plan_linear_finish(std::vector<Job>& jobs);   // its CTAs, from the jobs' pieces (chunks)
 struct VoleRounds {
     void* states;
     void* vole_states;

@@ -509,30 +509,197 @@ __global__ void __launch_bounds__(kRoundsThreads, 1) vec_rounds_kernel(const Job
 
 // ---- finish ---------------------------------------------------------------------
 
-// eq(challenges, c) for the copies c of a chunk: the products over bits 0..3 and 4..8
-// of c and over the chunk's higher bits, in shared memory (49 threads or more)
+// eq(point, c) for the copies c of up to 16 chunks of 512 in a row: the products over
+// bits 0..3 and 4..8 of c and over each chunk's higher bits, in shared memory (64
+// threads or more)
+constexpr int kMaxPieces = 16;
 struct EqParts {
     fp2 r[64];
-    fp2 lo[16], mid[32], hi;
+    fp2 lo[16], mid[32], hi[kMaxPieces];
 };
-__device__ void eq_parts(const Job& J, int chunk, EqParts& e)
+// from the first n entries of e.r
+__device__ void eq_parts(EqParts& e, int n, int chunk, int pieces)
 {
-    const int tid = threadIdx.x, kf = J.nf + (J.has_r != 0);
-    for (int k = tid; k < kf; k += blockDim.x) e.r[k] = k < J.nf ? ldcg2(J.rs + k) : J.r;
-    __syncthreads();
+    const int tid = threadIdx.x;
     const fp2 one = mk(1, 0);
     auto prod = [&](int idx, int first, int last) {
         fp2 v = one;
-        for (int b = first; b < last && b < kf; ++b)
+        for (int b = first; b < last && b < n; ++b)
             v = l2mul(v, ((idx >> (b - first)) & 1) ? e.r[b] : l2sub(one, e.r[b]));
         return v;
     };
     if (tid < 16) e.lo[tid] = prod(tid, 0, 4);
     else if (tid < 48) e.mid[tid - 16] = prod(tid - 16, 4, 9);
-    else if (tid == 48) e.hi = prod(chunk, 9, kf);
+    else if (tid < 48 + pieces) e.hi[tid - 48] = prod(chunk + tid - 48, 9, n);
+}
+// at a job's challenges
+__device__ void eq_parts(const Job& J, int chunk, int pieces, EqParts& e)
+{
+    const int kf = J.nf + (J.has_r != 0);
+    for (int k = threadIdx.x; k < kf; k += blockDim.x) e.r[k] = k < J.nf ? ldcg2(J.rs + k) : J.r;
+    __syncthreads();
+    eq_parts(e, kf, chunk, pieces);
     __syncthreads();
 }
-__device__ __forceinline__ fp2 eq_of(const EqParts& e, int c) { return l2mul(l2mul(e.lo[c & 15], e.mid[c >> 4]), e.hi); }
+// c: within the piece
+__device__ __forceinline__ fp2 eq_of(const EqParts& e, int c, int piece = 0)
+{
+    return l2mul(l2mul(e.lo[c & 15], e.mid[c >> 4]), e.hi[piece]);
+}
+
+// ---- bytes weighted over the copies --------------------------------------------
+// sum over copies of eq(c) byte(c, w), a warp per 32 wires: the 16 byte-planes of
+// eq are the mma's rows, the wires its columns (words of four copies' four wires,
+// transposed in registers), 512 copies' planes at a time.
+//
+// Read bandwidth is the bound on paper (64 1080p frames: 398 MB, 57 us); what is spent
+// besides are the products that make the weights and a CTA's serial start and end, 10
+// of 26 us of a CTA of 512 copies, so a CTA takes several such pieces in a row where
+// there are CTAs enough (row_pieces): the finish of 64 frames took 173 us with one piece
+// a CTA, 93 with eight (282 with each step's loads waited for, one CTA an SM).
+constexpr int kPlanePitch = kFinCopies + 16;
+
+// the planes of the piece's first lim copies' weights, zero behind; their sum added to
+// the thread's sum
+__device__ __forceinline__ void weight_planes(const EqParts& e, int piece, int lim, unsigned char* E, fp2& sum)
+{
+    for (int c = threadIdx.x; c < kFinCopies; c += blockDim.x) {
+        fp2 v = f2zero();
+        if (c < lim) {
+            v = l2canon(eq_of(e, c, piece));
+            sum = l2add(sum, v);
+        }
+#pragma unroll
+        for (int l = 0; l < 8; ++l) {
+            E[l * kPlanePitch + c] = (unsigned char)(v.re >> (8 * l));
+            E[(8 + l) * kPlanePitch + c] = (unsigned char)(v.im >> (8 * l));
+        }
+    }
+}
+
+// the wire of the warp's 32 whose sum a lane gets
+__device__ __forceinline__ int weighed_wire(int lane)
+{
+    const int g = lane >> 2, j = lane & 3;
+    return 4 * (2 * j + (g & 1)) + (g >> 1);
+}
+
+struct Weighed {
+    int d[4][4];
+
+    // v: the words of the wires 4g .. 4g + 3 of the copies k + 4j + i and k + 16 + 4j + i
+    __device__ __forceinline__ void step(const unsigned char* E, int k, const u32 (&v)[8])
+    {
+        const int lane = threadIdx.x & 31, g = lane >> 2, j = lane & 3;
+        const unsigned char* er = E + g * kPlanePitch + k + 4 * j;
+        auto word = [](const unsigned char* p) { return *reinterpret_cast<const u32*>(p); };
+        const u32 a0 = word(er), a1 = word(er + 8 * kPlanePitch), a2 = word(er + 16),
+                  a3 = word(er + 8 * kPlanePitch + 16);
+        const u32 lo[4] = {v[0], v[1], v[2], v[3]}, hi[4] = {v[4], v[5], v[6], v[7]};
+        u32 b0[4], b1[4];
+        transpose4(lo, b0);
+        transpose4(hi, b1);
+#pragma unroll
+        for (int m = 0; m < 4; ++m) mma_u8(d[m], a0, a1, a2, a3, b0[m], b1[m]);
+    }
+    __device__ __forceinline__ fp2 total() const;
+};
+
+// A warp's 32 columns of whole 16-byte vectors, by asynchronous copies: kRowStages - 1
+// steps of 32 copies are on their way from before the weights are made. Four copies'
+// 32 bytes lie together, and four times four in different banks.
+constexpr int kRowStages = 5, kRowStep = 8 * 160;
+
+struct RowCopies {
+    const unsigned char* src;   // column 0 of the warp's wires in the chunk's first copy
+    int pitch, copies, width;   // width: columns there are, 16 or 32 at least of them
+    unsigned char* ring;
+
+    __device__ __forceinline__ void fetch(int step) const
+    {
+        const int lane = threadIdx.x & 31, q = lane & 1;
+        if (32 * step < copies) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int r = 16 * h + (lane >> 1), c = min(32 * step + r, copies - 1);
+                const bool in = 16 * q < width;
+                async16(ring + (step % kRowStages) * kRowStep + (r >> 2) * 160 + (r & 3) * 32 + 16 * q,
+                        src + (size_t)c * pitch + (in ? 16 * q : 0), in);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    __device__ __forceinline__ void start() const
+    {
+#pragma unroll
+        for (int k = 0; k < kRowStages - 1; ++k) fetch(k);
+    }
+    // the piece's copies, E: its planes
+    __device__ __forceinline__ void sum(int piece, const unsigned char* E, Weighed& t) const
+    {
+        constexpr int kSteps = kFinCopies / 32;
+        const int lane = threadIdx.x & 31, g = lane >> 2, j = lane & 3;
+        for (int k = kSteps * piece; k < kSteps * (piece + 1) && 32 * k < copies; ++k) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kRowStages - 2) : "memory");
+            __syncwarp();   // the step is here, and the one before it read by all lanes
+            fetch(k + kRowStages - 1);
+            const unsigned char* p = ring + (k % kRowStages) * kRowStep + j * 160 + 4 * g;
+            u32 v[8];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                v[i] = *reinterpret_cast<const u32*>(p + 32 * i);
+                v[4 + i] = *reinterpret_cast<const u32*>(p + 4 * 160 + 32 * i);
+            }
+            t.step(E, 32 * (k % kSteps), v);
+        }
+    }
+};
+
+// any other rows' piece, with plain loads; load(c): the word of the wires 4g .. 4g + 3
+// of the piece's copy c
+template <class Load>
+__device__ __forceinline__ void weigh_words(const unsigned char* E, int copies, Weighed& t, Load load)
+{
+    const int j = threadIdx.x & 3;
+    for (int k = 0; k < copies; k += 32) {
+        u32 v[8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            v[i] = load(k + 4 * j + i);
+            v[4 + i] = load(k + 16 + 4 * j + i);
+        }
+        t.step(E, k, v);
+    }
+}
+
+__device__ __forceinline__ fp2 Weighed::total() const
+{
+    const int g = (threadIdx.x & 31) >> 2;
+    // lane (g, j): limb g of re (d[m][0, 1]) and im (d[m][2, 3]) of the wires
+    // 4 (2j) + m and 4 (2j + 1) + m; summed over g by halving
+    fp2 v[4][2];
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            v[m][h] = mk(shift_mod((u64)(u32)d[m][h], 8 * g), shift_mod((u64)(u32)d[m][2 + h], 8 * g));
+    auto halve = [](bool up, fp2 a, fp2 b, int o) {   // a of lanes without the bit, b of those with it
+        const fp2 keep = up ? b : a, send = up ? a : b;
+        return mk(keep.re + __shfl_xor_sync(0xffffffffu, send.re, o), keep.im + __shfl_xor_sync(0xffffffffu, send.im, o));
+    };
+    fp2 u[2][2], t[2];
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) u[m][h] = halve(g & 4, v[m][h], v[m + 2][h], 16);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        t[h] = halve(g & 2, u[0][h], u[1][h], 8);
+        t[h] = mk(fold61(t[h].re), fold61(t[h].im));
+    }
+    const fp2 s = halve(g & 1, t[0], t[1], 4);
+    return mk(fold61(s.re), fold61(s.im));
+}
 
 // beta's value: entry 0 after the pending fold
 __device__ __forceinline__ void finish_beta(const Job& J)
@@ -541,79 +708,44 @@ __device__ __forceinline__ void finish_beta(const Job& J)
     st2(J.fin_beta, l2canon(b));
 }
 
-// wires from the copied bytes. CTA = 512 copies, a warp per 32 wires: the planes of
-// eq are the mma's rows, the wires its columns (word loads of four copies' four
-// wires, transposed in registers); partial sums per chunk, the job's last CTA adds
-// them up.
-__global__ void __launch_bounds__(512) finish_bytes_kernel(const Job* __restrict__ jobs)
+// wires from the copied bytes. CTA = J.wpg pieces of 512 copies; partial sums per CTA,
+// the job's last one adds them up.
+__global__ void __maxnreg__(80) finish_bytes_kernel(const Job* __restrict__ jobs)
 {
-    constexpr int kPitch = kFinCopies + 16;
+    extern __shared__ __align__(16) unsigned char rings[];
     __shared__ __align__(16) Job J;
     __shared__ EqParts e;
-    __shared__ __align__(16) unsigned char E[16 * kPitch];
+    __shared__ __align__(16) unsigned char E[2][16 * kPlanePitch];
     __shared__ fp2 ws[16];
     __shared__ bool s_last;
     read_job(jobs, J);
     const int chunk = blockIdx.x;
     if (chunk >= J.chunks) return;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, j = lane & 3;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int kf = J.nf + (J.has_r != 0);
-    const int c0 = chunk * kFinCopies;
-    const int lim = min(J.n_real, 1 << kf) - c0;   // copies of this chunk that count
-    eq_parts(J, chunk, e);
+    const int c0 = chunk * J.wpg * kFinCopies;
+    const int lim = min(min(J.n_real, 1 << kf) - c0, J.wpg * kFinCopies);   // copies that count
+    const int kp = J.stride, warps = blockDim.x >> 5, w0 = 32 * warp;
+    const RowCopies rc = {J.bytes + (size_t)c0 * kp + w0, kp, w0 < kp ? lim : 0, 32,
+                          rings + warp * (kRowStages * kRowStep)};
+    rc.start();
+    eq_parts(J, chunk * J.wpg, J.wpg, e);
     fp2 sum = f2zero();
-    for (int c = tid; c < kFinCopies; c += blockDim.x) {
-        fp2 v = f2zero();
-        if (c < lim) {
-            v = l2canon(eq_of(e, c));
-            sum = l2add(sum, v);
-        }
-#pragma unroll
-        for (int l = 0; l < 8; ++l) {
-            E[l * kPitch + c] = (unsigned char)(v.re >> (8 * l));
-            E[(8 + l) * kPitch + c] = (unsigned char)(v.im >> (8 * l));
-        }
+    Weighed t = {};
+    for (int p = 0; p < J.wpg; ++p) {
+        weight_planes(e, p, lim - p * kFinCopies, E[p & 1], sum);
+        __syncthreads();
+        rc.sum(p, E[p & 1], t);
     }
     sum = warp_sum(l2canon(sum));
     if (lane == 0) ws[warp] = sum;
     __syncthreads();
     const int Wp = J.W_rows;
     fp2* part = J.fpart + (size_t)chunk * Wp;
-    const int kp = J.stride, warps = blockDim.x >> 5;
-    const int steps = min(kFinCopies, (lim + 31) & ~31);
-    for (int wb = warp; 32 * wb < kp; wb += warps) {
-        const unsigned char* src = J.bytes + (size_t)(c0 + 4 * j) * kp + 32 * wb + 4 * g;
-        int d[4][4] = {};
-        for (int k = 0; k < steps; k += 32) {
-            u32 x[4], y[4], b0[4], b1[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                x[i] = *reinterpret_cast<const u32*>(src + (size_t)(k + i) * kp);
-                y[i] = *reinterpret_cast<const u32*>(src + (size_t)(k + 16 + i) * kp);
-            }
-            const unsigned char* er = E + g * kPitch + k + 4 * j;
-            auto word = [](const unsigned char* p) { return *reinterpret_cast<const u32*>(p); };
-            const u32 a0 = word(er), a1 = word(er + 8 * kPitch), a2 = word(er + 16), a3 = word(er + 8 * kPitch + 16);
-            transpose4(x, b0);
-            transpose4(y, b1);
-#pragma unroll
-            for (int m = 0; m < 4; ++m) mma_u8(d[m], a0, a1, a2, a3, b0[m], b1[m]);
-        }
-        // lane (g, j): limb g of re (d[m][0, 1]) and im (d[m][2, 3]) of the wires
-        // 32 wb + 4 (2j) + m and 32 wb + 4 (2j + 1) + m
-#pragma unroll
-        for (int m = 0; m < 4; ++m)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                u64 re = shift_mod((u64)(u32)d[m][h], 8 * g), im = shift_mod((u64)(u32)d[m][2 + h], 8 * g);
-#pragma unroll
-                for (int o = 4; o < 32; o <<= 1) {
-                    re = fold61(re + __shfl_xor_sync(0xffffffffu, re, o));
-                    im = fold61(im + __shfl_xor_sync(0xffffffffu, im, o));
-                }
-                const int w = 32 * wb + 4 * (2 * j + h) + m;
-                if (g == 2 * (m & 1) + h && w < J.cs) stcg2(part + w, l2canon(mk(re, im)));
-            }
+    if (w0 < kp) {
+        const fp2 v = t.total();
+        const int w = w0 + weighed_wire(lane);
+        if (w < J.cs) stcg2(part + w, l2canon(v));
     }
     if (tid == 0) {
         fp2 s = f2zero();
@@ -630,13 +762,115 @@ __global__ void __launch_bounds__(512) finish_bytes_kernel(const Job* __restrict
     __threadfence();
     for (int w = tid; w < J.W; w += blockDim.x) {
         fp2 v = f2zero();
-        if (w < J.cs || (w == J.const_idx && w < Wp))
+        if (w < J.cs || (w == J.const_idx && w < Wp)) {
+#pragma unroll 8
             for (int k = 0; k < J.chunks; ++k) v = f2add(v, ldcg2(J.fpart + (size_t)k * Wp + w));
+        }
         st2(J.fin + w, v);
     }
     if (tid == 0) {
         finish_beta(J);
         *J.ticket = 0u;
+    }
+}
+
+// ---- MLE of a frame's input vector from its bytes -------------------------------
+//   sum_c hi[c] (sum_{w < cs} lo[w] byte(c, w) + const_val lo[const_idx]),
+// lo and hi the eq weights of the point's first h and further hb entries. The copies
+// are summed first, 512 to a CTA, on the tensor cores; what is left is a dot product
+// over the wires. Both weights are made by the CTA that uses them. Bound by reading
+// the bytes and by the weights (64 1080p frames, 398 MB: 133 us; a thread per copy with
+// four 32 x 32 multiplications a byte took 244, its eq tables 110).
+struct MleArgs {
+    const MleFrame* frames;
+    const fp2* points;
+    fp2* partials;
+    unsigned* tickets;
+    fp2* out;
+    u64 const_val;
+    int cs, h, hb, const_idx, pieces;   // pieces: a CTA's, of 512 copies
+};
+
+// kRows: what every frame's rows are: whole aligned 16-byte vectors, words, or bytes
+enum : int { kRowVectors, kRowWords, kRowBytes };
+template <int kRows>
+__global__ void __maxnreg__(80) mle_bytes_kernel(const MleArgs a)
+{
+    extern __shared__ __align__(16) unsigned char rings[];
+    __shared__ EqParts e, el;
+    __shared__ __align__(16) unsigned char E[2][16 * kPlanePitch];
+    __shared__ fp2 ws[16], wt[16];
+    __shared__ bool s_last;
+    const int f = blockIdx.y, chunk = blockIdx.x, per = a.pieces * kFinCopies;
+    const MleFrame fr = a.frames[f];
+    const int chunks = max(1, (fr.n_real + per - 1) / per);
+    if (chunk >= chunks) return;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, warps = blockDim.x >> 5;
+    const int cs = a.cs, w0 = 32 * warp;
+    const int c0 = chunk * per, lim = min(per, fr.n_real - c0);
+    const unsigned char* src = fr.pix + (size_t)c0 * cs + w0;
+    const RowCopies rc = {src, cs, w0 < cs ? lim : 0, cs - w0, rings + warp * (kRowStages * kRowStep)};
+    if (kRows == kRowVectors) rc.start();
+    const fp2* z = a.points + (size_t)f * (a.h + a.hb);
+    for (int k = tid; k < a.h + a.hb; k += blockDim.x) {
+        const fp2 v = ld2(z + k);
+        (k < a.h ? el.r[k] : e.r[k - a.h]) = mk(fold61(v.re), fold61(v.im));
+    }
+    __syncthreads();
+    eq_parts(e, a.hb, chunk * a.pieces, a.pieces);
+    eq_parts(el, a.h, 0, 1);
+    __syncthreads();
+    fp2 sum = f2zero(), acc = f2zero();
+    Weighed bytes = {};
+    for (int p = 0; p < a.pieces; ++p) {
+        const int at = p * kFinCopies;
+        weight_planes(e, p, lim - at, E[p & 1], sum);
+        __syncthreads();
+        if (kRows == kRowVectors)
+            rc.sum(p, E[p & 1], bytes);
+        else if (w0 < cs)
+            weigh_words(E[p & 1], min(kFinCopies, lim - at), bytes, [&](int c) -> u32 {   // rows past the last weigh nothing
+                const int col = 4 * (lane >> 2);
+                const unsigned char* q = src + (size_t)min(at + c, lim - 1) * cs + col;
+                if (kRows == kRowWords) return w0 + col < cs ? __ldg(reinterpret_cast<const u32*>(q)) : 0u;
+                u32 x = 0;
+#pragma unroll
+                for (int b = 0; b < 4; ++b)
+                    if (w0 + col + b < cs) x |= (u32)__ldg(q + b) << (8 * b);
+                return x;
+            });
+    }
+    sum = warp_sum(l2canon(sum));
+    if (lane == 0) ws[warp] = sum;
+    if (w0 < cs) {
+        const fp2 v = bytes.total();
+        const int w = w0 + weighed_wire(lane);
+        if (w < cs) acc = l2mul(eq_of(el, w), v);
+    }
+    acc = warp_sum(l2canon(acc));
+    if (lane == 0) wt[warp] = acc;
+    __syncthreads();
+    if (tid == 0) {
+        fp2 s = f2zero(), t = f2zero();
+        for (int k = 0; k < warps; ++k) {
+            s = f2add(s, ws[k]);
+            t = f2add(t, wt[k]);
+        }
+        if (a.const_idx >= 0) t = l2add(t, l2mul(eq_of(el, a.const_idx), l2canon(f2scale(s, a.const_val))));
+        t = l2canon(t);
+        stcg2(a.partials + (size_t)f * gridDim.x + chunk, t);
+        __threadfence();
+        s_last = atomicAdd(a.tickets + f, 1u) == (unsigned)(chunks - 1);
+    }
+    __syncthreads();
+    if (!s_last || warp != 0) return;
+    __threadfence();
+    fp2 t = f2zero();
+    for (int k = lane; k < chunks; k += 32) t = f2add(t, ldcg2(a.partials + (size_t)f * gridDim.x + k));
+    t = warp_sum(t);
+    if (lane == 0) {
+        st2(a.out + f, t);
+        a.tickets[f] = 0u;
     }
 }
 
@@ -649,7 +883,7 @@ __global__ void __launch_bounds__(kFinCopies) finish_eq_kernel(const Job* __rest
     const int kf = J.nf + (J.has_r != 0);
     const int c = blockIdx.x * kFinCopies + threadIdx.x;
     if ((long long)blockIdx.x * kFinCopies >= (1LL << kf)) return;
-    eq_parts(J, blockIdx.x, e);
+    eq_parts(J, blockIdx.x, 1, e);
     if (c < (1 << kf)) st2(J.fpart + c, eq_of(e, threadIdx.x));
     if (c == 0) finish_beta(J);
 }
@@ -674,6 +908,8 @@ __global__ void __launch_bounds__(kVecThreads) finish_table_kernel(const Job* __
     if (lane == 0) st2(J.fin + w, s);
 }
 
+size_t row_smem(unsigned threads) { return (size_t)(threads / 32) * kRowStages * kRowStep; }
+
 size_t form_smem(int kp) { return (size_t)(2 * kTileRows + 16) * (kp + 16); }
 
 }  // namespace
@@ -690,6 +926,36 @@ int lin_chunks(int n_real, int folds)
     return (int)std::max<long long>(1, (lim + kFinCopies - 1) / kFinCopies);
 }
 
+// Pieces of 512 copies per CTA of the weighted byte sums, chunks: the frames' pieces.
+// What a CTA spends besides its pieces is about one piece's time, and two CTAs fit an
+// SM: the number of pieces with the fewest (pieces + 1) x waves. 64 1080p frames, 2,048
+// pieces: 8 (256 CTAs); one frame or a few small ones: 1.
+int row_pieces(const std::vector<int>& chunks)
+{
+    Ctx* c = ctx();
+    const long long fit = 2LL * (c ? c->n_sm : 148);
+    int best = 1;
+    long long best_cost = 0;
+    for (int p = 1; p <= kMaxPieces; ++p) {
+        long long ctas = 0;
+        for (int k : chunks) ctas += (k + p - 1) / p;
+        const long long cost = (ctas + fit - 1) / fit * (p + 1);
+        if (p == 1 || cost < best_cost) best = p, best_cost = cost;
+    }
+    return best;
+}
+
+void plan_linear_finish(std::vector<Job>& jobs)
+{
+    std::vector<int> chunks;
+    for (const Job& j : jobs) chunks.push_back(j.chunks);
+    const int p = chunks.empty() ? 1 : row_pieces(chunks);
+    for (Job& j : jobs) {
+        j.wpg = p;
+        j.chunks = (j.chunks + p - 1) / p;
+    }
+}
+
 bool prepare_linear_kernels()
 {
     static bool done = false;
@@ -697,6 +963,12 @@ bool prepare_linear_kernels()
     TP_CUDA_OK(cudaFuncSetAttribute(forms_bytes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)form_smem(512)),
                "forms smem attr");
+    TP_CUDA_OK(cudaFuncSetAttribute(finish_bytes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)row_smem(512)),
+               "finish smem attr");
+    TP_CUDA_OK(cudaFuncSetAttribute(mle_bytes_kernel<kRowVectors>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)row_smem(512)),
+               "mle smem attr");
     done = true;
     return true;
 }
@@ -760,6 +1032,63 @@ bool launch_linear_rounds(const Job* d_jobs, int n_jobs, const VoleRounds* v, in
     return !cuda_failed(cudaGetLastError(), "linear rounds launch");
 }
 
+bool launch_mle_pixels_batch(const MleFrame* h_frames, int n, int n_pad, int cs, int W,
+                             int const_idx, u64 const_val, const fp2* d_points, fp2* d_out,
+                             cudaStream_t s, int* launches)
+{
+    if (n <= 0) return true;
+    if (!prepare_linear_kernels()) return false;
+    if ((W & (W - 1)) || (n_pad & (n_pad - 1)) || W > 512 || cs <= 0 || cs > W ||
+        const_idx >= W || (const_idx >= 0 && const_idx < cs) || const_val >= P61) {
+        set_error(TP_ERR_ARG, "mle over bytes: bad layout (wires %d, copies %d, copy_size %d)", W,
+                  n_pad, cs);
+        return false;
+    }
+    MleArgs a = {};
+    size_t bits = (size_t)cs;   // what the rows' addresses have in common
+    std::vector<int> chunks;
+    for (int i = 0; i < n; ++i) {
+        if (!h_frames[i].pix || h_frames[i].n_real < 0 || h_frames[i].n_real > n_pad) {
+            set_error(TP_ERR_ARG, "mle over bytes: frame %d has %d of %d copies", i,
+                      h_frames[i].n_real, n_pad);
+            return false;
+        }
+        chunks.push_back(lin_chunks(h_frames[i].n_real, 30));
+        bits |= reinterpret_cast<size_t>(h_frames[i].pix);
+    }
+    while ((1 << a.h) < W) ++a.h;
+    while ((1 << a.hb) < n_pad) ++a.hb;
+    a.cs = cs;
+    a.const_idx = const_idx;
+    a.const_val = const_val;
+    a.points = d_points;
+    a.out = d_out;
+    const int most = *std::max_element(chunks.begin(), chunks.end());
+    a.pieces = row_pieces(chunks);
+    const int ctas = (most + a.pieces - 1) / a.pieces;
+    const size_t np = (size_t)ctas * n;
+    const size_t bytes = sizeof(fp2) * np + (sizeof(MleFrame) + sizeof(unsigned)) * n;
+    unsigned char* ws = (unsigned char*)dev_alloc(bytes, s);
+    if (!ws) return false;
+    a.partials = reinterpret_cast<fp2*>(ws);
+    MleFrame* d_frames = reinterpret_cast<MleFrame*>(a.partials + np);
+    a.tickets = reinterpret_cast<unsigned*>(d_frames + n);
+    a.frames = d_frames;
+    bool ok = !cuda_failed(cudaMemsetAsync(a.tickets, 0, sizeof(unsigned) * n, s), "mle tickets") &&
+              upload_async(d_frames, h_frames, sizeof(MleFrame) * n, s);
+    if (ok) {
+        const unsigned threads = (unsigned)std::max(64, 32 * ((cs + 31) / 32));   // a warp per 32 wires
+        const dim3 grid((unsigned)ctas, (unsigned)n);
+        if ((bits & 15) == 0) mle_bytes_kernel<kRowVectors><<<grid, threads, row_smem(threads), s>>>(a);
+        else if ((bits & 3) == 0) mle_bytes_kernel<kRowWords><<<grid, threads, 0, s>>>(a);
+        else mle_bytes_kernel<kRowBytes><<<grid, threads, 0, s>>>(a);
+        ++*launches;
+        ok = !cuda_failed(cudaGetLastError(), "mle batch launch");
+    }
+    dev_free(ws, s);
+    return ok;
+}
+
 bool launch_linear_finish(const Job* d_jobs, const std::vector<Job>& jobs, bool bytes, cudaStream_t s, int* launches)
 {
     if (jobs.empty()) return true;
@@ -769,8 +1098,8 @@ bool launch_linear_finish(const Job* d_jobs, const std::vector<Job>& jobs, bool 
             chunks = std::max(chunks, j.chunks);
             kp = std::max(kp, j.stride);
         }
-        const unsigned threads = (unsigned)std::max(64, std::min(512, kp));   // a warp per 32 wires
-        finish_bytes_kernel<<<dim3((unsigned)chunks, (unsigned)jobs.size()), threads, 0, s>>>(d_jobs);
+        const unsigned threads = (unsigned)std::max(64, kp);   // a warp per 32 wires, 512 at most
+        finish_bytes_kernel<<<dim3((unsigned)chunks, (unsigned)jobs.size()), threads, row_smem(threads), s>>>(d_jobs);
         ++*launches;
     } else {
         int kf = 0, w = 1;

@@ -105,139 +105,6 @@ __global__ void __launch_bounds__(kT)
 
 }  // namespace
 
-// Batched MLE: frame blockIdx.y, one thread per copy (16-byte loads of its
-// bytes), hi[c] applied per copy, per-frame last-block reduction.
-__global__ void __launch_bounds__(kT)
-    mle_pixels_batch_kernel(const MleFrame* __restrict__ frames, int cs, int h, int hb,
-                            int const_idx, u64 const_val, const fp2* __restrict__ tabs,
-                            fp2* __restrict__ partials, unsigned* __restrict__ tickets,
-                            fp2* __restrict__ out)
-{
-    __shared__ uint4 los[512];
-    __shared__ fp2 red[kT / 32];
-    __shared__ bool s_last;
-    const int f = blockIdx.y;
-    const MleFrame fr = frames[f];
-    const size_t nt = ((size_t)1 << h) + ((size_t)1 << hb);
-    const fp2* lo = tabs + (size_t)f * nt;
-    const fp2* hi = lo + ((size_t)1 << h);
-    for (int w = threadIdx.x; w < cs; w += blockDim.x) los[w] = split4(l2canon(ld2c(lo + w)));
-    fp2 const_term = f2zero();
-    if (const_idx >= 0) {
-        const fp2 l = ld2c(lo + const_idx);
-        const_term = mk(lmul(l.re, const_val), lmul(l.im, const_val));
-    }
-    __syncthreads();
-    fp2 acc = f2zero();
-    const bool vec = (cs & 15) == 0 && ((reinterpret_cast<size_t>(fr.pix) & 15) == 0);
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < fr.n_real; c += gridDim.x * blockDim.x) {
-        const unsigned char* row = fr.pix + (size_t)c * cs;
-        u64 A0 = 0, A1 = 0, A2 = 0, A3 = 0;
-        if (vec) {
-            const uint4* r4 = reinterpret_cast<const uint4*>(row);
-            for (int q = 0; q < (cs >> 4); ++q) {
-                const uint4 v = __ldg(r4 + q);
-                const u32 words[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                for (int k = 0; k < 16; ++k) {
-                    const u32 x = (words[k >> 2] >> (8 * (k & 3))) & 0xFFu;
-                    const uint4 l = los[16 * q + k];
-                    A0 += (u64)l.x * x;
-                    A1 += (u64)l.y * x;
-                    A2 += (u64)l.z * x;
-                    A3 += (u64)l.w * x;
-                }
-            }
-        } else {
-            for (int w = 0; w < cs; ++w) {
-                const u32 x = __ldg(row + w);
-                const uint4 l = los[w];
-                A0 += (u64)l.x * x;
-                A1 += (u64)l.y * x;
-                A2 += (u64)l.z * x;
-                A3 += (u64)l.w * x;
-            }
-        }
-        const fp2 v = l2add(mk(combine(A0, A1), combine(A2, A3)), const_term);
-        acc = l2add(acc, l2mul(v, ld2c(hi + c)));
-    }
-    acc = warp_sum(l2canon(acc));
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) red[warp] = acc;
-    __syncthreads();
-    if (warp == 0) {
-        fp2 v = lane < (int)(blockDim.x >> 5) ? red[lane] : f2zero();
-        v = warp_sum(v);
-        if (lane == 0) {
-            stcg2(partials + (size_t)f * gridDim.x + blockIdx.x, v);
-            __threadfence();
-            s_last = atomicAdd(tickets + f, 1u) == gridDim.x - 1;
-        }
-    }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    fp2 t = f2zero();
-    for (unsigned i = threadIdx.x; i < gridDim.x; i += blockDim.x)
-        t = f2add(t, ldcg2(partials + (size_t)f * gridDim.x + i));
-    t = warp_sum(t);
-    __syncthreads();
-    if (lane == 0) red[warp] = t;
-    __syncthreads();
-    if (warp == 0) {
-        fp2 v = lane < (int)(blockDim.x >> 5) ? red[lane] : f2zero();
-        v = warp_sum(v);
-        if (lane == 0) {
-            st2(out + f, v);
-            tickets[f] = 0u;
-        }
-    }
-}
-
-bool launch_mle_pixels_batch(const MleFrame* h_frames, int n, int n_pad, int cs, int W,
-                             int const_idx, u64 const_val, const fp2* d_points, fp2* d_out,
-                             cudaStream_t s, int* launches)
-{
-    if (n <= 0) return true;
-    if ((W & (W - 1)) || (n_pad & (n_pad - 1)) || W > 512 || cs <= 0 || cs > W ||
-        const_idx >= W || (const_idx >= 0 && const_idx < cs) || const_val >= P61) {
-        set_error(TP_ERR_ARG, "mle over bytes: bad layout (wires %d, copies %d, copy_size %d)", W,
-                  n_pad, cs);
-        return false;
-    }
-    for (int i = 0; i < n; ++i)
-        if (!h_frames[i].pix || h_frames[i].n_real < 0 || h_frames[i].n_real > n_pad) {
-            set_error(TP_ERR_ARG, "mle over bytes: frame %d has %d of %d copies", i,
-                      h_frames[i].n_real, n_pad);
-            return false;
-        }
-    int h = 0, hb = 0;
-    while ((1 << h) < W) ++h;
-    while ((1 << hb) < n_pad) ++hb;
-    const size_t nt = ((size_t)1 << h) + ((size_t)1 << hb);
-    const unsigned blocks = (unsigned)std::max(1, std::min(64, (n_pad + kT - 1) / kT));
-    const size_t bytes = sizeof(fp2) * (nt * n + (size_t)blocks * n) + sizeof(MleFrame) * n +
-                         sizeof(unsigned) * n + 512;
-    unsigned char* ws = (unsigned char*)dev_alloc(bytes, s);
-    if (!ws) return false;
-    fp2* tabs = reinterpret_cast<fp2*>(ws);
-    fp2* partials = tabs + nt * n;
-    MleFrame* d_frames = reinterpret_cast<MleFrame*>(partials + (size_t)blocks * n);
-    unsigned* tickets = reinterpret_cast<unsigned*>(d_frames + n);
-    bool ok = !cuda_failed(cudaMemsetAsync(tickets, 0, sizeof(unsigned) * n, s), "mle tickets") &&
-              upload_async(d_frames, h_frames, sizeof(MleFrame) * n, s);
-    if (ok) {
-        launch_eq_tables_batch(d_points, h + hb, h, hb, mk(1, 0), tabs, n, s);
-        mle_pixels_batch_kernel<<<dim3(blocks, n), kT, 0, s>>>(d_frames, cs, h, hb, const_idx,
-                                                               const_val, tabs, partials, tickets,
-                                                               d_out);
-        *launches += 2;
-        ok = !cuda_failed(cudaGetLastError(), "mle batch launch");
-    }
-    dev_free(ws, s);
-    return ok;
-}
-
 bool pixsrc_valid(const PixSrc& px, int n_pad, int W)
 {
     if (!px.pix || px.n_real < 0 || px.n_real > n_pad || px.cs <= 0 || px.cs > W || px.cs > 512 ||

@@ -844,6 +844,7 @@ bool plan_finish(Batch* B, fp2* const* d_wires, fp2* const* d_beta, std::vector<
         if (f->linear && !f->forms_done && f->px.pix) fresh.push_back(f);   // their bytes are copied by the forms
         if (!plan_finish_frame(B, f, d_wires ? d_wires[i] : nullptr, d_beta ? d_beta[i] : nullptr, out)) return false;
     }
+    plan_linear_finish(out[1].jobs);
     plan_forms(fresh, forms, c->n_sm);
     return true;
 }
@@ -1188,6 +1189,7 @@ bool batch_finish_frame(Batch* B, int i, fp2* d_wires, fp2* d_beta)
     RoundLaunch fin[kFinishKinds];
     const bool fresh = f->linear && !f->forms_done && f->px.pix;
     if (!plan_finish_frame(B, f, d_wires, d_beta, fin)) return false;
+    plan_linear_finish(fin[1].jobs);
     if (fresh) plan_forms({f}, forms, c->n_sm);
     if (!launch_finishes(B, forms, fin)) return false;
     batch_release(B, i, false);

@@ -355,7 +355,7 @@ class BatchFrameProver:
             native.check(lib, lib.tp_mle_eval_pixels_batch(
                 len(fs), ptrs, ncop, C, L0.copy_size, L0.n_wires, L0.const_idx, L0.const_val,
                 points_dev[C].data_ptr(), out.data_ptr(), s), "mle")
-            launches += 2
+            launches += 1
             if len(self.groups) == 1:
                 self.mle.copy_(out)
             else:
