@@ -56,6 +56,8 @@ struct DevPar {
 __global__ void __launch_bounds__(kThreads) late_kernel(const Args a, const __grid_constant__ late::Gates G)
 {
     __shared__ late::Work w;
+    extern __shared__ uint32_t gates[];   // in shared memory: the lanes' reads of a constant bank would be one by one
+    for (int g = threadIdx.x; g < a.sh.n_gates; g += kThreads) gates[g] = G.g[g];
     const long long i = blockIdx.x;
     const int n = a.sh.n, W = 1 << n;
     late::Frame f;
@@ -78,7 +80,7 @@ __global__ void __launch_bounds__(kThreads) late_kernel(const Args a, const __gr
     f.closing = a.closing ? a.closing + i * (n + 10 + 5 * (a.sh.zk != 0)) : nullptr;
     f.point = a.closing ? a.point + i * (n + nb) : nullptr;
     f.tag = a.closing ? a.tag + i : nullptr;
-    late::run_frame(w, f, a.sh, G.g, DevPar{});
+    late::run_frame(w, f, a.sh, gates, DevPar{});
 }
 
 }  // namespace
@@ -141,7 +143,11 @@ int tp_late_rounds_dev(int n_frames, int n_in_bits, int n_gates, const int* gate
     a.sh.layer = layer;
     a.sh.round0 = round0;
     a.sh.zk = zk ? 1 : 0;
-    late_kernel<<<n_frames, kThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(a, G);
+    constexpr int kGateBytes = (int)sizeof(late::Gates);
+    static const cudaError_t attr =
+        cudaFuncSetAttribute(late_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGateBytes);
+    if (tp::cuda_failed(attr, "late rounds smem attr")) return -1;
+    late_kernel<<<n_frames, kThreads, kGateBytes, reinterpret_cast<cudaStream_t>(stream)>>>(a, G);
     return tp::cuda_failed(cudaGetLastError(), "late rounds") ? -1 : 0;
 }
 

@@ -496,18 +496,24 @@ TP_HD void step_close_sums(Work& w, const Frame& f, const uint32_t* gates, const
     w.red[2][tid] = f2zero();
 }
 
+// per early challenge w its value (Tn) and beta's factor 2 w z + 1 - (w + z) (T); both
+// tables are free by then
+TP_HD void step_close_load(Work& w, const Frame& f, const Shape& sh, int tid)
+{
+    if (tid >= sh.round0) return;
+    const fp2 wk = f.w3[tid * f.w3_stride], zk = f.z2[tid];
+    w.Tn[tid] = wk;
+    w.T[tid] = f2sub(f2add(f2dbl(f2mul(wk, zk)), mk(1, 0)), f2add(wk, zk));
+}
+
 // the equality proof against the last round's value, tau, the proof of knowledge
 // of all round coefficients, the input point and its value proof
 #pragma nv_exec_check_disable
 TP_HD void step_close_tail(Work& w, const Frame& f, const Shape& sh)
 {
     const int n = sh.n, nb = sh.round0;
-    // beta's factor: prod over the early challenges of 2 w z + 1 - (w + z)
     fp2 mz = mk(1, 0);
-    for (int k = 0; k < nb; ++k) {
-        const fp2 wk = f.w3[k * f.w3_stride], zk = f.z2[k];
-        mz = f2mul(mz, f2sub(f2add(f2dbl(f2mul(wk, zk)), mk(1, 0)), f2add(wk, zk)));
-    }
+    for (int k = 0; k < nb; ++k) mz = f2mul(mz, w.T[k]);
     const fp2 tv = f2mul(w.red[0][0], mz);
     warp_sync();
     fs::Writer st(w.st, &w.tx);
@@ -534,7 +540,7 @@ TP_HD void step_close_tail(Work& w, const Frame& f, const Shape& sh)
     // put(["gkr_input_point", [[re, im], ...]]): a string, then every coordinate's two ints
     st.put_label(fs::label_lit("gkr_input_point"));
     for (int k = 0; k < n + nb; ++k) {
-        const fp2 x = k < n ? f2add(w.w[k], f2mul(f2sub(w.w[n + k], w.w[k]), tau)) : f.w3[(k - n) * f.w3_stride];
+        const fp2 x = k < n ? f2add(w.w[k], f2mul(f2sub(w.w[n + k], w.w[k]), tau)) : w.Tn[k - n];
         if (fs::lead()) f.point[k] = x;
         st.absorb_le(0x02 | (x.re << 8), 8);
         st.absorb_le((x.re >> 56) | (0x02 << 8) | (x.im << 16), 8);
@@ -593,7 +599,10 @@ TP_HD void run_frame(Work& w, const Frame& f, const Shape& sh, const uint32_t* g
         if (f.closing) {
             par.one([&] { step_close_commit(w, f, sh); });
             if (!w.bad) {
-                par.all([&](int tid) { step_close_sums(w, f, gates, sh, tid); });
+                par.all([&](int tid) {
+                    step_close_load(w, f, sh, tid);
+                    step_close_sums(w, f, gates, sh, tid);
+                });
                 for (int left = kThreads / 4; left > 0; left >>= 2)
                     par.all([&](int tid) { step_reduce(w, left, tid); });
                 par.one([&] { step_close_tail(w, f, sh); });

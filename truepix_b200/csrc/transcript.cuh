@@ -136,11 +136,10 @@ TP_HD void label_decimal(Label& L, long long v)
         label_push(L, '-');
         v = -v;
     }
-    long long p = 1;
-    while (p <= v / 10) p *= 10;
-    for (; p > 0; p /= 10) {
-        label_push(L, (uint8_t)('0' + (v / p) % 10));
-    }
+    const uint32_t u = (uint32_t)v;   // 32-bit divisions: a 64-bit one costs the device ten times as much
+    uint32_t p = 1;
+    while (p <= u / 10) p *= 10;
+    for (; p > 0; p /= 10) label_push(L, (uint8_t)('0' + u / p % 10));
 }
 
 inline void init(State& s)
@@ -281,24 +280,31 @@ inline void rand_ext(State& s, const uint8_t* label, uint32_t len, uint64_t* re,
 // host form is the state itself.
 //
 // On the device a warp runs it: every lane makes the same calls. What is put gathers
-// in shared memory (TxMem) without being hashed; a draw hashes the whole stretch at
-// once. The message words of all its blocks are known by then, so their schedules
-// are made side by side, one lane per block, and the rounds run on k + w from shared
+// in shared memory (TxMem) without being hashed, a lane writing one byte of it, and a
+// draw's own 70 to 134 bytes are written by all lanes at once (a lane that appended
+// unit by unit spent a third of a round on that chain, and on fetching its code anew
+// each time); a draw hashes the whole stretch at once. The message words of all its
+// blocks are known by then, so their schedules are made side by side, one lane per block, and the rounds run on k + w from shared
 // memory: 31 cycles a round against 49 with the schedule in line. The real limb of a
 // draw does not enter the transcript, so the stretch runs on to the imaginary limb's
 // draw and an even and an odd lane close the two digests in the same instructions,
-// each with its own padding. Per committed round (243 bytes, two draws): ~5.6
-// compressions' rounds one after the other and two schedules, 11 us; a thread that
-// appended byte by byte and hashed block by block took 146 us.
+// each with its own padding. Per committed round (243 bytes, two draws): ~6
+// compressions' rounds one after the other and two schedules; a launch of one round
+// takes 16 us (22 with unit-wise appends; 146 with a thread that appended byte by byte
+// and hashed block by block).
 
 constexpr int kTxUnits = 72;     // 8-byte units a stretch may hold (9 blocks)
 constexpr int kTxBlocks = 8;     // blocks hashed at once, padding included
 
 struct TxMem {
     uint64_t buf[kTxUnits];      // the stretch, from the pending block's first byte
+    uint64_t label[4];           // the draw's label
     uint64_t prev[8];            // the block before it (what a state holds behind its pending bytes)
     uint32_t h[8], h_next[8];    // chaining words in front of the stretch; behind its last whole block
     uint64_t out[2];             // the two digests' low 61 bits
+    uint64_t total, rnum;        // a redrawn draw's end
+    uint32_t n;
+    uint32_t one;                // 1, for sha::AddMad
     __align__(16) uint32_t kw[2 * kTxBlocks][68];   // k + w of block b as digest v closes it: row 2 b + v
 };
 
@@ -312,7 +318,7 @@ static __device__ __noinline__ void tx_hash(TxMem* m, uint32_t n0, uint32_t n1, 
     const uint32_t lane = threadIdx.x & 31, v = lane & 1;
     const int n = (int)(v ? n1 : n0), whole = n >> 6;
     const int blocks = close ? whole + ((n & 63) >= 56 ? 2 : 1) : whole;
-    const sha::AddMad add{sha::kShaOne};
+    const sha::AddMad add{m->one};
     __syncwarp();
     {
         const int b = (int)(lane >> 1);
@@ -331,18 +337,23 @@ static __device__ __noinline__ void tx_hash(TxMem* m, uint32_t n0, uint32_t n1, 
                 w[14] = (uint32_t)(bits >> 32);
                 w[15] = (uint32_t)bits;
             }
-            uint32_t* kw = m->kw[lane];
+            uint4* kw = reinterpret_cast<uint4*>(m->kw[lane]);
 #pragma unroll 1
-            for (int i = 0; i < 48; i += 16)
+            for (int i = 0; i < 64; i += 16) {
 #pragma unroll
-                for (int t = 0; t < 16; ++t) {
-                    kw[i + t] = add(w[t], sha::kShaTables.k[i + t]);
-                    const uint32_t x = w[(t + 1) & 15], y = w[(t + 14) & 15];
-                    w[t] = add(sha::rotr(y, 17) ^ sha::rotr(y, 19) ^ (y >> 10),
-                               add(sha::rotr(x, 7) ^ sha::rotr(x, 18) ^ (x >> 3), add(w[t], w[(t + 9) & 15])));
+                for (int q = 0; q < 4; ++q) {
+                    uint32_t o[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const int t = 4 * q + j;
+                        o[j] = add(w[t], sha::kShaTables.k[i + t]);
+                        const uint32_t x = w[(t + 1) & 15], y = w[(t + 14) & 15];
+                        w[t] = add(sha::rotr(y, 17) ^ sha::rotr(y, 19) ^ (y >> 10),
+                                   add(sha::rotr(x, 7) ^ sha::rotr(x, 18) ^ (x >> 3), add(w[t], w[(t + 9) & 15])));
+                    }
+                    kw[i / 4 + q] = make_uint4(o[0], o[1], o[2], o[3]);
                 }
-#pragma unroll
-            for (int t = 0; t < 16; ++t) kw[48 + t] = add(w[t], sha::kShaTables.k[48 + t]);
+            }
         }
     }
     __syncwarp();
@@ -358,21 +369,15 @@ static __device__ __noinline__ void tx_hash(TxMem* m, uint32_t n0, uint32_t n1, 
         uint32_t s[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) s[i] = st[i];
+        uint4 ka = kw[0], kb = kw[1];
+        // eight rounds a pass: 16 are as fast in a small kernel, but this one's other code
+        // lies between two calls, and their 7 KB are fetched anew each time
 #pragma unroll 1
-        for (int i = 0; i < 16; i += 4) {
-            uint32_t k[16];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const uint4 x = kw[i + q];
-                k[4 * q] = x.x;
-                k[4 * q + 1] = x.y;
-                k[4 * q + 2] = x.z;
-                k[4 * q + 3] = x.w;
-            }
-#pragma unroll
-            for (int t = 0; t < 16; ++t)
-                sha::round_step(s[(0 - t) & 7], s[(1 - t) & 7], s[(2 - t) & 7], s[(3 - t) & 7], s[(4 - t) & 7],
-                                s[(5 - t) & 7], s[(6 - t) & 7], s[(7 - t) & 7], k[t], add);
+        for (int i = 2; i <= 16; i += 2) {
+            const uint4 x = ka, y = kb;
+            ka = kw[i & 15];
+            kb = kw[(i & 15) + 1];
+            sha::eight_rounds(s, x, y, add);
         }
 #pragma unroll
         for (int i = 0; i < 8; ++i) st[i] = add(st[i], s[i]);
@@ -403,84 +408,147 @@ static __device__ __noinline__ void tx_advance(TxMem* m, uint32_t n)
     __syncwarp();
 }
 
+// One limb of a draw put behind the stretch's n bytes: "ext", the label (in m->label),
+// "real" or "imag", [rnum]; 35 + len bytes. No branches: a lane writes one byte of each
+// of three pieces.
+static __device__ __forceinline__ void tx_draw_bytes(TxMem* m, uint32_t n, uint32_t len, uint64_t rnum, int limb)
+{
+    const int i = (int)(threadIdx.x & 31);
+    uint8_t* to = reinterpret_cast<uint8_t*>(m->buf) + n + i;
+    const uint64_t head = i < 8 ? 0x7478650000000304ull : 0x04 | ((uint64_t)len << 8);   // 04, 3, "ext"; 04, len
+    if (i < 13) to[0] = (uint8_t)(head >> (8 * (i & 7)));
+    to += 13;
+    if (i < (int)len) to[0] = reinterpret_cast<const uint8_t*>(m->label)[i];
+    to += len;
+    const uint64_t name = limb ? 0x616d690000000404ull : 0x6165720000000404ull;          // 04, 4, "ima" / "rea"
+    const uint64_t last = (limb ? 'g' : 'l') | 0x010100ull;                               // "g" / "l", 01, 1
+    const uint64_t tail = i < 8 ? name : i < 14 ? last : rnum;
+    if (i < 22) to[0] = (uint8_t)(tail >> (8 * (i < 8 ? i : i < 14 ? i - 8 : i - 14)));
+}
+
+// A draw on the stretch's n bytes: m->out, and the stretch moved on. False when a limb
+// has to be drawn again (nothing moved).
+static __device__ __noinline__ bool tx_draw(TxMem* m, uint32_t n, uint64_t total, uint64_t rnum, uint32_t len)
+{
+    const uint32_t per = 35 + len;
+    __syncwarp();
+    tx_draw_bytes(m, n, len, rnum, 0);
+    tx_draw_bytes(m, n + per, len, rnum + 1, 1);
+    tx_hash(m, n + per, n + 2 * per, total + 2 * per, true);
+    const bool ok = m->out[0] < P61 && m->out[1] < P61;
+    if (ok) tx_advance(m, n + 2 * per);
+    return ok;
+}
+
+// The same limb by limb, each again while it is all ones (probability 2^-61; the loop
+// is bounded all the same, and past the bound the value is reduced).
+static __device__ __noinline__ void tx_redraw(TxMem* m, uint32_t n, uint64_t total, uint64_t rnum, uint32_t len)
+{
+    uint64_t limb[2];
+#pragma unroll 1
+    for (int k = 0; k < 2; ++k) {
+        uint64_t v = 0;
+#pragma unroll 1
+        for (int it = 0; it < 1000; ++it) {
+            __syncwarp();
+            if (it == 0) {
+                tx_draw_bytes(m, n, len, rnum, k);
+                n += 35 + len;
+                total += 35 + len;
+            } else {   // the counter again
+                const int q = threadIdx.x & 31;
+                if (q < 13)
+                    reinterpret_cast<uint8_t*>(m->buf)[n + q] =
+                        (uint8_t)(q < 5 ? 0x0101u >> (8 * q) : rnum >> (8 * (q - 5)));
+                n += 13;
+                total += 13;
+            }
+            ++rnum;
+            tx_hash(m, n, n, total, true);
+            v = m->out[1];
+            tx_advance(m, n);
+            n &= 63;
+            if (v < P61) break;
+        }
+        limb[k] = v % P61;
+    }
+    __syncwarp();
+    if (lead()) {
+        m->out[0] = limb[0];
+        m->out[1] = limb[1];
+        m->total = total;
+        m->rnum = rnum;
+        m->n = n;
+    }
+    __syncwarp();
+}
+
 class Writer {
 public:
     __device__ Writer(const State& s, TxMem* mem) : m(mem), total(s.total), rnum(s.rnum), n(s.nbuf)
     {
         const uint32_t lane = threadIdx.x & 31;
-        cur = n & 7 ? s.unit[n >> 3] & low_bytes(n & 7) : 0;
         __syncwarp();
         if (lane < 8) {
             m->buf[lane] = m->prev[lane] = s.unit[lane];
             m->h[lane] = s.h[lane];
         }
+        if (lead()) m->one = 1;
         __syncwarp();
     }
+    // the low `bytes` bytes of v (1 <= bytes <= 8)
     __device__ void absorb_le(uint64_t v, int bytes)
     {
-        if (bytes < 8) v &= low_bytes(bytes);
-        const int r = (int)(n & 7);
-        cur |= v << (8 * r);
-        total += (uint64_t)bytes;
-        n += (uint32_t)bytes;
-        if (r + bytes >= 8) {
-            if (lead()) m->buf[(n >> 3) - 1] = cur;
-            cur = r ? v >> (8 * (8 - r)) : 0;
-            if (n >= 64 * (kTxBlocks - 1)) take_whole();
-        }
+        const int i = (int)(threadIdx.x & 31);
+        room((uint32_t)bytes);
+        if (i < bytes) byte(i) = (uint8_t)(v >> (8 * i));
+        moved((uint32_t)bytes);
     }
     __device__ void put_fp2(uint64_t re, uint64_t im)
     {
-        absorb_le(0x03 | (re << 8), 8);
-        absorb_le((re >> 56) | (im << 8), 8);
-        absorb_le(im >> 56, 1);
+        const int i = (int)(threadIdx.x & 31);
+        room(17);
+        const uint64_t v = i < 9 ? re : im;
+        if (i < 17) byte(i) = i == 0 ? 0x03 : (uint8_t)(v >> (8 * ((i - 1) & 7)));
+        moved(17);
     }
     __device__ void put_label(const Label& L)
     {
+        const int i = (int)(threadIdx.x & 31), q = i & 7;
         absorb_le(0x04 | ((uint64_t)L.len << 8), 5);
-        const uint64_t w[4] = {L.w0, L.w1, L.w2, L.w3};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int left = (int)L.len - 8 * i;
-            if (left > 0) absorb_le(w[i], left < 8 ? left : 8);
-        }
+        room(32);
+        const uint64_t v = i < 8 ? L.w0 : i < 16 ? L.w1 : i < 24 ? L.w2 : L.w3;
+        if (i < (int)L.len) byte(i) = (uint8_t)(v >> (8 * q));
+        moved(L.len);
     }
     // rand_ext(label)
     __device__ fp2 rand_fp2(const Label& L)
     {
         if (n > 256) take_whole();   // a draw puts at most 134 bytes, its padding at most 72
-        const uint32_t n_start = n;
-        const uint64_t total_start = total, rnum_start = rnum;
-        part(L, label_lit("real"));
-        put_counter();
-        const uint32_t n_real = n;
-        part(L, label_lit("imag"));
-        put_counter();
-        if (lead()) m->buf[n >> 3] = cur;
-        tx_hash(m, n_real, n, total, true);
-        uint64_t re = m->out[0], im = m->out[1];
-        if (re < P61 && im < P61) {
-            tx_advance(m, n);
-            n &= 63;
-            return mk(re, im);
+        if (lead()) {
+            m->label[0] = L.w0;
+            m->label[1] = L.w1;
+            m->label[2] = L.w2;
+            m->label[3] = L.w3;
         }
-        // a limb of all ones is drawn again (probability 2^-60): one after the other
-        n = n_start;
-        total = total_start;
-        rnum = rnum_start;
-        cur = n & 7 ? m->buf[n >> 3] & low_bytes(n & 7) : 0;
-        part(L, label_lit("real"));
-        re = scalar();
-        part(L, label_lit("imag"));
-        im = scalar();
-        return mk(re, im);
+        if (tx_draw(m, n, total, rnum, L.len)) {
+            const uint32_t size = 2 * (35 + L.len);
+            total += size;
+            rnum += 2;
+            n = (n + size) & 63;
+        } else {
+            tx_redraw(m, n, total, rnum, L.len);
+            total = m->total;
+            rnum = m->rnum;
+            n = m->n;
+        }
+        return mk(m->out[0], m->out[1]);
     }
     // the state at this point back to s (lanes 0..7 write)
     __device__ void store(State& s)
     {
         if (n >= 64) take_whole();
         const uint32_t lane = threadIdx.x & 31;
-        if (lead()) m->buf[n >> 3] = cur;
         __syncwarp();
         if (lane < 8) {
             const int k = (int)n - 8 * (int)lane;
@@ -497,17 +565,15 @@ public:
     }
 
 private:
-    __device__ void part(const Label& L, const Label& limb)
+    __device__ uint8_t& byte(int i) { return reinterpret_cast<uint8_t*>(m->buf)[n + i]; }
+    __device__ void room(uint32_t bytes)   // whole blocks leave a stretch before it holds kTxBlocks
     {
-        put_label(label_lit("ext"));
-        put_label(L);
-        put_label(limb);
+        if (n + bytes >= 64 * (kTxBlocks - 1)) take_whole();
     }
-    __device__ void put_counter()
+    __device__ void moved(uint32_t bytes)
     {
-        absorb_le(0x01 | (1ull << 8) | (rnum << 40), 8);
-        absorb_le(rnum >> 24, 5);
-        rnum += 1;
+        n += bytes;
+        total += bytes;
     }
     __device__ void take_whole()
     {
@@ -515,22 +581,8 @@ private:
         tx_advance(m, n);
         n &= 63;
     }
-    __device__ uint64_t scalar()
-    {
-        uint64_t v = 0;
-        for (int it = 0; it < 1000; ++it) {
-            put_counter();
-            if (lead()) m->buf[n >> 3] = cur;
-            tx_hash(m, n, n, total, true);
-            v = m->out[1];
-            tx_advance(m, n);
-            n &= 63;
-            if (v < P61) return v;
-        }
-        return v % P61;
-    }
     TxMem* m;
-    uint64_t total, rnum, cur;   // cur: the unit that is not full yet
+    uint64_t total, rnum;
     uint32_t n;                  // bytes of the stretch
 };
 #else
