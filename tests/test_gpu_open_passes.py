@@ -59,3 +59,25 @@ def test_answer(n):
         native.check(lib, lib.tp_orion_answer_dev(d_x.data_ptr(), n, d_r1.data_ptr(), out.data_ptr(),
                                                   torch.cuda.current_stream().cuda_stream), "answer")
     assert tuple(out.cpu().numpy().view(np.uint64).tolist()) == dot(x.reshape(-1, 2), r1.reshape(-1, 2))
+
+
+@pytest.mark.parametrize("col_len", [1, 2, 3, 130, 300, 16000, 40000])   # 1 to 256 CTAs in the tree's first launch
+def test_combined_tree(col_len):
+    import hashlib
+    import torch
+    from truepix_b200 import native
+    lib = native.gkr()
+    n = 128 * col_len
+    cw = lib.tp_orion_codeword_len(col_len)
+    leaves = lib.tp_orion_tree_leaves(n)
+    d_rows, d_r0 = dev(elements(col_len, 128 * cw)), dev(elements(7, 128))
+    comb = torch.zeros(2 * cw, dtype=torch.int64, device="cuda")
+    tree = torch.full((64 * leaves,), 7, dtype=torch.uint8, device="cuda")
+    native.check(lib, lib.tp_orion_combine_dev(d_rows.data_ptr(), n, d_r0.data_ptr(), comb.data_ptr(), tree.data_ptr(),
+                                               torch.cuda.current_stream().cuda_stream), "combine")
+    x = comb.cpu().numpy().tobytes() + bytes(16 * max(0, leaves - cw))
+    want = [None] * leaves + [hashlib.sha256(x[16 * i:16 * i + 16] + bytes(48)).digest() for i in range(leaves)]
+    for k in range(leaves - 1, 0, -1):
+        want[k] = hashlib.sha256(want[2 * k] + want[2 * k + 1]).digest()
+    t = tree.cpu().numpy().tobytes()
+    assert t[32:] == b"".join(want[1:])

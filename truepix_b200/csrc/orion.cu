@@ -442,7 +442,7 @@ __global__ void __launch_bounds__(sha::kFewThreads) leaf_few_kernel(const ulongl
     const long long r = (long long)blockIdx.x * sha::kFewRows + (threadIdx.x & 31);
     const ulonglong2* p = rows + (r < cw_len ? r : cw_len - 1) * kColumns;
     uint32_t st[8];
-    const bool mine = sha::chain_pair<false>(mem, kColumns / 2, st, sha::AddMad{one}, [&](int n, uint32_t w[8]) {
+    const bool mine = sha::chain_pair<false>(mem, kColumns / 2, st, sha::AddAlu{}, [&](int n, uint32_t w[8]) {
         const ulonglong2 x = ldg16(p + 2 * n), y = ldg16(p + 2 * n + 1);
         sha::fe_words(x.x, x.y, w);
         sha::fe_words(y.x, y.y, w + 4);
@@ -465,9 +465,10 @@ __global__ void fill_leaves_kernel(unsigned char* __restrict__ tree, long long l
 // `levels` tree levels above the n_in nodes at heap positions [n_in, 2 n_in):
 // CTA b reduces the 2^levels nodes from n_in + b * 2^levels to one node
 // (merkle_tree.cpp:64-83: node k = SHA256(node 2k || node 2k + 1)). Bound by the
-// latency of one hash after another up the levels.
+// latency of one hash after another up the levels; Add: build_tree.
+template <class Add>
 __global__ void __launch_bounds__(256) tree_kernel(unsigned char* __restrict__ tree, long long n_in, int levels,
-                                                   uint32_t one)
+                                                   Add add)
 {
     __shared__ uint32_t s[2][256][9];
     const int t = threadIdx.x;
@@ -490,7 +491,7 @@ __global__ void __launch_bounds__(256) tree_kernel(unsigned char* __restrict__ t
             }
             // one copy of the rounds for all levels, so that they stay in the
             // instruction cache (68 us for the 17 levels of a 1080p tree with two)
-            sha::hash64(w, st, sha::AddMad{one});
+            sha::hash64(w, st, add);
 #pragma unroll
             for (int i = 0; i < 8; ++i) s[(lv + 1) & 1][t][i] = st[i];
             store_digest(tree, (base >> 1) + t, st);
@@ -1154,6 +1155,9 @@ bool leaf_digests(const ulonglong2* rows, long long count, unsigned char* digest
 
 bool build_tree(unsigned char* tree, long long leaves, cudaStream_t s)
 {
+    Ctx* c = ctx();
+    if (!c) return false;
+    const long long n_sm = c->n_sm;
     // nine levels per launch
     long long n_in = leaves;
     while (n_in > 1) {
@@ -1161,7 +1165,13 @@ bool build_tree(unsigned char* tree, long long leaves, cudaStream_t s)
         while (levels < 9 && (1LL << (levels + 1)) <= n_in) ++levels;
         const long long blocks = n_in >> levels;
         timer_begin(s, kTagTree);
-        tree_kernel<<<(unsigned)blocks, 1 << (levels - 1), 0, s>>>(tree, n_in, levels, 1u);
+        // With more CTAs than SMs the lowest level's warps share the schedulers, and
+        // the additions are better off that pipe; else a level is one hash's latency
+        // (opening of a 1080p frame, two trees of 256 CTAs and 1: 65 us against 75 with
+        // plain additions throughout; a 2^16 Reed-Solomon commit's 15 trees: 394 against 356).
+        const unsigned threads = 1u << (levels - 1);
+        if (blocks > n_sm) tree_kernel<<<(unsigned)blocks, threads, 0, s>>>(tree, n_in, levels, sha::AddMad{1u});
+        else tree_kernel<<<(unsigned)blocks, threads, 0, s>>>(tree, n_in, levels, sha::AddAlu{});
         timer_end(s);
         if (!launch_ok("merkle tree")) return false;
         n_in >>= levels;

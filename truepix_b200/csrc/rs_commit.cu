@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(sha::kFewThreads) pair_leaf_few_kernel(const u
     const long long t = (long long)blockIdx.x * sha::kFewRows + (threadIdx.x & 31);
     const ulonglong2* p = src + (t < n_leaves ? t : n_leaves - 1) * leaf_step;
     uint32_t st[8];
-    const bool mine = sha::chain_pair<true>(mem, kSlices, st, sha::AddMad{one}, [&](int n, uint32_t w[8]) {
+    const bool mine = sha::chain_pair<true>(mem, kSlices, st, sha::AddAlu{}, [&](int n, uint32_t w[8]) {
         const ulonglong2 x = __ldg(p + n * slice_step), y = __ldg(p + n * slice_step + y_off);
         sha::fe_words(x.x, x.y, w);
         sha::fe_words(y.x, y.y, w + 4);

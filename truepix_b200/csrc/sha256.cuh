@@ -150,8 +150,6 @@ __host__ __device__ __forceinline__ void compress_pad64(uint32_t st[8], Add add)
 #ifdef __CUDACC__
 // round constants (and the padding block's k + w) for the device's compact form
 static __constant__ Tables kShaTables = make_tables();
-// AddMad's `one` where no launch hands it in
-static __constant__ uint32_t kShaOne = 1u;
 
 // One round. The additions are grouped so that behind e only Sigma1 and two of them
 // stand before the next e, and behind a Sigma0 and one before the next a; no group
@@ -171,6 +169,22 @@ __device__ __forceinline__ void round_step(uint32_t a, uint32_t b, uint32_t c, u
     const uint32_t t1 = add(s1, add(ch, add(h, kw)));
     d = add(d, t1);
     h = add(s0, add(mj, t1));
+}
+
+// The same on plain additions, three operands to one: behind e only Sigma1 and one of
+// them; its 15 instructions a round keep the ALU pipe busy for 30 cycles, and one warp
+// alone takes 30.6 (32.1 with the form above, which is ahead from three warps a
+// scheduler on: 103 against 105 at four, 145 against 157 at six).
+__device__ __forceinline__ void round_step(uint32_t a, uint32_t b, uint32_t c, uint32_t& d, uint32_t e, uint32_t f,
+                                           uint32_t g, uint32_t& h, uint32_t kw, AddAlu)
+{
+    const uint32_t s1 = rotr(e, 6) ^ rotr(e, 11) ^ rotr(e, 25);
+    const uint32_t ch = (e & f) ^ (~e & g);
+    const uint32_t s0 = rotr(a, 2) ^ rotr(a, 13) ^ rotr(a, 22);
+    const uint32_t mj = (a & b) ^ (a & c) ^ (b & c);
+    const uint32_t hk = h + kw, dk = d + hk, u = s0 + mj + hk;
+    d = s1 + ch + dk;
+    h = s1 + ch + u;
 }
 
 // Sixteen rounds from round i0 (a multiple of 16); kUpdate: each schedule word is

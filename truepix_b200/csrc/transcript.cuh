@@ -304,7 +304,6 @@ struct TxMem {
     uint64_t out[2];             // the two digests' low 61 bits
     uint64_t total, rnum;        // a redrawn draw's end
     uint32_t n;
-    uint32_t one;                // 1, for sha::AddMad
     __align__(16) uint32_t kw[2 * kTxBlocks][68];   // k + w of block b as digest v closes it: row 2 b + v
 };
 
@@ -318,7 +317,7 @@ static __device__ __noinline__ void tx_hash(TxMem* m, uint32_t n0, uint32_t n1, 
     const uint32_t lane = threadIdx.x & 31, v = lane & 1;
     const int n = (int)(v ? n1 : n0), whole = n >> 6;
     const int blocks = close ? whole + ((n & 63) >= 56 ? 2 : 1) : whole;
-    const sha::AddMad add{m->one};
+    const sha::AddAlu add;
     __syncwarp();
     {
         const int b = (int)(lane >> 1);
@@ -493,7 +492,6 @@ public:
             m->buf[lane] = m->prev[lane] = s.unit[lane];
             m->h[lane] = s.h[lane];
         }
-        if (lead()) m->one = 1;
         __syncwarp();
     }
     // the low `bytes` bytes of v (1 <= bytes <= 8)
