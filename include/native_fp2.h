@@ -172,6 +172,13 @@ int tp_batch_set_pixels(void* batch, int i, int n_gates, const int* gate_type, c
                         const int* in1, const uint64_t* z1_real, const uint64_t* z1_imag,
                         const void* d_pixels, int n_copies, int n_copies_padded, int copy_size,
                         int n_wires, int const_idx, uint64_t const_val, const void* d_beta);
+/* every frame of the batch at once, all of one circuit: frame i's weights z1[i] =
+   {real[n_gates], imag[n_gates]}, pixels, copy counts and beta; as tp_batch_set_pixels
+   for each in turn (no frame is set when one is refused) */
+int tp_batch_set_pixels_all(void* batch, int n_gates, const int* gate_type, const int* in0, const int* in1,
+                            const uint64_t* z1, const void* const* d_pixels, const int* n_copies,
+                            const int* n_copies_padded, int copy_size, int n_wires, int const_idx,
+                            uint64_t const_val, const void* const* d_betas);
 /* frame i from a packed device table (borrow as in tp_early_create_dev) */
 int tp_batch_set_table(void* batch, int i, int n_gates, const int* gate_type, const int* in0,
                        const int* in1, const uint64_t* z1_real, const uint64_t* z1_imag,

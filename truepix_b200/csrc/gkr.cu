@@ -516,12 +516,11 @@ bool build_gate_form(int n_gates, const int* type, const int* in0, const int* in
     return true;
 }
 
-bool upload_gate_form(const GateForm& g, DevGateForm& d, cudaStream_t s)
+void pack_gate_form(const GateForm& g, DevGateForm& d, std::vector<unsigned char>& h)
 {
     d.K0 = g.K0;
     d.n_wires = (int)g.L.size();
     d.n_terms = (int)g.tc.size();
-    // one upload: L, then the terms' coefficients and wires, then the groups
     std::vector<int> gptr, gb;
     for (int i = 0; i < d.n_terms; ++i)
         if (i == 0 || g.tb[(size_t)i] != g.tb[(size_t)i - 1]) {
@@ -530,30 +529,48 @@ bool upload_gate_form(const GateForm& g, DevGateForm& d, cudaStream_t s)
         }
     d.groups = (int)gb.size();
     gptr.push_back(d.n_terms);
-    const size_t oL = 0, oc = oL + sizeof(fp2) * g.L.size(), oab = oc + sizeof(fp2) * g.tc.size(),
-                 op = oab + sizeof(int2) * g.tc.size(), ob = op + sizeof(int) * gptr.size(),
-                 bytes = ob + sizeof(int) * gb.size();
-    if (bytes > d.cap) {
+    // L, then the terms' coefficients and wires, then the groups; whole 16 bytes
+    h.resize((h.size() + 15) & ~(size_t)15);
+    auto put = [&](const void* p, size_t bytes) {
+        const size_t at = h.size();
+        h.resize(at + bytes);
+        if (bytes) memcpy(h.data() + at, p, bytes);
+        return at;
+    };
+    d.at[0] = put(g.L.data(), sizeof(fp2) * g.L.size());
+    d.at[1] = put(g.tc.data(), sizeof(fp2) * g.tc.size());
+    d.at[2] = h.size();
+    for (int i = 0; i < d.n_terms; ++i) {
+        const int2 ab = make_int2(g.ta[(size_t)i], g.tb[(size_t)i]);
+        put(&ab, sizeof ab);
+    }
+    d.at[3] = put(gptr.data(), sizeof(int) * gptr.size());
+    d.at[4] = put(gb.data(), sizeof(int) * gb.size());
+}
+
+void place_gate_form(DevGateForm& d, void* base)
+{
+    unsigned char* m = static_cast<unsigned char*>(base);
+    d.L = reinterpret_cast<fp2*>(m + d.at[0]);
+    d.c = reinterpret_cast<fp2*>(m + d.at[1]);
+    d.ab = reinterpret_cast<int2*>(m + d.at[2]);
+    d.gptr = reinterpret_cast<int*>(m + d.at[3]);
+    d.gb = reinterpret_cast<int*>(m + d.at[4]);
+}
+
+bool upload_gate_form(const GateForm& g, DevGateForm& d, cudaStream_t s)
+{
+    std::vector<unsigned char> h;
+    pack_gate_form(g, d, h);
+    if (h.size() > d.cap) {
         dev_free(d.mem, s);
         d.cap = 0;
-        d.mem = dev_alloc(bytes, s);
+        d.mem = dev_alloc(h.size(), s);
         if (!d.mem) return false;
-        d.cap = bytes;
+        d.cap = h.size();
     }
-    unsigned char* m = static_cast<unsigned char*>(d.mem);
-    d.L = reinterpret_cast<fp2*>(m + oL);
-    d.c = reinterpret_cast<fp2*>(m + oc);
-    d.ab = reinterpret_cast<int2*>(m + oab);
-    d.gptr = reinterpret_cast<int*>(m + op);
-    d.gb = reinterpret_cast<int*>(m + ob);
-    std::vector<unsigned char> h(bytes);
-    memcpy(h.data() + oL, g.L.data(), sizeof(fp2) * g.L.size());
-    if (d.n_terms) memcpy(h.data() + oc, g.tc.data(), sizeof(fp2) * g.tc.size());
-    int2* ab = reinterpret_cast<int2*>(h.data() + oab);
-    for (int i = 0; i < d.n_terms; ++i) ab[i] = make_int2(g.ta[(size_t)i], g.tb[(size_t)i]);
-    memcpy(h.data() + op, gptr.data(), sizeof(int) * gptr.size());
-    if (d.groups) memcpy(h.data() + ob, gb.data(), sizeof(int) * gb.size());
-    return upload_async(d.mem, h.data(), bytes, s);
+    place_gate_form(d, d.mem);
+    return upload_async(d.mem, h.data(), h.size(), s);
 }
 
 void free_gate_form(DevGateForm& d, cudaStream_t s)

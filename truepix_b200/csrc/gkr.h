@@ -36,9 +36,13 @@ struct DevGateForm {
     int n_terms = 0;
     int n_wires = 0;
     int groups = 0;
-    void* mem = nullptr;
+    size_t at[5] = {};     // the arrays' offsets in their block
+    void* mem = nullptr;   // the form's own block
     size_t cap = 0;
 };
+// the form's arrays appended to a host block (d.at), and found in its device copy
+void pack_gate_form(const GateForm& g, DevGateForm& d, std::vector<unsigned char>& h);
+void place_gate_form(DevGateForm& d, void* base);
 bool upload_gate_form(const GateForm& g, DevGateForm& d, cudaStream_t s);
 void free_gate_form(DevGateForm& d, cudaStream_t s);
 
@@ -101,6 +105,8 @@ struct Batch {
     void* d_patch = nullptr;   // (job, device challenge) pairs patched into the job array
     size_t cap_patch = 0;
     int launches = 0;
+    void* forms = nullptr;     // all frames' forms, set in one call
+    size_t cap_forms = 0;
     // the graph path (batch_vole_rounds_graph): every round's jobs in one device
     // table, uploaded from a pinned stage, and the captured graph of the rounds
     Job* d_table = nullptr;
@@ -124,6 +130,10 @@ bool batch_load_host(Batch* B, int i, const u64* v_re, const u64* v_im, const u6
                      const u64* b_im);
 bool batch_load_device(Batch* B, int i, const fp2* d_values, const fp2* d_beta, bool borrow);
 bool batch_load_pixels(Batch* B, int i, const PixSrc& px, const fp2* d_beta);
+// every frame of a batch at once, all of one circuit: frame i from z1[i] = {real[n_gates],
+// imag[n_gates]}, px[i], n_copies[i] and d_betas[i]
+bool batch_set_pixels_all(Batch* B, int n_gates, const int* type, const int* in0, const int* in1, const u64* z1,
+                          const PixSrc* px, const int* n_copies, int n_wires, const fp2* const* d_betas);
 // claims of all unfinished frames; d_claims[i] (8 u64, device) or the frame's slot
 bool batch_claim(Batch* B, u64* const* d_claims);
 bool batch_fold(Batch* B, int i, fp2 r);

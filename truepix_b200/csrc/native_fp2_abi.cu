@@ -491,6 +491,32 @@ int tp_batch_set_pixels(void* batch, int i, int n_gates, const int* gate_type, c
     return tp::batch_load_pixels(B, i, px, static_cast<const fp2*>(d_beta)) ? 0 : -1;
 }
 
+int tp_batch_set_pixels_all(void* batch, int n_gates, const int* gate_type, const int* in0, const int* in1,
+                            const uint64_t* z1, const void* const* d_pixels, const int* n_copies,
+                            const int* n_copies_padded, int copy_size, int n_wires, int const_idx, uint64_t const_val,
+                            const void* const* d_betas)
+{
+    tp::clear_error();
+    if (!batch) return -1;
+    tp::Batch* B = static_cast<tp::Batch*>(batch);
+    if (!gate_type || !in0 || !in1 || !z1 || !d_pixels || !n_copies || !n_copies_padded || !d_betas) {
+        tp::set_error(tp::TP_ERR_ARG, "tp_batch_set_pixels_all: null argument");
+        return -1;
+    }
+    std::vector<tp::PixSrc> px(B->frames.size());
+    for (size_t i = 0; i < px.size(); ++i) {
+        px[i].pix = static_cast<const unsigned char*>(d_pixels[i]);
+        px[i].n_real = n_copies[i];
+        px[i].cs = copy_size;
+        px[i].const_idx = const_idx;
+        px[i].const_val = const_val;
+    }
+    return tp::batch_set_pixels_all(B, n_gates, gate_type, in0, in1, U(z1), px.data(), n_copies_padded, n_wires,
+                                    reinterpret_cast<const tp::fp2* const*>(d_betas))
+               ? 0
+               : -1;
+}
+
 int tp_batch_set_table(void* batch, int i, int n_gates, const int* gate_type, const int* in0,
                        const int* in1, const uint64_t* z1_real, const uint64_t* z1_imag,
                        int n_copies, int n_wires, const void* d_values, const void* d_beta,

@@ -232,9 +232,24 @@ class BatchFrameProver:
         self.fin_beta = torch.zeros(self.B * 2, dtype=i64, device=self.dev)
         self.mle = torch.zeros(self.B * 2, dtype=i64, device=self.dev)
         self.launches_last = 0
+        self._group_index = {C: torch.tensor(fs, dtype=i64, device=self.dev) for C, fs in self.groups.items()}
+        self._copies = np.array([L.copies for L in self.layouts], np.int32)
+        self._padded = np.array([L.padded_copies for L in self.layouts], np.int32)
         self.handle = self.lib.tp_batch_create(self.B, self._s())
         if not self.handle:
             native.check(self.lib, -1, "batch_create")
+
+    def _gate_weights(self, z1s):
+        """the frames' z1 as one array [B, 2, n_gates]"""
+        G = self.gt.size
+        zs = [z1s[f] for f in range(self.B)]
+        if all(type(z) is np.ndarray and z.dtype == np.uint64 and z.shape == (2, G) for z in zs):
+            return np.stack(zs)
+        out = np.empty((self.B, 2, G), np.uint64)
+        for f, z in enumerate(zs):
+            for part in (0, 1):
+                out[f, part] = np.asarray(z[part], np.uint64).reshape(-1)[:G]
+        return out
 
     def __del__(self):
         try:
@@ -288,16 +303,15 @@ class BatchFrameProver:
             for q, f in enumerate(fs):
                 beta_of[f] = self.betas[C].data_ptr() + 16 * C * q
         lib.tp_batch_reset(b)
-        keep = []
-        quick = native.gkr_launcher()     # per-frame setup calls keep the interpreter lock
-        for f, L in enumerate(self.layouts):
-            z1r = np.ascontiguousarray(z1s[f][0], np.uint64)
-            z1i = np.ascontiguousarray(z1s[f][1], np.uint64)
-            keep += [z1r, z1i]
-            native.check(lib, quick.tp_batch_set_pixels(
-                b, f, self.gt.size, self.gt.ctypes.data, self.i0.ctypes.data, self.i1.ctypes.data,
-                z1r.ctypes.data, z1i.ctypes.data, pixels[f].data_ptr(), L.copies, L.padded_copies,
-                L.copy_size, L.n_wires, L.const_idx, L.const_val, beta_of[f]), "batch_set_pixels")
+        L = self.layouts[0]
+        z1 = self._gate_weights(z1s)
+        pix = np.array([pixels[f].data_ptr() for f in range(self.B)], np.uint64)
+        betas = np.array([beta_of[f] for f in range(self.B)], np.uint64)
+        native.check(lib, lib.tp_batch_set_pixels_all(
+            b, self.gt.size, self.gt.ctypes.data, self.i0.ctypes.data, self.i1.ctypes.data, z1.ctypes.data,
+            pix.ctypes.data, self._copies.ctypes.data, self._padded.ctypes.data, L.copy_size, L.n_wires, L.const_idx,
+            L.const_val, betas.ctypes.data), "batch_set_pixels")
+        launches += 1
         base = self.claims.data_ptr()
         use_graph = graph and transcripts is not None and vole is not None and self.stream is not None
         if transcripts is not None:
@@ -359,8 +373,7 @@ class BatchFrameProver:
             if len(self.groups) == 1:
                 self.mle.copy_(out)
             else:
-                for q, f in enumerate(fs):
-                    self.mle[2 * f:2 * f + 2].copy_(out[2 * q:2 * q + 2])
+                self.mle.view(-1, 2).index_copy_(0, self._group_index[C], out.view(-1, 2))
         self.launches_last = launches
 
     def prove_late(self, z1s, challenges=None, transcripts=None, vole=None, layer: int = 0, zk: bool = False) -> None:
@@ -379,13 +392,13 @@ class BatchFrameProver:
         torch, lib, s = self.torch, self.lib, self._s()
         n = int(math.log2(self.W))
         G = self.gt.size
-        zg = np.stack([np.stack([np.asarray(z[0], np.uint64), np.asarray(z[1], np.uint64)], axis=1)
-                       for z in z1s]).reshape(-1)
+        zg = torch.empty(self.B * G * 2, dtype=torch.int64, pin_memory=True)
+        zg.numpy().view(np.uint64).reshape(self.B, G, 2)[...] = self._gate_weights(z1s).transpose(0, 2, 1)
         # uploads on the launch stream, so that the kernel is ordered after them
         def on_stream():
             return torch.cuda.stream(self.stream) if self.stream is not None else contextlib.nullcontext()
         with on_stream():    # from pinned memory, asynchronously: no wait for the launch stream to drain
-            d_zg = torch.from_numpy(zg.view(np.int64)).pin_memory().to(self.dev, non_blocking=True)
+            d_zg = zg.to(self.dev, non_blocking=True)
         i64 = torch.int64
         with on_stream():
             self.late_coefs = torch.zeros(self.B * 2 * n * 3 * 2, dtype=i64, device=self.dev)

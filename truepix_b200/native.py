@@ -57,6 +57,7 @@ GKR_SIGNATURES = {
     "tp_batch_create": (_VP, [_I32, _VP]),
     "tp_batch_set_pixels": (_I32, [_VP, _I32, _I32, _VP, _VP, _VP, _VP, _VP, _VP, _I32, _I32, _I32,
                                    _I32, _I32, _U64, _VP]),
+    "tp_batch_set_pixels_all": (_I32, [_VP, _I32, _VP, _VP, _VP, _VP, _VP, _VP, _VP, _I32, _I32, _I32, _U64, _VP]),
     "tp_batch_set_table": (_I32, [_VP, _I32, _I32, _VP, _VP, _VP, _VP, _VP, _I32, _I32, _VP, _VP,
                                   _I32]),
     "tp_batch_claim": (_I32, [_VP, _VP]),
