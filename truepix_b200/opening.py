@@ -164,24 +164,37 @@ def opening_proof(committer, f: int, point, polynomial: str = None, stream=None)
     s = stream.cuda_stream if stream is not None else torch.cuda.current_stream(dev).cuda_stream
     as_dev = lambda a: torch.from_numpy(np.ascontiguousarray(a[:, ::-1]).view(np.int64).reshape(-1).copy()).to(dev)
     d_r0, d_r1 = as_dev(r0), as_dev(r1)          # (img, real), the codeword's element order
-    comb = torch.empty(2 * cw_len, dtype=torch.int64, device=dev)
+    # what the file needs of the device, side by side for one copy back: the combined
+    # codeword, the answer, the queried columns and both trees' siblings (their roots
+    # behind them), taken on the device instead of downloading the trees
+    col_q = np.ascontiguousarray(col_q, np.int64)
+    nodes = np.empty(qc * (leaves.bit_length() - 1) + 1, np.int32)
+    n = lib.tp_orion_path_nodes(leaves, col_q.ctypes.data, qc, nodes.ctypes.data, nodes.size - 1)
+    native.check(lib, 0 if n >= 0 else -1, "tp_orion_path_nodes")
+    nodes[n] = 1
+    sizes = (2 * cw_len, 2, 2 * COLUMN_SIZE * qc, 4 * (n + 1), 4 * (n + 1))
+    out = torch.empty(sum(sizes), dtype=torch.int64, device=dev)
+    comb, ans, cols, com_digs, comb_digs = out.split(sizes)
     ctree = torch.empty(64 * leaves, dtype=torch.uint8, device=dev)
-    ans = torch.empty(2, dtype=torch.int64, device=dev)
-    q = torch.tensor(col_q, dtype=torch.int64, device=dev)
-    cols = torch.empty(2 * COLUMN_SIZE * qc, dtype=torch.int64, device=dev)
+    q, idx = torch.from_numpy(col_q).to(dev), torch.from_numpy(nodes[:n + 1]).to(dev)
     rows = (committer.mask_rows[f] if mask else committer.rows[f]).data_ptr()
+    tree = committer.mask_trees[f] if mask else committer.trees[f]
     native.check(lib, lib.tp_orion_combine_dev(rows, N, d_r0.data_ptr(), comb.data_ptr(), ctree.data_ptr(), s),
                  "tp_orion_combine_dev")
     native.check(lib, lib.tp_orion_answer_dev(comb.data_ptr(), msg_len, d_r1.data_ptr(), ans.data_ptr(), s),
                  "tp_orion_answer_dev")
     native.check(lib, lib.tp_orion_query_columns_dev(rows, N, q.data_ptr(), qc, cols.data_ptr(), s),
                  "tp_orion_query_columns_dev")
+    for t, digs in ((tree, com_digs), (ctree, comb_digs)):
+        native.check(lib, lib.tp_orion_gather_nodes_dev(t.data_ptr(), 2 * leaves, idx.data_ptr(), n + 1,
+                                                        digs.data_ptr(), s), "tp_orion_gather_nodes_dev")
     if stream is not None:
         stream.synchronize()
     torch.cuda.synchronize(dev)
-    combined = comb.cpu().numpy().view(np.uint64).reshape(cw_len, 2)
-    tree = (committer.mask_trees[f] if mask else committer.trees[f]).cpu().numpy().reshape(-1, 32)
-    ct = ctree.cpu().numpy().reshape(-1, 32)
-    return opening_bytes(N, msg_len, cw_len, ans.cpu().numpy().view(np.uint64), com_root, ct[1].tobytes(), col_q,
-                         cols.cpu().numpy().view(np.uint64), combined, merkle_siblings(tree, leaves, col_q),
-                         merkle_siblings(ct, leaves, col_q), use_group1=0 if mask else 1)
+    host = torch.empty(out.numel(), dtype=torch.int64, pin_memory=True)
+    host.copy_(out)
+    h_comb, h_ans, h_cols, h_com, h_cdigs = (x.numpy() for x in host.split(sizes))
+    h_com, h_cdigs = h_com.view(np.uint8).reshape(-1, 32), h_cdigs.view(np.uint8).reshape(-1, 32)
+    return opening_bytes(N, msg_len, cw_len, h_ans.view(np.uint64), com_root, h_cdigs[n].tobytes(), col_q,
+                         h_cols.view(np.uint64), h_comb.view(np.uint64), (nodes[:n], h_com[:n]),
+                         (nodes[:n], h_cdigs[:n]), use_group1=0 if mask else 1)
