@@ -76,3 +76,52 @@ def test_mle(cs, const, W, n_pad, counts, offset, extreme):
             s = sum(v[0] for v in hi) % P61, sum(v[1] for v in hi) % P61
             terms.append(mul(lo[const], mul(s, (const_val, 0))))
         assert got[f] == [sum(t[0] for t in terms) % P61, sum(t[1] for t in terms) % P61], f
+
+
+def test_slots():
+    """the values placed at given indices; a negative one is refused"""
+    import torch
+    from truepix_b200 import native
+    lib = native.gkr()
+    rng = np.random.default_rng(5)
+    x = torch.from_numpy(rng.integers(0, 256, (3, 4 * 16), dtype=np.uint8)).cuda()
+    z = torch.from_numpy(rng.integers(0, P61, (3, 6, 2)).astype(np.int64)).cuda()
+    s = torch.cuda.current_stream().cuda_stream
+    args = (3, (ctypes.c_void_p * 3)(*[x[i].data_ptr() for i in range(3)]), (ctypes.c_int * 3)(4, 3, 4), 4, 16, 16, -1, 0,
+            z.data_ptr())
+    a = torch.zeros(3, 2, dtype=torch.int64, device="cuda")
+    b = torch.full((7, 2), -1, dtype=torch.int64, device="cuda")
+    native.check(lib, lib.tp_mle_eval_pixels_batch(*args, a.data_ptr(), s), "mle")
+    native.check(lib, lib.tp_mle_eval_pixels_batch_at(*args, (ctypes.c_int * 3)(6, 0, 3), b.data_ptr(), s), "mle at")
+    assert torch.equal(b[[6, 0, 3]], a) and bool((b[[1, 2, 4, 5]] == -1).all())
+    assert lib.tp_mle_eval_pixels_batch_at(*args, (ctypes.c_int * 3)(0, -1, 2), b.data_ptr(), s) != 0
+
+
+def test_beside_the_rounds(monkeypatch):
+    """MLEs on a stream of their own (large batches) and behind the rounds: the same
+    values in two passes over different bytes, for one padded size and for two"""
+    import torch
+    from truepix_b200.frame import BatchFrameProver, FrameLayout
+    rng = np.random.default_rng(9)
+    G = 300
+    gt, i0, i1 = rng.choice([1, 2, 3], size=G), rng.integers(0, 384, G), rng.integers(0, 384, G)
+    for counts in ([100, 128, 90], [100, 60, 128, 33]):
+        layouts = [FrameLayout(copies=c, copy_size=384, const_idx=400, const_val=7) for c in counts]
+        got = {}
+        for aside in (False, True):
+            monkeypatch.setattr(BatchFrameProver, "MLE_ASIDE", 1 if aside else 1 << 62)
+            p = BatchFrameProver(layouts, gt, i0, i1)
+            rng = np.random.default_rng(11)
+            field = lambda *shape: rng.integers(0, P61, shape).astype(np.int64)
+            for _ in range(2):
+                pix = [torch.from_numpy(rng.integers(0, 256, c * 384, dtype=np.uint8)).cuda() for c in counts]
+                z1 = [field(2, G).astype(np.uint64) for _ in counts]
+                z2, pt = {}, {}
+                for C, fs in p.groups.items():
+                    nb = C.bit_length() - 1
+                    z2[C] = torch.from_numpy(field(len(fs), nb, 2)).cuda()
+                    pt[C] = torch.from_numpy(field(len(fs), layouts[0].n_in_bits + nb, 2)).cuda()
+                p.prove(pix, z1, z2, pt, field(p.max_rounds, len(counts), 2).astype(np.uint64))
+                got.setdefault(aside, []).append((p.mle.cpu(), p.claims.cpu(), p.wires.cpu()))
+        for a, b in zip(got[False], got[True]):
+            assert all(torch.equal(x, y) for x, y in zip(a, b))

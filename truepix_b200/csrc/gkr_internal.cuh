@@ -210,7 +210,7 @@ bool launch_beta_batch(const fp2* d_z, int n_z, int n, fp2* d_out, cudaStream_t 
 struct MleFrame {
     const unsigned char* pix;
     int n_real;
-    int pad_;
+    int slot;   // where its value goes
 };
 bool launch_mle_pixels_batch(const MleFrame* h_frames, int n, int n_pad, int cs, int W,
                              int const_idx, u64 const_val, const fp2* d_points, fp2* d_out,

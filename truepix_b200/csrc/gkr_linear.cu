@@ -889,7 +889,7 @@ __global__ void __maxnreg__(80) mle_bytes_kernel(const MleArgs a)
     for (int k = lane; k < chunks; k += 32) t = f2add(t, ldcg2(a.partials + (size_t)f * gridDim.x + k));
     t = warp_sum(t);
     if (lane == 0) {
-        st2(a.out + f, t);
+        st2(a.out + fr.slot, t);
         a.tickets[f] = 0u;
     }
 }

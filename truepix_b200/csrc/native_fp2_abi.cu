@@ -694,6 +694,14 @@ int tp_mle_eval_pixels_batch(int n_frames, const void* const* d_pixels, const in
                              int n_copies_padded, int copy_size, int n_wires, int const_idx,
                              uint64_t const_val, const void* d_points, void* d_out, void* stream)
 {
+    return tp_mle_eval_pixels_batch_at(n_frames, d_pixels, n_copies, n_copies_padded, copy_size, n_wires, const_idx,
+                                       const_val, d_points, nullptr, d_out, stream);
+}
+
+int tp_mle_eval_pixels_batch_at(int n_frames, const void* const* d_pixels, const int* n_copies,
+                                int n_copies_padded, int copy_size, int n_wires, int const_idx,
+                                uint64_t const_val, const void* d_points, const int* slots, void* d_out, void* stream)
+{
     tp::clear_error();
     tp::Ctx* c = tp::ctx();
     if (!c) return -1;
@@ -701,12 +709,16 @@ int tp_mle_eval_pixels_batch(int n_frames, const void* const* d_pixels, const in
     for (int i = 0; i < n_frames; ++i) {
         fr[(size_t)i].pix = static_cast<const unsigned char*>(d_pixels[i]);
         fr[(size_t)i].n_real = n_copies[i];
-        fr[(size_t)i].pad_ = 0;
+        fr[(size_t)i].slot = slots ? slots[i] : i;
+        if (fr[(size_t)i].slot < 0) {
+            tp::set_error(tp::TP_ERR_ARG, "mle over bytes: frame %d at %d", i, fr[(size_t)i].slot);
+            return -1;
+        }
     }
     int launches = 0;
     return tp::launch_mle_pixels_batch(fr.data(), n_frames, n_copies_padded, copy_size, n_wires,
-                                       const_idx, const_val, static_cast<const fp2*>(d_points),
-                                       static_cast<fp2*>(d_out), pick(stream, c), &launches) ? 0 : -1;
+                                       const_idx, const_val, static_cast<const tp::fp2*>(d_points),
+                                       static_cast<tp::fp2*>(d_out), pick(stream, c), &launches) ? 0 : -1;
 }
 
 }  // extern "C"

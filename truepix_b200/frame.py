@@ -232,7 +232,10 @@ class BatchFrameProver:
         self.fin_beta = torch.zeros(self.B * 2, dtype=i64, device=self.dev)
         self.mle = torch.zeros(self.B * 2, dtype=i64, device=self.dev)
         self.launches_last = 0
-        self._group_index = {C: torch.tensor(fs, dtype=i64, device=self.dev) for C, fs in self.groups.items()}
+        self._mle_groups = {C: (fs, np.array(fs, np.int32), np.array([self.layouts[f].copies for f in fs], np.int32))
+                            for C, fs in self.groups.items()}
+        large = sum(L.copies * L.copy_size for L in self.layouts) >= self.MLE_ASIDE
+        self._mle_stream = torch.cuda.Stream(self.dev) if large else None
         self._copies = np.array([L.copies for L in self.layouts], np.int32)
         self._padded = np.array([L.padded_copies for L in self.layouts], np.int32)
         self.handle = self.lib.tp_batch_create(self.B, self._s())
@@ -250,6 +253,23 @@ class BatchFrameProver:
             for part in (0, 1):
                 out[f, part] = np.asarray(z[part], np.uint64).reshape(-1)[:G]
         return out
+
+    # From this many bytes on, the MLEs' time (64 1080p frames, 398 MB: 133 us) is worth
+    # the four event calls (10 us of the host's time) that put them beside the rounds: that
+    # batch took 1347 us with them behind the finish and takes 1258 so, with the late
+    # outputs zeroed in one launch instead of seven
+    MLE_ASIDE = 64 << 20
+
+    def _input_mles(self, pixels, points_dev, stream) -> int:
+        """the input MLE of every frame into self.mle, on a stream; the launches made"""
+        L0 = self.layouts[0]
+        for C, (fs, slots, copies) in self._mle_groups.items():
+            ptrs = np.array([pixels[f].data_ptr() for f in fs], np.uint64)
+            native.check(self.lib, self.lib.tp_mle_eval_pixels_batch_at(
+                len(fs), ptrs.ctypes.data, copies.ctypes.data, C, L0.copy_size, L0.n_wires, L0.const_idx,
+                L0.const_val, points_dev[C].data_ptr(), slots.ctypes.data, self.mle.data_ptr(), stream.cuda_stream),
+                "mle")
+        return len(self.groups)
 
     def __del__(self):
         try:
@@ -287,12 +307,31 @@ class BatchFrameProver:
         graph: with transcripts and vole on a stream of the caller's, every round
         and the finish run as one CUDA graph (tp_batch_vole_rounds_graph), captured
         on the first call and replayed after."""
-        lib, s, b = self.lib, self._s(), self.handle
         if not isinstance(z2s_dev, dict):
             assert len(self.groups) == 1
             C = next(iter(self.groups))
             z2s_dev, points_dev = {C: z2s_dev}, {C: points_dev}
         self._z2s_dev = z2s_dev      # the layer's closing proofs read the copy part of the point
+        launches = 0
+        # the input MLEs need the bytes and points alone: those of a large batch run beside
+        # the rounds, whose one CTA per frame leaves the chip half idle
+        launch = self.stream if self.stream is not None else self.torch.cuda.current_stream(self.dev)
+        aside = self._mle_stream is not None
+        if aside:
+            self._mle_stream.wait_stream(launch)
+            launches += self._input_mles(pixels, points_dev, self._mle_stream)
+        try:
+            launches += self._rounds(pixels, z1s, z2s_dev, challenges, round_hook, transcripts, layer, vole, graph)
+        finally:             # also when a round is refused: the caller's tensors are free behind this
+            if aside:
+                launch.wait_stream(self._mle_stream)
+        if not aside:
+            launches += self._input_mles(pixels, points_dev, launch)
+        self.launches_last = launches
+
+    def _rounds(self, pixels, z1s, z2s_dev, challenges, round_hook, transcripts, layer, vole, graph) -> int:
+        """prove() but for the input MLEs: betas, early rounds and finish; the launches made"""
+        lib, s, b = self.lib, self._s(), self.handle
         launches = 0
         beta_of = {}
         for C, fs in self.groups.items():
@@ -361,20 +400,7 @@ class BatchFrameProver:
             native.check(lib, lib.tp_batch_finish(b, self.wires.data_ptr(), self.fin_beta.data_ptr()),
                          "batch_finish")
         launches += lib.tp_batch_launches(b) - l0
-        L0 = self.layouts[0]
-        for C, fs in self.groups.items():
-            ptrs = (ctypes.c_void_p * len(fs))(*[pixels[f].data_ptr() for f in fs])
-            ncop = (ctypes.c_int * len(fs))(*[self.layouts[f].copies for f in fs])
-            out = self.torch.empty(2 * len(fs), dtype=self.torch.int64, device=self.dev)
-            native.check(lib, lib.tp_mle_eval_pixels_batch(
-                len(fs), ptrs, ncop, C, L0.copy_size, L0.n_wires, L0.const_idx, L0.const_val,
-                points_dev[C].data_ptr(), out.data_ptr(), s), "mle")
-            launches += 1
-            if len(self.groups) == 1:
-                self.mle.copy_(out)
-            else:
-                self.mle.view(-1, 2).index_copy_(0, self._group_index[C], out.view(-1, 2))
-        self.launches_last = launches
+        return launches
 
     def prove_late(self, z1s, challenges=None, transcripts=None, vole=None, layer: int = 0, zk: bool = False) -> None:
         """The late rounds and the line projection of every frame, after prove():
@@ -399,15 +425,16 @@ class BatchFrameProver:
             return torch.cuda.stream(self.stream) if self.stream is not None else contextlib.nullcontext()
         with on_stream():    # from pinned memory, asynchronously: no wait for the launch stream to drain
             d_zg = zg.to(self.dev, non_blocking=True)
-        i64 = torch.int64
-        with on_stream():
-            self.late_coefs = torch.zeros(self.B * 2 * n * 3 * 2, dtype=i64, device=self.dev)
-            self.line = torch.zeros(self.B * (n + 1) * 2, dtype=i64, device=self.dev)
-            self.late_challenges = torch.zeros(self.B * 2 * n * 2, dtype=i64, device=self.dev)
+        def zeros(*elements):   # one launch for all outputs; parts of 16-byte elements
+            with on_stream():
+                whole = torch.zeros(2 * sum(elements), dtype=torch.int64, device=self.dev)
+            return whole.split([2 * e for e in elements])
+        sizes = [self.B * 2 * n * 3, self.B * (n + 1), self.B * 2 * n]
         I32P = ctypes.POINTER(ctypes.c_int)
         gt, i0, i1 = (a.ctypes.data_as(I32P) for a in (self.gt, self.i0, self.i1))
         keep = [d_zg]
         if transcripts is None:
+            self.late_coefs, self.line, self.late_challenges = zeros(*sizes)
             ch = np.ascontiguousarray(challenges, np.uint64).reshape(-1)
             if ch.size != self.B * 2 * n * 2:
                 raise ValueError("challenges: [B, 2 log2 W, 2] expected")
@@ -426,11 +453,9 @@ class BatchFrameProver:
             if any(L.n_copy_bits != self.max_rounds for L in self.layouts):
                 raise ValueError("device transcripts need frames with the same number of rounds")
             nb = self.max_rounds
-            with on_stream():
-                self.late_proof = torch.zeros(self.B * 2 * n * 4 * 2, dtype=i64, device=self.dev)
-                self.closing = torch.zeros(self.B * (n + (15 if zk else 10)) * 2, dtype=i64, device=self.dev)
-                self.input_point = torch.zeros(self.B * (n + nb) * 2, dtype=i64, device=self.dev)
-                self.input_tag = torch.zeros(self.B * 2, dtype=i64, device=self.dev)
+            (self.late_coefs, self.line, self.late_challenges, self.late_proof, self.closing, self.input_point,
+             self.input_tag) = zeros(*sizes, self.B * 2 * n * 4, self.B * (n + (15 if zk else 10)), self.B * (n + nb),
+                                     self.B)
             z2 = next(iter(self._z2s_dev.values()))
             # early challenges: self.device_challenges [round][frame]
             rc = lib.tp_late_rounds_dev(self.B, n, G, gt, i0, i1, self.wires.data_ptr(), self.fin_beta.data_ptr(),
