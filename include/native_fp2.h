@@ -251,10 +251,13 @@ int tp_compute_beta_batch_dev(const void* d_z, int n_z, int n_frames, void* d_ou
 int tp_mle_eval_pixels_batch(int n_frames, const void* const* d_pixels, const int* n_copies,
                              int n_copies_padded, int copy_size, int n_wires, int const_idx,
                              uint64_t const_val, const void* d_points, void* d_out, void* stream);
-/* the same, frame i's value at d_out[slots[i]] (slots null: i) */
+/* the same, frame i's value at d_out[slots[i]] (slots null: i), and with the caller's
+ * workspace d_ws (null: one from the library's pool; 16-byte aligned, at least
+ * 16 ceil(c / 512) + 20 bytes for every frame, c the largest of n_copies) */
 int tp_mle_eval_pixels_batch_at(int n_frames, const void* const* d_pixels, const int* n_copies,
                                 int n_copies_padded, int copy_size, int n_wires, int const_idx,
-                                uint64_t const_val, const void* d_points, const int* slots, void* d_out, void* stream);
+                                uint64_t const_val, const void* d_points, const int* slots, void* d_out, void* d_ws,
+                                size_t ws_bytes, void* stream);
 
 /* Claim-kernel timer: when enabled, every session claim records a CUDA event pair
  * with tag 1000*(reads pixels) + 100*(fold fused) + log2(copies claimed).

@@ -79,7 +79,8 @@ def test_mle(cs, const, W, n_pad, counts, offset, extreme):
 
 
 def test_slots():
-    """the values placed at given indices; a negative one is refused"""
+    """the values placed at given indices, in the caller's workspace; a negative index and
+    a workspace too small are refused"""
     import torch
     from truepix_b200 import native
     lib = native.gkr()
@@ -90,11 +91,14 @@ def test_slots():
     args = (3, (ctypes.c_void_p * 3)(*[x[i].data_ptr() for i in range(3)]), (ctypes.c_int * 3)(4, 3, 4), 4, 16, 16, -1, 0,
             z.data_ptr())
     a = torch.zeros(3, 2, dtype=torch.int64, device="cuda")
+    ws = torch.empty(3 * 36, dtype=torch.uint8, device="cuda")
     b = torch.full((7, 2), -1, dtype=torch.int64, device="cuda")
     native.check(lib, lib.tp_mle_eval_pixels_batch(*args, a.data_ptr(), s), "mle")
-    native.check(lib, lib.tp_mle_eval_pixels_batch_at(*args, (ctypes.c_int * 3)(6, 0, 3), b.data_ptr(), s), "mle at")
+    native.check(lib, lib.tp_mle_eval_pixels_batch_at(*args, (ctypes.c_int * 3)(6, 0, 3), b.data_ptr(), ws.data_ptr(),
+                                                      ws.numel(), s), "mle at")
     assert torch.equal(b[[6, 0, 3]], a) and bool((b[[1, 2, 4, 5]] == -1).all())
-    assert lib.tp_mle_eval_pixels_batch_at(*args, (ctypes.c_int * 3)(0, -1, 2), b.data_ptr(), s) != 0
+    assert lib.tp_mle_eval_pixels_batch_at(*args, (ctypes.c_int * 3)(0, -1, 2), b.data_ptr(), None, 0, s) != 0
+    assert lib.tp_mle_eval_pixels_batch_at(*args, None, b.data_ptr(), ws.data_ptr(), 3 * 36 - 1, s) != 0
 
 
 def test_beside_the_rounds(monkeypatch):

@@ -206,7 +206,8 @@ void launch_eq_tables_batch(const fp2* d_z, int z_stride, int h, int hb, fp2 ini
 // beta tables of n frames: d_z packed [n][n_z], d_out packed [n][2^n_z]
 bool launch_beta_batch(const fp2* d_z, int n_z, int n, fp2* d_out, cudaStream_t s, int* launches);
 // MLE of n frames' input vectors (same padded size) from their bytes:
-// frames[i] = {pix, n_real}; points packed [n][log2 W + log2 n_pad]; out packed [n]
+// frames[i] = {pix, n_real, slot}; points packed [n][log2 W + log2 n_pad]; value i at
+// out[slot]; d_ws (16-byte aligned): the caller's workspace in place of one from the pool
 struct MleFrame {
     const unsigned char* pix;
     int n_real;
@@ -214,6 +215,6 @@ struct MleFrame {
 };
 bool launch_mle_pixels_batch(const MleFrame* h_frames, int n, int n_pad, int cs, int W,
                              int const_idx, u64 const_val, const fp2* d_points, fp2* d_out,
-                             cudaStream_t s, int* launches);
+                             cudaStream_t s, int* launches, void* d_ws = nullptr, size_t ws_bytes = 0);
 
 }  // namespace tp

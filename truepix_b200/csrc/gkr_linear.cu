@@ -1054,7 +1054,7 @@ bool launch_linear_rounds(const Job* d_jobs, int n_jobs, const VoleRounds* v, in
 
 bool launch_mle_pixels_batch(const MleFrame* h_frames, int n, int n_pad, int cs, int W,
                              int const_idx, u64 const_val, const fp2* d_points, fp2* d_out,
-                             cudaStream_t s, int* launches)
+                             cudaStream_t s, int* launches, void* d_ws, size_t ws_bytes)
 {
     if (n <= 0) return true;
     if (!prepare_linear_kernels()) return false;
@@ -1088,7 +1088,11 @@ bool launch_mle_pixels_batch(const MleFrame* h_frames, int n, int n_pad, int cs,
     const int ctas = (most + a.pieces - 1) / a.pieces;
     const size_t np = (size_t)ctas * n;
     const size_t bytes = sizeof(fp2) * np + (sizeof(MleFrame) + sizeof(unsigned)) * n;
-    unsigned char* ws = (unsigned char*)dev_alloc(bytes, s);
+    if (d_ws && ws_bytes < bytes) {
+        set_error(TP_ERR_ARG, "mle over bytes: a workspace of %zu bytes, %zu needed", ws_bytes, bytes);
+        return false;
+    }
+    unsigned char* ws = (unsigned char*)(d_ws ? d_ws : dev_alloc(bytes, s));
     if (!ws) return false;
     a.partials = reinterpret_cast<fp2*>(ws);
     MleFrame* d_frames = reinterpret_cast<MleFrame*>(a.partials + np);
@@ -1105,7 +1109,7 @@ bool launch_mle_pixels_batch(const MleFrame* h_frames, int n, int n_pad, int cs,
         ++*launches;
         ok = !cuda_failed(cudaGetLastError(), "mle batch launch");
     }
-    dev_free(ws, s);
+    if (!d_ws) dev_free(ws, s);
     return ok;
 }
 

@@ -695,12 +695,13 @@ int tp_mle_eval_pixels_batch(int n_frames, const void* const* d_pixels, const in
                              uint64_t const_val, const void* d_points, void* d_out, void* stream)
 {
     return tp_mle_eval_pixels_batch_at(n_frames, d_pixels, n_copies, n_copies_padded, copy_size, n_wires, const_idx,
-                                       const_val, d_points, nullptr, d_out, stream);
+                                       const_val, d_points, nullptr, d_out, nullptr, 0, stream);
 }
 
 int tp_mle_eval_pixels_batch_at(int n_frames, const void* const* d_pixels, const int* n_copies,
                                 int n_copies_padded, int copy_size, int n_wires, int const_idx,
-                                uint64_t const_val, const void* d_points, const int* slots, void* d_out, void* stream)
+                                uint64_t const_val, const void* d_points, const int* slots, void* d_out, void* d_ws,
+                                size_t ws_bytes, void* stream)
 {
     tp::clear_error();
     tp::Ctx* c = tp::ctx();
@@ -718,7 +719,8 @@ int tp_mle_eval_pixels_batch_at(int n_frames, const void* const* d_pixels, const
     int launches = 0;
     return tp::launch_mle_pixels_batch(fr.data(), n_frames, n_copies_padded, copy_size, n_wires,
                                        const_idx, const_val, static_cast<const tp::fp2*>(d_points),
-                                       static_cast<tp::fp2*>(d_out), pick(stream, c), &launches) ? 0 : -1;
+                                       static_cast<tp::fp2*>(d_out), pick(stream, c), &launches, d_ws,
+                                       ws_bytes) ? 0 : -1;
 }
 
 }  // extern "C"
