@@ -29,7 +29,7 @@ the GKR rounds and openings of the previous batch run on the main stream.
                 commit per frame from resident bytes, challenges given): its
                 kernels with their time shares and the roofline of the dominant
                 ones (the SHA-256 leaf kernel against the integer-ALU pipe, the
-                fold kernel against HBM)
+                byte forms against HBM)
   cpu_baseline  the reference implementation's proved frame on one host core
                 (oracle/reference_proof.py: the reference's compiled commit,
                 native_fp2.cpp and linearPC_multi_prove + fft_gkr programs, its
@@ -332,8 +332,9 @@ def kernel_groups(ms, tags, layout, batch=1, cw_len=0, leaves=0):
     """Per kernel kind: launches, total time, algorithmic bytes, folded elements,
     SHA-256 compressions.
     Claim kernels: tag = 1000*(reads bytes) + 100*(fold fused) + log2(copies
-    claimed per frame); algorithmic bytes per frame = bytes read once + folded Fp2
-    rows written (16 B per element) + table rows read (16 B per element) + beta.
+    claimed per frame). The gray circuit has no product gates, so a frame's rounds run on
+    one vector and beta: the forms read the bytes and write them aside, with 16 B per
+    copy; a round reads 32 B per copy claimed, a fused fold twice that and writes 32 B.
     Commit kernels (tags 9100-9104), per frame: pixel rows = bytes read + 16 B per
     codeword-message element written; leaves = 2 KB read + 32 B written per
     codeword row, 128 compressions per row; tree = 64 B read + 32 B written and 2
@@ -362,13 +363,13 @@ def kernel_groups(ms, tags, layout, batch=1, cw_len=0, leaves=0):
             pix, fold, lg = tag // 1000, (tag // 100) % 10, tag % 100
             n = 1 << lg                                    # copies claimed
             if pix and not fold:
-                name, byt, el = "pix_claim_kernel", pix_bytes + 16 * n, 0
+                name, byt, el = "forms_bytes_kernel", 2 * pix_bytes + 16 * n, 0
             elif pix and fold:
                 name, byt, el = "pix_fold_claim_kernel", pix_bytes + 16 * rows * n + 48 * n, rows * n
             elif fold:
-                name, byt, el = "table_round_kernel<fold>", 48 * rows * n + 48 * n, rows * n
+                name, byt, el = "vec_round_kernel<fold>", 96 * n, 2 * n
             else:
-                name, byt, el = "table_round_kernel<claim>", 16 * rows * n + 16 * n, 0
+                name, byt, el = "vec_round_kernel<claim>", 32 * n, 0
         g = groups.setdefault(name, {"launches": 0, "ms": 0.0, "bytes": 0.0, "folded": 0,
                                      "compressions": 0.0, "by_copies": {}})
         per_launch = batch if tag < 9000 else 1    # a claim launch serves the whole batch
@@ -709,7 +710,7 @@ def ours_arm(args, rank, world, local_rank):
 
     kernels = summarize(groups, ms)
     roof = roof_of(kernels[0], groups) if kernels else None
-    hbm_kernel = next((k for k in kernels if k["kernel"] == "table_round_kernel<fold>"), None)
+    hbm_kernel = next((k for k in kernels if k["kernel"] == "forms_bytes_kernel"), None)
     roof_fold = roof_of(hbm_kernel, groups) if hbm_kernel else None
 
     # One more step, outside the timed region, with the commits serialised on the

@@ -66,8 +66,8 @@ __device__ __forceinline__ int at(int r, int c, int log_g) { return (r << log_g)
 // where lo = 0), and what is left is a plain 2^K-point DFT. Up to 8 points that needs
 // no multiplication in this field: the 4th root is -i (forward; +i inverse) and the
 // 8th 2^30 (1 -+ i), since 2^61 = 1 makes 2^30 = 2^(-31) a square root of 1/2, so
-// they are swaps, negations and rotations by 30 bits. (12 multiplications per 8 rows
-// and group before, two in the first: 2^20 points 47.4 -> see ntt.h.)
+// they are swaps, negations and rotations by 30 bits. (With 12 multiplications per 8
+// rows and group, two in the first, 2^20 points forward and inverse took 196 us, now 165.)
 //
 // Bounds: rows come in below 2^61 + 8. The first two levels are left unreduced
 // (differences add 2p, then 4p, and stay below 2^64), folded, and the third level's

@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(kLeafRows) leaf_kernel(const ulonglong2* __res
 __global__ void __launch_bounds__(sha::kFewThreads) leaf_few_kernel(const ulonglong2* __restrict__ rows,
                                                                     long long cw_len,
                                                                     unsigned char* __restrict__ tree,
-                                                                    long long leaf0, uint32_t one)
+                                                                    long long leaf0)
 {
     __shared__ sha::ChainMem mem;
     const long long r = (long long)blockIdx.x * sha::kFewRows + (threadIdx.x & 31);
@@ -529,10 +529,10 @@ __global__ void __launch_bounds__(kLeafRows) sha_peak_kernel(int iters, uint32_t
 // three 32-bit words each (two 32 x 32 multiply-adds per product, no fold per
 // product). a c and b d (< 2^92) are folded mod 2^61 - 1 back below 2^61 + 8 every 8
 // edges, the third every 4: a + b is not reduced, its products are at most
-// (2^62 - 4)(2^32 - 2), and four of them with the fold's rest stay below 2^96.
-// (Reducing a + b first, with one fold per 8 edges,
-// a 1080p commit took 1183 us, now 1164; a 720p zero-knowledge pair 1543, now 1506.)
-// The result is (a c - b d) + (s (c + d) - a c - b d) i.
+// (2^62 - 4)(2^32 - 2), and four of them with the fold's rest stay below 2^96. The
+// result is (a c - b d) + (s (c + d) - a c - b d) i. Reducing a + b first, with one fold
+// per 8 edges, took 1183 us for a 1080p commit (now 1164) and 1543 us for a 720p
+// zero-knowledge pair (now 1506).
 struct Acc3 {
     u32 w0, w1, w2;
 };
@@ -819,7 +819,7 @@ void launch_leaves(const ulonglong2* rows, long long count, unsigned char* diges
     const long long few = (count + sha::kFewRows - 1) / sha::kFewRows;
     Ctx* c = ctx();
     if (c && few <= (long long)sha::kFewPerSm * c->n_sm && pair0 == 0 && pair1 == kColumns / 2)
-        leaf_few_kernel<<<(unsigned)few, sha::kFewThreads, 0, s>>>(rows, count, digests, leaf0, 1u);
+        leaf_few_kernel<<<(unsigned)few, sha::kFewThreads, 0, s>>>(rows, count, digests, leaf0);
     else
         leaf_kernel<<<(unsigned)((count + kLeafRows - 1) / kLeafRows), kLeafRows, 0, s>>>(rows, count, digests, leaf0,
                                                                                          1u, pair0, pair1);

@@ -66,8 +66,7 @@ __global__ void __launch_bounds__(kLeafThreads) pair_leaf_kernel(const ulonglong
 __global__ void __launch_bounds__(sha::kFewThreads) pair_leaf_few_kernel(const ulonglong2* __restrict__ src,
                                                                          long long n_leaves, long long leaf_step,
                                                                          long long slice_step, long long y_off,
-                                                                         unsigned char* __restrict__ tree,
-                                                                         uint32_t one)
+                                                                         unsigned char* __restrict__ tree)
 {
     __shared__ sha::ChainMem mem;
     const long long t = (long long)blockIdx.x * sha::kFewRows + (threadIdx.x & 31);
@@ -89,7 +88,7 @@ bool launch_pair_leaves(const ulonglong2* src, long long n_leaves, long long lea
     const long long few = (n_leaves + sha::kFewRows - 1) / sha::kFewRows;
     if (few <= (long long)sha::kFewPerSm * c->n_sm)
         pair_leaf_few_kernel<<<(unsigned)few, sha::kFewThreads, 0, s>>>(src, n_leaves, leaf_step, slice_step, y_off,
-                                                                        tree, 1u);
+                                                                        tree);
     else
         pair_leaf_kernel<<<(unsigned)((n_leaves + kLeafThreads - 1) / kLeafThreads), kLeafThreads, 0, s>>>(
             src, n_leaves, leaf_step, slice_step, y_off, tree, 1u);

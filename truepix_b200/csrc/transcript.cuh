@@ -284,12 +284,13 @@ inline void rand_ext(State& s, const uint8_t* label, uint32_t len, uint64_t* re,
 // draw's own 70 to 134 bytes are written by all lanes at once (a lane that appended
 // unit by unit spent a third of a round on that chain, and on fetching its code anew
 // each time); a draw hashes the whole stretch at once. The message words of all its
-// blocks are known by then, so their schedules are made side by side, one lane per block, and the rounds run on k + w from shared
-// memory: 31 cycles a round against 49 with the schedule in line. The real limb of a
-// draw does not enter the transcript, so the stretch runs on to the imaginary limb's
-// draw and an even and an odd lane close the two digests in the same instructions,
-// each with its own padding. Per committed round (243 bytes, two draws): ~6
-// compressions' rounds one after the other and two schedules; a launch of one round
+// blocks are known by then, so their schedules are made side by side, one lane per
+// block, and the rounds run on k + w from shared memory: 33 cycles a round against 49
+// with the schedule in line. The real limb of a draw does not enter the transcript, so
+// the stretch runs on to the imaginary limb's draw and an even and an odd lane close the
+// two digests in the same instructions, each with its own padding. Per committed round
+// (243 bytes, two draws): ~6 compressions' rounds one after the other and two schedules,
+// 10 to 13 thousand cycles a draw by the bytes before it; a launch of one round
 // takes 16 us (22 with unit-wise appends; 146 with a thread that appended byte by byte
 // and hashed block by block).
 
