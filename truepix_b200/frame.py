@@ -350,7 +350,8 @@ class BatchFrameProver:
         z1 = self._gate_weights(z1s)
         pix = np.array([pixels[f].data_ptr() for f in range(self.B)], np.uint64)
         betas = np.array([beta_of[f] for f in range(self.B)], np.uint64)
-        native.check(lib, lib.tp_batch_set_pixels_all(
+        quick = native.gkr_launcher()     # a short call: it keeps the interpreter lock
+        native.check(lib, quick.tp_batch_set_pixels_all(
             b, self.gt.size, self.gt.ctypes.data, self.i0.ctypes.data, self.i1.ctypes.data, z1.ctypes.data,
             pix.ctypes.data, self._copies.ctypes.data, self._padded.ctypes.data, L.copy_size, L.n_wires, L.const_idx,
             L.const_val, betas.ctypes.data), "batch_set_pixels")
