@@ -122,6 +122,9 @@ __device__ __forceinline__ void store_poly(ulonglong2* ret, fp2 qa, fp2 qb, fp2 
 // entry, the CTAs' sums added in the first one's shared memory: no partial sums in
 // memory, no ticket to clear. A round of so few entries is launch latency: 10.6 us
 // with the cleared ticket and the grid's sum added up by three threads, 6.5 us so.
+// A CTA's shared memory may be written by another only once it runs, so every CTA
+// arrives at the cluster's barrier as it starts and waits there before its store, by
+// when the others have long arrived.
 constexpr int kClusterMax = 8, kSmall = kClusterMax * kThreads;
 
 __global__ void __launch_bounds__(kThreads) update_small_kernel(const ulonglong2* __restrict__ vma,
@@ -136,10 +139,12 @@ __global__ void __launch_bounds__(kThreads) update_small_kernel(const ulonglong2
     __shared__ fp2 red[kThreads / 32][3];
     __shared__ fp2 sums[kClusterMax][3];
     const cg::cluster_group cluster = cg::this_cluster();
+    cluster.barrier_arrive();
     fp2 qa = f2zero(), qb = f2zero(), qc = f2zero();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < half) update_entry(vma, addv, ams, i, r, bit, vma_out, addv_out, ams_out, qa, qb, qc);
     cta_sum3(qa, qb, qc, red);
+    cluster.barrier_wait();
     if (threadIdx.x == 0) {
         fp2* to = cluster.map_shared_rank(&sums[blockIdx.x][0], 0);
         to[0] = qa;
