@@ -21,7 +21,8 @@ namespace tp {
 
 namespace {
 
-// (re)use the frame's buffers: grow only when a configuration needs more
+// (re)use the frame's buffers: grow only when a configuration needs more. The frame
+// counts as loaded once its loader has put everything in place, not before.
 bool frame_alloc(Frame* f, size_t rows0, size_t rows1, cudaStream_t s)
 {
     const size_t n = (size_t)f->n_copies0;
@@ -51,9 +52,8 @@ bool frame_alloc(Frame* f, size_t rows0, size_t rows1, cudaStream_t s)
     f->pending = false;
     f->r_dev = nullptr;
     f->pix_cur = false;
-    f->linear = false;
-    f->loaded = (!rows0 || f->buf[0]) && (!rows1 || f->buf[1]) && f->beta[0] && f->beta[1];
-    return f->loaded;
+    f->linear = f->loaded = false;
+    return (!rows0 || f->buf[0]) && (!rows1 || f->buf[1]) && f->beta[0] && f->beta[1];
 }
 
 template <class T>
@@ -355,7 +355,8 @@ bool batch_load_host(Batch* B, int i, const u64* v_re, const u64* v_im, const u6
     B->launches += launches;
     dev_free(stage_im, s);
     // the reference contract: host inputs are consumed before the call returns
-    return ok && !cuda_failed(cudaStreamSynchronize(s), "load tables");
+    f->loaded = ok && !cuda_failed(cudaStreamSynchronize(s), "load tables");
+    return f->loaded;
 }
 
 bool batch_load_device(Batch* B, int i, const fp2* d_values, const fp2* d_beta, bool borrow)
@@ -376,6 +377,7 @@ bool batch_load_device(Batch* B, int i, const fp2* d_values, const fp2* d_beta, 
     }
     TP_CUDA_OK(cudaMemcpyAsync(f->beta[0], d_beta, sizeof(fp2) * (size_t)f->n_copies0,
                                cudaMemcpyDeviceToDevice, s), "copy beta");
+    f->loaded = true;
     return true;
 }
 
@@ -392,10 +394,8 @@ bool start_load_pixels(Batch* B, int i, const PixSrc& px)
     const size_t C = (size_t)f->n_copies0, R = (size_t)f->W_rows;
     if (wants_linear(f)) {
         if (!frame_alloc(f, 0, 0, s) || !linear_alloc(f, (size_t)lin_chunks(px.n_real, 30) * R, s) ||
-            !grow(f->bytes, f->cap_bytes, lin_bytes(px.cs, px.n_real), s)) {
-            f->loaded = false;
+            !grow(f->bytes, f->cap_bytes, lin_bytes(px.cs, px.n_real), s))
             return false;
-        }
     } else {
         // first fold writes R x C/2 into buf[1]; later folds alternate with buf[0]
         if (!frame_alloc(f, R * std::max<size_t>(1, C / 4), R * (C / 2), s)) return false;
@@ -427,6 +427,7 @@ bool batch_load_pixels(Batch* B, int i, const PixSrc& px, const fp2* d_beta)
     TP_CUDA_OK(cudaMemcpyAsync(f->beta[0], d_beta, sizeof(fp2) * (size_t)f->n_copies0, cudaMemcpyDeviceToDevice,
                                B->stream),
                "copy beta");
+    f->loaded = true;
     return true;
 }
 
@@ -469,7 +470,9 @@ bool batch_set_pixels_all(Batch* B, int n_gates, const int* type, const int* in0
         copy_betas_kernel<<<dim3((unsigned)std::max(1, std::min(64, (most + 255) / 256)), (unsigned)n), 256, 0, s>>>(
             reinterpret_cast<const BetaCopy*>(forms + at));
         ++B->launches;
-        return !cuda_failed(cudaGetLastError(), "copy betas");
+        if (cuda_failed(cudaGetLastError(), "copy betas")) return false;
+        for (Frame* f : B->frames) f->loaded = true;
+        return true;
     };
     if (all()) return true;
     batch_reset(B);   // no frame is left half set
@@ -858,6 +861,10 @@ bool batch_fold(Batch* B, int i, fp2 r)
         return false;
     }
     if (device_fold_blocked(f)) return false;
+    if (f->pending && !f->loaded) {
+        set_error(TP_ERR_ARG, "frame %d has no table", i);
+        return false;
+    }
     if (f->pending && !(f->linear ? apply_fold_linear(B, f) : apply_fold(f, B->stream, &B->launches))) return false;
     f->pending = true;
     f->r = r;

@@ -96,6 +96,7 @@ void* dev_alloc(size_t bytes, cudaStream_t s)
     cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, c->pool, s);
     if (e != cudaSuccess) {
         cuda_failed(e, "device allocation");
+        cudaGetLastError();   // reported here, not by the next launch's check
         return nullptr;
     }
     return p;
