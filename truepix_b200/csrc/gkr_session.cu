@@ -433,7 +433,7 @@ bool batch_load_pixels(Batch* B, int i, const PixSrc& px, const fp2* d_beta)
 
 // One upload in a few pieces and one launch for all frames, where a call per frame made
 // two copies and an event each (64 1080p frames: 1.98 ms of the host's time a proof, now
-// 1.03).
+// 1.03). A beta that 16-byte loads cannot read is copied by itself.
 bool batch_set_pixels_all(Batch* B, int n_gates, const int* type, const int* in0, const int* in1, const u64* z1,
                           const PixSrc* px, const int* n_copies, int n_wires, const fp2* const* d_betas)
 {
@@ -441,6 +441,12 @@ bool batch_set_pixels_all(Batch* B, int n_gates, const int* type, const int* in0
     const int n = (int)B->frames.size();
     std::vector<unsigned char> h;
     std::vector<BetaCopy> betas;
+    for (int i = 0; i < n; ++i)
+        if (!d_betas[i]) {
+            set_error(TP_ERR_ARG, "frame %d has no beta", i);
+            return false;
+        }
+    auto aligned = [&](int i) { return (reinterpret_cast<size_t>(d_betas[i]) & 15) == 0; };
     auto all = [&]() -> bool {
         int most = 0;
         for (int i = 0; i < n; ++i) {
@@ -450,7 +456,7 @@ bool batch_set_pixels_all(Batch* B, int n_gates, const int* type, const int* in0
             if (!start_set_gates(B, i, n_gates, type, in0, in1, z, z + n_gates, n_copies[i], n_wires, g)) return false;
             pack_gate_form(g, f->form, h);
             if (!finish_set_gates(B, f) || !start_load_pixels(B, i, px[i])) return false;
-            betas.push_back(BetaCopy{d_betas[i], f->beta[0], n_copies[i]});
+            betas.push_back(BetaCopy{d_betas[i], f->beta[0], aligned(i) ? n_copies[i] : 0});
             most = std::max(most, n_copies[i]);
         }
         h.resize((h.size() + 15) & ~(size_t)15);
@@ -471,6 +477,12 @@ bool batch_set_pixels_all(Batch* B, int n_gates, const int* type, const int* in0
             reinterpret_cast<const BetaCopy*>(forms + at));
         ++B->launches;
         if (cuda_failed(cudaGetLastError(), "copy betas")) return false;
+        for (int i = 0; i < n; ++i)
+            if (!aligned(i) &&
+                cuda_failed(cudaMemcpyAsync(B->frames[(size_t)i]->beta[0], d_betas[i], sizeof(fp2) * (size_t)n_copies[i],
+                                            cudaMemcpyDeviceToDevice, s),
+                            "copy beta"))
+                return false;
         for (Frame* f : B->frames) f->loaded = true;
         return true;
     };
