@@ -174,7 +174,8 @@ int tp_batch_set_pixels(void* batch, int i, int n_gates, const int* gate_type, c
                         int n_wires, int const_idx, uint64_t const_val, const void* d_beta);
 /* every frame of the batch at once, all of one circuit: frame i's weights z1[i] =
    {real[n_gates], imag[n_gates]}, pixels, copy counts and beta; as tp_batch_set_pixels
-   for each in turn (no frame is set when one is refused) */
+   for each in turn, except that no frame is set when one is refused; a batch with a
+   configured frame is refused and stays as it is */
 int tp_batch_set_pixels_all(void* batch, int n_gates, const int* gate_type, const int* in0, const int* in1,
                             const uint64_t* z1, const void* const* d_pixels, const int* n_copies,
                             const int* n_copies_padded, int copy_size, int n_wires, int const_idx,

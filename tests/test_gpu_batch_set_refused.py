@@ -1,5 +1,6 @@
 """What tp_batch_set_pixels_all refuses and takes, against tp_batch_set_pixels for each
-frame in turn: betas that are missing or at any address."""
+frame in turn: betas that are missing or at any address, and a batch in its rounds,
+which a refused call leaves as it is."""
 import ctypes
 
 import numpy as np
@@ -91,4 +92,36 @@ def test_beta_at_odd_addresses():
     assert fr.set_all(b, betas) == 0, fr.lib.tp_last_error()
     for w in want:
         np.testing.assert_array_equal(fr.round(b), w)
+    fr.lib.tp_batch_destroy(b)
+
+
+def test_refused_in_the_middle_of_the_rounds():
+    fr = Frames(3)
+    b = fr.batch()
+    fr.set_each(b)
+    want = [fr.round(b) for _ in range(3)]
+    fr.lib.tp_batch_destroy(b)
+    b = fr.batch()
+    assert fr.set_all(b) == 0, fr.lib.tp_last_error()
+    for k, w in enumerate(want):
+        np.testing.assert_array_equal(fr.round(b), w)
+        assert fr.set_all(b) != 0 and b"already configured" in fr.lib.tp_last_error()
+        assert [fr.lib.tp_batch_n_copies(b, f) for f in range(3)] == [int(p) >> (k + 1) for p in fr.padded]
+    fr.lib.tp_batch_reset(b)
+    assert fr.set_all(b) == 0, fr.lib.tp_last_error()
+    np.testing.assert_array_equal(fr.round(b), want[0])
+    fr.lib.tp_batch_destroy(b)
+
+
+@pytest.mark.parametrize("one_set", [0, 2])
+def test_refused_beside_a_single_frame(one_set):
+    fr = Frames(3)
+    b = fr.batch()
+    f = one_set
+    assert fr.lib.tp_batch_set_pixels(
+        b, f, G, fr.gt.ctypes.data, fr.i0.ctypes.data, fr.i1.ctypes.data, fr.z[f, 0].ctypes.data,
+        fr.z[f, 1].ctypes.data, fr.pix[f].data_ptr(), int(fr.copies[f]), int(fr.padded[f]), CS, W, CONST, 77,
+        fr.beta[f].data_ptr()) == 0, fr.lib.tp_last_error()
+    assert fr.set_all(b) != 0
+    assert [fr.lib.tp_batch_n_copies(b, k) for k in range(3)] == [int(fr.padded[k]) if k == f else 0 for k in range(3)]
     fr.lib.tp_batch_destroy(b)

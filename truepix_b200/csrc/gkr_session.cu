@@ -441,11 +441,16 @@ bool batch_set_pixels_all(Batch* B, int n_gates, const int* type, const int* in0
     const int n = (int)B->frames.size();
     std::vector<unsigned char> h;
     std::vector<BetaCopy> betas;
-    for (int i = 0; i < n; ++i)
+    for (int i = 0; i < n; ++i) {
+        if (B->frames[(size_t)i]->configured) {   // in the middle of its rounds, perhaps: the batch stays as it is
+            set_error(TP_ERR_ARG, "frame %d is already configured (tp_batch_reset first)", i);
+            return false;
+        }
         if (!d_betas[i]) {
             set_error(TP_ERR_ARG, "frame %d has no beta", i);
             return false;
         }
+    }
     auto aligned = [&](int i) { return (reinterpret_cast<size_t>(d_betas[i]) & 15) == 0; };
     auto all = [&]() -> bool {
         int most = 0;
@@ -487,7 +492,7 @@ bool batch_set_pixels_all(Batch* B, int n_gates, const int* type, const int* in0
         return true;
     };
     if (all()) return true;
-    batch_reset(B);   // no frame is left half set
+    batch_reset(B);   // no frame was set before, none is left half set
     return false;
 }
 
