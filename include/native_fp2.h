@@ -254,7 +254,7 @@ int tp_mle_eval_pixels_batch(int n_frames, const void* const* d_pixels, const in
                              uint64_t const_val, const void* d_points, void* d_out, void* stream);
 /* the same, frame i's value at d_out[slots[i]] (slots null: i), and with the caller's
  * workspace d_ws (null: one from the library's pool; 16-byte aligned, at least
- * 16 ceil(c / 512) + 20 bytes for every frame, c the largest of n_copies) */
+ * 16 max(1, ceil(c / 512)) + 20 bytes for every frame, c the largest of n_copies) */
 int tp_mle_eval_pixels_batch_at(int n_frames, const void* const* d_pixels, const int* n_copies,
                                 int n_copies_padded, int copy_size, int n_wires, int const_idx,
                                 uint64_t const_val, const void* d_points, const int* slots, void* d_out, void* d_ws,

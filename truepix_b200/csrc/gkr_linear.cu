@@ -1113,6 +1113,10 @@ bool launch_mle_pixels_batch(const MleFrame* h_frames, int n, int n_pad, int cs,
         set_error(TP_ERR_ARG, "mle over bytes: a workspace of %zu bytes, %zu needed", ws_bytes, bytes);
         return false;
     }
+    if (reinterpret_cast<size_t>(d_ws) & 15) {
+        set_error(TP_ERR_ARG, "mle over bytes: a workspace that is not 16-byte aligned");
+        return false;
+    }
     unsigned char* ws = (unsigned char*)(d_ws ? d_ws : dev_alloc(bytes, s));
     if (!ws) return false;
     a.partials = reinterpret_cast<fp2*>(ws);
