@@ -320,13 +320,13 @@ class BatchFrameProver:
         # the rounds, whose one CTA per frame leaves the chip half idle.
         launch = self.stream if self.stream is not None else self.torch.cuda.current_stream(self.dev)
         launches = 0
-        if self._mle_stream is not None:
-            self._mle_stream.wait_stream(launch)
-            launches += self._input_mles(pixels, points_dev, self._mle_stream)
         try:
+            if self._mle_stream is not None:
+                self._mle_stream.wait_stream(launch)
+                launches += self._input_mles(pixels, points_dev, self._mle_stream)
             launches += self._set_frames(pixels, z1s, z2s_dev)
             launches += self._rounds(challenges, round_hook, transcripts, layer, vole, graph)
-        finally:             # also when a round is refused: the caller's tensors are free behind this
+        finally:             # also when a call is refused: the caller's tensors are free behind this
             if self._mle_stream is not None:
                 launch.wait_stream(self._mle_stream)
         if self._mle_stream is None:
