@@ -276,7 +276,7 @@ struct ChainMem {
 };
 
 // The pair's named barriers (0 is the CTA's own): the digest is there; words 16..23
-// are; 24..39; 40..63; the next hash's pair is. At each, one warp only arrives and the
+// are; 24..39; 40..63; a hash's pair is. At each, one warp only arrives and the
 // other waits. None may be shared and the rounds' warp takes kBarPair before it hands
 // over the digest: the schedule's warp runs on up to the next digest without waiting,
 // so only a digest not yet handed over keeps its next arrival (or its wait for that
@@ -311,7 +311,7 @@ __device__ __forceinline__ void chain_rounds(ChainMem& m, int hashes, uint32_t s
     for (int i = 0; i < 8; ++i) st[i] = 0;
 #pragma unroll 1
     for (int n = 0; n < hashes; ++n) {
-        if (n > 0) bar_wait(kBarPair);    // this hash's pair, made behind the last padding block's rounds
+        bar_wait(kBarPair);    // this hash's pair, made behind the last padding block's rounds
         m.h[0][lane] = make_uint4(st[0], st[1], st[2], st[3]);
         m.h[1][lane] = make_uint4(st[4], st[5], st[6], st[7]);
         bar_arrive(kBarH);
@@ -371,7 +371,7 @@ __device__ __forceinline__ void chain_schedule(ChainMem& m, int hashes, Add add,
     };
     pair(0, next);
     place(0);
-    __syncthreads();   // the first pair is in place (the rounds' warp waits here too)
+    bar_arrive(kBarPair);
 #pragma unroll 1
     for (int n = 0; n < hashes; ++n) {
         uint32_t w[16];
@@ -426,7 +426,6 @@ template <bool kPairFirst, class Add, class Pair>
 __device__ __forceinline__ bool chain_pair(ChainMem& m, int hashes, uint32_t st[8], Add add, Pair pair)
 {
     if (threadIdx.x < 32) {
-        __syncthreads();
         chain_rounds<kPairFirst>(m, hashes, st, add);
         return true;
     }
