@@ -15,15 +15,25 @@
 //
 // The state is a plain struct (the SHA-256 chaining words, the pending partial
 // block, the byte count and the challenge counter), so it can move between host
-// and device memory by a copy; host and device share the code.
+// and device memory by a copy. The host appends to the state itself, a warp of the
+// device to a stretch in shared memory (Writer): two pieces of code with the same
+// bytes, draws and states.
 #pragma once
 #include <stdint.h>
 
 #include "fp2.cuh"
 #include "sha256.cuh"
 
+// A draw below this is taken, one from here on is drawn again (2^-61 of them); tests
+// compile with a smaller one.
+#ifndef TP_FS_DRAW_BOUND
+#define TP_FS_DRAW_BOUND P61
+#endif
+
 namespace tp {
 namespace fs {
+
+constexpr uint64_t kDrawBound = TP_FS_DRAW_BOUND;
 
 struct State {
     uint32_t h[8];
@@ -240,7 +250,7 @@ inline uint64_t rand_scalar(State& s)
     for (int it = 0; it < 1000; ++it) {
         put_counter(s);
         v = draw_bits(s);
-        if (v < P61) return v;
+        if (v < kDrawBound) return v;
     }
     return v % P61;
 }
@@ -435,7 +445,7 @@ static __device__ __noinline__ bool tx_draw(TxMem* m, uint32_t n, uint64_t total
     tx_draw_bytes(m, n, len, rnum, 0);
     tx_draw_bytes(m, n + per, len, rnum + 1, 1);
     tx_hash(m, n + per, n + 2 * per, total + 2 * per, true);
-    const bool ok = m->out[0] < P61 && m->out[1] < P61;
+    const bool ok = m->out[0] < kDrawBound && m->out[1] < kDrawBound;
     if (ok) tx_advance(m, n + 2 * per);
     return ok;
 }
@@ -459,7 +469,7 @@ static __device__ __noinline__ void tx_redraw(TxMem* m, uint32_t n, uint64_t tot
                 const int q = threadIdx.x & 31;
                 if (q < 13)
                     reinterpret_cast<uint8_t*>(m->buf)[n + q] =
-                        (uint8_t)(q < 5 ? 0x0101u >> (8 * q) : rnum >> (8 * (q - 5)));
+                        (uint8_t)(q < 5 ? 0x0101ull >> (8 * q) : rnum >> (8 * (q - 5)));
                 n += 13;
                 total += 13;
             }
@@ -468,7 +478,7 @@ static __device__ __noinline__ void tx_redraw(TxMem* m, uint32_t n, uint64_t tot
             v = m->out[1];
             tx_advance(m, n);
             n &= 63;
-            if (v < P61) break;
+            if (v < kDrawBound) break;
         }
         limb[k] = v % P61;
     }
