@@ -1,5 +1,5 @@
-"""A frame whose table could not be loaded (the vectors of its rounds do not fit the
-device) takes no claim, no second fold and no finish, and its batch can be set anew."""
+"""A frame that could not be loaded (the vectors of its rounds do not fit the device)
+takes no claim, no second fold and no finish, and its batch can be set anew."""
 import ctypes
 
 import numpy as np
@@ -23,15 +23,15 @@ def test_a_frame_that_did_not_fit():
     z = np.array([rand_fp(rng, groups), rand_fp(rng, groups)], np.uint64)
     s = torch.cuda.current_stream().cuda_stream
     copies = 8
-    values = torch.from_numpy(rng.integers(0, P61, 2 * W * copies).astype(np.int64)).cuda()
+    pixels = torch.from_numpy(rng.integers(0, 256, W * copies, dtype=np.uint8)).cuda()
     beta = torch.from_numpy(rng.integers(0, P61, 2 * copies).astype(np.int64)).cuda()
     claims = torch.zeros(8, dtype=torch.int64, device="cuda")
     out = torch.zeros(2 * W + 2, dtype=torch.int64, device="cuda")
     ch = np.array([3, 5], np.uint64)
 
     def load(b, n):
-        return lib.tp_batch_set_table(b, 0, groups, gt.ctypes.data, i0.ctypes.data, i1.ctypes.data, z[0].ctypes.data,
-                                      z[1].ctypes.data, n, W, values.data_ptr(), beta.data_ptr(), 1)
+        return lib.tp_batch_set_pixels(b, 0, groups, gt.ctypes.data, i0.ctypes.data, i1.ctypes.data, z[0].ctypes.data,
+                                       z[1].ctypes.data, pixels.data_ptr(), copies, n, W, W, -1, 0, beta.data_ptr())
 
     def first_claim(b):
         assert lib.tp_batch_claim(b, claims.data_ptr()) == 0, lib.tp_last_error()

@@ -80,8 +80,8 @@ struct Frame {
     bool configured = false;
     bool loaded = false;   // its table, bytes or vectors are in place
     size_t cap0 = 0, cap1 = 0, capb = 0, capfin = 0;  // element capacities kept across resets
-    // rounds on vectors (gkr_linear.cu): the source stays as it is (bytes copied
-    // aside by the forms launch, or the table in buf[0]) until the finish
+    // a byte frame's rounds on vectors (gkr_linear.cu): its bytes, copied aside by the
+    // forms launch, stay until the finish
     bool linear = false, forms_done = false;
     int folds = 0;                            // folds applied to the vectors, recorded in rs
     fp2* vec[2] = {nullptr, nullptr};         // 1 + 2 groups vectors of n / n/2 copies

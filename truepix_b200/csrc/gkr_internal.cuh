@@ -140,18 +140,17 @@ struct Job {
     int vec;                // byte rows are whole 16-byte vectors (copy_size % 16 == 0, aligned)
     // rounds on vectors (gkr_linear.cu): A / Aout hold 1 + 2 G vectors of n_in copies
     int G, stride;          // product groups; row length of `bytes`
-    const fp2* src;         // a table source's table [W_rows][n_table]
     unsigned char* bytes;   // a byte source's copied rows
     const int* gptr;        // [G + 1] the groups' terms in ab / cf
     const int* gb;          // [G] their wires b
     fp2* rs;                // challenges of the folds applied so far
     const fp2* given;       // challenges of the next rounds (all rounds in one launch)
-    fp2* fpart;             // finish: partial sums per chunk of copies, or eq of every copy
-    int n_table, nf, has_r; // nf: recorded folds; has_r: r is pending
+    fp2* fpart;             // finish: partial sums per chunk of copies
+    int nf, has_r;          // nf: recorded folds; has_r: r is pending
     int chunks, n_rounds, frame, pad_;
 };
 
-enum : int { kVecClaim = 4, kVecFold = 5, kFormsBytes = 6, kFormsTable = 7 };
+enum : int { kVecClaim = 4, kVecFold = 5, kFormsBytes = 6 };
 
 void plan_job(Job& j, int target_ctas);
 // gkr_linear.cu: the rounds on vectors
@@ -177,7 +176,7 @@ bool launch_linear(const Job* d_jobs, const std::vector<Job>& jobs, int kind, cu
 // J.n_rounds rounds of every job in one launch; v null: the challenges J.given
 bool launch_linear_rounds(const Job* d_jobs, int n_jobs, const VoleRounds* v, int k0, long long claim_stride,
                           cudaStream_t s, int* launches);
-bool launch_linear_finish(const Job* d_jobs, const std::vector<Job>& jobs, bool bytes, cudaStream_t s, int* launches);
+bool launch_linear_finish(const Job* d_jobs, const std::vector<Job>& jobs, cudaStream_t s, int* launches);
 bool launch_round(const Job* d_jobs, const std::vector<Job>& jobs, int kind, cudaStream_t s,
                   int* launches);
 bool launch_finish(const Job* d_jobs, int n_jobs, int max_w, cudaStream_t s, int* launches);

@@ -1,4 +1,4 @@
-// Early rounds whose per-copy sums stay in vectors.
+// Early rounds of byte frames whose per-copy sums stay in vectors.
 //
 // A round's claim at copy c needs, besides beta, only
 //   s(c) = sum_w L[w] V[w][c]                     (the layer's linear part)
@@ -7,25 +7,24 @@
 // challenge is linear, so these 1 + 2 G vectors fold by themselves, and the table
 // of all wires is not needed until the end, where the wire values are sums over
 // the copies weighted with eq(challenges, c). For the layers of TruePix's circuits
-// (G = 0, or 1 to 3 for mask and crop) a round then moves 32 B per copy and vector
-// instead of 32 B per copy and wire: over 64 1080p frames the rounds after the
+// (G = 0 for gray, inv and mask, 1 for crop) a round then moves 32 B per copy and
+// vector instead of 32 B per copy and wire: over 64 1080p frames the rounds after the
 // first took 2.95 ms (12.9 GB of folded tables written and read) and now 0.1 ms.
 // The sums are exact field sums, so every value is the same.
 //
-//   forms     the vectors from the source. From bytes: an integer matrix product
+//   forms     the vectors from the bytes: an integer matrix product
 //             (copies x wires bytes) x (wires x 16 byte-planes of a form's
 //             coefficients, eight for each limb) on the tensor cores, u8 x u8
 //             accumulated in 32 bits (512 * 255 * 255 < 2^31), recombined mod p;
 //             bound by reading the bytes. The bytes are also copied aside (rows of
 //             a multiple of 32 bytes), so that the caller's buffer is free after
-//             the first claim or fold as before. From a table: one warp a slice of
-//             rows, 32 copies wide; bound by reading the table.
+//             the first claim or fold as before.
 //   rounds    one thread a pair of copies, one launch a round (vec_round_kernel), or
 //             all rounds of a frame in one CTA once few pairs are left
 //             (vec_rounds_kernel), with the challenges given or drawn by the
 //             VOLE-committed round on the frame's transcript.
-//   finish    wires from bytes: (16 byte-planes of eq) x (copies x wires) the same
-//             way; from a table: a warp per wire.
+//   finish    the wires from the bytes: (16 byte-planes of eq) x (copies x wires) the
+//             same way.
 #include "gkr.h"
 #include "gkr_internal.cuh"
 #include "runtime.h"
@@ -256,63 +255,6 @@ __global__ void __launch_bounds__(kFormThreads) forms_bytes_kernel(const Job* __
             }
             __syncthreads();
         }
-    }
-}
-
-// ---- forms from a table ---------------------------------------------------------
-// CTA = 32 copies; its warps take slices of the rows and of each group's terms
-__global__ void __launch_bounds__(kVecThreads) forms_table_kernel(const Job* __restrict__ jobs)
-{
-    __shared__ __align__(16) Job J;
-    __shared__ fp2 red[kVecThreads / 32][32];
-    read_job(jobs, J);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    constexpr int kW = kVecThreads / 32;
-    if ((int)blockIdx.x * 32 >= J.n_in) return;
-    const int c = blockIdx.x * 32 + lane;
-    const bool live = c < J.n_in;
-    const fp2* src = J.src + (live ? c : 0);
-    fp2* out = const_cast<fp2*>(J.A);
-    auto at = [&](int w) {
-        const fp2 v = w < J.W_rows ? ld2(src + (size_t)w * J.n_in) : f2zero();
-        return mk(fold61(v.re), fold61(v.im));
-    };
-    for (int form = 0; form <= J.G; ++form) {
-        const int n = form == 0 ? J.W_rows : J.gptr[form] - J.gptr[form - 1];
-        const int base = form == 0 ? 0 : J.gptr[form - 1];
-        const int per = (n + kW - 1) / kW;
-        const int e0 = min(n, warp * per), e1 = min(n, e0 + per);
-        u64 re = 0, im = 0;
-        int e = e0;
-        for (; e + 4 <= e1; e += 4) {   // four rows' loads before their products
-            fp2 x[4], l[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                x[k] = at(form == 0 ? e + k : J.ab[base + e + k].x);
-                l[k] = ld2((form == 0 ? J.L : J.cf + base) + e + k);
-            }
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const fp2 v = l2mul(l[k], x[k]);
-                re = fold61(re + v.re);
-                im = fold61(im + v.im);
-            }
-        }
-        for (; e < e1; ++e) {
-            const fp2 v = l2mul(ld2((form == 0 ? J.L : J.cf + base) + e), at(form == 0 ? e : J.ab[base + e].x));
-            re = fold61(re + v.re);
-            im = fold61(im + v.im);
-        }
-        red[warp][lane] = mk(re, im);
-        __syncthreads();
-        fp2* o = out + (size_t)(form == 0 ? 0 : 2 * form - 1) * J.n_in;
-        if (warp == 0 && live) {
-            fp2 s = red[0][lane];
-            for (int k = 1; k < kW; ++k) s = l2add(s, red[k][lane]);
-            st2(o + c, s);
-        }
-        if (form > 0 && warp == 1 && live) st2(o + J.n_in + c, at(J.gb[form - 1]));
-        __syncthreads();
     }
 }
 
@@ -915,40 +857,6 @@ __global__ void __maxnreg__(80) mle_bytes_kernel(const MleArgs a)
     }
 }
 
-// eq(challenges, c) of all copies of a table's frame
-__global__ void __launch_bounds__(kFinCopies) finish_eq_kernel(const Job* __restrict__ jobs)
-{
-    __shared__ __align__(16) Job J;
-    __shared__ EqParts e;
-    read_job(jobs, J);
-    const int kf = J.nf + (J.has_r != 0);
-    const int c = blockIdx.x * kFinCopies + threadIdx.x;
-    if ((long long)blockIdx.x * kFinCopies >= (1LL << kf)) return;
-    eq_parts(J, blockIdx.x, 1, e);
-    if (c < (1 << kf)) st2(J.fpart + c, eq_of(e, threadIdx.x));
-    if (c == 0) finish_beta(J);
-}
-
-// wires from a table: a warp per wire
-__global__ void __launch_bounds__(kVecThreads) finish_table_kernel(const Job* __restrict__ jobs)
-{
-    __shared__ __align__(16) Job J;
-    read_job(jobs, J);
-    const int w = blockIdx.x * (kVecThreads / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (w >= J.W) return;
-    const int n = 1 << (J.nf + (J.has_r != 0));
-    fp2 s = f2zero();
-    if (w < J.W_rows) {
-        const fp2* row = J.src + (size_t)w * J.n_table;
-        for (int c = lane; c < n; c += 32) {
-            const fp2 v = ld2(row + c);
-            s = l2add(s, l2mul(ld2(J.fpart + c), mk(fold61(v.re), fold61(v.im))));
-        }
-    }
-    s = warp_sum(l2canon(s));
-    if (lane == 0) st2(J.fin + w, s);
-}
-
 size_t row_smem(unsigned threads) { return (size_t)(threads / 32) * kRowStages * kRowStep; }
 
 size_t form_smem(int kp) { return (size_t)(2 * kTileRows + 16) * (kp + 16); }
@@ -1021,8 +929,6 @@ void plan_linear_job(Job& j, int kind, int target)
         const int tiles = (j.n_in + kTileRows - 1) / kTileRows;
         j.wpg = std::max(1, std::min(16, tiles / target));
         j.tiles = (tiles + j.wpg - 1) / j.wpg;
-    } else if (kind == kFormsTable) {
-        j.tiles = (j.n_in + 31) / 32;
     } else {
         j.tiles = std::max(1, (j.n_pairs + kVecThreads - 1) / kVecThreads);
     }
@@ -1041,7 +947,6 @@ bool launch_linear(const Job* d_jobs, const std::vector<Job>& jobs, int kind, cu
     }
     const dim3 grid(ctas, (unsigned)jobs.size());
     if (kind == kFormsBytes) forms_bytes_kernel<<<grid, kFormThreads, form_smem(kp), s>>>(d_jobs);
-    else if (kind == kFormsTable) forms_table_kernel<<<grid, kVecThreads, 0, s>>>(d_jobs);
     else if (kind == kVecClaim) vec_round_kernel<false><<<grid, kVecThreads, 0, s>>>(d_jobs);
     else vec_round_kernel<true><<<grid, kVecThreads, 0, s>>>(d_jobs);
     ++*launches;
@@ -1138,30 +1043,17 @@ bool launch_mle_pixels_batch(const MleFrame* h_frames, int n, int n_pad, int cs,
     return ok;
 }
 
-bool launch_linear_finish(const Job* d_jobs, const std::vector<Job>& jobs, bool bytes, cudaStream_t s, int* launches)
+bool launch_linear_finish(const Job* d_jobs, const std::vector<Job>& jobs, cudaStream_t s, int* launches)
 {
     if (jobs.empty()) return true;
-    if (bytes) {
-        int chunks = 1, kp = 32;
-        for (const Job& j : jobs) {
-            chunks = std::max(chunks, j.chunks);
-            kp = std::max(kp, j.stride);
-        }
-        const unsigned threads = (unsigned)std::max(64, kp);   // a warp per 32 wires, 512 at most
-        finish_bytes_kernel<<<dim3((unsigned)chunks, (unsigned)jobs.size()), threads, row_smem(threads), s>>>(d_jobs);
-        ++*launches;
-    } else {
-        int kf = 0, w = 1;
-        for (const Job& j : jobs) {
-            kf = std::max(kf, j.nf + (j.has_r != 0));
-            w = std::max(w, j.W);
-        }
-        const unsigned eq = (unsigned)(((1LL << kf) + kFinCopies - 1) / kFinCopies);
-        finish_eq_kernel<<<dim3(eq, (unsigned)jobs.size()), kFinCopies, 0, s>>>(d_jobs);
-        finish_table_kernel<<<dim3(blocks_for((size_t)w, kVecThreads / 32), (unsigned)jobs.size()), kVecThreads, 0, s>>>(
-            d_jobs);
-        *launches += 2;
+    int chunks = 1, kp = 32;
+    for (const Job& j : jobs) {
+        chunks = std::max(chunks, j.chunks);
+        kp = std::max(kp, j.stride);
     }
+    const unsigned threads = (unsigned)std::max(64, kp);   // a warp per 32 wires, 512 at most
+    finish_bytes_kernel<<<dim3((unsigned)chunks, (unsigned)jobs.size()), threads, row_smem(threads), s>>>(d_jobs);
+    ++*launches;
     return !cuda_failed(cudaGetLastError(), "linear finish launch");
 }
 

@@ -66,13 +66,21 @@ bool grow(T*& p, size_t& cap, size_t n, cudaStream_t s)
     return p != nullptr;
 }
 
-// Whether the frame's rounds run on vectors (gkr_linear.cu): 1 + 2 groups vectors
-// in place of W_rows rows. A round moves so many times less, against one more pass
-// over the source at the end; below a quarter of the rows that always pays (gray
-// and crop: 1 and 3 against 385 and 386).
+// Whether a byte frame's rounds run on vectors (gkr_linear.cu): 1 + 2 groups vectors in
+// place of W_rows rows. A round moves so many times less, against a pass over the bytes
+// for every group and one more at the end. 384 bytes a copy, one frame, a call a round,
+// rows -> vectors in us: no group, 2 copies 46 -> 54, 4 copies 70 -> 67, 8,192 copies
+// 271 -> 198; one group 182 -> 168 and 456 -> 313; 4 groups 255 -> 250 and 538 -> 448;
+// 8 groups 281 -> 291, 552 -> 552, and from 16,384 copies on 673 -> 592.
+// A frame given as a table stays on its rows: its vectors cost two passes over 16 bytes a
+// wire and won nothing in the same rounds (512 wires: 32 copies 98 -> 118, 2,048 copies
+// 203 -> 196, 8,192 copies 319 -> 329; 16 wires and 32,768 copies 246 -> 582; 2^18 wires
+// and 2 copies 0.8 -> 17 ms).
 bool wants_linear(const Frame* f)
 {
-    return f->form.groups <= kMaxLinGroups && 4 * (1 + 2 * f->form.groups) <= f->W_rows;
+    const int G = f->form.groups;
+    return f->n_copies0 >= 4 && G <= kMaxLinGroups && 4 * (1 + 2 * G) <= f->W_rows &&
+           (G <= 4 || f->n_copies0 >= 2048 * G);
 }
 
 // the vectors' buffers of a frame; `part`: elements of the finish's scratch
@@ -223,21 +231,15 @@ Job base_job(const Frame* f)
         j.nf = f->folds;
         j.has_r = f->pending ? 1 : 0;
         j.fpart = f->fpart;
-        j.n_table = f->n_copies0;
-        j.const_idx = -1;
-        if (f->px.pix) {
-            j.pix = f->px.pix;
-            j.n_real = f->px.n_real;
-            j.cs = f->px.cs;
-            j.const_idx = f->px.const_idx;
-            j.const_val = f->px.const_val;
-            j.bytes = f->bytes;
-            j.stride = lin_stride(f->px.cs);
-            j.chunks = lin_chunks(f->px.n_real, f->folds + j.has_r);
-            j.vec = ((j.cs & 15) == 0 && (reinterpret_cast<size_t>(j.pix) & 15) == 0) ? 1 : 0;
-        } else {
-            j.src = f->buf[0];
-        }
+        j.pix = f->px.pix;
+        j.n_real = f->px.n_real;
+        j.cs = f->px.cs;
+        j.const_idx = f->px.const_idx;
+        j.const_val = f->px.const_val;
+        j.bytes = f->bytes;
+        j.stride = lin_stride(f->px.cs);
+        j.chunks = lin_chunks(f->px.n_real, f->folds + j.has_r);
+        j.vec = ((j.cs & 15) == 0 && (reinterpret_cast<size_t>(j.pix) & 15) == 0) ? 1 : 0;
     } else if (f->pix_cur) {
         j.pix = f->px.pix;
         j.n_real = f->px.n_real;
@@ -337,8 +339,6 @@ bool batch_load_host(Batch* B, int i, const u64* v_re, const u64* v_im, const u6
     cudaStream_t s = B->stream;
     const size_t vn = (size_t)f->n_wires * (size_t)f->n_copies0;
     if (!frame_alloc(f, vn, vn / 2, s)) return false;
-    f->px = PixSrc{};
-    if (wants_linear(f) && !linear_alloc(f, (size_t)f->n_copies0, s)) return false;
     // stage the real limbs in the half-size buffer (exactly vn u64), the
     // imaginary limbs in a temporary, then pack
     u64* stage_re = reinterpret_cast<u64*>(f->buf[1]);
@@ -364,10 +364,7 @@ bool batch_load_device(Batch* B, int i, const fp2* d_values, const fp2* d_beta, 
     Frame* f = B->frames[(size_t)i];
     cudaStream_t s = B->stream;
     const size_t vn = (size_t)f->n_wires * (size_t)f->n_copies0;
-    f->px = PixSrc{};
-    const bool linear = wants_linear(f);
-    if (!frame_alloc(f, borrow ? 0 : vn, linear ? 0 : vn / 2, s)) return false;
-    if (linear && !linear_alloc(f, (size_t)f->n_copies0, s)) return false;
+    if (!frame_alloc(f, borrow ? 0 : vn, vn / 2, s)) return false;
     if (borrow) {
         f->buf[0] = const_cast<fp2*>(d_values);
         f->borrowed0 = true;
@@ -620,26 +617,24 @@ void set_workspace_ptrs(Batch* B, std::vector<Job>& jobs)
 // the launch that makes the vectors of frames which have none yet; appended to out
 void plan_forms(const std::vector<Frame*>& frames, std::vector<RoundLaunch>& out, int n_sm)
 {
-    for (int kind : {(int)kFormsBytes, (int)kFormsTable}) {
-        RoundLaunch L;
-        L.kind = kind;
-        int lg = 0;
-        for (Frame* f : frames) {
-            if (!f->linear || f->forms_done || (f->px.pix != nullptr) != (kind == kFormsBytes)) continue;
-            Job j = base_job(f);
-            j.kind = kind;
-            L.jobs.push_back(j);
-            L.rdev.push_back(nullptr);
-            f->forms_done = true;
-            lg = 0;
-            while ((1 << lg) < f->n_copies0) ++lg;
-        }
-        if (L.jobs.empty()) continue;
-        if (kind == kFormsBytes) L.bucket = work_bucket(L.jobs, kind);
-        plan_linear_jobs(L.jobs, kind, (kind == kFormsBytes ? tuned_mult(2, L.bucket) : 4) * n_sm);
-        L.timer_tag = (kind == kFormsBytes ? 1000 : 0) + lg;
-        out.push_back(std::move(L));
+    RoundLaunch L;
+    L.kind = kFormsBytes;
+    int lg = 0;
+    for (Frame* f : frames) {
+        if (!f->linear || f->forms_done) continue;
+        Job j = base_job(f);
+        j.kind = kFormsBytes;
+        L.jobs.push_back(j);
+        L.rdev.push_back(nullptr);
+        f->forms_done = true;
+        lg = 0;
+        while ((1 << lg) < f->n_copies0) ++lg;
     }
+    if (L.jobs.empty()) return;
+    L.bucket = work_bucket(L.jobs, kFormsBytes);
+    plan_linear_jobs(L.jobs, kFormsBytes, tuned_mult(2, L.bucket) * n_sm);
+    L.timer_tag = 1000 + lg;
+    out.push_back(std::move(L));
 }
 
 constexpr int kKinds = 6;   // 0..3 on tables and bytes, kVecClaim, kVecFold
@@ -921,9 +916,9 @@ namespace {
 // The finish launches: wires and beta of every configured frame (a pending fold of
 // the last two copies applied by it). A pending fold of more copies is applied
 // first (host challenges only) on a table of all wires; linear frames take copy 0
-// after the pending fold from the source at once. out: [0] frames on tables, [1]
-// linear ones from bytes, [2] from a table; `forms` (if any) come before them.
-constexpr int kFinishKinds = 3;
+// after the pending fold from the bytes at once. out: [0] frames on tables, [1]
+// linear ones; `forms` (if any) come before them.
+constexpr int kFinishKinds = 2;
 
 bool plan_finish_frame(Batch* B, Frame* f, fp2* d_wires, fp2* d_beta, RoundLaunch (&out)[kFinishKinds])
 {
@@ -934,7 +929,7 @@ bool plan_finish_frame(Batch* B, Frame* f, fp2* d_wires, fp2* d_beta, RoundLaunc
     j.kind = f->pending ? 1 : 0;  // a pending fold of the last two copies
     j.fin = d_wires ? d_wires : f->fin;
     j.fin_beta = d_beta ? d_beta : f->fin + f->n_wires;
-    RoundLaunch& L = out[!f->linear ? 0 : f->px.pix ? 1 : 2];
+    RoundLaunch& L = out[f->linear ? 1 : 0];
     L.kind = 8;
     j.tiles = j.groups = 1;
     L.max_w = std::max(L.max_w, f->n_wires);
@@ -956,7 +951,7 @@ bool plan_finish(Batch* B, fp2* const* d_wires, fp2* const* d_beta, std::vector<
             set_error(TP_ERR_ARG, "frame %zu has no table", i);
             return false;
         }
-        if (f->linear && !f->forms_done && f->px.pix) fresh.push_back(f);   // their bytes are copied by the forms
+        if (f->linear && !f->forms_done) fresh.push_back(f);   // their bytes are copied by the forms
         if (!plan_finish_frame(B, f, d_wires ? d_wires[i] : nullptr, d_beta ? d_beta[i] : nullptr, out)) return false;
     }
     plan_linear_finish(out[1].jobs);
@@ -967,7 +962,7 @@ bool plan_finish(Batch* B, fp2* const* d_wires, fp2* const* d_beta, std::vector<
 bool launch_finish_kind(const Job* d_jobs, const RoundLaunch& L, int which, cudaStream_t s, int* launches)
 {
     return which == 0 ? launch_finish(d_jobs, (int)L.jobs.size(), L.max_w, s, launches)
-                      : launch_linear_finish(d_jobs, L.jobs, which == 1, s, launches);
+                      : launch_linear_finish(d_jobs, L.jobs, s, launches);
 }
 
 bool launch_finishes(Batch* B, std::vector<RoundLaunch>& forms, RoundLaunch (&fin)[kFinishKinds])
@@ -1196,7 +1191,7 @@ bool batch_vole_rounds_graph(Batch* B, u64* d_claims, void* d_states, void* d_vo
             key.push_back(j.W);
             key.push_back(j.nf + j.has_r);
         }
-        kernels += (op.type == 1) ? 1 : 1 + (op.n_patch ? 1 : 0) + (op.type == 2 && op.fin == 2 ? 1 : 0);
+        kernels += (op.type == 1) ? 1 : 1 + (op.n_patch ? 1 : 0);
     }
     if (!B->graph || key != B->graph_key) {
         if (B->graph) {
@@ -1302,7 +1297,7 @@ bool batch_finish_frame(Batch* B, int i, fp2* d_wires, fp2* d_beta)
     if (!c) return false;
     std::vector<RoundLaunch> forms;
     RoundLaunch fin[kFinishKinds];
-    const bool fresh = f->linear && !f->forms_done && f->px.pix;
+    const bool fresh = f->linear && !f->forms_done;
     if (!plan_finish_frame(B, f, d_wires, d_beta, fin)) return false;
     plan_linear_finish(fin[1].jobs);
     if (fresh) plan_forms({f}, forms, c->n_sm);
