@@ -516,7 +516,10 @@ bool build_gate_form(int n_gates, const int* type, const int* in0, const int* in
     return true;
 }
 
-void pack_gate_form(const GateForm& g, DevGateForm& d, std::vector<unsigned char>& h)
+namespace {
+
+// the form's arrays behind h's bytes; L itself only when asked for
+void pack_form(const GateForm& g, DevGateForm& d, std::vector<unsigned char>& h, bool with_L)
 {
     d.K0 = g.K0;
     d.n_wires = (int)g.L.size();
@@ -537,16 +540,18 @@ void pack_gate_form(const GateForm& g, DevGateForm& d, std::vector<unsigned char
         if (bytes) memcpy(h.data() + at, p, bytes);
         return at;
     };
-    d.at[0] = put(g.L.data(), sizeof(fp2) * g.L.size());
+    if (with_L) d.at[0] = put(g.L.data(), sizeof(fp2) * g.L.size());
     d.at[1] = put(g.tc.data(), sizeof(fp2) * g.tc.size());
-    d.at[2] = h.size();
-    for (int i = 0; i < d.n_terms; ++i) {
-        const int2 ab = make_int2(g.ta[(size_t)i], g.tb[(size_t)i]);
-        put(&ab, sizeof ab);
-    }
+    std::vector<int2> ab((size_t)d.n_terms);
+    for (size_t i = 0; i < ab.size(); ++i) ab[i] = make_int2(g.ta[i], g.tb[i]);
+    d.at[2] = put(ab.data(), sizeof(int2) * ab.size());
     d.at[3] = put(gptr.data(), sizeof(int) * gptr.size());
     d.at[4] = put(gb.data(), sizeof(int) * gb.size());
 }
+
+}  // namespace
+
+void pack_gate_form(const GateForm& g, DevGateForm& d, std::vector<unsigned char>& h) { pack_form(g, d, h, true); }
 
 void place_gate_form(DevGateForm& d, void* base)
 {
@@ -558,19 +563,29 @@ void place_gate_form(DevGateForm& d, void* base)
     d.gb = reinterpret_cast<int*>(m + d.at[4]);
 }
 
+// Up to 1,024 wires in one upload; the L of more is uploaded from where it stands, behind
+// the terms (packed with them, the 4 MB of 2^18 wires cost 3 ms of page faults a call).
 bool upload_gate_form(const GateForm& g, DevGateForm& d, cudaStream_t s)
 {
     std::vector<unsigned char> h;
-    pack_gate_form(g, d, h);
-    if (h.size() > d.cap) {
+    const bool apart = g.L.size() > 1024;
+    pack_form(g, d, h, !apart);
+    size_t total = h.size();
+    if (apart) {
+        d.at[0] = (h.size() + 15) & ~(size_t)15;
+        total = d.at[0] + sizeof(fp2) * g.L.size();
+    }
+    if (total > d.cap) {
         dev_free(d.mem, s);
         d.cap = 0;
-        d.mem = dev_alloc(h.size(), s);
+        d.mem = dev_alloc(total, s);
         if (!d.mem) return false;
-        d.cap = h.size();
+        d.cap = total;
     }
     place_gate_form(d, d.mem);
-    return upload_async(d.mem, h.data(), h.size(), s);
+    if (!apart) return upload_async(d.mem, h.data(), total, s);
+    return (!d.n_terms || upload_async(d.mem, h.data(), h.size(), s)) &&
+           upload_async(d.L, g.L.data(), sizeof(fp2) * g.L.size(), s);
 }
 
 void free_gate_form(DevGateForm& d, cudaStream_t s)
