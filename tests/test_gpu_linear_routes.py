@@ -1,6 +1,6 @@
 """Byte frames on both sides of the lines between rounds on vectors and on the table of
-all wires (copies, product groups, copies per group), against the oracle's session;
-frames of both kinds in one batch."""
+all wires, and between a launch a round and all rounds in one (copies, product groups,
+copies per group), against the oracle's session; frames of both kinds in one batch."""
 import ctypes
 
 import numpy as np
@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("W,cs,real,C,groups", [
     (64, 48, 2, 2, 0), (64, 48, 4, 4, 0), (64, 48, 4, 4, 4), (64, 48, 900, 1024, 4), (64, 48, 900, 1024, 5),
-    (64, 48, 8100, 8192, 5), (64, 48, 16000, 16384, 5), (128, 72, 8192, 8192, 8), (128, 72, 16384, 16384, 8),
+    (64, 48, 8100, 8192, 2), (64, 48, 4096, 4096, 4), (64, 48, 8100, 8192, 5), (64, 48, 16000, 16384, 5), (128, 72, 8192, 8192, 8), (128, 72, 16384, 16384, 8),
     (256, 140, 32000, 32768, 16), (64, 35, 100, 128, 4), (64, 36, 100, 128, 4)])
 def test_byte_frames(lib, oracle, W, cs, real, C, groups):  # noqa: F811
     rounds.test_bytes_source(lib, oracle, W, cs, real, C, -1, groups, 0)

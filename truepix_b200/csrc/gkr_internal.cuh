@@ -155,7 +155,11 @@ enum : int { kVecClaim = 4, kVecFold = 5, kFormsBytes = 6 };
 void plan_job(Job& j, int target_ctas);
 // gkr_linear.cu: the rounds on vectors
 constexpr int kMaxLinGroups = 16;   // more product groups keep the table of all wires
-constexpr int kFusePairs = 4096;    // from this many pairs on a frame's rounds run in one CTA
+// A frame's rounds run in one CTA once it has this few pairs, and this few pairs times
+// vectors (1 + 2 groups). 384 bytes a copy, all rounds given, in one CTA from 4,096 pairs
+// on -> a launch a round, in us: no group 131 -> 198, one 288 -> 313, 2 groups 366 -> 365,
+// 4 groups 483 -> 448, 8 groups 679 -> 552; 2,048 pairs and 4 groups 391 -> 414.
+constexpr int kFusePairs = 4096, kFuseEntries = 16384;
 int lin_stride(int cs);
 size_t lin_bytes(int cs, int n_real);        // bytes of a frame's copied rows
 int lin_chunks(int n_real, int folds);       // pieces of 512 copies of the finish from bytes

@@ -788,6 +788,13 @@ bool apply_fold_linear(Batch* B, Frame* f)
     return true;
 }
 
+// whether a linear frame's rounds that are left run in one CTA
+bool few_left(const Frame* f)
+{
+    const long long pairs = f->n_copies / 2;
+    return pairs <= kFusePairs && pairs * (1 + 2 * f->form.groups) <= kFuseEntries;
+}
+
 // Rounds of a linear frame whose challenges (device memory at its given[]) are all
 // known: n_rounds claims, each followed by its fold, in one launch; the last fold
 // stays recorded (host challenge `last`). Planned into L.
@@ -820,7 +827,7 @@ bool batch_given_rounds(Batch* B, int n_rounds, const u64* challenges, u64* d_cl
         // from here on in one launch: few pairs left, two rounds or more to go
         const int left = n_rounds - k;
         if (f->configured && f->loaded && f->linear && d_claims && left > 1 && left <= 63 &&
-            f->n_copies / 2 <= kFusePairs && (f->n_copies >> left) >= 1) {
+            few_left(f) && (f->n_copies >> left) >= 1) {
             std::vector<fp2> r;
             for (int q = k; q < n_rounds; ++q) {
                 r.push_back(mk(challenges[2 * q], challenges[2 * q + 1]));
@@ -1045,8 +1052,6 @@ bool batch_vole_rounds_graph(Batch* B, u64* d_claims, void* d_states, void* d_vo
     // ---- plan every launch (advances the frames as the launches will)
     std::vector<GraphOp> ops;
     std::vector<u64*> claim_ptrs((size_t)nB);
-    bool all_linear = true;
-    for (const Frame* f : B->frames) all_linear = all_linear && f->loaded && f->linear;
     auto push = [&](RoundLaunch& L, int type) {
         GraphOp op;
         op.type = type;
@@ -1055,11 +1060,12 @@ bool batch_vole_rounds_graph(Batch* B, u64* d_claims, void* d_states, void* d_vo
     };
     int k = 0;
     for (; k < rounds; ++k) {
-        // frames on vectors: once no frame has many pairs left, each runs the rest of
-        // its rounds, transcript included, in one CTA
-        int most = 0;
-        for (const Frame* f : B->frames) most = std::max(most, f->n_copies / 2);
-        if (all_linear && most <= kFusePairs) break;
+        // once only frames on vectors have rounds left, and few pairs, each runs the rest
+        // of its rounds, transcript included, in one CTA
+        bool fuse = true;
+        for (const Frame* f : B->frames)
+            fuse = fuse && f->loaded && (f->n_copies < 2 || (f->linear && few_left(f)));
+        if (fuse) break;
         for (int i = 0; i < nB; ++i) claim_ptrs[(size_t)i] = d_claims + 8 * ((size_t)nB * k + i);
         std::vector<RoundLaunch> plan;
         if (!plan_claims(B, claim_ptrs.data(), plan)) return false;
