@@ -9,6 +9,7 @@
 
 #include <algorithm>
 #include <array>
+#include <type_traits>
 #include <vector>
 
 #include "gkr_internal.cuh"
@@ -75,15 +76,48 @@ bool make_device_label(const char* label, tp::fs::Label* L, const char* who)
 
 // Device transcripts: one warp (a CTA of 32 threads) per state, see Writer in
 // transcript.cuh. The kernels are bound by the latency of the hash's round chain, so
-// a warp of its own costs nothing and transcripts at different offsets do not diverge.
-constexpr int kFsThreads = 32;
+// a warp of its own costs nothing and transcripts at different offsets do not diverge,
+// while a scheduler has a few. Of more states each has a thread: a warp a state hashes
+// every block 32 times over. Four elements put and one drawn, warp / thread a state: 1,184
+// states 31 / 34 us, 4,096 53 / 29, 16,384 136 / 30, 65,536 490 / 55; a VOLE-committed
+// round 44 / 52, 85 / 44, 243 / 46 and 898 / 95.
+constexpr int kFsThreads = 32, kManyThreads = 128;
 
-__global__ void __launch_bounds__(kFsThreads) put_fp2s_kernel(State* __restrict__ st,
-                                                              const ulonglong2* __restrict__ vals, int k)
+bool many_states(int n)
 {
-    __shared__ tp::fs::TxMem mem;
-    const int i = blockIdx.x;
-    tp::fs::Writer s(st[i], &mem);
+    tp::Ctx* c = tp::ctx();
+    return c && n > 8LL * c->n_sm;
+}
+int fs_threads(bool many) { return many ? kManyThreads : kFsThreads; }
+int fs_blocks(bool many, int n) { return many ? (n + kManyThreads - 1) / kManyThreads : n; }
+
+template <bool kMany>
+using Tx = std::conditional_t<kMany, tp::fs::Alone, tp::fs::Writer>;
+
+// the state of the thread, or of the CTA's warp
+template <bool kMany>
+__device__ __forceinline__ int my_state()
+{
+    return kMany ? blockIdx.x * kManyThreads + threadIdx.x : blockIdx.x;
+}
+template <bool kMany>
+__device__ __forceinline__ Tx<kMany> open_state(const State& st)
+{
+    if constexpr (kMany) {
+        return tp::fs::Alone(st);
+    } else {
+        __shared__ tp::fs::TxMem mem;
+        return tp::fs::Writer(st, &mem);
+    }
+}
+
+template <bool kMany>
+__global__ void __launch_bounds__(kMany ? kManyThreads : kFsThreads)
+    put_fp2s_kernel(State* __restrict__ st, int n, const ulonglong2* __restrict__ vals, int k)
+{
+    const int i = my_state<kMany>();
+    if (i >= n) return;
+    auto s = open_state<kMany>(st[i]);
     for (int j = 0; j < k; ++j) {
         const ulonglong2 v = vals[(long long)i * k + j];   // packed {re, im}
         s.put_fp2(v.x, v.y);
@@ -91,50 +125,52 @@ __global__ void __launch_bounds__(kFsThreads) put_fp2s_kernel(State* __restrict_
     s.store(st[i]);
 }
 
-__global__ void __launch_bounds__(kFsThreads) rand_ext_kernel(State* __restrict__ st, tp::fs::Label L,
-                                                              ulonglong2* __restrict__ out)
+template <bool kMany>
+__global__ void __launch_bounds__(kMany ? kManyThreads : kFsThreads)
+    rand_ext_kernel(State* __restrict__ st, int n, tp::fs::Label L, ulonglong2* __restrict__ out)
 {
-    __shared__ tp::fs::TxMem mem;
-    const int i = blockIdx.x;
-    tp::fs::Writer s(st[i], &mem);
+    const int i = my_state<kMany>();
+    if (i >= n) return;
+    auto s = open_state<kMany>(st[i]);
     const tp::fp2 r = s.rand_fp2(L);
     s.store(st[i]);
-    if (tp::fs::lead()) out[i] = make_ulonglong2(r.re, r.im);
+    if (s.lead()) out[i] = make_ulonglong2(r.re, r.im);
 }
 
-// ---- VOLE-committed early round (vole.cuh), one warp per frame ------------------
+// ---- VOLE-committed early round (vole.cuh) --------------------------------------
 using VoleState = tp::vole::State;
 
 // the round of frame i on its four claims: the states updated in place, the
 // challenge returned (on every lane)
+template <bool kMany>
 __device__ __forceinline__ tp::fp2 vole_round_frame(State* st, VoleState* vs, const tp::fp2* claims,
                                                     const tp::fp2* u, const tp::fp2* v, long long count,
                                                     const tp::fs::Label& L, tp::fp2* proof)
 {
     using namespace tp;
-    __shared__ fs::TxMem mem;
     VoleState w = *vs;
-    fs::Writer s(*st, &mem);
+    auto s = open_state<kMany>(*st);
     fp2 coef[4], r;
     vole::interpolate_cubic(claims[0], claims[1], claims[2], claims[3], coef);
     vole::round(s, w, coef, 4, u, v, count, L, proof, &r);
     s.store(*st);
-    if (fs::lead()) *vs = w;
+    if (s.lead()) *vs = w;
     return r;
 }
 
 // rounds (optional): frame i takes part only while this round k < rounds[i]
-__global__ void __launch_bounds__(kFsThreads) vole_round_kernel(
-    State* __restrict__ st, VoleState* __restrict__ vs, const tp::fp2* __restrict__ claims,
+template <bool kMany>
+__global__ void __launch_bounds__(kMany ? kManyThreads : kFsThreads) vole_round_kernel(
+    State* __restrict__ st, VoleState* __restrict__ vs, int n, const tp::fp2* __restrict__ claims,
     const tp::fp2* __restrict__ u, const tp::fp2* __restrict__ v, long long count, tp::fs::Label L,
     tp::fp2* __restrict__ chal, tp::fp2* __restrict__ proof, const int* __restrict__ rounds, int k)
 {
-    const int i = blockIdx.x;
-    if (rounds && k >= rounds[i]) return;
+    const int i = my_state<kMany>();
+    if (i >= n || (rounds && k >= rounds[i])) return;
     const long long base = (long long)i * count;
-    const tp::fp2 r = vole_round_frame(st + i, vs + i, claims + 4 * i, u + base, v + base, count, L,
-                                       proof ? proof + 5 * i : nullptr);
-    if (tp::fs::lead()) chal[i] = r;
+    const tp::fp2 r = vole_round_frame<kMany>(st + i, vs + i, claims + 4 * (long long)i, u + base, v + base, count, L,
+                                              proof ? proof + 5 * (long long)i : nullptr);
+    if (kMany || tp::fs::lead()) chal[i] = r;
 }
 
 // ---- VOLE-committed rounds of frames each at its own round (the serving loop) ----
@@ -150,8 +186,8 @@ __global__ void __launch_bounds__(kFsThreads) vole_round_slots_kernel(
     if (m.x < 0 || m.x >= m.y || m.x >= max_rounds) return;
     const long long base = (long long)i * count;
     const long long at = (long long)i * max_rounds + m.x;
-    const tp::fp2 r = vole_round_frame(st + i, vs + i, claims + 4 * i, u + base, v + base, count,
-                                       tp::vole::sc_label(layer, m.x), proof ? proof + 5 * at : nullptr);
+    const tp::fp2 r = vole_round_frame<false>(st + i, vs + i, claims + 4 * i, u + base, v + base, count,
+                                              tp::vole::sc_label(layer, m.x), proof ? proof + 5 * at : nullptr);
     if (tp::fs::lead()) {
         chal_cur[i] = r;
         chal_hist[at] = r;
@@ -394,8 +430,10 @@ bool launch_vole_round_batch(void* d_states, void* d_vole_states, int n, const v
 {
     fs::Label L;
     if (!make_device_label(label, &L, "vole round")) return false;
-    vole_round_kernel<<<n, kFsThreads, 0, s>>>(
-        static_cast<State*>(d_states), static_cast<VoleState*>(d_vole_states), static_cast<const fp2*>(d_claims),
+    const bool many = many_states(n);
+    const auto kernel = many ? vole_round_kernel<true> : vole_round_kernel<false>;
+    kernel<<<fs_blocks(many, n), fs_threads(many), 0, s>>>(
+        static_cast<State*>(d_states), static_cast<VoleState*>(d_vole_states), n, static_cast<const fp2*>(d_claims),
         static_cast<const fp2*>(d_u), static_cast<const fp2*>(d_v), count, L, static_cast<fp2*>(d_chal),
         static_cast<fp2*>(d_proof), d_rounds, k);
     return !cuda_failed(cudaGetLastError(), "vole round");
@@ -599,8 +637,10 @@ int tp_fs_put_fp2s_dev(void* d_states, int n, const void* d_vals, int k, void* s
         return -1;
     }
     if (k == 0) return 0;
-    put_fp2s_kernel<<<n, kFsThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        static_cast<State*>(d_states), static_cast<const ulonglong2*>(d_vals), k);
+    const bool many = many_states(n);
+    const auto kernel = many ? put_fp2s_kernel<true> : put_fp2s_kernel<false>;
+    kernel<<<fs_blocks(many, n), fs_threads(many), 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+        static_cast<State*>(d_states), n, static_cast<const ulonglong2*>(d_vals), k);
     return tp::cuda_failed(cudaGetLastError(), "transcript put") ? -1 : 0;
 }
 
@@ -614,8 +654,10 @@ int tp_fs_rand_ext_dev(void* d_states, int n, const char* label, void* d_out, vo
         tp::set_error(tp::TP_ERR_ARG, "tp_fs_rand_ext_dev: bad arguments");
         return -1;
     }
-    rand_ext_kernel<<<n, kFsThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        static_cast<State*>(d_states), L, static_cast<ulonglong2*>(d_out));
+    const bool many = many_states(n);
+    const auto kernel = many ? rand_ext_kernel<true> : rand_ext_kernel<false>;
+    kernel<<<fs_blocks(many, n), fs_threads(many), 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+        static_cast<State*>(d_states), n, L, static_cast<ulonglong2*>(d_out));
     return tp::cuda_failed(cudaGetLastError(), "transcript rand_ext") ? -1 : 0;
 }
 
@@ -791,8 +833,10 @@ int tp_vole_round_dev(void* d_fs_states, void* d_vole_states, int n, const void*
         tp::set_error(tp::TP_ERR_ARG, "tp_vole_round_dev: bad arguments");
         return -1;
     }
-    vole_round_kernel<<<n, kFsThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        static_cast<State*>(d_fs_states), static_cast<VoleState*>(d_vole_states),
+    const bool many = many_states(n);
+    const auto kernel = many ? vole_round_kernel<true> : vole_round_kernel<false>;
+    kernel<<<fs_blocks(many, n), fs_threads(many), 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+        static_cast<State*>(d_fs_states), static_cast<VoleState*>(d_vole_states), n,
         static_cast<const tp::fp2*>(d_claims), static_cast<const tp::fp2*>(d_u), static_cast<const tp::fp2*>(d_v),
         count, L, static_cast<tp::fp2*>(d_chal), static_cast<tp::fp2*>(d_proof), nullptr, 0);
     return tp::cuda_failed(cudaGetLastError(), "vole round") ? -1 : 0;

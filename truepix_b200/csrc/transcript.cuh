@@ -15,9 +15,9 @@
 //
 // The state is a plain struct (the SHA-256 chaining words, the pending partial
 // block, the byte count and the challenge counter), so it can move between host
-// and device memory by a copy. The host appends to the state itself, a warp of the
-// device to a stretch in shared memory (Writer): two pieces of code with the same
-// bytes, draws and states.
+// and device memory by a copy. The host, and a device thread that has a transcript to
+// itself, append to the state; a warp of the device appends to a stretch in shared
+// memory (Writer): two pieces of code with the same bytes, draws and states.
 #pragma once
 #include <stdint.h>
 
@@ -58,21 +58,45 @@ TP_HD bool lead()
 #endif
 }
 
-// ---- the state's operations (host) ----------------------------------------------
+// ---- the state's operations (host, or one thread of the device) ------------------
 
-inline void compress_units(uint32_t* h, const uint64_t* unit)
+TP_HD void unit_words(uint32_t w[16], const uint64_t* unit)
 {
-    uint32_t w[16];
+#pragma unroll
     for (int i = 0; i < 8; ++i) {
         w[2 * i] = sha::bswap32((uint32_t)unit[i]);
         w[2 * i + 1] = sha::bswap32((uint32_t)(unit[i] >> 32));
     }
+}
+
+#ifdef __CUDACC__
+// one copy for all the places that put bytes
+static __device__ __noinline__ void compress_units_dev(uint32_t* h, const uint64_t* unit)
+{
+    uint32_t w[16], st[8];
+    unit_words(w, unit);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) st[i] = h[i];
+    sha::compress_compact<true>(st, w, sha::kShaTables.k, sha::AddAlu{});
+#pragma unroll
+    for (int i = 0; i < 8; ++i) h[i] = st[i];
+}
+#endif
+
+TP_HD void compress_units(uint32_t* h, const uint64_t* unit)
+{
+#ifdef __CUDA_ARCH__
+    compress_units_dev(h, unit);
+#else
+    uint32_t w[16];
+    unit_words(w, unit);
     sha::compress(h, w, sha::AddAlu{});
+#endif
 }
 
 // The low `bytes` bytes of v (1 <= bytes <= 8), least significant first. Bytes
 // behind the pending ones keep what they held.
-inline void absorb_le(State& s, uint64_t v, int bytes)
+TP_HD void absorb_le(State& s, uint64_t v, int bytes)
 {
     const uint64_t all = bytes < 8 ? low_bytes(bytes) : ~(uint64_t)0;
     const int q = (int)(s.nbuf >> 3), r = (int)(s.nbuf & 7);
@@ -169,7 +193,7 @@ inline void put_u64s(State& s, const uint64_t* v, uint64_t n)
     for (uint64_t i = 0; i < n; ++i) absorb_le(s, v[i], 8);
 }
 
-inline void put_fp2(State& s, uint64_t re, uint64_t im)
+TP_HD void put_fp2(State& s, uint64_t re, uint64_t im)
 {
     absorb_le(s, 0x03 | (re << 8), 8);
     absorb_le(s, (re >> 56) | (im << 8), 8);
@@ -184,19 +208,18 @@ inline void put_str(State& s, const uint8_t* p, uint32_t len)
 }
 
 // put(str) of a label held by value
-inline void put_label(State& s, const Label& L)
+TP_HD void put_label(State& s, const Label& L)
 {
     absorb_le(s, 0x04 | ((uint64_t)L.len << 8), 5);
-    const uint64_t w[4] = {L.w0, L.w1, L.w2, L.w3};
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; 8 * i < (int)L.len; ++i) {
         const int left = (int)L.len - 8 * i;
-        if (left > 0) absorb_le(s, w[i], left < 8 ? left : 8);
+        absorb_le(s, i == 0 ? L.w0 : i == 1 ? L.w1 : i == 2 ? L.w2 : L.w3, left < 8 ? left : 8);
     }
 }
 
 // The chaining words after the SHA-256 padding: the digest of everything
 // absorbed so far. The running state is unchanged.
-inline void digest_words(const State& s, uint32_t h[8])
+TP_HD void digest_words(const State& s, uint32_t h[8])
 {
     uint64_t u[8];
     for (int i = 0; i < 8; ++i) {
@@ -227,7 +250,7 @@ inline void digest(const State& s, uint8_t out[32])
 }
 
 // put([rnum]): a one-int list of the counter, which then moves on
-inline void put_counter(State& s)
+TP_HD void put_counter(State& s)
 {
     absorb_le(s, 0x01 | (1ull << 8) | (s.rnum << 40), 8);
     absorb_le(s, s.rnum >> 24, 5);
@@ -235,7 +258,7 @@ inline void put_counter(State& s)
 }
 
 // the low 61 bits of the big-endian digest (its last two words)
-inline uint64_t draw_bits(const State& s)
+TP_HD uint64_t draw_bits(const State& s)
 {
     uint32_t h[8];
     digest_words(s, h);
@@ -244,7 +267,7 @@ inline uint64_t draw_bits(const State& s)
 
 // A draw is redrawn only when its 61 bits are all ones (probability 2^-61); the
 // loop is bounded all the same, and past the bound returns the value reduced.
-inline uint64_t rand_scalar(State& s)
+TP_HD uint64_t rand_scalar(State& s)
 {
     uint64_t v = 0;
     for (int it = 0; it < 1000; ++it) {
@@ -257,7 +280,7 @@ inline uint64_t rand_scalar(State& s)
 
 // rand_ext(label) as an Fp2: "ext", label, "real" -> the real limb; "ext",
 // label, "imag" -> the imaginary limb
-inline fp2 rand_fp2(State& s, const Label& L)
+TP_HD fp2 rand_fp2(State& s, const Label& L)
 {
     const Label ext = label_lit("ext"), real = label_lit("real"), imag = label_lit("imag");
     put_label(s, ext);
@@ -286,8 +309,9 @@ inline void rand_ext(State& s, const uint8_t* label, uint32_t len, uint64_t* re,
 }
 
 // ---- a transcript at work ---------------------------------------------------------
-// Writer runs a state: opened from it, put to and drawn from, stored back to it. The
-// host form is the state itself.
+// Alone and Writer run a state: opened from it, put to and drawn from, stored back to it.
+// Alone is the state itself, on the host or in one thread of the device, and the host's
+// form of Writer.
 //
 // On the device a warp runs it: every lane makes the same calls. What is put gathers
 // in shared memory (TxMem) without being hashed, a lane writing one byte of it, and a
@@ -316,6 +340,18 @@ struct TxMem {
     uint64_t total, rnum;        // a redrawn draw's end
     uint32_t n;
     __align__(16) uint32_t kw[2 * kTxBlocks][68];   // k + w of block b as digest v closes it: row 2 b + v
+};
+
+class Alone {
+public:
+    TP_HD explicit Alone(const State& state) : s(state) {}
+    TP_HD void put_fp2(uint64_t re, uint64_t im) { fs::put_fp2(s, re, im); }
+    TP_HD fp2 rand_fp2(const Label& L) { return fs::rand_fp2(s, L); }
+    TP_HD void store(State& out) const { out = s; }
+    TP_HD bool lead() const { return true; }
+
+protected:
+    State s;
 };
 
 #ifdef __CUDACC__
@@ -553,6 +589,7 @@ public:
         }
         return mk(m->out[0], m->out[1]);
     }
+    __device__ bool lead() const { return fs::lead(); }
     // the state at this point back to s (lanes 0..7 write)
     __device__ void store(State& s)
     {
@@ -595,17 +632,11 @@ private:
     uint32_t n;                  // bytes of the stretch
 };
 #else
-class Writer {
+class Writer : public Alone {
 public:
-    Writer(const State& state, TxMem*) : s(state) {}
+    Writer(const State& state, TxMem*) : Alone(state) {}
     void absorb_le(uint64_t v, int bytes) { fs::absorb_le(s, v, bytes); }
-    void put_fp2(uint64_t re, uint64_t im) { fs::put_fp2(s, re, im); }
     void put_label(const Label& L) { fs::put_label(s, L); }
-    fp2 rand_fp2(const Label& L) { return fs::rand_fp2(s, L); }
-    void store(State& out) { out = s; }
-
-private:
-    State s;
 };
 #endif
 #endif
