@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(kMany ? kManyThreads : kFsThreads)
     auto s = open_state<kMany>(st[i]);
     const tp::fp2 r = s.rand_fp2(L);
     s.store(st[i]);
-    if (s.lead()) out[i] = make_ulonglong2(r.re, r.im);
+    if (tp::fs::writes<Tx<kMany>>()) out[i] = make_ulonglong2(r.re, r.im);
 }
 
 // ---- VOLE-committed early round (vole.cuh) --------------------------------------
@@ -154,7 +154,7 @@ __device__ __forceinline__ tp::fp2 vole_round_frame(State* st, VoleState* vs, co
     vole::interpolate_cubic(claims[0], claims[1], claims[2], claims[3], coef);
     vole::round(s, w, coef, 4, u, v, count, L, proof, &r);
     s.store(*st);
-    if (s.lead()) *vs = w;
+    if (fs::writes<Tx<kMany>>()) *vs = w;
     return r;
 }
 
@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(kMany ? kManyThreads : kFsThreads) vole_round_
     const long long base = (long long)i * count;
     const tp::fp2 r = vole_round_frame<kMany>(st + i, vs + i, claims + 4 * (long long)i, u + base, v + base, count, L,
                                               proof ? proof + 5 * (long long)i : nullptr);
-    if (kMany || tp::fs::lead()) chal[i] = r;
+    if (tp::fs::writes<Tx<kMany>>()) chal[i] = r;
 }
 
 // ---- VOLE-committed rounds of frames each at its own round (the serving loop) ----

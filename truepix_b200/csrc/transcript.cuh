@@ -21,6 +21,8 @@
 #pragma once
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "fp2.cuh"
 #include "sha256.cuh"
 
@@ -342,17 +344,24 @@ struct TxMem {
     __align__(16) uint32_t kw[2 * kTxBlocks][68];   // k + w of block b as digest v closes it: row 2 b + v
 };
 
+// a state by itself
 class Alone {
 public:
     TP_HD explicit Alone(const State& state) : s(state) {}
     TP_HD void put_fp2(uint64_t re, uint64_t im) { fs::put_fp2(s, re, im); }
     TP_HD fp2 rand_fp2(const Label& L) { return fs::rand_fp2(s, L); }
     TP_HD void store(State& out) const { out = s; }
-    TP_HD bool lead() const { return true; }
 
 protected:
     State s;
 };
+
+// whether this thread writes what leaves the one, or the warp, that runs a transcript
+template <class Tx>
+TP_HD bool writes()
+{
+    return std::is_same<Tx, Alone>::value || lead();
+}
 
 #ifdef __CUDACC__
 #ifdef __CUDA_ARCH__
@@ -589,7 +598,6 @@ public:
         }
         return mk(m->out[0], m->out[1]);
     }
-    __device__ bool lead() const { return fs::lead(); }
     // the state at this point back to s (lanes 0..7 write)
     __device__ void store(State& s)
     {

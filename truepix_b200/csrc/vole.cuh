@@ -110,14 +110,14 @@ TP_HD bool round(Tx& s, State& w, const fp2* c, int n_coef, const fp2* u, const 
     w.idx += (unsigned long long)n_coef;
     for (int k = 0; k < n_coef; ++k) {
         s.put_fp2(dm[k].re, dm[k].im);
-        if (proof && s.lead()) proof[k] = dm[k];
+        if (proof && fs::writes<Tx>()) proof[k] = dm[k];
     }
     fp2 now = tag[0];
     for (int k = 0; k < n_coef; ++k) now = f2add(now, tag[k]);
     const fp2 e = s.rand_fp2(fs::label_lit("eq"));
     const fp2 vz = w.has_prev ? f2mul(f2sub(w.prev, now), e) : f2mul(now, e);
     s.put_fp2(vz.re, vz.im);
-    if (proof && s.lead()) proof[n_coef] = vz;
+    if (proof && fs::writes<Tx>()) proof[n_coef] = vz;
     const fp2 r = s.rand_fp2(label);
     fp2 p = tag[n_coef - 1];
     for (int k = n_coef - 2; k >= 0; --k) p = f2add(f2mul(p, r), tag[k]);
