@@ -314,7 +314,7 @@ def int_alu_roof(ms_per_launch, rows_per_launch, sm_mhz, n_sm):
 def profiled_traffic():
     """DRAM bytes (read + write) per launch of each round kernel of the 64-frame
     1080p step, from the committed ncu summary (profiles/gkr_batch_1080p_traffic.json;
-    measured at 4 frames per launch and scaled by the frames per launch)."""
+    measured at 24 frames per launch and scaled by the frames per launch)."""
     p = os.path.join(ROOT, "profiles", "gkr_batch_1080p_traffic.json")
     if os.path.exists(p):
         try:
