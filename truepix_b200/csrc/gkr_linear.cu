@@ -764,7 +764,7 @@ __global__ void __maxnreg__(80) finish_bytes_kernel(const Job* __restrict__ jobs
 // lo and hi the eq weights of the point's first h and further hb entries. The copies
 // are summed first, 512 to a CTA, on the tensor cores; what is left is a dot product
 // over the wires. Both weights are made by the CTA that uses them. Bound by reading
-// the bytes and by the weights (64 1080p frames, 398 MB: 133 us; a thread per copy with
+// the bytes and by the weights (64 1080p frames, 398 MB: 96 us; a thread per copy with
 // four 32 x 32 multiplications a byte took 244, its eq tables 110).
 struct MleArgs {
     const MleFrame* frames;

@@ -531,7 +531,7 @@ __global__ void __launch_bounds__(kLeafRows) sha_peak_kernel(int iters, uint32_t
 // edges, the third every 4: a + b is not reduced, its products are at most
 // (2^62 - 4)(2^32 - 2), and four of them with the fold's rest stay below 2^96. The
 // result is (a c - b d) + (s (c + d) - a c - b d) i. Reducing a + b first, with one fold
-// per 8 edges, took 1183 us for a 1080p commit (now 1164) and 1543 us for a 720p
+// per 8 edges, took 4731 us for four 1080p commits (now 4655) and 1543 us for a 720p
 // zero-knowledge pair (now 1506).
 struct Acc3 {
     u32 w0, w1, w2;

@@ -315,14 +315,14 @@ inline void rand_ext(State& s, const uint8_t* label, uint32_t len, uint64_t* re,
 // Alone is the state itself, on the host or in one thread of the device, and the host's
 // form of Writer.
 //
-// On the device a warp runs it: every lane makes the same calls. What is put gathers
+// On the device a warp runs Writer: every lane makes the same calls. What is put gathers
 // in shared memory (TxMem) without being hashed, a lane writing one byte of it, and a
 // draw's own 70 to 134 bytes are written by all lanes at once (a lane that appended
 // unit by unit spent a third of a round on that chain, and on fetching its code anew
 // each time); a draw hashes the whole stretch at once. The message words of all its
 // blocks are known by then, so their schedules are made side by side, one lane per
-// block, and the rounds run on k + w from shared memory: 33 cycles a round against 49
-// with the schedule in line. The real limb of a draw does not enter the transcript, so
+// block, and the rounds run on k + w from shared memory: about 37 cycles a round (33 in a
+// kernel of nothing else) against 49 with the schedule in line. The real limb of a draw does not enter the transcript, so
 // the stretch runs on to the imaginary limb's draw and an even and an odd lane close the
 // two digests in the same instructions, each with its own padding. Per committed round
 // (243 bytes, two draws): ~6 compressions' rounds one after the other and two schedules,

@@ -258,7 +258,7 @@ class BatchFrameProver:
                 out[f, part] = np.asarray(z[part], np.uint64).reshape(-1)[:G]
         return out
 
-    # From this many bytes on, the MLEs' time (64 1080p frames, 398 MB: 133 us) is worth
+    # From this many bytes on, the MLEs' time (64 1080p frames, 398 MB: 96 us) is worth
     # the four event calls (10 us of the host's time) that put them beside the rounds: that
     # batch took 1347 us with them behind the finish and takes 1258 so, with the late
     # outputs zeroed in one launch instead of seven
@@ -350,8 +350,9 @@ class BatchFrameProver:
         z1 = self._gate_weights(z1s)
         pix = np.array([pixels[f].data_ptr() for f in range(self.B)], np.uint64)
         betas = np.array([beta_of[f] for f in range(self.B)], np.uint64)
-        quick = native.gkr_launcher()     # a short call: it keeps the interpreter lock
-        native.check(lib, quick.tp_batch_set_pixels_all(
+        # builds every frame's form and may wait for the staging ring: the interpreter lock is
+        # free meanwhile (kept, 1080p proved frames/s were 288 to 327; free, 268 to 326)
+        native.check(lib, lib.tp_batch_set_pixels_all(
             b, self.gt.size, self.gt.ctypes.data, self.i0.ctypes.data, self.i1.ctypes.data, z1.ctypes.data,
             pix.ctypes.data, self._copies.ctypes.data, self._padded.ctypes.data, L.copy_size, L.n_wires, L.const_idx,
             L.const_val, betas.ctypes.data), "batch_set_pixels")
