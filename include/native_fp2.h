@@ -261,7 +261,10 @@ int tp_mle_eval_pixels_batch_at(int n_frames, const void* const* d_pixels, const
                                 size_t ws_bytes, void* stream);
 
 /* Claim-kernel timer: when enabled, every session claim records a CUDA event pair
- * with tag 1000*(reads pixels) + 100*(fold fused) + log2(copies claimed).
+ * with tag 1000*(reads pixels) + 100*(fold fused) + log2(copies claimed). Of a byte
+ * frame whose rounds run on per-copy sums the launch that makes the sums has the tag
+ * 1000 + log2(copies), a pair of its own in front of the first claim's; its claims read
+ * no pixels. Rounds that share a launch have no pairs.
  * tp_timer_read (after a synchronise) returns the number of pairs and their ms. */
 int tp_timer_enable(int max_pairs);
 void tp_timer_disable(void);

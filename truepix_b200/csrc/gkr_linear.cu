@@ -31,6 +31,7 @@
 #include "vole.cuh"
 
 #include <algorithm>
+#include <atomic>
 
 namespace tp {
 
@@ -909,8 +910,8 @@ void plan_linear_finish(std::vector<Job>& jobs)
 
 bool prepare_linear_kernels()
 {
-    static bool done = false;
-    if (done) return true;
+    static std::atomic<bool> done{false};   // sessions of several threads come here
+    if (done.load()) return true;
     TP_CUDA_OK(cudaFuncSetAttribute(forms_bytes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)form_smem(512)),
                "forms smem attr");
@@ -920,7 +921,7 @@ bool prepare_linear_kernels()
     TP_CUDA_OK(cudaFuncSetAttribute(mle_bytes_kernel<kRowVectors>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)row_smem(512)),
                "mle smem attr");
-    done = true;
+    done.store(true);
     return true;
 }
 
